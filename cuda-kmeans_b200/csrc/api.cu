@@ -152,7 +152,7 @@ Workspace carve(char* base, uint64_t n, uint32_t k, uint32_t dim, bool with_tc_p
 	w.tm.b_lo = reinterpret_cast<float*>(take(plane));
 	w.tm.cnorm = reinterpret_cast<float*>(take((size_t)w.tm.k_pad * sizeof(float)));
 	w.tm.b_aug = reinterpret_cast<float*>(take((size_t)w.tm.k_pad * 8 * sizeof(float)));
-	w.tm.center = reinterpret_cast<float*>(take((size_t)w.tm.d_pad * sizeof(float)));
+	w.tm.center = reinterpret_cast<float*>(take((size_t)dim * sizeof(float)));
 	w.sm.center = w.tm.center;
 	w.flag_list = reinterpret_cast<uint32_t*>(take(n * sizeof(uint32_t)));
 	w.asg_scratch = reinterpret_cast<uint32_t*>(take(n * sizeof(uint32_t)));
@@ -412,7 +412,7 @@ static bkm::TcPlan* cached_plan(const bkm::Shape& s, const Workspace& w, int dev
 }
 
 // One assignment pass on a caller's workspace.  The operands derived from the (immutable) points -
-// centre vector, largest norm, tf32 planes - stay in the workspace; a call that finds the same
+// centre vector, largest norm, fp16 planes - stay in the workspace; a call that finds the same
 // point set there (address, shape and a fingerprint of a sample of the values) skips them.
 // Whether the fast assignment pass should accumulate the update sums itself.  On CTA pairs the
 // epilogue warps send the reductions, which pays where the update would otherwise be the row-wise
@@ -448,7 +448,7 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 		CUDA_TRY(cudaMemsetAsync(&key->fp_new, 0, sizeof(key->fp_new), st));
 		CUDA_TRY(bkm::launch_points_fingerprint(points, s.n * s.dim, key, sm_count, st));
 		CUDA_TRY(bkm::launch_points_key_decide(key, points, s, v, w.ctl, st));
-		CUDA_TRY(bkm::launch_compute_center(points, s, w.tm.center, st, skip));
+		CUDA_TRY(bkm::launch_compute_center(points, s, w.tm.center, w.ctl, st, skip));
 		if (v == BKM_ASSIGN_SIMT) {
 			CUDA_TRY(cudaMemsetAsync(w.sm.rows, 0, w.cprep_bytes, st));
 			CUDA_TRY(bkm::launch_points_norm_max(points, s, w.tm.center, w.ctl, sm_count, st, skip));
@@ -551,7 +551,7 @@ int bkm_iterate_f32(const float* points, const float* means_in, float* means_out
 	// otherwise be the row-wise kernel) the points are read once.
 	int vu = 0;
 	if ((rc = resolve_update(variant_update, s, device, &vu))) return rc;
-	bkm::FusedAcc fa{w.acc, w.counts, w.replicas, bkm::acc_replica_stride(k, dim), w.tm.center};
+	bkm::FusedAcc fa{w.acc, w.counts, w.replicas, bkm::acc_replica_stride(k, dim), w.tm.center, points, s.soa};
 	bool fused = false;
 	rc = stateless_assign(points, means_in, asg, s, w, variant_assign, device, sm, st, &fa, vu, &fused);
 	if (rc) return rc;
@@ -828,18 +828,34 @@ static int initialize_finish(bkm_handle_t h, bool points_done)
 	const bkm::Shape& s = h->shape;
 	cudaStream_t st = h->stream;
 	if (h->assign_variant == BKM_ASSIGN_SIMT) {
-		CUDA_TRY(bkm::launch_compute_center(h->d_points, s, h->ws.tm.center, st));
+		CUDA_TRY(bkm::launch_compute_center(h->d_points, s, h->ws.tm.center, h->ws.ctl, st));
 		CUDA_TRY(bkm::launch_points_norm_max(h->d_points, s, h->ws.tm.center, h->ws.ctl, h->sm_count, st));
 	}
 	if (!points_done) {
 		if (h->assign_variant == BKM_ASSIGN_TC) {
-			CUDA_TRY(bkm::launch_compute_center(h->d_points, s, h->ws.tm.center, st));
+			CUDA_TRY(bkm::launch_compute_center(h->d_points, s, h->ws.tm.center, h->ws.ctl, st));
 			CUDA_TRY(bkm::launch_split_points(h->d_points, s, h->ws.tp, h->ws.tm.center, h->ws.ctl, st));
 		}
 		const int rc = prepare_plan_and_means(h);
 		if (rc) return rc;
 	}
 	CUDA_TRY(cudaGetLastError());
+	if (points_done) {
+		// The scale of the operands came from the first chunk.  Where it turns out too small for what
+		// followed (points that grow by orders of magnitude towards the end), they are derived again
+		// from a sample of all points; a few outliers are left to the exact kernel.
+		bkm::Control c;
+		CUDA_TRY(cudaMemcpyAsync(&c, h->ws.ctl, sizeof(c), cudaMemcpyDeviceToHost, st));
+		CUDA_TRY(cudaStreamSynchronize(st));
+		if (c.beyond > s.n / 256) {
+			int rc = drop_first_pass(h);
+			if (rc) return rc;
+			CUDA_TRY(cudaMemsetAsync(h->ws.ctl, 0, sizeof(bkm::Control), st));
+			CUDA_TRY(bkm::launch_compute_center(h->d_points, s, h->ws.tm.center, h->ws.ctl, st));
+			CUDA_TRY(bkm::launch_split_points(h->d_points, s, h->ws.tp, h->ws.tm.center, h->ws.ctl, st));
+			if ((rc = prepare_plan_and_means(h))) return rc;
+		}
+	}
 	CUDA_TRY(cudaStreamSynchronize(st));
 	h->initialized = true;
 	return BKM_OK;
@@ -862,7 +878,7 @@ static int upload_and_split(bkm_handle_t h, const float* host_points)
 	for (cudaEvent_t& e : h->copy_ev)
 		if (!e) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
 	const uint64_t chunk = bkm::round_up64((s.n + bkm_handle_s::UPLOAD_CHUNKS - 1) / bkm_handle_s::UPLOAD_CHUNKS, 4096);
-	bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(s.k, s.dim), h->ws.tm.center};
+	bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(s.k, s.dim), h->ws.tm.center, h->d_points, s.soa};
 	bool fused = false, early_pass = false;
 	// the copies must not overtake the clearing of the workspace and of what the previous use left in the planes' consumers
 	CUDA_TRY(cudaEventRecord(h->copy_ev[0], h->stream));
@@ -879,7 +895,7 @@ static int upload_and_split(bkm_handle_t h, const float* host_points)
 		CUDA_TRY(cudaEventRecord(h->copy_ev[c], h->copy_stream));
 		CUDA_TRY(cudaStreamWaitEvent(h->stream, h->copy_ev[c], 0));
 		if (c == 0) {
-			CUDA_TRY(bkm::launch_compute_center(h->d_points, s, h->ws.tm.center, h->stream, nullptr, count));
+			CUDA_TRY(bkm::launch_compute_center(h->d_points, s, h->ws.tm.center, h->ws.ctl, h->stream, nullptr, count));
 			const int rc = prepare_plan_and_means(h);
 			if (rc) return rc;
 			// On CTA pairs the fast pass of the first iteration follows the upload chunk by chunk as well
@@ -994,7 +1010,7 @@ static int enqueue_iteration(bkm_handle_t h, cudaEvent_t* ev)
 	if (ev) CUDA_TRY(cudaEventRecord(ev[0], st));
 	// The CTA-pair tensor-core pass and the CUDA-core pass can add every point to its cluster's sum on
 	// the way (the accumulators are zero between iterations: the finalize pass clears what it has read).
-	bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(s.k, s.dim), h->ws.tm.center};
+	bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(s.k, s.dim), h->ws.tm.center, h->d_points, s.soa};
 	const bool fused = h->fuse_update && fuse_pays(h->assign_variant, h->update_variant, h->plan, fa, s, h->fuse_update >= 2);
 	h->last_fused = fused;
 	h->launches_per_iter = (h->assign_variant == BKM_ASSIGN_EXACT ? 1u : 2u) + (fused ? 0u : 1u) + 1u;

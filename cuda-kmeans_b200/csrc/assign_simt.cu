@@ -262,7 +262,9 @@ __global__ void __launch_bounds__(LIST_THREADS, PB > LIST_PB ? 2 : 3) assign_exa
 				for (int p = 0; p < PB; ++p) {
 					const float dist = __fsqrt_rn(sum[p]);
 					// (the chunks come in rotated order: the lower index wins a tie explicitly)
-					if (bidx[p] == 0xffffffffu || dist < best[p] || (dist == best[p] && m < bidx[p])) { best[p] = dist; bidx[p] = m; }
+					if (dist < best[p] || (dist == best[p] && m < bidx[p])) { best[p] = dist; bidx[p] = m; }
+					// what is not a number never wins, but nothing replaces it as the first distance of the sequential scan
+					if (m == 0 && dist != dist) { best[p] = 0.0f; bidx[p] = 0; }
 				}
 			}
 		}
@@ -321,13 +323,14 @@ __global__ void __launch_bounds__(LIST_THREADS, PB > LIST_PB ? 2 : 3) assign_exa
 			__syncthreads();
 			for (uint32_t p = 0; p < np; ++p) {
 				const uint32_t from = smoved[p][0], to = smoved[p][1];
-				if (from == to || from >= k) continue;
+				if (from == to) continue;
+				// (no previous cluster: the fast pass could not hold the point and has not added it)
 				for (uint32_t j = tid; j < d; j += LIST_THREADS) {
 					const float x = sx[p * dpad + j];
-					atomicAdd(&fix_acc[(size_t)from * d + j], -x);
+					if (from < k) atomicAdd(&fix_acc[(size_t)from * d + j], -x);
 					atomicAdd(&fix_acc[(size_t)to * d + j], x);
 				}
-				if (tid == 0) { atomicSub(&fix_counts[from], 1u); atomicAdd(&fix_counts[to], 1u); }
+				if (tid == 0) { if (from < k) atomicSub(&fix_counts[from], 1u); atomicAdd(&fix_counts[to], 1u); }
 			}
 		}
 	}
@@ -395,13 +398,13 @@ __global__ void __launch_bounds__(256) assign_exact_list_small_kernel(const floa
 		if (fix_acc) {
 			// the fast pass has already added this point to the sum of the cluster it picked
 			const uint32_t from = asg[i];
-			if (from != bidx && from < k) {
+			if (from != bidx) {
 				#pragma unroll
 				for (int j = 0; j < D; ++j) {
-					atomicAdd(&fix_acc[(size_t)from * D + j], -x[j]);
+					if (from < k) atomicAdd(&fix_acc[(size_t)from * D + j], -x[j]);
 					atomicAdd(&fix_acc[(size_t)bidx * D + j], x[j]);
 				}
-				atomicSub(&fix_counts[from], 1u);
+				if (from < k) atomicSub(&fix_counts[from], 1u);
 				atomicAdd(&fix_counts[bidx], 1u);
 			}
 		}
@@ -470,9 +473,10 @@ cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* 
 		const uint32_t resident_ok = resident_bytes <= 64 * 1024 ? 1u : 0u;
 		if (resident_ok && resident_bytes > lsmem) lsmem = resident_bytes;
 		const uint32_t lgrid = (uint32_t)sm_count * 8;
+		// (the 48 KiB that need no permission include the kernel's static arrays, less than 4 KiB)
 #define BKM_LAUNCH_LIST_PB(SOA, SOAM, PBV) do { \
 		auto kern = assign_exact_list_kernel<SOA, SOAM, PBV>; \
-		if (lsmem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem); if (e != cudaSuccess) return e; } \
+		if (lsmem > 44 * 1024) { cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem); if (e != cudaSuccess) return e; } \
 		kern<<<lgrid, LIST_THREADS, lsmem, stream>>>(pts, means, asg, s.n, s.k, s.dim, list, list_count, \
 			fix ? fix->acc : nullptr, fix ? fix->counts : nullptr, resident_ok, split_keys, split_arrive); \
 	} while (0)

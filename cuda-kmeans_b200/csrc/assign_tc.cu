@@ -2,11 +2,13 @@
 //
 //   |x - c|^2 = |x|^2 + ( |c|^2 - 2 x.c )          argmin over c ignores |x|^2
 //
-// The x.c contraction runs as split-TF32 ("3xTF32"): every fp32 operand is split once into a
-// tf32 high part and a tf32 low part (x = xh + xl), and xl*ch + xh*cl + xh*ch is accumulated in
-// fp32 in tensor memory, which restores fp32-level accuracy of the products.  |c|^2 and an offset
-// constant enter the same accumulator through one more K step whose A operand is a constant
-// tile, so the accumulator holds |c|^2 - 2 x.c + C, all values positive with one exponent, and
+// The x.c contraction runs on fp16 pairs: every fp32 operand, centred and multiplied by a power of
+// two of the data set (tc_scale), is split once into an fp16 high part and an fp16 low part
+// (x = xh + xl, 22 bits as with tf32 pairs), and xl*ch + xh*cl + xh*ch is accumulated in fp32 in
+// tensor memory, which restores fp32-level accuracy of the products.  A K step holds 16 dimensions
+// where tf32 has 8 at the same cost, so the three products take half the tensor time and the operands
+// half the bytes.  |c|^2 and an offset constant enter the same accumulator through one more K step
+// whose A operand is a constant tile, so the accumulator holds |c|^2 - 2 x.c + C, all values positive with one exponent, and
 // the epilogue is a pure arg-min on integer keys.  The N x k distance
 // matrix never exists in HBM.  Because the GEMM form cancels, a point whose best and
 // second-best values are closer than the error band of this formulation is queued for the
@@ -15,12 +17,12 @@
 // the shape range of the reference's cachedRegsAssignmentKernel (kernels/kernels.cu:548-661).
 //
 // Kernel organisation (one persistent CTA per SM, 18 warps):
-//   warp 0      : TMA producer.  dim <= 32: point tiles (128 points, hi and lo plane) go through a
+//   warp 0      : TMA producer.  dim <= 64: point tiles (128 points, hi and lo plane) go through a
 //                 ring and stay for all mean tiles; mean tiles (up to 256 means, hi and lo, plus
 //                 their |c|^2 K step) stream through a 2-stage ring, or stay when there is only
-//                 one.  dim > 32: both operands stream in 32-dimension slices.
+//                 one.  dim > 64: both operands stream in 32-dimension slices.
 //   warp 1      : allocates the 512 TMEM columns and issues the tcgen05.mma instructions
-//                 (kind::tf32, M=128, N<=256, K=8) into two accumulators, one per point tile of
+//                 (kind::f16, M=128, N<=256, K=16) into two accumulators, one per point tile of
 //                 a block.  The whole warp walks the loop; one elected lane issues.
 //   warps 2..17 : epilogue.  Eight warps per accumulator (TMEM lane quarter x column half), so
 //                 that one accumulator is reduced while the other is being multiplied.  A warp
@@ -28,7 +30,7 @@
 //                 accumulator back after its last load, and reduces each chunk to (best, second)
 //                 on integer keys; (best, second, chunk of best) per point stay in registers
 //                 across all mean tiles and are merged through shared memory at the end.
-// Mean sets of 2..4 tiles of 256 with 17 <= dim <= 32 run on CTA pairs instead, with all means
+// Mean sets of 2..4 tiles of 256 with 17 <= dim <= 64 run on CTA pairs instead, with all means
 // resident in shared memory (assign_tc_pair.cu).
 // All mbarrier waits are bounded; a wait that runs out sets STATUS_WAIT_TIMEOUT and lets every
 // role fall through to the end, where TMEM is released.
@@ -51,9 +53,9 @@ constexpr uint32_t A_PLANE_BYTES = TC_MTILE * TC_KCHUNK * 4;     // 16 KiB: 128 
 constexpr uint32_t B_PLANE_BYTES = TC_NT_MAX * TC_KCHUNK * 4;    // 32 KiB: 256 rows x 128 B
 constexpr uint32_t A_TILE_BYTES = 2 * A_PLANE_BYTES;             // hi + lo
 constexpr uint32_t B_STAGE_BYTES = 2 * B_PLANE_BYTES;
-constexpr uint32_t AUG_BYTES = TC_NT_MAX * 8 * 4;                // 8 KiB: 256 rows x one K step of 8
-// K-loop mode (dim > 32): both operands stream in 16-dimension slices (rows of 64 B, 64-byte
-// swizzle).  A stage holds the slice of BOTH point tiles of the block and of one mean tile:
+constexpr uint32_t AUG_BYTES = TC_NT_MAX * 8 * 4;                // 8 KiB: 256 rows x one K step of 16 fp16
+// K-loop mode (dim > 64): both operands stream in 32-dimension slices (16 words = rows of 64 B,
+// 64-byte swizzle).  A stage holds the slice of BOTH point tiles of the block and of one mean tile:
 // [A0 hi | A0 lo | A1 hi | A1 lo | B hi | B lo], and feeds both accumulators, so every byte of
 // the mean tile that crosses from L2 is used for 256 points.  Three stages; the |c|^2 steps of
 // the current and the next mean tile sit behind them.
@@ -87,94 +89,220 @@ bool assign_tc_supported(const Shape& s)
 // one-off split of the points
 // ------------------------------------------------------------------------------------------
 
-// 32 points x 32 dims per step through a padded shared tile, so that both the read (along
-// points for SoA, along dims for AoS) and the write (along dims) are coalesced.
-template<bool SOA>
-__global__ void __launch_bounds__(256) split_points_kernel(const float* __restrict__ pts, float* __restrict__ a_hi,
-	float* __restrict__ a_lo, float* __restrict__ xnorm, uint64_t n, uint64_t p_begin, uint64_t p_end, uint32_t d, uint32_t d_pad,
+// Largest |x|^2 of a block's points -> ctl->xmax2, one atomic per block: one per warp kept the line that
+// every block reads its scale from busy (82 us for 100 003 points of 128 dimensions).
+__device__ __forceinline__ void block_norm_max(float local_max, Control* __restrict__ ctl)
+{
+	__shared__ float warp_max[8];
+	#pragma unroll
+	for (int off = 16; off > 0; off >>= 1) local_max = fmaxf(local_max, __shfl_xor_sync(0xffffffffu, local_max, off));
+	if ((threadIdx.x & 31u) == 0) warp_max[threadIdx.x >> 5] = local_max;
+	__syncthreads();
+	if (threadIdx.x != 0) return;
+	#pragma unroll
+	for (int w = 1; w < 8; ++w) local_max = fmaxf(local_max, warp_max[w]);
+	// non-negative floats order like their bit patterns
+	atomicMax(reinterpret_cast<int*>(&ctl->xmax2), __float_as_int(local_max));
+}
+
+// Row-major points: a lane per operand word (two dimensions), 16 or 32 lanes per row, so that reads and
+// writes are coalesced; a warp has the words of SPLIT_ROWS (pairs of) rows in flight.  Rows
+// [p_begin, p_end) of the planes (both multiples of 32); rows at or behind n are padding.
+constexpr uint32_t SPLIT_ROWS = 4;
+
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ pts, uint32_t* __restrict__ a_hi,
+	uint32_t* __restrict__ a_lo, float* __restrict__ xnorm, uint64_t n, uint64_t p_begin, uint64_t p_end, uint32_t d, uint32_t d_pad, int vec,
 	const float* __restrict__ center, Control* __restrict__ ctl, const uint32_t* __restrict__ skip_if)
 {
 	if (skip_if && *skip_if) return;
+	const float scale = tc_scale(ctl->xdev);
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	const uint32_t lanes = d_pad == 16 ? 16u : 32u, word = lane & (lanes - 1u);
+	const uint32_t per_warp = SPLIT_ROWS * (32u / lanes);                // 4 or 8 rows
 	float local_max = 0.0f;
-	__shared__ float tile[32][33];
-	const uint32_t tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
-	// rows [p_begin, p_end) of the planes (both multiples of 32); rows at or behind n are padding
-	for (uint64_t p0 = p_begin + (uint64_t)blockIdx.x * 32; p0 < p_end; p0 += (uint64_t)gridDim.x * 32) {
-		float norm[4] = {0.f, 0.f, 0.f, 0.f};
-		for (uint32_t c0 = 0; c0 < d_pad; c0 += 32) {
-			__syncthreads();
+	for (uint64_t r0 = p_begin + ((uint64_t)blockIdx.x * 8 + warp) * per_warp; r0 < p_end; r0 += (uint64_t)gridDim.x * 8 * per_warp) {
+		const uint64_t first = r0 + (lane >= lanes ? SPLIT_ROWS : 0u);
+		float norm[SPLIT_ROWS] = {};
+		for (uint32_t w = word; w < d_pad; w += lanes) {
+			const uint32_t j = 2 * w;
+			const float c0 = j < d ? center[j] : 0.0f, c1 = j + 1 < d ? center[j + 1] : 0.0f;
+			float x0[SPLIT_ROWS], x1[SPLIT_ROWS];
 			#pragma unroll
-			for (uint32_t r = 0; r < 4; ++r) {
-				const uint32_t rr = ty + r * 8;
-				if (SOA) {
-					const uint64_t p = p0 + tx;
-					const uint32_t j = c0 + rr;
-					tile[tx][rr] = (p < n && j < d) ? pts[(size_t)j * n + p] - center[j] : 0.0f;     // tile[point][dim]
-				} else {
-					const uint64_t p = p0 + rr;
-					const uint32_t j = c0 + tx;
-					tile[rr][tx] = (p < n && j < d) ? pts[(size_t)p * d + j] - center[j] : 0.0f;
+			for (uint32_t u = 0; u < SPLIT_ROWS; ++u) {
+				const uint64_t p = first + u;
+				const float* src = pts + (size_t)p * d + j;
+				x0[u] = c0; x1[u] = c1;
+				if (p < n && vec && j < d) {                                 // rows on 8-byte boundaries, dim even
+					const float2 v = *reinterpret_cast<const float2*>(src);
+					x0[u] = v.x; x1[u] = v.y;
+				} else if (p < n) {
+					if (j < d) x0[u] = src[0];
+					if (j + 1 < d) x1[u] = src[1];
 				}
 			}
-			__syncthreads();
 			#pragma unroll
-			for (uint32_t r = 0; r < 4; ++r) {
-				const uint32_t rr = ty + r * 8;     // point within the group
-				const float x = tile[rr][tx];
-				const float hi = to_tf32(x);
-				const float lo = to_tf32(x - hi);
-				const size_t o = (size_t)(p0 + rr) * d_pad + c0 + tx;
-				if (c0 + tx < d_pad) {          // rows are shorter than the 32-wide step when d_pad = 16
-					a_hi[o] = hi;
-					a_lo[o] = lo;
-				}
-				norm[r] = fmaf(x, x, norm[r]);
+			for (uint32_t u = 0; u < SPLIT_ROWS; ++u) {
+				const float y0 = (x0[u] - c0) * scale, y1 = (x1[u] - c1) * scale;
+				uint32_t hi, lo;
+				tc_split2(y0, y1, hi, lo);
+				const size_t o = (size_t)(first + u) * d_pad + w;
+				a_hi[o] = hi;
+				a_lo[o] = lo;
+				norm[u] = fmaf(y0, y0, fmaf(y1, y1, norm[u]));
 			}
 		}
 		#pragma unroll
-		for (uint32_t r = 0; r < 4; ++r) {
-			float s = norm[r];
+		for (uint32_t u = 0; u < SPLIT_ROWS; ++u) {
+			float s = norm[u];
 			#pragma unroll
-			for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-			if (tx == 0) xnorm[p0 + ty + r * 8] = s;
-			local_max = fmaxf(local_max, s);
+			for (uint32_t off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+			const float other = __shfl_xor_sync(0xffffffffu, s, 16);
+			if (lanes == 32) s += other;
+			if (!(s <= TC_NORM2_MAX)) {
+				// beyond what the planes hold, or not a number: a zero row whose |x|^2 sends the point to the exact kernel
+				s = INFINITY;
+				for (uint32_t w = word; w < d_pad; w += lanes) { a_hi[(size_t)(first + u) * d_pad + w] = 0u; a_lo[(size_t)(first + u) * d_pad + w] = 0u; }
+				if (word == 0) atomicAdd(&ctl->beyond, 1u);
+			} else {
+				local_max = fmaxf(local_max, s);
+			}
+			if (word == 0) xnorm[first + u] = s;
 		}
 	}
-	// non-negative floats order like their bit patterns
-	if (tx == 0) atomicMax(reinterpret_cast<int*>(&ctl->xmax2), __float_as_int(local_max));
+	block_norm_max(local_max, ctl);
 }
 
-// One block per dimension: mean of that coordinate over at most 65536 evenly spaced points.
-template<bool SOA>
-__global__ void __launch_bounds__(256) compute_center_kernel(const float* __restrict__ pts, float* __restrict__ center,
-	uint64_t n, uint64_t n_sampled, uint32_t d, const uint32_t* __restrict__ skip_if)
+// Dimension-major points: a lane per point (reads coalesced along the points), 32 dimensions in flight.
+// The 64-byte slices of a warp's 32 points pass through shared memory (16-byte pieces, swizzled so that
+// neither side meets a bank twice) and leave as whole rows: written straight from the lanes, 16 bytes
+// every 64, the stores cost 1.3 ms for 2^21 points of 32 dimensions.
+__global__ void __launch_bounds__(256) split_columns_kernel(const float* __restrict__ pts, uint32_t* __restrict__ a_hi,
+	uint32_t* __restrict__ a_lo, float* __restrict__ xnorm, uint64_t n, uint64_t p_begin, uint64_t p_end, uint32_t d, uint32_t d_pad,
+	const float* __restrict__ center, Control* __restrict__ ctl, const uint32_t* __restrict__ skip_if)
 {
 	if (skip_if && *skip_if) return;
-	__shared__ float part[256];
-	const uint32_t j = blockIdx.x;
-	// the sample is taken from the first n_sampled points
-	const uint64_t samples = n_sampled < 65536 ? n_sampled : 65536;
-	const uint64_t stride = n_sampled / samples;
-	float sum = 0.0f;
-	for (uint64_t t = threadIdx.x; t < samples; t += 256) {
-		const uint64_t i = t * stride;
-		sum += SOA ? pts[(size_t)j * n + i] : pts[(size_t)i * d + j];
+	__shared__ uint4 s_hi[8][128], s_lo[8][128];
+	const float scale = tc_scale(ctl->xdev);
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	float local_max = 0.0f;
+	for (uint64_t p0 = p_begin + ((uint64_t)blockIdx.x * 8 + warp) * 32; p0 < p_end; p0 += (uint64_t)gridDim.x * 256) {
+		const uint64_t p = p0 + lane;
+		uint4* out_hi = reinterpret_cast<uint4*>(a_hi + (size_t)p0 * d_pad);
+		uint4* out_lo = reinterpret_cast<uint4*>(a_lo + (size_t)p0 * d_pad);
+		const uint32_t pitch = d_pad / 4;           // 16-byte pieces of a row
+		float s = 0.0f;
+		for (uint32_t w0 = 0; w0 < d_pad; w0 += 16) {
+			float x[32];
+			#pragma unroll
+			for (uint32_t i = 0; i < 32; ++i) {
+				const uint32_t j = 2 * w0 + i;
+				x[i] = (p < n && j < d) ? pts[(size_t)j * n + p] : 0.0f;
+			}
+			#pragma unroll
+			for (uint32_t i = 0; i < 32; ++i) {
+				const uint32_t j = 2 * w0 + i;
+				x[i] = (p < n && j < d) ? (x[i] - center[j]) * scale : 0.0f;
+				s = fmaf(x[i], x[i], s);
+			}
+			__syncwarp();                           // the previous slice has been read
+			#pragma unroll
+			for (uint32_t q = 0; q < 4; ++q) {
+				uint4 hi, lo;
+				tc_split2(x[8 * q + 0], x[8 * q + 1], hi.x, lo.x);
+				tc_split2(x[8 * q + 2], x[8 * q + 3], hi.y, lo.y);
+				tc_split2(x[8 * q + 4], x[8 * q + 5], hi.z, lo.z);
+				tc_split2(x[8 * q + 6], x[8 * q + 7], hi.w, lo.w);
+				const uint32_t e = lane * 4 + (q ^ ((lane >> 1) & 3u));
+				s_hi[warp][e] = hi;
+				s_lo[warp][e] = lo;
+			}
+			__syncwarp();
+			#pragma unroll
+			for (uint32_t r = 0; r < 4; ++r) {
+				const uint32_t row = r * 8 + (lane >> 2), q = lane & 3u, e = row * 4 + (q ^ ((row >> 1) & 3u));
+				out_hi[(size_t)row * pitch + w0 / 4 + q] = s_hi[warp][e];
+				out_lo[(size_t)row * pitch + w0 / 4 + q] = s_lo[warp][e];
+			}
+		}
+		if (!(s <= TC_NORM2_MAX)) s = INFINITY;     // (as above)
+		else local_max = fmaxf(local_max, s);
+		__syncwarp();
+		if (s == INFINITY) {
+			for (uint32_t q = 0; q < pitch; ++q) { out_hi[(size_t)lane * pitch + q] = make_uint4(0u, 0u, 0u, 0u); out_lo[(size_t)lane * pitch + q] = make_uint4(0u, 0u, 0u, 0u); }
+			atomicAdd(&ctl->beyond, 1u);
+		}
+		xnorm[p] = s;
 	}
-	part[threadIdx.x] = sum;
-	__syncthreads();
-	for (uint32_t w = 128; w > 0; w >>= 1) {
-		if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-		__syncthreads();
-	}
-	if (threadIdx.x == 0) center[j] = part[0] / (float)samples;
+	block_norm_max(local_max, ctl);
 }
 
-cudaError_t launch_compute_center(const float* pts, const Shape& s, float* center, cudaStream_t stream, const uint32_t* skip_if,
+// One block per dimension: mean of that coordinate over at most 8192 evenly spaced points (any vector
+// near the points serves), and the sample's largest distance from it.  Bound by the latency of strided
+// reads: a thread has all of its samples in flight together (65536 samples in a loop of 256 threads
+// took 28-39 us per new batch of a stateless call).
+constexpr uint32_t CENTER_THREADS = 1024, CENTER_PER_THREAD = 8;
+
+template<bool SOA>
+__global__ void __launch_bounds__(CENTER_THREADS) compute_center_kernel(const float* __restrict__ pts, float* __restrict__ center,
+	uint64_t n, uint64_t n_sampled, uint32_t d, Control* __restrict__ ctl, const uint32_t* __restrict__ skip_if)
+{
+	if (skip_if && *skip_if) return;
+	__shared__ float part[4][CENTER_THREADS / 32];
+	const uint32_t j = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	// the sample is taken from the first n_sampled points
+	constexpr uint32_t MAX_SAMPLES = CENTER_THREADS * CENTER_PER_THREAD;
+	const uint32_t samples = n_sampled < MAX_SAMPLES ? (uint32_t)n_sampled : MAX_SAMPLES;
+	float x[CENTER_PER_THREAD];
+	#pragma unroll
+	for (uint32_t r = 0; r < CENTER_PER_THREAD; ++r) {
+		const uint32_t t = threadIdx.x + r * CENTER_THREADS;
+		const uint64_t i = samples == MAX_SAMPLES ? (uint64_t)t * n_sampled / MAX_SAMPLES : (t < samples ? t : 0u);
+		x[r] = SOA ? pts[(size_t)j * n + i] : pts[(size_t)i * d + j];
+	}
+	// (values that are not finite are left out: one of them must not spoil the centre for all points)
+	float sum = 0.0f, cnt = 0.0f, mn = INFINITY, mx = -INFINITY;
+	#pragma unroll
+	for (uint32_t r = 0; r < CENTER_PER_THREAD; ++r) {
+		if (threadIdx.x + r * CENTER_THREADS < samples && fabsf(x[r]) < INFINITY) {
+			sum += x[r];
+			cnt += 1.0f;
+			mn = fminf(mn, x[r]);
+			mx = fmaxf(mx, x[r]);
+		}
+	}
+	#pragma unroll
+	for (int off = 16; off > 0; off >>= 1) {
+		sum += __shfl_xor_sync(0xffffffffu, sum, off);
+		cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
+		mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+		mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+	}
+	if (lane == 0) { part[0][warp] = sum; part[1][warp] = mn; part[2][warp] = mx; part[3][warp] = cnt; }
+	__syncthreads();
+	if (warp != 0) return;
+	sum = part[0][lane]; mn = part[1][lane]; mx = part[2][lane]; cnt = part[3][lane];
+	#pragma unroll
+	for (int off = 16; off > 0; off >>= 1) {
+		sum += __shfl_xor_sync(0xffffffffu, sum, off);
+		cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
+		mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+		mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+	}
+	if (lane == 0) {
+		float c = sum / cnt;
+		if (!(fabsf(c) < INFINITY)) c = 0.0f;
+		center[j] = c;
+		const float dev = fmaxf(fmaxf(mx - c, c - mn), 0.0f);
+		if (dev < 3.0e38f) atomicMax(reinterpret_cast<int*>(&ctl->xdev), __float_as_int(dev));
+	}
+}
+
+cudaError_t launch_compute_center(const float* pts, const Shape& s, float* center, Control* ctl, cudaStream_t stream, const uint32_t* skip_if,
 	uint64_t n_sampled)
 {
 	if (n_sampled == 0 || n_sampled > s.n) n_sampled = s.n;
-	if (s.soa) compute_center_kernel<true><<<s.dim, 256, 0, stream>>>(pts, center, s.n, n_sampled, s.dim, skip_if);
-	else compute_center_kernel<false><<<s.dim, 256, 0, stream>>>(pts, center, s.n, n_sampled, s.dim, skip_if);
+	if (s.soa) compute_center_kernel<true><<<s.dim, CENTER_THREADS, 0, stream>>>(pts, center, s.n, n_sampled, s.dim, ctl, skip_if);
+	else compute_center_kernel<false><<<s.dim, CENTER_THREADS, 0, stream>>>(pts, center, s.n, n_sampled, s.dim, ctl, skip_if);
 	return cudaGetLastError();
 }
 
@@ -183,10 +311,13 @@ cudaError_t launch_split_points(const float* pts, const Shape& s, const TcPoints
 {
 	if (p_end == 0 || p_end > tp.n_pad) p_end = tp.n_pad;
 	if ((p_begin & 31u) != 0 || (p_end & 31u) != 0 || p_begin >= p_end) return cudaErrorInvalidValue;
-	const uint64_t groups = (p_end - p_begin) / 32;
-	const uint32_t grid = (uint32_t)std::min<uint64_t>(groups, (uint64_t)current_sm_count() * 16);
-	if (s.soa) split_points_kernel<true><<<grid, 256, 0, stream>>>(pts, tp.a_hi, tp.a_lo, tp.xnorm, s.n, p_begin, p_end, s.dim, tp.d_pad, center, ctl, skip_if);
-	else split_points_kernel<false><<<grid, 256, 0, stream>>>(pts, tp.a_hi, tp.a_lo, tp.xnorm, s.n, p_begin, p_end, s.dim, tp.d_pad, center, ctl, skip_if);
+	uint32_t* a_hi = reinterpret_cast<uint32_t*>(tp.a_hi);
+	uint32_t* a_lo = reinterpret_cast<uint32_t*>(tp.a_lo);
+	const uint64_t rows_pb = s.soa ? 256 : 8 * SPLIT_ROWS * (tp.d_pad == 16 ? 2 : 1);
+	const uint32_t grid = (uint32_t)std::min<uint64_t>((p_end - p_begin + rows_pb - 1) / rows_pb, (uint64_t)current_sm_count() * 8);
+	const int vec = s.dim % 2 == 0 && (reinterpret_cast<uintptr_t>(pts) & 7u) == 0 ? 1 : 0;
+	if (s.soa) split_columns_kernel<<<grid, 256, 0, stream>>>(pts, a_hi, a_lo, tp.xnorm, s.n, p_begin, p_end, s.dim, tp.d_pad, center, ctl, skip_if);
+	else split_rows_kernel<<<grid, 256, 0, stream>>>(pts, a_hi, a_lo, tp.xnorm, s.n, p_begin, p_end, s.dim, tp.d_pad, vec, center, ctl, skip_if);
 	return cudaGetLastError();
 }
 
@@ -195,26 +326,6 @@ cudaError_t launch_split_points(const float* pts, const Shape& s, const TcPoints
 // ------------------------------------------------------------------------------------------
 
 constexpr uint32_t TC_NA_MAX = 8;        // most point-tile buffers (single resident centroid tile, 16-float rows)
-
-// The 3xTF32 products of one operand-tile pair over KS steps of 8 dimensions: the small cross
-// terms lo*hi and hi*lo first, then the dominant hi*hi.  Operands are the low halves of the
-// descriptors (+2 in the address field = 32 bytes = one K step), `hi_word` their common high half.
-// `acc_first` = accumulate the very first product onto the destination.
-template<uint32_t KS>
-__device__ __forceinline__ void issue_products(uint32_t d_tmem, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi, uint32_t b_lo,
-	uint32_t hi_word, uint32_t idesc, uint32_t acc_first)
-{
-	ptx::mma_tf32_halves(d_tmem, a_lo, hi_word, b_hi, hi_word, idesc, acc_first);
-	#pragma unroll
-	for (uint32_t ks = 1; ks < KS; ++ks)
-		ptx::mma_tf32_halves(d_tmem, a_lo + 2 * ks, hi_word, b_hi + 2 * ks, hi_word, idesc, 1);
-	#pragma unroll
-	for (uint32_t ks = 0; ks < KS; ++ks)
-		ptx::mma_tf32_halves(d_tmem, a_hi + 2 * ks, hi_word, b_lo + 2 * ks, hi_word, idesc, 1);
-	#pragma unroll
-	for (uint32_t ks = 0; ks < KS; ++ks)
-		ptx::mma_tf32_halves(d_tmem, a_hi + 2 * ks, hi_word, b_hi + 2 * ks, hi_word, idesc, 1);
-}
 
 struct TcBars {
 	uint64_t a_full[TC_NA_MAX];
@@ -232,27 +343,15 @@ static_assert(sizeof(TcBars) <= 256, "barrier block too large");
 static_assert(SM_ALLOC <= 227 * 1024, "shared memory budget exceeded");
 static_assert(KL_AUG_OFF + 2 * AUG_BYTES <= SM_AAUG_OFF, "K-loop stages overlap the constant tile");
 
-// The end of a point's arg-min: decode the winning key (key - key_base = M * mantissa + column) and
-// write the assignment.  Returns whether best and second are closer than `margin`, i.e. whether
-// the point has to be queued for the exact kernel (the caller appends, a warp at a time).
-__device__ __forceinline__ bool finish_point(uint32_t best, uint32_t second, uint32_t bchunk, uint32_t key_base, uint32_t key_mult, uint32_t key_magic,
-	float ulp, float margin, uint64_t p, uint32_t* __restrict__ asg)
-{
-	const uint32_t bm = div_key(best - key_base, key_magic);
-	asg[p] = bchunk * 32u + ((best - key_base) - bm * key_mult);
-	// keys are (mantissa * M + column): the difference of the quotients counts value spacings
-	const float gap = second == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second - key_base, key_magic) - bm) * ulp;
-	return gap <= margin;
-}
-
 // Combines the partial arg-min results of the CTAs that shared the mean tiles of a point block.
 __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __restrict__ partial, uint64_t partial_stride, uint32_t parts,
-	const float* __restrict__ xnorm, uint32_t* __restrict__ asg, uint64_t n, Control* __restrict__ ctl, int slot,
-	uint32_t* __restrict__ flag_list, float margin_coef)
+	const float* __restrict__ xnorm, uint32_t* __restrict__ asg, uint64_t n, uint32_t k, Control* __restrict__ ctl, int slot,
+	uint32_t* __restrict__ flag_list, float margin_coef, float sqrt_dim)
 {
-	const float c2max = ctl->cmax2[slot];
-	const KeyConsts kc = make_key_consts(ctl->xmax2, c2max);
+	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
+	const KeyConsts kc = tc_key_consts(x2max, c2max);
 	const float ulp = kc.pow2 * 1.1920929e-07f;
+	const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim);
 	const uint64_t n32 = (n + 31) & ~(uint64_t)31;      // whole warps walk the loop together (the append is a warp operation)
 	for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n32; p += (uint64_t)gridDim.x * blockDim.x) {
 		bool flag = false;
@@ -265,7 +364,7 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __r
 				bchunk = ob < best ? oc : bchunk;
 				best = min(best, ob);
 			}
-			flag = finish_point(best, second, bchunk, kc.key_base, kc.key_mult, kc.key_magic, ulp, margin_coef * (xnorm[p] + c2max) + 4.0f * ulp, p, asg);
+			flag = finish_point(best, second, bchunk, kc.key_base, kc.key_mult, kc.key_magic, ulp, margin_coef * (xnorm[p] + c2max) + margin_floor, k, p, asg);
 		}
 		append_flagged(flag, (uint32_t)p, ctl, flag_list, n);
 	}
@@ -280,7 +379,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 	const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
 	const float* __restrict__ b_aug, const float* __restrict__ xnorm, uint32_t* __restrict__ asg,
 	uint64_t n, uint32_t n_tiles, uint32_t k, uint32_t k_pad, uint32_t nt_cols, uint32_t kw, uint32_t kchunks, uint32_t ksteps, uint32_t idesc,
-	Control* __restrict__ ctl, int slot, uint32_t* __restrict__ flag_list, float margin_coef,
+	Control* __restrict__ ctl, int slot, uint32_t* __restrict__ flag_list, float margin_coef, float sqrt_dim,
 	uint32_t jsplit, uint32_t* __restrict__ partial, uint64_t partial_stride)
 {
 	extern __shared__ uint8_t smem_raw[];
@@ -299,10 +398,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 	const uint32_t jpart = blockIdx.x % jsplit, bid = blockIdx.x / jsplit, nbid = gridDim.x / jsplit;
 	const uint32_t jper = (n_ctiles + jsplit - 1) / jsplit;
 	const uint32_t j_begin = min(n_ctiles, jpart * jper), j_end = min(n_ctiles, j_begin + jper);
-	// Resident-points layout (dim <= 32).  With a single centroid tile (k <= 256) that tile is loaded
+	// Resident-points layout (dim <= 64).  With a single centroid tile (k <= 256) that tile is loaded
 	// once and stays, and the space of the second stage holds two more point tiles, so that the
 	// next block's points arrive while this block is still being multiplied.
-	// Rows are kw = 32 floats (128 B) or, for dim <= 16, kw = 16 floats (64 B): half-size tiles.
+	// Rows are kw = 32 words (128 B) or, for dim <= 32, kw = 16 words (64 B): half-size tiles.
 	const bool b_resident = n_ctiles == 1;
 	const uint32_t a_plane = TC_MTILE * kw * 4, a_tile = 2 * a_plane;
 	const uint32_t b_plane = TC_NT_MAX * kw * 4, b_stage = 2 * b_plane;
@@ -336,10 +435,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 		ptx::tmem_relinquish();
 	}
 	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
-	const KeyConsts kc = make_key_consts(x2max, c2max);
+	const KeyConsts kc = tc_key_consts(x2max, c2max);
 	const float pow2 = kc.pow2;
 	const uint32_t key_mult = kc.key_mult, key_base = kc.key_base, key_magic = kc.key_magic;
-	fill_a_aug(reinterpret_cast<float*>(smem + SM_AAUG_OFF), kc.offset_c, threadIdx.x, TC_THREADS);
+	fill_a_aug(smem + SM_AAUG_OFF, kc.offset_c, threadIdx.x, TC_THREADS);
 	ptx::fence_proxy_async();
 	ptx::tc_fence_before();
 	__syncthreads();
@@ -356,7 +455,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 			bool ok = true;
 			uint32_t aug_count = 0;
 			if (kchunks > 1) {
-				// K-loop mode: one (block of two point tiles, mean tile, 16-dimension slice) per stage
+				// K-loop mode: one (block of two point tiles, mean tile, 32-dimension slice) per stage
 				for (uint32_t blk = bid; blk < nblocks && ok; blk += nbid) {
 					const uint32_t tiles = min(TC_MA, n_tiles - blk * TC_MA);
 					for (uint32_t j = j_begin; j < j_end && ok; ++j) {
@@ -475,15 +574,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 									const uint64_t a_hi = make_desc_kw(base + i * KL_A1_OFF, KL_KW), a_lo = make_desc_kw(base + i * KL_A1_OFF + KL_A_PLANE, KL_KW);
 									#pragma unroll
 									for (uint32_t ks = 0; ks < 2; ++ks)
-										if (ks < steps) ptx::mma_tf32(d_tmem, a_lo + 2 * ks, b_hi + 2 * ks, idesc, (kc | ks) > 0);
+										if (ks < steps) ptx::mma_f16(d_tmem, a_lo + 2 * ks, b_hi + 2 * ks, idesc, (kc | ks) > 0);
 									#pragma unroll
 									for (uint32_t ks = 0; ks < 2; ++ks)
-										if (ks < steps) ptx::mma_tf32(d_tmem, a_hi + 2 * ks, b_lo + 2 * ks, idesc, 1);
+										if (ks < steps) ptx::mma_f16(d_tmem, a_hi + 2 * ks, b_lo + 2 * ks, idesc, 1);
 									#pragma unroll
 									for (uint32_t ks = 0; ks < 2; ++ks)
-										if (ks < steps) ptx::mma_tf32(d_tmem, a_hi + 2 * ks, b_hi + 2 * ks, idesc, 1);
+										if (ks < steps) ptx::mma_f16(d_tmem, a_hi + 2 * ks, b_hi + 2 * ks, idesc, 1);
 									if (last) {
-										ptx::mma_tf32(d_tmem, make_desc_aug(ptx::smem_u32(smem + SM_AAUG_OFF)), make_desc_aug(ptx::smem_u32(smem + KL_AUG_OFF + as * AUG_BYTES)), idesc, 1);
+										ptx::mma_f16(d_tmem, make_desc_aug(ptx::smem_u32(smem + SM_AAUG_OFF)), make_desc_aug(ptx::smem_u32(smem + KL_AUG_OFF + as * AUG_BYTES)), idesc, 1);
 										ptx::mma_commit(&bars->acc_full[i]);
 									}
 								}
@@ -530,7 +629,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 								case 2: issue_products<2>(d_tmem, a_hi, a_lo, b_hi, b_lo, desc_hi, idesc, 0); break;
 								default: issue_products<1>(d_tmem, a_hi, a_lo, b_hi, b_lo, desc_hi, idesc, 0); break;
 								}
-								ptx::mma_tf32_halves(d_tmem, a_aug_lo, DESC_HI_AUG, b_aug_lo, DESC_HI_AUG, idesc, 1);
+								ptx::mma_f16_halves(d_tmem, a_aug_lo, DESC_HI_AUG, b_aug_lo, DESC_HI_AUG, idesc, 1);
 								ptx::mma_commit(&bars->acc_full[i]);
 								if (j == j_end - 1) ptx::mma_commit(&bars->a_empty[buf]);
 							}
@@ -563,6 +662,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 		const uint32_t half = part & 1u;
 		const uint32_t row = q * 32 + lane;
 		const float ulp = pow2 * 1.1920929e-07f;   // spacing of the values inside [P, 2P)
+		const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim);
 		const uint32_t chunks_total = nt_cols >> 5;                    // 1..8
 		const uint32_t per_half = (chunks_total + 1) / 2;              // 1..4
 		const uint32_t first_chunk = half * per_half;
@@ -642,7 +742,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 					uint32_t* dst = partial + (size_t)jpart * 3 * partial_stride + p;
 					dst[0] = best; dst[partial_stride] = second; dst[2 * partial_stride] = bchunk;
 				} else {
-					flag = finish_point(best, second, bchunk, key_base, key_mult, key_magic, ulp, margin_coef * (xn + c2max) + 4.0f * ulp, p, asg);
+					flag = finish_point(best, second, bchunk, key_base, key_mult, key_magic, ulp, margin_coef * (xn + c2max) + margin_floor, k, p, asg);
 				}
 			}
 			if (half == 0 && partial == nullptr) buffered_append(flag, (uint32_t)p, flag_buf, flag_cnt, ctl, flag_list, n);
@@ -715,9 +815,9 @@ static PFN_cuTensorMapEncodeTiled_v12000 get_encode()
 	return fn;
 }
 
-// [rows][cols] fp32 row-major, box = box_rows x 32 columns with 128-byte swizzle, or, when the
-// rows are only 16 floats long or the K loop runs (rows longer than 32 floats, 16-dimension
-// slices), box_rows x 16 columns with 64-byte swizzle.
+// [rows][cols] 32-bit words (two fp16 each) row-major, box = box_rows x 32 columns with 128-byte
+// swizzle, or, when the rows are only 16 words long or the K loop runs (rows longer than 32 words,
+// 16-word slices), box_rows x 16 columns with 64-byte swizzle.
 static bool encode_plane(CUtensorMap* out, const float* base, uint64_t rows, uint32_t cols, uint32_t box_rows)
 {
 	const uint32_t kw = (cols == 16 || cols > TC_KCHUNK) ? 16u : TC_KCHUNK;
@@ -738,13 +838,13 @@ TcPlan* tc_plan_create(const Shape& s, const TcPoints& tp, const TcMeans& tm, in
 	static const char* e_sup = "shape not supported by the tensor-core assignment";
 	static const char* e_map = "cuTensorMapEncodeTiled failed or is unavailable";
 	static const char* e_attr = "cannot set the shared-memory size of the tensor-core kernel";
-	if (!assign_tc_supported(s) || tp.d_pad != tm.d_pad || (tp.d_pad != 16 && tp.d_pad % TC_KCHUNK != 0)) { if (err) *err = e_sup; return nullptr; }
+	if (!assign_tc_supported(s) || tp.d_pad != tm.d_pad || tp.d_pad % 16 != 0) { if (err) *err = e_sup; return nullptr; }
 	TcPlan* p = new (std::nothrow) TcPlan();
 	if (!p) return nullptr;
 	p->s = s; p->tp = tp; p->tm = tm;
 	p->nt_cols = tc_nt_cols(s.k);
-	// c_format = f32 (bit 4), a/b format = tf32 (bits 7.., 10..), K-major both, N>>3 at bit 17, M>>4 at bit 24
-	p->idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((p->nt_cols >> 3) << 17) | ((TC_MTILE >> 4) << 24);
+	// c_format = f32 (bit 4), a/b format = fp16 (0 at bits 7.., 10..), K-major both, N>>3 at bit 17, M>>4 at bit 24
+	p->idesc = (1u << 4) | ((p->nt_cols >> 3) << 17) | ((TC_MTILE >> 4) << 24);
 	if (cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || p->sm_count < 1) { cudaGetLastError(); if (err) *err = e_attr; delete p; return nullptr; }
 	if (!encode_plane(&p->a_hi, tp.a_hi, tp.n_pad, tp.d_pad, TC_MTILE) ||
 		!encode_plane(&p->a_lo, tp.a_lo, tp.n_pad, tp.d_pad, TC_MTILE) ||
@@ -762,7 +862,7 @@ TcPlan* tc_plan_create(const Shape& s, const TcPoints& tp, const TcMeans& tm, in
 		return nullptr;
 	}
 	p->pair_allowed = true;
-	p->pair_ok = assign_tc_pair_supported(s.k, tm.k_pad, tp.d_pad, p->nt_cols, p->sm_count) &&
+	p->pair_ok = assign_tc_pair_supported(s.k, tm.k_pad, s.dim, tp.d_pad, p->nt_cols, p->sm_count) &&
 		encode_plane(&p->bh_hi, tm.b_hi, tm.k_pad, tm.d_pad, TC_NT_MAX / 2) &&
 		encode_plane(&p->bh_lo, tm.b_lo, tm.k_pad, tm.d_pad, TC_NT_MAX / 2);
 	p->max_pairs = 0;
@@ -782,7 +882,7 @@ void tc_plan_destroy(TcPlan* plan) { delete plan; }
 // reductions: dim a multiple of 4 and 16-byte aligned accumulators.
 bool tc_plan_can_fuse(const TcPlan* p, const FusedAcc& f)
 {
-	return tc_plan_uses_pair(p) && p->s.dim % 4 == 0 && f.acc != nullptr && f.counts != nullptr && f.center != nullptr &&
+	return tc_plan_uses_pair(p) && assign_tc_pair_can_fuse(p->tm.k_pad, p->s.dim, p->tp.d_pad) && f.acc != nullptr && f.counts != nullptr && f.points != nullptr &&
 		(reinterpret_cast<uintptr_t>(f.acc) & 15u) == 0 && (f.rep_stride * sizeof(float)) % 16 == 0;
 }
 
@@ -814,18 +914,19 @@ cudaError_t launch_assign_tc(TcPlan* p, uint32_t* asg, Control* ctl, int slot, u
 	const uint32_t n_tiles = (uint32_t)(p->tp.n_pad / TC_MTILE);
 	const uint32_t nblocks = (n_tiles + TC_MA - 1) / TC_MA;
 	const uint32_t grid = std::min<uint32_t>(nblocks, (uint32_t)p->sm_count);
-	// error band of the split-TF32 GEMM form relative to |x|^2 + max|c|^2
-	const float margin_coef = margin_scale * (48.0f + 0.5f * (float)p->tp.d_pad) * 1.1920929e-07f;
-	// rows of 16 or 32 floats stay resident whole; longer rows stream in 16-dimension slices, and
-	// slices that hold padding only are skipped
+	// error band of the split GEMM form relative to |x|^2 + max|c|^2
+	const uint32_t dim_band = p->s.dim <= 16 ? 16u : round_up(p->s.dim, 32);
+	const float margin_coef = margin_scale * (48.0f + 0.5f * (float)dim_band) * 1.1920929e-07f;
+	const float sqrt_dim = sqrtf((float)p->s.dim);
+	// rows of 16 or 32 words stay resident whole; longer rows stream in slices of 16 words
 	const bool kloop = p->tp.d_pad > TC_KCHUNK;
 	const uint32_t kw = (p->tp.d_pad == 16 || kloop) ? 16u : TC_KCHUNK;
-	const uint32_t kchunks = kloop ? (p->s.dim + kw - 1) / kw : 1u;
-	const uint32_t ksteps_last = (p->s.dim - (kchunks - 1) * kw + 7) / 8;    // K steps of the last slice
+	const uint32_t kchunks = kloop ? p->tp.d_pad / kw : 1u;
+	const uint32_t ksteps_last = (p->s.dim - (kchunks - 1) * 2 * kw + 15) / 16;    // K steps (16 dimensions) of the last slice
 	const uint32_t idesc = p->idesc;
 	if (tc_plan_uses_pair(p))
 		return launch_assign_tc_pair(p->a_hi, p->a_lo, p->bh_hi, p->bh_lo, p->tm.b_aug, p->tp.xnorm, asg, p->s.n, n_tiles,
-			p->s.k, p->tm.k_pad, p->tp.d_pad, ksteps_last, p->max_pairs, ctl, slot, flag_list, margin_coef, stream, fused, p->s.dim,
+			p->s.k, p->tm.k_pad, p->tp.d_pad, ksteps_last, p->max_pairs, ctl, slot, flag_list, margin_coef, sqrt_dim, stream, fused, p->s.dim,
 			ranged ? (uint32_t)(p_begin / (2 * TC_MTILE)) : 0u,
 			ranged ? (uint32_t)((std::min<uint64_t>(p_end, p->tp.n_pad) + 2 * TC_MTILE - 1) / (2 * TC_MTILE)) : 0u);
 	const uint32_t jsplit = plan_jsplit(p);
@@ -833,11 +934,11 @@ cudaError_t launch_assign_tc(TcPlan* p, uint32_t* asg, Control* ctl, int slot, u
 	auto kern = (p->s.k == p->tm.k_pad && p->nt_cols % 128 == 0) ? assign_tc_kernel<true> : assign_tc_kernel<false>;
 	kern<<<jsplit > 1 ? grid_j : grid, TC_THREADS, SM_ALLOC, stream>>>(p->a_hi, p->a_lo, p->b_hi, p->b_lo,
 		p->tm.b_aug, p->tp.xnorm, asg, p->s.n, n_tiles, p->s.k, p->tm.k_pad, p->nt_cols, kw, kchunks, ksteps_last, idesc,
-		ctl, slot, flag_list, margin_coef, jsplit, jsplit > 1 ? p->tp.partial : nullptr, p->tp.n_pad);
+		ctl, slot, flag_list, margin_coef, sqrt_dim, jsplit, jsplit > 1 ? p->tp.partial : nullptr, p->tp.n_pad);
 	if (jsplit > 1) {
 		const uint32_t mgrid = (uint32_t)std::min<uint64_t>((p->s.n + 255) / 256, (uint64_t)p->sm_count * 8);
-		merge_partials_kernel<<<mgrid, 256, 0, stream>>>(p->tp.partial, p->tp.n_pad, jsplit, p->tp.xnorm, asg, p->s.n, ctl, slot,
-			flag_list, margin_coef);
+		merge_partials_kernel<<<mgrid, 256, 0, stream>>>(p->tp.partial, p->tp.n_pad, jsplit, p->tp.xnorm, asg, p->s.n, p->s.k, ctl, slot,
+			flag_list, margin_coef, sqrt_dim);
 	}
 	return cudaGetLastError();
 }

@@ -22,12 +22,14 @@ struct Control {
 	float cmax2[2];        // max over clusters of |mean|^2; the preparation of iteration t
 	                       // writes slot (t+1)&1 with atomicMax and clears slot t&1
 	uint32_t last_flag_count; // flag_count of the last finished iteration (for reporting)
-	float xmax2;           // max over the points of |x|^2 (written by the one-off split of the points)
-	uint32_t pad[2];
+	float xmax2;           // max over the points of |x|^2 (written by the one-off preprocessing of the points;
+	                       // in units of the operand scale, see tc_scale, when the operands are the fp16 planes)
+	float xdev;            // largest |x_j - centre_j| over a sample of the points
+	uint32_t beyond;       // points that the fp16 planes cannot hold at the scale of that sample
 };
 
 // What a stateless workspace remembers about the point set its one-off operands (centre vector,
-// largest norm, tf32 planes) were derived from; it lives at byte 64 of the workspace.  `valid` is
+// largest norm, fp16 planes) were derived from; it lives at byte 64 of the workspace.  `valid` is
 // rewritten by every call: 1 when the points of this call are the remembered ones.
 struct PointsKey {
 	unsigned long long fp_new;   // fingerprint of the points of the current call (accumulated, then compared)
@@ -61,12 +63,33 @@ __host__ __device__ __forceinline__ uint32_t simt_row_stride(uint32_t dim) { ret
 // Rows of the prepared means: k rounded to the 32-mean chunk the kernel walks.
 __host__ __device__ __forceinline__ uint32_t simt_rows(uint32_t k) { return round_up(k, 32); }
 
-// Geometry of the tensor-core operands: K (dimension) padded to 32 floats (one 128-byte
-// swizzle row), point rows padded to 128, mean rows padded to 16.
+// Geometry of the tensor-core operands: planes of fp16 values, two dimensions to a 32-bit word.
+// Operand rows are counted in words: 32 (one 128-byte swizzle row, 64 dimensions) or, for dim <= 32,
+// 16 (64-byte swizzle: half the operand bytes); longer rows are whole 16-word slices.  Point rows are
+// padded to 128, mean rows to the mean tile.
 constexpr uint32_t TC_KCHUNK = 32;
 constexpr uint32_t TC_MTILE = 128;
-// dim <= 16 uses rows of 16 floats (64-byte swizzle): half the operand bytes of a 32-float row
-__host__ __device__ __forceinline__ uint32_t tc_dpad(uint32_t dim) { return dim <= 16 ? 16u : round_up(dim, TC_KCHUNK); }
+__host__ __device__ __forceinline__ uint32_t tc_dpad(uint32_t dim)
+{
+	const uint32_t words = (dim + 1) / 2;
+	return words <= 16 ? 16u : (words <= TC_KCHUNK ? TC_KCHUNK : round_up(words, 16));
+}
+
+// The power of two that points and means (relative to the centre) are multiplied by before they are
+// split into fp16 pairs hi + lo.  The largest deviation of the sample lands in [16, 32): values down
+// to 2^-2 keep all 22 bits of the pair, smaller ones an absolute 2^-25, and there is room for
+// vectors of 256 times that deviation (TC_NORM2_MAX), beyond which a point is left to the exact pass.
+__host__ __device__ __forceinline__ float tc_scale(float xdev)
+{
+	if (!(xdev > 0.0f && xdev < 3.0e38f)) return 1.0995116e12f;      // 2^40: nothing seen but the centre itself
+	int e;
+	frexpf(xdev, &e);
+	e = 5 - e;
+	return ldexpf(1.0f, e < -100 ? -100 : (e > 100 ? 100 : e));
+}
+// Largest scaled |x|^2 and |c|^2 that the operands hold (2^26: the offset constant of the keys, at
+// most eight times this, must fit one fp16 product).
+constexpr float TC_NORM2_MAX = 67108864.0f;
 
 // The per-iteration accumulators (k*dim float sums directly followed by k integer sizes) exist in
 // `acc_replicas` copies so that concurrent global reductions spread over more cache lines; a
@@ -82,12 +105,12 @@ __host__ __device__ __forceinline__ uint32_t acc_replicas(uint32_t k, uint32_t d
 	return (uint32_t)(r < 1 ? 1 : (r > 16 ? 16 : r));
 }
 
-// The |c|^2 operand of the tensor-core assignment is one K step (8 tf32) wide and stored
+// The |c|^2 operand of the tensor-core assignment is one K step (16 fp16) wide and stored
 // K-major without swizzle: 8-row x 16-byte core matrices, the two 16-byte chunks of a row group
-// 128 B apart, row groups 256 B apart.  Float offset of element (row, k):
-__host__ __device__ __forceinline__ uint32_t aug_offset(uint32_t row, uint32_t k)
+// 128 B apart, row groups 256 B apart.  Offset, in 32-bit words, of the 16-byte chunk (row, chunk):
+__host__ __device__ __forceinline__ uint32_t aug_offset(uint32_t row, uint32_t chunk)
 {
-	return (row >> 3) * 64 + (k >> 2) * 32 + (row & 7) * 4 + (k & 3);
+	return (row >> 3) * 64 + chunk * 32 + (row & 7) * 4;
 }
 
 } // namespace bkm

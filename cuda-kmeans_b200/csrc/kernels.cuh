@@ -15,15 +15,14 @@ struct Shape {
 
 // Operands of the tensor-core assignment derived from the means (rewritten every iteration).
 struct TcMeans {
-	float* b_hi;     // [k_pad][d_pad] tf32 high part of -2*mean, K-major
-	float* b_lo;     // [k_pad][d_pad] tf32 low part
-	float* cnorm;    // [k_pad] |mean|^2, +inf for padding rows
-	float* b_aug;    // [k_pad x 8] one K step (aug_offset layout): columns 0,1 = tf32 (hi, lo) of |mean|^2,
-	                 // columns 2,3 = 1 (they meet the kernel's offset constant), rest 0; padding rows 0,0,1,1
-	float* center;   // [d_pad] vector subtracted from points and means alike before the split (distances do
+	float* b_hi;     // [k_pad][d_pad words] fp16 high part of -2*mean (centred, scaled by tc_scale), K-major
+	float* b_lo;     // [k_pad][d_pad words] fp16 low part
+	float* cnorm;    // [k_pad] |mean|^2 in units of the scale, +inf for padding rows
+	float* b_aug;    // [k_pad x 8 words] one K step of |mean|^2 (aug_offset layout, see tc_aug_row); padding rows: 0
+	float* center;   // [dim] vector subtracted from points and means alike before the split (distances do
 	                 // not change; the norms, and with them the cancellation of the GEMM form, shrink)
 	uint32_t k_pad;  // k rounded up to the centroid tile
-	uint32_t d_pad;  // dim rounded up to TC_KCHUNK
+	uint32_t d_pad;  // 32-bit words of an operand row (two dimensions each), see tc_dpad
 };
 
 // Operand of the CUDA-core fast pass derived from the means (rewritten every iteration).
@@ -34,9 +33,9 @@ struct SimtMeans {
 
 // Operands derived from the points (written once per initialize).
 struct TcPoints {
-	float* a_hi;     // [n_pad][d_pad]
-	float* a_lo;     // [n_pad][d_pad]
-	float* xnorm;    // [n_pad] |x|^2
+	float* a_hi;     // [n_pad][d_pad words] fp16 high part of the centred, scaled coordinates
+	float* a_lo;     // [n_pad][d_pad words] fp16 low part
+	float* xnorm;    // [n_pad] |x|^2 in units of the scale; +inf (and zero rows) for points the planes cannot hold
 	uint64_t n_pad;  // n rounded up to TC_MTILE
 	uint32_t d_pad;
 	uint32_t* partial; // K loop only (d_pad > 32): [TC_JSPLIT][3][n_pad] partial arg-min keys, else null
@@ -111,6 +110,8 @@ struct FusedAcc {
 	uint32_t replicas;
 	size_t rep_stride;
 	const float* center;  // the vector the split operands were centred by
+	const float* points;  // the points themselves (in the layout `soa`): what the tensor-core pass adds up
+	int soa;
 };
 // `split_scratch` (optional): list_split_scratch_bytes() of zeroed device memory, 8-byte aligned,
 // through which the blocks share the groups of a short list; the kernel leaves it zeroed.
@@ -134,15 +135,16 @@ cudaError_t launch_assign_simt(const float* pts, const SimtMeans& sm, uint32_t* 
 // ---- assignment on tensor cores (assign_tc.cu) ----
 bool assign_tc_supported(const Shape& s);
 uint32_t tc_kpad(uint32_t k);
-// One-off split of the points into tf32 hi/lo K-major planes + |x|^2.
+// One-off split of the points into fp16 hi/lo K-major planes + |x|^2 (after launch_compute_center).
 // `p_begin`, `p_end` (multiples of 32; 0, 0 = all): only these rows of the planes, so that a host upload
 // can be split chunk by chunk while the next chunk is on its way.
 cudaError_t launch_split_points(const float* pts, const Shape& s, const TcPoints& tp, const float* center, Control* ctl, cudaStream_t stream,
 	const uint32_t* skip_if = nullptr, uint64_t p_begin = 0, uint64_t p_end = 0);
 // center[j] = mean of dimension j over a strided sample of the points (any vector would do; the
-// sample mean keeps the shifted norms small).
+// sample mean keeps the shifted norms small), and ctl->xdev (zero on entry) = the sample's largest
+// deviation from it, which sets the scale of the fp16 operands.
 // `n_sampled` (0 = all): the sample is taken from the first n_sampled points only.
-cudaError_t launch_compute_center(const float* pts, const Shape& s, float* center, cudaStream_t stream, const uint32_t* skip_if = nullptr,
+cudaError_t launch_compute_center(const float* pts, const Shape& s, float* center, Control* ctl, cudaStream_t stream, const uint32_t* skip_if = nullptr,
 	uint64_t n_sampled = 0);
 // Opaque per-handle state (tensor maps).  Created once the operand buffers exist.
 struct TcPlan;

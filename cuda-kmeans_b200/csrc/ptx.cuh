@@ -109,6 +109,28 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
 		:: "r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
+// Asynchronous copies of one thread, global -> shared (both sides aligned to the size).
+__device__ __forceinline__ void cp_async16(uint32_t smem_addr, const void* gmem_src)
+{
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_addr), "l"(gmem_src) : "memory");
+}
+
+__device__ __forceinline__ void cp_async4(uint32_t smem_addr, const void* gmem_src)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(smem_addr), "l"(gmem_src) : "memory");
+}
+
+// Arrives on `bar` once all asynchronous copies this thread has issued so far are complete.
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar)
+{
+	asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_wait_all()
+{
+	asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // 2-D tiled TMA load: box at (x = innermost coordinate, y) of the tensor map -> shared.
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, int32_t x, int32_t y, uint64_t* bar)
 {
@@ -164,14 +186,14 @@ __device__ __forceinline__ bool elect_one()
 	return pred != 0;
 }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc], kind::tf32, issued by one thread.
-__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+// D[tmem] (+)= A[smem desc] * B[smem desc], kind::f16, issued by one thread.
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
 	asm volatile(
 		"{\n"
 		".reg .pred p;\n"
 		"setp.ne.b32 p, %4, 0;\n"
-		"tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n"
+		"tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
 		"}\n"
 		:: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
@@ -179,7 +201,7 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint6
 // The same with the two 64-bit shared-memory descriptors given as 32-bit halves: within one
 // operand tile only the low half (the address field) changes from instruction to instruction, so
 // the issuing thread spends one 32-bit add per operand and MMA instead of 64-bit arithmetic.
-__device__ __forceinline__ void mma_tf32_halves(uint32_t d_tmem, uint32_t a_lo32, uint32_t a_hi32, uint32_t b_lo32, uint32_t b_hi32, uint32_t idesc, uint32_t accumulate)
+__device__ __forceinline__ void mma_f16_halves(uint32_t d_tmem, uint32_t a_lo32, uint32_t a_hi32, uint32_t b_lo32, uint32_t b_hi32, uint32_t idesc, uint32_t accumulate)
 {
 	asm volatile(
 		"{\n"
@@ -188,7 +210,7 @@ __device__ __forceinline__ void mma_tf32_halves(uint32_t d_tmem, uint32_t a_lo32
 		"mov.b64 da, {%1, %2};\n"
 		"mov.b64 db, {%3, %4};\n"
 		"setp.ne.b32 p, %6, 0;\n"
-		"tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %5, p;\n"
+		"tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n"
 		"}\n"
 		:: "r"(d_tmem), "r"(a_lo32), "r"(a_hi32), "r"(b_lo32), "r"(b_hi32), "r"(idesc), "r"(accumulate) : "memory");
 }
@@ -282,13 +304,13 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols)
 // One MMA over both CTAs of the pair (M = 256: 128 accumulator rows in each CTA's tensor memory;
 // each CTA's shared memory holds its 128 rows of A and its half of the N rows of B at the
 // descriptor's address).  Issued by one thread of the pair's first CTA.
-__device__ __forceinline__ void mma_tf32_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
 	asm volatile(
 		"{\n"
 		".reg .pred p;\n"
 		"setp.ne.b32 p, %4, 0;\n"
-		"tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n"
+		"tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
 		"}\n"
 		:: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
@@ -298,7 +320,7 @@ __device__ __forceinline__ void mma_tf32_pair(uint32_t d_tmem, uint64_t a_desc, 
 // the high half is a constant of the layout, which leaves the issuing thread one 32-bit add per
 // operand and MMA instead of 64-bit descriptor arithmetic.  ACC = accumulate onto the destination.
 template<bool ACC>
-__device__ __forceinline__ void mma_tf32_pair_halves(uint32_t d_tmem, uint32_t a_lo32, uint32_t a_hi32, uint32_t b_lo32, uint32_t b_hi32, uint32_t idesc)
+__device__ __forceinline__ void mma_f16_pair_halves(uint32_t d_tmem, uint32_t a_lo32, uint32_t a_hi32, uint32_t b_lo32, uint32_t b_hi32, uint32_t idesc)
 {
 	asm volatile(
 		"{\n"
@@ -307,7 +329,7 @@ __device__ __forceinline__ void mma_tf32_pair_halves(uint32_t d_tmem, uint32_t a
 		"mov.b64 da, {%1, %2};\n"
 		"mov.b64 db, {%3, %4};\n"
 		"setp.ne.b32 p, %6, 0;\n"
-		"tcgen05.mma.cta_group::2.kind::tf32 [%0], da, db, %5, p;\n"
+		"tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n"
 		"}\n"
 		:: "r"(d_tmem), "r"(a_lo32), "r"(a_hi32), "r"(b_lo32), "r"(b_hi32), "r"(idesc), "n"(ACC ? 1 : 0) : "memory");
 }

@@ -8,6 +8,7 @@
 #include "kernels.cuh"
 #include "ptx.cuh"
 #include "keys.cuh"
+#include "tc_split.cuh"
 
 namespace bkm {
 
@@ -19,13 +20,6 @@ constexpr uint32_t TC_THREADS = (2 + TC_EPI_WARPS) * 32;
 constexpr uint32_t TC_MAX_KPAD = 1u << 20;
 constexpr uint32_t TC_TMEM_COLS = 512;
 
-
-__device__ __forceinline__ float to_tf32(float x)
-{
-	uint32_t u;
-	asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
-	return __uint_as_float(u);
-}
 
 // Bounded wait that also gives up when another role already failed.  try_wait suspends the
 // thread for a while by itself but comes back early often, so the loop around it decides how
@@ -78,7 +72,7 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr)
 	return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
-// Same for rows of `kw` floats: kw = 32 as above, kw = 16 -> 64-byte swizzle, rows of 64 B,
+// Same for rows of `kw` words: kw = 32 as above, kw = 16 -> 64-byte swizzle, rows of 64 B,
 // 8-row groups 512 B apart.
 __device__ __forceinline__ uint64_t make_desc_kw(uint32_t smem_addr, uint32_t kw)
 {
@@ -86,7 +80,7 @@ __device__ __forceinline__ uint64_t make_desc_kw(uint32_t smem_addr, uint32_t kw
 		: ((uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61));
 }
 
-// K-major operand without swizzle, one K step (8 tf32 = two 16-byte chunks) wide: 8x16-byte core
+// K-major operand without swizzle, one K step (16 fp16 = two 16-byte chunks) wide: 8x16-byte core
 // matrices; the two chunks of a row group are 128 B apart, row groups 256 B apart.
 __device__ __forceinline__ uint64_t make_desc_aug(uint32_t smem_addr)
 {
@@ -101,24 +95,76 @@ constexpr uint32_t DESC_HI_SW64 = 32u | (1u << 14) | (4u << 29);      // 64-byte
 __device__ __forceinline__ uint32_t desc_lo_sw128(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3FFFu) | (1u << 16); }
 __device__ __forceinline__ uint32_t desc_lo_aug(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3FFFu) | (8u << 16); }
 
-// The constant A operand of the extra K step (128 rows, no-swizzle layout): columns 0 and 1 are
-// one (they meet the high and the low part of |c|^2), columns 2 and 3 hold the offset constant as
-// tf32 hi/lo (they meet ones on the B side), the rest is zero.
-__device__ __forceinline__ void fill_a_aug(float* a_aug, float offset_c, uint32_t tid, uint32_t nthreads)
+// The constant A operand of the extra K step (128 rows, no-swizzle layout): see tc_aug_row.
+__device__ __forceinline__ void fill_a_aug(uint8_t* a_aug, float offset_c, uint32_t tid, uint32_t nthreads)
 {
-	const float c_hi = to_tf32(offset_c), c_lo = to_tf32(offset_c - c_hi);
-	for (uint32_t e = tid; e < TC_MTILE * 8; e += nthreads) {
-		const uint32_t row = e >> 3, kk = e & 7u;
-		a_aug[aug_offset(row, kk)] = kk < 2 ? 1.0f : (kk == 2 ? c_hi : (kk == 3 ? c_lo : 0.0f));
+	const __half a0 = __float2half_rn(TC_AUG_A0), a1 = __float2half_rn(TC_AUG_A1), a2 = __float2half_rn(TC_AUG_A2);
+	const __half a3 = __float2half_rn(offset_c * (1.0f / TC_AUG_B3));
+	const uint4 row = make_uint4((uint32_t)__half_as_ushort(a0) | ((uint32_t)__half_as_ushort(a1) << 16),
+		(uint32_t)__half_as_ushort(a2) | ((uint32_t)__half_as_ushort(a3) << 16), 0u, 0u);
+	uint32_t* words = reinterpret_cast<uint32_t*>(a_aug);
+	for (uint32_t r = tid; r < TC_MTILE; r += nthreads) {
+		*reinterpret_cast<uint4*>(words + aug_offset(r, 0)) = row;
+		*reinterpret_cast<uint4*>(words + aug_offset(r, 1)) = make_uint4(0u, 0u, 0u, 0u);
 	}
 }
 
+// Key constants of the scaled values.  The norms are taken as at least 1 so that the offset constant
+// is a normal fp16 value; that it is rounded to 11 bits there (P / 1024 at most) is covered by the
+// head-room of P / 32.
+__device__ __forceinline__ KeyConsts tc_key_consts(float x2max, float c2max) { return make_key_consts(fmaxf(x2max, 1.0f), c2max); }
+
+// The part of the near-tie band that does not depend on the point: four value spacings, plus what the
+// absolute 2^-25 of small operand values can move a product sum by (2 * 2^-25 * sqrt(dim) * (|x| + |c|)
+// for each side).  Means beyond what the operands hold make it infinite: every point goes to the
+// exact kernel.  (A point beyond it has an infinite |x|^2, which does the same for that point.)
+__device__ __forceinline__ float tc_margin_floor(float ulp, float x2max, float c2max, float sqrt_dim)
+{
+	if (!(c2max <= TC_NORM2_MAX)) return INFINITY;
+	return 4.0f * ulp + 2.4e-7f * sqrt_dim * sqrtf(x2max + c2max);
+}
+
+// The three products of one operand-tile pair over KS steps of 16 dimensions: the small cross
+// terms lo*hi and hi*lo first, then the dominant hi*hi.  Operands are the low halves of the
+// descriptors (+2 in the address field = 32 bytes = one K step), `hi_word` their common high half.
+// `acc_first` = accumulate the very first product onto the destination.
+template<uint32_t KS>
+__device__ __forceinline__ void issue_products(uint32_t d_tmem, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi, uint32_t b_lo,
+	uint32_t hi_word, uint32_t idesc, uint32_t acc_first)
+{
+	ptx::mma_f16_halves(d_tmem, a_lo, hi_word, b_hi, hi_word, idesc, acc_first);
+	#pragma unroll
+	for (uint32_t ks = 1; ks < KS; ++ks)
+		ptx::mma_f16_halves(d_tmem, a_lo + 2 * ks, hi_word, b_hi + 2 * ks, hi_word, idesc, 1);
+	#pragma unroll
+	for (uint32_t ks = 0; ks < KS; ++ks)
+		ptx::mma_f16_halves(d_tmem, a_hi + 2 * ks, hi_word, b_lo + 2 * ks, hi_word, idesc, 1);
+	#pragma unroll
+	for (uint32_t ks = 0; ks < KS; ++ks)
+		ptx::mma_f16_halves(d_tmem, a_hi + 2 * ks, hi_word, b_hi + 2 * ks, hi_word, idesc, 1);
+}
+
+// The end of a point's arg-min: decode the winning key (key - key_base = M * mantissa + column) and
+// write the assignment.  Returns whether best and second are closer than `margin`, i.e. whether
+// the point has to be queued for the exact kernel (the caller appends, a warp at a time).
+__device__ __forceinline__ bool finish_point(uint32_t best, uint32_t second, uint32_t bchunk, uint32_t key_base, uint32_t key_mult, uint32_t key_magic,
+	float ulp, float margin, uint32_t k, uint64_t p, uint32_t* __restrict__ asg)
+{
+	const uint32_t bm = div_key(best - key_base, key_magic);
+	// (with means beyond the operands' range the keys mean nothing: any index, the exact kernel follows)
+	asg[p] = min(bchunk * 32u + ((best - key_base) - bm * key_mult), k - 1);
+	// keys are (mantissa * M + column): the difference of the quotients counts value spacings
+	const float gap = second == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second - key_base, key_magic) - bm) * ulp;
+	return !(gap > margin);                  // (a margin that is not a number sends the point to the exact kernel as well)
+}
+
 // ---- the CTA-pair kernel (assign_tc_pair.cu), used through the plan of assign_tc.cu ----
-bool assign_tc_pair_supported(uint32_t k, uint32_t k_pad, uint32_t d_pad, uint32_t nt_cols, int sm_count);
+bool assign_tc_pair_supported(uint32_t k, uint32_t k_pad, uint32_t dim, uint32_t d_pad, uint32_t nt_cols, int sm_count);
+bool assign_tc_pair_can_fuse(uint32_t k_pad, uint32_t dim, uint32_t d_pad);
 cudaError_t assign_tc_pair_prepare(int sm_count, int* max_pairs);
 cudaError_t launch_assign_tc_pair(const CUtensorMap& a_hi, const CUtensorMap& a_lo, const CUtensorMap& b_hi, const CUtensorMap& b_lo,
 	const float* b_aug, const float* xnorm, uint32_t* asg, uint64_t n, uint32_t n_tiles, uint32_t k, uint32_t k_pad, uint32_t d_pad,
-	uint32_t ksteps, int max_pairs, Control* ctl, int slot, uint32_t* flag_list, float margin_coef, cudaStream_t stream,
+	uint32_t ksteps, int max_pairs, Control* ctl, int slot, uint32_t* flag_list, float margin_coef, float sqrt_dim, cudaStream_t stream,
 	const FusedAcc* fused, uint32_t dim, uint32_t step_begin = 0, uint32_t step_end = 0);
 
 } // namespace bkm

@@ -15,6 +15,7 @@
 //    (kernels/kernels.cu:116-135, 150-163) - fused with the derivation of the operands the
 //    next assignment reads and with clearing the accumulators (fillZeros, :13-17).
 #include "kernels.cuh"
+#include "tc_split.cuh"
 #include "../../include/bkm.h"
 
 #include <algorithm>
@@ -47,13 +48,6 @@ int current_sm_count()
 constexpr int UPD_THREADS = 512;
 constexpr size_t SMEM_LIMIT = 227 * 1024;
 
-__device__ __forceinline__ float tf32_rna(float x)
-{
-	uint32_t u;
-	asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
-	return __uint_as_float(u);
-}
-
 // ------------------------------------------------------------------------------------------
 // finalize / prepare
 // ------------------------------------------------------------------------------------------
@@ -64,7 +58,7 @@ struct RowSinks {
 	float* means_out; uint32_t* sizes_out;
 	uint32_t k, d; int soa_means;
 	float* cprep; uint32_t rs, srows;
-	float* b_hi; float* b_lo; float* cnorm; float* b_aug; const float* center; uint32_t k_pad, d_pad;
+	__half* b_hi; __half* b_lo; float* cnorm; float* b_aug; const float* center; uint32_t k_pad, d_pad;   // d_pad in words
 	Control* ctl; int slot;
 	int divide;            // 0: the rows are written as sums (bucketing), 1: as means
 };
@@ -74,19 +68,20 @@ template<class MEAN>
 __device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32_t lane, bool write_means, uint32_t cnt, MEAN mean_of)
 {
 	float s2 = 0.0f;
+	const float scale = o.b_hi ? tc_scale(o.ctl->xdev) : 1.0f;
 	for (uint32_t j = lane; j < o.d; j += 32) {
 		const float mean = mean_of(j);
 		if (write_means) o.means_out[at_rt(o.soa_means, c, j, o.k, o.d)] = mean;
 		// the tensor-core operands and the norms use the mean relative to the common centre
-		const float shifted = o.center ? mean - o.center[j] : mean;
+		const float shifted = (o.center ? mean - o.center[j] : mean) * scale;
 		s2 = fmaf(shifted, shifted, s2);
 		const float b = -2.0f * shifted;
 		if (o.cprep) o.cprep[(size_t)c * o.rs + 1 + j] = b;
 		if (o.b_hi) {
-			const float hi = tf32_rna(b);
-			const float lo = tf32_rna(b - hi);
-			o.b_hi[(size_t)c * o.d_pad + j] = hi;
-			o.b_lo[(size_t)c * o.d_pad + j] = lo;
+			__half hi, lo;
+			tc_split(b, hi, lo);
+			o.b_hi[(size_t)c * o.d_pad * 2 + j] = hi;
+			o.b_lo[(size_t)c * o.d_pad * 2 + j] = lo;
 		}
 	}
 	#pragma unroll
@@ -96,11 +91,8 @@ __device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32
 		if (o.cprep) o.cprep[(size_t)c * o.rs] = s2;
 		if (o.cnorm) o.cnorm[c] = s2;
 		if (o.b_aug) {
-			const float hi = tf32_rna(s2);
-			const float lo = tf32_rna(s2 - hi);
-			float4* dst = reinterpret_cast<float4*>(o.b_aug + aug_offset(c, 0));
-			dst[0] = make_float4(hi, lo, 1.0f, 1.0f);
-			dst[8] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);    // columns 4..7 sit 32 floats further
+			*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 0)) = tc_aug_row(s2);
+			*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 1)) = make_uint4(0u, 0u, 0u, 0u);
 		}
 		atomicMax(reinterpret_cast<int*>(&o.ctl->cmax2[o.slot]), __float_as_int(s2));
 		if (write_means && o.sizes_out) o.sizes_out[c] = cnt;
@@ -113,9 +105,8 @@ __device__ __forceinline__ void finish_padding_row(const RowSinks& o, uint32_t c
 	if (o.cprep && c < o.srows) o.cprep[(size_t)c * o.rs] = INFINITY;
 	if (o.cnorm && c < o.k_pad) o.cnorm[c] = INFINITY;
 	if (o.b_aug && c < o.k_pad) {
-		float4* dst = reinterpret_cast<float4*>(o.b_aug + aug_offset(c, 0));
-		dst[0] = make_float4(0.0f, 0.0f, 1.0f, 1.0f);
-		dst[8] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+		*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 0)) = tc_aug_row(0.0f);
+		*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 1)) = make_uint4(0u, 0u, 0u, 0u);
 	}
 }
 
@@ -308,7 +299,7 @@ static RowSinks make_sinks(float* means_out, uint32_t* sizes_out, const Shape& s
 	o.means_out = means_out; o.sizes_out = sizes_out;
 	o.k = s.k; o.d = s.dim; o.soa_means = s.soa_means;
 	o.cprep = sm ? sm->rows : nullptr; o.rs = simt_row_stride(s.dim); o.srows = simt_rows(s.k);
-	o.b_hi = tc ? tc->b_hi : nullptr; o.b_lo = tc ? tc->b_lo : nullptr;
+	o.b_hi = tc ? reinterpret_cast<__half*>(tc->b_hi) : nullptr; o.b_lo = tc ? reinterpret_cast<__half*>(tc->b_lo) : nullptr;
 	o.cnorm = tc ? tc->cnorm : nullptr; o.b_aug = tc ? tc->b_aug : nullptr;
 	o.center = tc ? tc->center : (sm ? sm->center : nullptr);
 	o.k_pad = tc ? tc->k_pad : 0; o.d_pad = tc ? tc->d_pad : 0;
@@ -461,7 +452,7 @@ __global__ void points_key_decide_kernel(PointsKey* key, unsigned long long ptr,
 	key->valid = same ? 1u : 0u;
 	key->fp_old = key->fp_new;
 	key->ptr = ptr; key->n = n; key->dim = dim; key->layout = layout; key->variant = variant;
-	if (!same) ctl->xmax2 = 0.0f;
+	if (!same) { ctl->xmax2 = 0.0f; ctl->xdev = 0.0f; ctl->beyond = 0u; }
 }
 
 cudaError_t launch_points_fingerprint(const float* pts, uint64_t words, PointsKey* key, int sm_count, cudaStream_t stream)

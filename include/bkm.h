@@ -73,7 +73,7 @@ int bkm_device_count(void);
  *
  * The reference's drivers call their runners once per iteration on the same, immutable points
  * (headers/cuda.hpp:70-88).  bkm_assign_f32 and bkm_iterate_f32 therefore leave what they derive
- * from the points alone (a centre vector, the largest norm, tf32 operand planes) in the
+ * from the points alone (a centre vector, the largest norm, fp16 operand planes) in the
  * workspace, and a later call on the same workspace skips that work when it finds the same
  * points: same address, shape and variant, and the same fingerprint of a sample of the values
  * (every 16th 128-byte line and the last).  New data at the same address is therefore noticed;
@@ -292,8 +292,8 @@ int bkm_counters(bkm_handle_t h, uint64_t out[4]);
  * pass also accumulated the update sums.  Valid after bkm_initialize. */
 #define BKM_PLAN_EXACT 0        /* CUDA cores, reference arithmetic */
 #define BKM_PLAN_SIMT 1         /* CUDA cores, small-dim fast pass */
-#define BKM_PLAN_TC_RESIDENT 2  /* tcgen05, one CTA per SM, point tiles resident (dim <= 32) */
-#define BKM_PLAN_TC_KLOOP 3     /* tcgen05, one CTA per SM, both operands stream in slices (dim > 32) */
+#define BKM_PLAN_TC_RESIDENT 2  /* tcgen05, one CTA per SM, point tiles resident (dim <= 64) */
+#define BKM_PLAN_TC_KLOOP 3     /* tcgen05, one CTA per SM, both operands stream in slices (dim > 64) */
 #define BKM_PLAN_TC_PAIR 4      /* tcgen05 on CTA pairs, all means resident in shared memory */
 int bkm_assign_plan(bkm_handle_t h, uint32_t out[4]);
 
