@@ -63,25 +63,34 @@ struct RowSinks {
 	int divide;            // 0: the rows are written as sums (bucketing), 1: as means
 };
 
-// One warp finishes row c < k.  `mean_of(j)` yields coordinate j of the mean (lane-strided calls).
-template<class MEAN>
-__device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32_t lane, bool write_means, uint32_t cnt, MEAN mean_of)
+// One warp finishes row c < k.  `means_of(j, m)` yields coordinates j, j + 32, j + 64, j + 96 of the
+// mean as far as they exist (j lane-strided): four at a time, so that a long row has the loads of
+// several of them in flight.
+template<class MEANS>
+__device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32_t lane, bool write_means, uint32_t cnt, MEANS means_of)
 {
 	float s2 = 0.0f;
 	const float scale = o.b_hi ? tc_scale(o.ctl->xdev) : 1.0f;
-	for (uint32_t j = lane; j < o.d; j += 32) {
-		const float mean = mean_of(j);
-		if (write_means) o.means_out[at_rt(o.soa_means, c, j, o.k, o.d)] = mean;
-		// the tensor-core operands and the norms use the mean relative to the common centre
-		const float shifted = (o.center ? mean - o.center[j] : mean) * scale;
-		s2 = fmaf(shifted, shifted, s2);
-		const float b = -2.0f * shifted;
-		if (o.cprep) o.cprep[(size_t)c * o.rs + 1 + j] = b;
-		if (o.b_hi) {
-			__half hi, lo;
-			tc_split(b, hi, lo);
-			o.b_hi[(size_t)c * o.d_pad * 2 + j] = hi;
-			o.b_lo[(size_t)c * o.d_pad * 2 + j] = lo;
+	for (uint32_t j0 = lane; j0 < o.d; j0 += 128) {
+		float m[4];
+		means_of(j0, m);
+		#pragma unroll
+		for (uint32_t q = 0; q < 4; ++q) {
+			const uint32_t j = j0 + 32 * q;
+			if (j >= o.d) break;
+			const float mean = m[q];
+			if (write_means) o.means_out[at_rt(o.soa_means, c, j, o.k, o.d)] = mean;
+			// the tensor-core operands and the norms use the mean relative to the common centre
+			const float shifted = (o.center ? mean - o.center[j] : mean) * scale;
+			s2 = fmaf(shifted, shifted, s2);
+			const float b = -2.0f * shifted;
+			if (o.cprep) o.cprep[(size_t)c * o.rs + 1 + j] = b;
+			if (o.b_hi) {
+				__half hi, lo;
+				tc_split(b, hi, lo);
+				o.b_hi[(size_t)c * o.d_pad * 2 + j] = hi;
+				o.b_lo[(size_t)c * o.d_pad * 2 + j] = lo;
+			}
 		}
 	}
 	#pragma unroll
@@ -153,18 +162,44 @@ __global__ void __launch_bounds__(256) finalize_prepare_kernel(float* __restrict
 	for (uint32_t c = blockIdx.x * wpb + (threadIdx.x >> 5); c < rows_total; c += gridDim.x * wpb) {
 		if (c < o.k) {
 			if (FINALIZE) {
-				uint32_t cnt = 0;
-				for (uint32_t r = 0; r < replicas; ++r) cnt += counts[c + r * rep_stride];
+				// (at most 16 copies: one per lane)
+				uint32_t cnt = lane < replicas ? counts[c + lane * rep_stride] : 0u;
+				cnt = __reduce_add_sync(0xffffffffu, cnt);
+				if (lane < replicas) counts[c + lane * rep_stride] = 0u;
 				const float divisor = (float)cnt;
-				finish_row(o, c, lane, true, cnt, [&](uint32_t j) {
-					const float sum = sum_and_clear(acc + (size_t)c * o.d + j, replicas, rep_stride);
-					if (!o.divide) return sum;
-					return cnt ? __fdiv_rn(sum, divisor) : 0.0f;
+				finish_row(o, c, lane, true, cnt, [&](uint32_t j, float (&m)[4]) {
+					const float* src = acc + (size_t)c * o.d + j;
+					float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+					uint32_t r = 0;
+					#pragma unroll 4
+					for (; r + 4 <= replicas; r += 4) {
+						#pragma unroll
+						for (uint32_t q = 0; q < 4; ++q) {
+							if (j + 32 * q < o.d) {
+								const float* p = src + r * rep_stride + 32 * q;
+								const float s0 = p[0], s1 = p[rep_stride], s2 = p[2 * rep_stride], s3 = p[3 * rep_stride];
+								sum[q] += (s0 + s1) + (s2 + s3);
+							}
+						}
+					}
+					for (; r < replicas; ++r) {
+						#pragma unroll
+						for (uint32_t q = 0; q < 4; ++q) if (j + 32 * q < o.d) sum[q] += src[r * rep_stride + 32 * q];
+					}
+					// cleared for the next iteration only after all loads, which therefore travel together
+					float* dst = acc + (size_t)c * o.d + j;
+					for (r = 0; r < replicas; ++r) {
+						#pragma unroll
+						for (uint32_t q = 0; q < 4; ++q) if (j + 32 * q < o.d) dst[r * rep_stride + 32 * q] = 0.0f;
+					}
+					#pragma unroll
+					for (uint32_t q = 0; q < 4; ++q) m[q] = !o.divide ? sum[q] : (cnt ? __fdiv_rn(sum[q], divisor) : 0.0f);
 				});
-				__syncwarp();
-				if (lane == 0) for (uint32_t r = 0; r < replicas; ++r) counts[c + r * rep_stride] = 0;
 			} else {
-				finish_row(o, c, lane, false, 0u, [&](uint32_t j) { return means_in[at_rt(o.soa_means, c, j, o.k, o.d)]; });
+				finish_row(o, c, lane, false, 0u, [&](uint32_t j, float (&m)[4]) {
+					#pragma unroll
+					for (uint32_t q = 0; q < 4; ++q) m[q] = j + 32 * q < o.d ? means_in[at_rt(o.soa_means, c, j + 32 * q, o.k, o.d)] : 0.0f;
+				});
 			}
 		} else if (lane == 0) {
 			finish_padding_row(o, c);
@@ -276,13 +311,17 @@ __global__ void __launch_bounds__(256) exchange_finalize_kernel(float* __restric
 			#pragma unroll
 			for (uint32_t r = 0; r < EXCHANGE_MAX_RANKS; ++r) if (r < world) cnt += part[r];
 			const float divisor = (float)cnt;
-			finish_row(o, c, lane, true, cnt, [&](uint32_t j) {
-				uint32_t bits[EXCHANGE_MAX_RANKS];
-				poll_packets(slot, words, (size_t)c * o.d + j, world, epoch, wait_limit_ns, &s_timeout, bits);
-				float sum = 0.0f;
+			finish_row(o, c, lane, true, cnt, [&](uint32_t j0, float (&m)[4]) {
 				#pragma unroll
-				for (uint32_t r = 0; r < EXCHANGE_MAX_RANKS; ++r) if (r < world) sum += __uint_as_float(bits[r]);
-				return cnt ? __fdiv_rn(sum, divisor) : 0.0f;
+				for (uint32_t q = 0; q < 4; ++q) {
+					if (j0 + 32 * q >= o.d) break;
+					uint32_t bits[EXCHANGE_MAX_RANKS];
+					poll_packets(slot, words, (size_t)c * o.d + j0 + 32 * q, world, epoch, wait_limit_ns, &s_timeout, bits);
+					float sum = 0.0f;
+					#pragma unroll
+					for (uint32_t r = 0; r < EXCHANGE_MAX_RANKS; ++r) if (r < world) sum += __uint_as_float(bits[r]);
+					m[q] = cnt ? __fdiv_rn(sum, divisor) : 0.0f;
+				}
 			});
 		} else if (lane == 0) {
 			finish_padding_row(o, c);
