@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) update_rows_kernel(const float* 
 //
 // With few clusters every global or shared-memory reduction of the row-wise kernels lands on
 // one of a few hundred hot rows, and the memory system serialises them.  Here a block takes a
-// chunk of SORT_CHUNK consecutive points and sorts their positions by cluster in shared memory
+// chunk of CHUNK consecutive points and sorts their positions by cluster in shared memory
 // (histogram, prefix sum, scatter).  Groups of `dg` lanes (one lane per dimension) then walk
 // equal shares of the sorted order, adding rows into a register while the cluster stays the
 // same and sending one row of reductions when it changes.  The number of reductions drops by
@@ -737,14 +737,18 @@ __global__ void __launch_bounds__(ROWS_THREADS) update_rows_kernel(const float* 
 // accumulators pre-added in a fixed small tree, which also keeps the rounding error down.
 
 constexpr uint32_t SORT_THREADS = 256;
-constexpr uint32_t SORT_CHUNK = 2048;
-constexpr uint32_t SORT_PER_THREAD = SORT_CHUNK / SORT_THREADS;
 constexpr uint32_t SORT_MAX_K = 1024;
 constexpr uint32_t SORT_SCAN = (SORT_MAX_K + 1 + SORT_THREADS - 1) / SORT_THREADS;   // buckets per thread in the scan
 
 bool update_sorted_supported(const Shape& s) { return s.k <= SORT_MAX_K; }
 
-template<bool SOA, int VW>
+static uint32_t sorted_chunk(uint64_t n, int sm_count)
+{
+	const uint64_t blocks = (uint64_t)sm_count * 4;
+	return n >= blocks * 2048 ? 2048u : (n >= blocks * 1024 ? 1024u : 512u);
+}
+
+template<bool SOA, int VW, uint32_t CHUNK>
 __global__ void __launch_bounds__(SORT_THREADS) update_sorted_kernel(const float* __restrict__ pts,
 	const uint32_t* __restrict__ asg, float* __restrict__ acc, uint32_t* __restrict__ counts,
 	uint64_t n, uint32_t k, uint32_t d, uint32_t dg, uint32_t replicas, size_t rep_stride, Control* __restrict__ ctl)
@@ -752,28 +756,31 @@ __global__ void __launch_bounds__(SORT_THREADS) update_sorted_kernel(const float
 	acc += (blockIdx.x % replicas) * rep_stride;
 	counts += (blockIdx.x % replicas) * rep_stride;
 	__shared__ uint32_t start[SORT_MAX_K + 2];      // after the scan: first sorted position of each cluster (k = trash bucket)
-	__shared__ __align__(8) uint16_t order[SORT_CHUNK];     // sorted position -> point within the chunk
-	__shared__ __align__(8) uint16_t cl_sorted[SORT_CHUNK]; // sorted position -> cluster
+	__shared__ __align__(8) uint16_t order[CHUNK];     // sorted position -> point within the chunk
+	__shared__ __align__(8) uint16_t cl_sorted[CHUNK]; // sorted position -> cluster
 	__shared__ uint32_t warp_sums[SORT_THREADS / 32];
 	const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
 	const uint32_t nsub = 32 / dg;                  // lane groups per warp
 	const uint32_t dl = lane % dg, sub = lane / dg;
 	const uint32_t walker = warp * nsub + sub, walkers = (SORT_THREADS / 32) * nsub;
-	const uint64_t chunks = (n + SORT_CHUNK - 1) / SORT_CHUNK;
+	const uint64_t chunks = (n + CHUNK - 1) / CHUNK;
+// A walker has four rows in flight, so few blocks leave the kernel waiting for memory: the chunk is the
+// largest of 2048, 1024 and 512 points that still gives four blocks per SM (sorted_chunk).
 	bool bad = false;
 	for (uint64_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
-		const uint64_t base = chunk * SORT_CHUNK;
-		const uint32_t cnt = (uint32_t)(n - base < SORT_CHUNK ? n - base : SORT_CHUNK);
+		const uint64_t base = chunk * CHUNK;
+		const uint32_t cnt = (uint32_t)(n - base < CHUNK ? n - base : CHUNK);
 		__syncthreads();                            // the previous chunk's walkers are done
 		for (uint32_t c = tid; c <= k; c += SORT_THREADS) start[c] = 0;
 		__syncthreads();
-		uint32_t mine[SORT_PER_THREAD], rank[SORT_PER_THREAD];
+		uint32_t mine[PER_THREAD], rank[PER_THREAD];
 		#pragma unroll
-		for (uint32_t r = 0; r < SORT_PER_THREAD; ++r) {
+		for (uint32_t r = 0; r < PER_THREAD; ++r) {
 			const uint32_t i = r * SORT_THREADS + tid;
 			uint32_t c = k;                         // trash bucket: beyond the chunk or a bad index
 			if (i < cnt) {
 				c = asg[base + i];
+	constexpr uint32_t PER_THREAD = CHUNK / SORT_THREADS;
 				if (c >= k) { bad = true; c = k; }
 			}
 			mine[r] = c;
@@ -807,7 +814,7 @@ __global__ void __launch_bounds__(SORT_THREADS) update_sorted_kernel(const float
 			if (sz) atomicAdd(&counts[c], sz);
 		}
 		#pragma unroll
-		for (uint32_t r = 0; r < SORT_PER_THREAD; ++r) {
+		for (uint32_t r = 0; r < PER_THREAD; ++r) {
 			const uint32_t pos = start[mine[r]] + rank[r];
 			order[pos] = (uint16_t)(r * SORT_THREADS + tid);
 			cl_sorted[pos] = (uint16_t)mine[r];
@@ -946,13 +953,19 @@ void launch_update(const float* pts, const uint32_t* asg, float* acc, uint32_t* 
 		const uint32_t per_point = s.dim / (uint32_t)vw;
 		uint32_t dg = vw == 1 ? 2 : 1;              // lanes per point: the power of two that covers a row, at most 32
 		while (dg < 32 && dg < per_point) dg <<= 1;
-		const uint64_t chunks = (s.n + SORT_CHUNK - 1) / SORT_CHUNK;
+		const uint32_t chunk = sorted_chunk(s.n, sm_count);
+		const uint64_t chunks = (s.n + chunk - 1) / chunk;
 		const uint32_t grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(chunks, 1), (uint64_t)sm_count * 8);
 		const size_t rep_stride = acc_replica_stride(s.k, s.dim);
-		if (s.soa) update_sorted_kernel<true, 1><<<grid, SORT_THREADS, 0, stream>>>(pts, asg, acc, counts, s.n, s.k, s.dim, dg, replicas, rep_stride, ctl);
-		else if (vw == 4) update_sorted_kernel<false, 4><<<grid, SORT_THREADS, 0, stream>>>(pts, asg, acc, counts, s.n, s.k, s.dim, dg, replicas, rep_stride, ctl);
-		else if (vw == 2) update_sorted_kernel<false, 2><<<grid, SORT_THREADS, 0, stream>>>(pts, asg, acc, counts, s.n, s.k, s.dim, dg, replicas, rep_stride, ctl);
-		else update_sorted_kernel<false, 1><<<grid, SORT_THREADS, 0, stream>>>(pts, asg, acc, counts, s.n, s.k, s.dim, dg, replicas, rep_stride, ctl);
+#define BKM_LAUNCH_SORTED(SOA, VW) do { \
+		auto kern = chunk == 2048 ? update_sorted_kernel<SOA, VW, 2048> : (chunk == 1024 ? update_sorted_kernel<SOA, VW, 1024> : update_sorted_kernel<SOA, VW, 512>); \
+		kern<<<grid, SORT_THREADS, 0, stream>>>(pts, asg, acc, counts, s.n, s.k, s.dim, dg, replicas, rep_stride, ctl); \
+	} while (0)
+		if (s.soa) BKM_LAUNCH_SORTED(true, 1);
+		else if (vw == 4) BKM_LAUNCH_SORTED(false, 4);
+		else if (vw == 2) BKM_LAUNCH_SORTED(false, 2);
+		else BKM_LAUNCH_SORTED(false, 1);
+#undef BKM_LAUNCH_SORTED
 		return;
 	}
 	if (variant == BKM_UPDATE_ROWS) {
