@@ -735,6 +735,8 @@ __global__ void __launch_bounds__(ROWS_THREADS) update_rows_kernel(const float* 
 // same and sending one row of reductions when it changes.  The number of reductions drops by
 // about the number of points per cluster and chunk (8 for 256 clusters), and the sums reach the
 // accumulators pre-added in a fixed small tree, which also keeps the rounding error down.
+// A walker has four rows in flight, so few blocks leave the kernel waiting for memory: the chunk is the
+// largest of 2048, 1024 and 512 points that still gives four blocks per SM (sorted_chunk).
 
 constexpr uint32_t SORT_THREADS = 256;
 constexpr uint32_t SORT_MAX_K = 1024;
@@ -753,6 +755,7 @@ __global__ void __launch_bounds__(SORT_THREADS) update_sorted_kernel(const float
 	const uint32_t* __restrict__ asg, float* __restrict__ acc, uint32_t* __restrict__ counts,
 	uint64_t n, uint32_t k, uint32_t d, uint32_t dg, uint32_t replicas, size_t rep_stride, Control* __restrict__ ctl)
 {
+	constexpr uint32_t PER_THREAD = CHUNK / SORT_THREADS;
 	acc += (blockIdx.x % replicas) * rep_stride;
 	counts += (blockIdx.x % replicas) * rep_stride;
 	__shared__ uint32_t start[SORT_MAX_K + 2];      // after the scan: first sorted position of each cluster (k = trash bucket)
@@ -764,8 +767,6 @@ __global__ void __launch_bounds__(SORT_THREADS) update_sorted_kernel(const float
 	const uint32_t dl = lane % dg, sub = lane / dg;
 	const uint32_t walker = warp * nsub + sub, walkers = (SORT_THREADS / 32) * nsub;
 	const uint64_t chunks = (n + CHUNK - 1) / CHUNK;
-// A walker has four rows in flight, so few blocks leave the kernel waiting for memory: the chunk is the
-// largest of 2048, 1024 and 512 points that still gives four blocks per SM (sorted_chunk).
 	bool bad = false;
 	for (uint64_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
 		const uint64_t base = chunk * CHUNK;
@@ -780,7 +781,6 @@ __global__ void __launch_bounds__(SORT_THREADS) update_sorted_kernel(const float
 			uint32_t c = k;                         // trash bucket: beyond the chunk or a bad index
 			if (i < cnt) {
 				c = asg[base + i];
-	constexpr uint32_t PER_THREAD = CHUNK / SORT_THREADS;
 				if (c >= k) { bad = true; c = k; }
 			}
 			mine[r] = c;
