@@ -378,10 +378,6 @@ static int stateless_common(uint64_t n, uint32_t k, uint32_t dim, int layout, in
 	return device_sm_count(*device, sm_count);
 }
 
-// Bytes of the control block that every stateless call clears: status, flag count and the two
-// max |c|^2 slots.  last_flag_count and xmax2 behind them survive (xmax2 belongs to the points).
-constexpr size_t CONTROL_CLEAR_BYTES = 16;
-
 // Tensor maps are a function of the workspace address and the shape, so the stateless calls keep
 // the few most recent plans instead of encoding six maps per call.
 struct PlanSlot {
@@ -438,33 +434,36 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 	int rc = resolve_assign(variant, s, &v);
 	if (rc) return rc;
 	if (fused_out) *fused_out = false;
-	CUDA_TRY(cudaMemsetAsync(w.ctl, 0, CONTROL_CLEAR_BYTES, st));
-	CUDA_TRY(cudaMemsetAsync(w.split_scratch, 0, bkm::list_split_scratch_bytes(), st));
 	bkm::TcPlan* plan = nullptr;
 	bool fused = false;
-	if (v == BKM_ASSIGN_SIMT || v == BKM_ASSIGN_TC) {
-		bkm::PointsKey* key = reinterpret_cast<bkm::PointsKey*>(reinterpret_cast<char*>(w.ctl) + bkm::POINTS_KEY_OFFSET);
+	bkm::PointsKey* key = nullptr;
+	if (v == BKM_ASSIGN_SIMT) {
+		fused = fa != nullptr && fuse_pays(v, variant_update, nullptr, *fa, s, true);     // the caller asked for the one-pass form
+	} else if (v == BKM_ASSIGN_TC) {
+		const char* err = nullptr;
+		plan = cached_plan(s, w, device, &err);
+		if (!plan) return fail(BKM_ERR_CUDA, "tensor-core plan: %s", err ? err : "unknown");
+		bkm::tc_plan_allow_pair(plan, true);
+		fused = fa != nullptr && fuse_pays(v, variant_update, plan, *fa, s);
+	}
+	// the re-check's scratch, the accumulators (also those of a separate update that follows) and the
+	// padding of the operands derived from the means (workspace ranges are multiples of 256 bytes)
+	bkm::ClearRanges clear = {{w.split_scratch, w.acc, nullptr}, {bkm::list_split_scratch_bytes(), fa ? align256(w.acc_bytes) : 0, 0}};
+	if (v == BKM_ASSIGN_SIMT) { clear.base[2] = w.sm.rows; clear.bytes[2] = align256(w.cprep_bytes); }
+	if (v == BKM_ASSIGN_TC) { clear.base[2] = w.tm.b_hi; clear.bytes[2] = w.tm_bytes; }
+	if (v != BKM_ASSIGN_EXACT) key = reinterpret_cast<bkm::PointsKey*>(reinterpret_cast<char*>(w.ctl) + bkm::POINTS_KEY_OFFSET);
+	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, key, clear, sm_count, st));
+	if (key) {
 		const uint32_t* skip = &key->valid;
-		CUDA_TRY(cudaMemsetAsync(&key->fp_new, 0, sizeof(key->fp_new), st));
-		CUDA_TRY(bkm::launch_points_fingerprint(points, s.n * s.dim, key, sm_count, st));
-		CUDA_TRY(bkm::launch_points_key_decide(key, points, s, v, w.ctl, st));
+		CUDA_TRY(bkm::launch_points_fingerprint(points, s, v, key, w.ctl, sm_count, st));
 		CUDA_TRY(bkm::launch_compute_center(points, s, w.tm.center, w.ctl, st, skip));
 		if (v == BKM_ASSIGN_SIMT) {
-			CUDA_TRY(cudaMemsetAsync(w.sm.rows, 0, w.cprep_bytes, st));
 			CUDA_TRY(bkm::launch_points_norm_max(points, s, w.tm.center, w.ctl, sm_count, st, skip));
 			bkm::launch_prepare_means(means, s, &w.sm, nullptr, w.ctl, 0, st);
-			fused = fa != nullptr && fuse_pays(v, variant_update, nullptr, *fa, s, true);     // the caller asked for the one-pass form
 		} else {
-			CUDA_TRY(cudaMemsetAsync(w.tm.b_hi, 0, w.tm_bytes, st));
 			bkm::launch_prepare_means(means, s, nullptr, &w.tm, w.ctl, 0, st);
 			CUDA_TRY(bkm::launch_split_points(points, s, w.tp, w.tm.center, w.ctl, st, skip));
-			const char* err = nullptr;
-			plan = cached_plan(s, w, device, &err);
-			if (!plan) return fail(BKM_ERR_CUDA, "tensor-core plan: %s", err ? err : "unknown");
-			bkm::tc_plan_allow_pair(plan, true);
-			fused = fa != nullptr && fuse_pays(v, variant_update, plan, *fa, s);
 		}
-		if (fused) CUDA_TRY(cudaMemsetAsync(w.acc, 0, w.acc_bytes, st));
 	}
 	CUDA_TRY(cudaGetLastError());
 	if (fused_out) *fused_out = fused;
@@ -472,13 +471,13 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 }
 
 static int stateless_update(const float* points, const uint32_t* assignment, float* means, uint32_t* sizes,
-	const bkm::Shape& s, const Workspace& w, int variant, int device, int sm_count, cudaStream_t st, bool clear_ctl)
+	const bkm::Shape& s, const Workspace& w, int variant, int device, int sm_count, cudaStream_t st, bool clear)
 {
 	int v = 0;
 	int rc = resolve_update(variant, s, device, &v);
 	if (rc) return rc;
-	if (clear_ctl) CUDA_TRY(cudaMemsetAsync(w.ctl, 0, CONTROL_CLEAR_BYTES, st));
-	CUDA_TRY(cudaMemsetAsync(w.acc, 0, w.acc_bytes, st));
+	// (an assignment in front of it has cleared the accumulators as well)
+	if (clear) CUDA_TRY(bkm::launch_stateless_begin(w.ctl, nullptr, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, sm_count, st));
 	bkm::launch_update(points, assignment, w.acc, w.counts, w.replicas, s, v, w.ctl, sm_count, st);
 	bkm::launch_finalize(w.acc, w.counts, w.replicas, means, sizes, s, nullptr, nullptr, w.ctl, 1, st);
 	CUDA_TRY(cudaGetLastError());
@@ -517,8 +516,7 @@ int bkm_bucket_sums_f32(const float* points, const uint32_t* indices, float* sum
 	int v = 0;
 	if ((rc = resolve_update(variant, s, device, &v))) return rc;
 	cudaStream_t st = static_cast<cudaStream_t>(stream);
-	CUDA_TRY(cudaMemsetAsync(w.ctl, 0, CONTROL_CLEAR_BYTES, st));
-	CUDA_TRY(cudaMemsetAsync(w.acc, 0, w.acc_bytes, st));
+	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, nullptr, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, sm, st));
 	bkm::launch_update(points, indices, w.acc, w.counts, w.replicas, s, v, w.ctl, sm, st);
 	bkm::launch_finalize_sums(w.acc, w.counts, w.replicas, sums, s, w.ctl, st);
 	CUDA_TRY(cudaGetLastError());

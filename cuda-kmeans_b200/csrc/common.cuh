@@ -36,6 +36,7 @@ struct PointsKey {
 	unsigned long long fp_old;   // fingerprint the operands in the workspace belong to
 	unsigned long long ptr, n;
 	uint32_t dim, layout, variant, valid;
+	uint32_t arrive, pad;        // blocks of the fingerprint that are done
 };
 constexpr size_t POINTS_KEY_OFFSET = 64;
 

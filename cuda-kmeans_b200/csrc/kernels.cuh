@@ -81,13 +81,16 @@ void launch_finalize_sums(float* acc, uint32_t* counts, uint32_t replicas, float
 cudaError_t launch_probe_atomics(float* result, uint64_t n, uint32_t k, uint32_t dim, int soa, bool shared_cache, uint32_t items_per_thread,
 	cudaStream_t stream);
 
-// ---- recognising the point set of a stateless call (update.cu) ----
-// Adds a fingerprint of the points (every 16th 128-byte line and the last one; order-independent
-// sum of mixed (value, position) words) to key->fp_new, which must be zero on entry.
-cudaError_t launch_points_fingerprint(const float* pts, uint64_t words, PointsKey* key, int sm_count, cudaStream_t stream);
-// Sets key->valid (same address, shape, variant and fingerprint as remembered) and remembers the
-// current call's; when the points are new it also clears ctl->xmax2, which their preprocessing refills.
-cudaError_t launch_points_key_decide(PointsKey* key, const float* pts, const Shape& s, int variant, Control* ctl, cudaStream_t stream);
+// ---- the beginning of a stateless call (update.cu) ----
+// Ranges of the workspace to clear (16-byte aligned, whole multiples of 16 bytes; 0 bytes = unused).
+struct ClearRanges { void* base[3]; size_t bytes[3]; };
+// Clears status, near-tie count, |c|^2 slots, the fingerprint of `key` (may be null) and the ranges.
+cudaError_t launch_stateless_begin(Control* ctl, PointsKey* key, const ClearRanges& ranges, int sm_count, cudaStream_t stream);
+// Fingerprints the points (every 16th 128-byte line and the last one; order-independent sum of mixed
+// (value, position) words), sets key->valid (same address, shape, variant and fingerprint as
+// remembered) and remembers the current call's; when the points are new it also clears what their
+// preprocessing refills in `ctl`.  Behind launch_stateless_begin with the same key.
+cudaError_t launch_points_fingerprint(const float* pts, const Shape& s, int variant, PointsKey* key, Control* ctl, int sm_count, cudaStream_t stream);
 
 // ---- update (update.cu) ----
 // variant: BKM_UPDATE_SHARED or BKM_UPDATE_GLOBAL (already resolved).  acc/counts must be zero.
