@@ -336,65 +336,113 @@ __global__ void __launch_bounds__(LIST_THREADS, PB > LIST_PB ? 2 : 3) assign_exa
 	}
 }
 
-// The same arithmetic with one THREAD per queued point and all means in shared memory, for mean sets
-// of a few thousand floats and at most 16 dimensions: there a block per four points spends its time
-// in barriers and reductions, while a thread walks the whole set in microseconds and a long list
-// fills the machine by itself.
+// The same arithmetic with all means in shared memory and the lanes of a warp shared out over points:
+// for mean sets of a few thousand floats and at most 16 dimensions, where a block per four points
+// spends its time in barriers and reductions.  A long list gives every point one thread and fills the
+// machine by itself; a short one gives a point 2 to 32 lanes, each of which walks every 2nd to 32nd
+// mean.  A thread is bound by the latency of its D dependent additions, so it keeps four sums going at
+// a time (encode of 250 000 8-dimensional vectors against 256 means, a few thousand of them queued:
+// 31 us with one thread per point and one sum at a time).
 constexpr uint32_t LIST_SMALL_MAX_FLOATS = 4096;
 constexpr uint32_t LIST_SMALL_MAX_DIM = 16;
+constexpr uint32_t LIST_SMALL_SUMS = 4;
+
+// Exact distances of one point to the means sub, sub + lanes, ... in shared memory (rows of RS floats,
+// LIST_SMALL_SUMS - 1 rows of infinities behind the last), four at a time.
+// The reference compares square roots.  The correctly rounded square root never decreases with its
+// argument, so a sum that is not below the best sum cannot give a smaller root: only the few
+// candidates that are below it need the root itself (equal roots of different sums keep the earlier
+// mean, as the reference's strict comparison does).
+template<int D, uint32_t RS>
+__device__ __forceinline__ void scan_means(const float* sm, const float (&x)[D], uint32_t k, uint32_t sub, uint32_t lanes,
+	float& best, float& best_sum, uint32_t& bidx)
+{
+	for (uint32_t m0 = sub; m0 < k; m0 += lanes * LIST_SMALL_SUMS) {
+		float sum[LIST_SMALL_SUMS];
+		#pragma unroll
+		for (uint32_t u = 0; u < LIST_SMALL_SUMS; ++u) {
+			const float* row = sm + (lanes == 1 ? m0 + u : min(m0 + u * lanes, k - 1u)) * RS;
+			float c[D];
+			if (D % 4 == 0) {
+				#pragma unroll
+				for (int q = 0; q < D / 4; ++q) {
+					const float4 v = *reinterpret_cast<const float4*>(row + 4 * q);
+					c[4 * q] = v.x; c[4 * q + 1] = v.y; c[4 * q + 2] = v.z; c[4 * q + 3] = v.w;
+				}
+			} else if (D % 2 == 0) {
+				#pragma unroll
+				for (int q = 0; q < D / 2; ++q) {
+					const float2 v = *reinterpret_cast<const float2*>(row + 2 * q);
+					c[2 * q] = v.x; c[2 * q + 1] = v.y;
+				}
+			} else {
+				#pragma unroll
+				for (int j = 0; j < D; ++j) c[j] = row[j];
+			}
+			sum[u] = 0.0f;
+			#pragma unroll
+			for (int j = 0; j < D; ++j) {
+				const float diff = __fsub_rn(x[j], c[j]);
+				sum[u] = __fadd_rn(sum[u], __fmul_rn(diff, diff));
+			}
+		}
+		// the first mean is taken whatever its distance, as in the sequential scan
+		if (m0 == 0) { best_sum = sum[0]; best = __fsqrt_rn(sum[0]); bidx = 0; }
+		// (a row of infinities is not below the best, nor is anything below what is not a number; behind the last
+		// mean of a lane the very last mean is looked at again)
+		if (fminf(fminf(sum[0], sum[1]), fminf(sum[2], sum[3])) < best_sum) {
+			#pragma unroll
+			for (uint32_t u = 0; u < LIST_SMALL_SUMS; ++u) {
+				if (sum[u] < best_sum) {
+					const float dist = __fsqrt_rn(sum[u]);
+					if (dist < best) { best = dist; best_sum = sum[u]; bidx = min(m0 + u * lanes, k - 1u); }
+				}
+			}
+		}
+	}
+}
 
 template<int D, bool SOA, bool SOAM>
 __global__ void __launch_bounds__(256) assign_exact_list_small_kernel(const float* __restrict__ pts, const float* __restrict__ means,
 	uint32_t* __restrict__ asg, uint64_t n, uint32_t k, const uint32_t* __restrict__ list, const uint32_t* __restrict__ list_count,
 	float* __restrict__ fix_acc, uint32_t* __restrict__ fix_counts)
 {
-	__shared__ __align__(16) float sm[LIST_SMALL_MAX_FLOATS];          // [mean][dimension]
+	// [mean][dimension], read as vectors of VW floats; a row is an odd number of them, so that lanes on
+	// neighbouring means meet different banks
+	constexpr uint32_t VW = D % 4 == 0 ? 4 : (D % 2 == 0 ? 2 : 1), RS = (D / VW) % 2 == 0 ? D + VW : D;
+	__shared__ __align__(16) float sm[(LIST_SMALL_MAX_FLOATS / D + LIST_SMALL_SUMS - 1) * RS];
 	uint64_t total = *list_count;
 	if (total > n) total = n;
-	if ((uint64_t)blockIdx.x * blockDim.x >= total) return;            // the grid is sized for long lists: most blocks of a short one have nothing to do
+	const uint64_t threads = (uint64_t)gridDim.x * blockDim.x;
+	uint32_t shift = 0;                                                // 2^shift lanes per point
+	while (shift < 5 && (total << (shift + 1)) <= threads && (2u << shift) * LIST_SMALL_SUMS <= k) ++shift;
+	if ((((uint64_t)blockIdx.x * blockDim.x) >> shift) >= total) return;  // the grid is sized for long lists: most blocks of a short one have nothing to do
 	for (uint32_t e = threadIdx.x; e < k * D; e += blockDim.x) {
 		const uint32_t m = e / D, j = e - m * D;
-		sm[e] = means[at<SOAM>(m, j, k, D)];
+		sm[m * RS + j] = means[at<SOAM>(m, j, k, D)];
 	}
+	for (uint32_t e = threadIdx.x; e < (LIST_SMALL_SUMS - 1) * RS; e += blockDim.x) sm[k * RS + e] = INFINITY;
 	__syncthreads();
-	for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (uint64_t)gridDim.x * blockDim.x) {
-		const uint64_t i = list[w];
+	const uint32_t lanes = 1u << shift, sub = threadIdx.x & (lanes - 1u);
+	const uint64_t step = threads >> shift, rounds = (total + step - 1) / step;
+	uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> shift;
+	for (uint64_t round = 0; round < rounds; ++round, w += step) {       // whole warps: the lanes of a point meet in shuffles
+		const uint64_t i = list[w < total ? w : 0];
 		float x[D];
 		#pragma unroll
 		for (int j = 0; j < D; ++j) x[j] = pts[at<SOA>(i, j, n, D)];
-		float best = 0.0f, best_sum = 0.0f;
-		uint32_t bidx = 0;
-		for (uint32_t m = 0; m < k; ++m) {
-			float c[D];
-			if (D % 4 == 0) {
-				// whole rows as 128-bit loads (the same address for all threads: broadcast)
-				#pragma unroll
-				for (int q = 0; q < D / 4; ++q) {
-					const float4 v = reinterpret_cast<const float4*>(sm + m * D)[q];
-					c[4 * q] = v.x; c[4 * q + 1] = v.y; c[4 * q + 2] = v.z; c[4 * q + 3] = v.w;
-				}
-			} else {
-				#pragma unroll
-				for (int j = 0; j < D; ++j) c[j] = sm[m * D + j];
-			}
-			float sum = 0.0f;
-			#pragma unroll
-			for (int j = 0; j < D; ++j) {
-				const float diff = __fsub_rn(x[j], c[j]);
-				sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-			}
-			// The reference compares square roots.  The correctly rounded square root never decreases
-			// with its argument, so a sum that is not below the best sum cannot give a smaller root:
-			// only the few candidates that are below it need the root itself (equal roots of different
-			// sums keep the earlier mean, as the reference's strict comparison does).
-			if (m == 0) {
-				best_sum = sum;
-				best = __fsqrt_rn(sum);
-			} else if (sum < best_sum) {
-				const float dist = __fsqrt_rn(sum);
-				if (dist < best) { best = dist; best_sum = sum; bidx = m; }
-			}
+		float best = INFINITY, best_sum = INFINITY;
+		uint32_t bidx = 0xffffffffu;
+		// (one lane per point: the stride is a constant and the four rows are one address away from each other)
+		if (lanes == 1) scan_means<D, RS>(sm, x, k, 0u, 1u, best, best_sum, bidx);
+		else scan_means<D, RS>(sm, x, k, sub, lanes, best, best_sum, bidx);
+		// lowest (distance, index) over the lanes of the point; lane 0 of them has seen mean 0
+		for (uint32_t off = lanes >> 1; off > 0; off >>= 1) {
+			const float ob = __shfl_down_sync(0xffffffffu, best, off, lanes);
+			const uint32_t oi = __shfl_down_sync(0xffffffffu, bidx, off, lanes);
+			if (oi != 0xffffffffu && (ob < best || (ob == best && oi < bidx))) { best = ob; bidx = oi; }
 		}
+		if (sub != 0 || w >= total) continue;
 		if (fix_acc) {
 			// the fast pass has already added this point to the sum of the cluster it picked
 			const uint32_t from = asg[i];
