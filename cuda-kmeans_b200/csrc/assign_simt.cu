@@ -7,8 +7,7 @@
 //    (kernels/kernels.cu:182-199 of the reference) and follows serial.hpp:21-35.
 //
 //  * assign_simt_kernel<D, SOA, P>: small-d fast pass (see the comment above the kernel): the
-//    means staged into shared memory with a bulk TMA copy, P points per thread in registers,
-//    |c|^2 - 2 x.c on the FMA pipe, arg-min on integer keys, near-ties queued for the exact
+//    means in shared memory, P points per thread in registers, |c|^2 - 2 x.c on the FMA pipe, arg-min on integer keys, near-ties queued for the exact
 //    kernel.  Covers the shape range of cachedFixedAssignmentKernel (kernels/kernels.cu:218-273)
 //    and cachedAllMeansAssignmentKernel (:330-374).
 #include "kernels.cuh"
@@ -509,7 +508,8 @@ cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* 
 	}
 	if (list != nullptr && (size_t)s.dim * sizeof(float) * LIST_PB <= 120 * 1024) {
 		// Every group of points walks all means: with long rows and many means (megabytes of them) the
-		// re-reads through L2 dominate, and sixteen points per group cut them fourfold.
+		// re-reads through L2 dominate, and sixteen points per group cut them fourfold (from 64 KiB of
+		// means on: 51 instead of 49 us for 1000 x 50, 19 instead of 11.5 us for 1024 x 128).
 		const bool wide = fix == nullptr && (size_t)s.k * s.dim * sizeof(float) >= (1u << 20) &&
 			(size_t)LIST_PB_WIDE * ((s.dim + 3) & ~3u) * sizeof(float) <= 64 * 1024;
 		const int pb = wide ? LIST_PB_WIDE : LIST_PB;
@@ -564,8 +564,11 @@ cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* 
 // ------------------------------------------------------------------------------------------
 //
 // Every thread keeps P points in registers (shifted by the common centre vector) and walks the
-// means in chunks of 32.  A mean's row in shared memory is [ |c|^2 + C, -2c_0 .. -2c_{D-1} ], so a
-// point's value |c|^2 - 2 x.c + C costs D fused multiply-adds per mean; the constant C (from the
+// means in chunks of 32.  A mean's row is [ |c|^2 + C, -2c_0 .. -2c_{D-1} ], so a point's value
+// |c|^2 - 2 x.c + C costs D fused multiply-adds per mean.  The rows of two neighbouring means are
+// interleaved in shared memory, and one instruction does the multiply-add of both (fma.rn.f32x2, the
+// point's coordinate in both halves): the pass is bound by instruction issue, and this halves the D
+// instructions per mean and point.  The constant C (from the
 // largest |x|^2 and |c|^2, see make_key_consts) puts all values into one binade, where their bit
 // patterns order like the values.  The 32 values of a chunk become integer keys (bits * M + column)
 // and are reduced to the smallest and second smallest with plain integer minima (chunk_update):
@@ -612,14 +615,13 @@ __device__ __forceinline__ void send_row(float* dst, const float (&sum)[D], floa
 }
 
 template<int D, bool SOA, int P, bool FUSE>
-__global__ void __launch_bounds__(SIMT_THREADS) assign_simt_kernel(const float* __restrict__ pts,
+__global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const float* __restrict__ pts,
 	const float* __restrict__ cprep, const float* __restrict__ center, uint32_t* __restrict__ asg, uint64_t n, uint32_t rows,
 	Control* __restrict__ ctl, int slot, uint32_t* __restrict__ flag_list, float margin_ulps, int vec_ok,
 	uint32_t k, float* __restrict__ fuse_acc, uint32_t* __restrict__ fuse_counts)
 {
-	constexpr int RS = (D + 1 + 3) / 4 * 4;
-	extern __shared__ __align__(128) float tile[];
-	__shared__ __align__(8) uint64_t bar;
+	constexpr int RS = (D + 1 + 3) / 4 * 4;      // floats of a prepared row in global memory
+	extern __shared__ __align__(128) float tile[];  // rows of two means interleaved: (D + 1) pairs
 	// fused update sums: see above
 	__shared__ uint32_t s_hist[FUSE ? SIMT_THREADS / 32 : 1][FUSE ? (SIMT_FUSE_MAX_K + 2) / 2 : 1];   // per warp: points per cluster, 16 bits each
 	__shared__ uint32_t s_cnt[FUSE ? SIMT_FUSE_MAX_K : 1];                  // sizes counted by this block
@@ -641,33 +643,27 @@ __global__ void __launch_bounds__(SIMT_THREADS) assign_simt_kernel(const float* 
 	const KeyConsts kc = make_key_consts(ctl->xmax2, ctl->cmax2[slot]);
 	const uint32_t key_mult = kc.key_mult, key_base = kc.key_base, key_magic = kc.key_magic;
 	const float pad_value = kc.pow2 * (2.0f - 1.0f / 32.0f);     // padding rows: above every real value, inside [P, 2P)
-	uint32_t phase = 0;
-	bool ok = true;
 	float cen[D];
 	#pragma unroll
 	for (int j = 0; j < D; ++j) cen[j] = center[j];
 
-	if (tid == 0) {
-		ptx::mbar_init(&bar, 1);
-		ptx::fence_mbar_init();
-	}
-	__syncthreads();
-
-	// Brings tile t of the prepared means into shared memory and adds the offset constant to its
-	// |c|^2 column (padding rows, marked by +inf there, get the top of the value band).
+	// Brings tile t of the prepared means into shared memory, interleaved by pairs, and adds the offset
+	// constant to its |c|^2 column (padding rows, marked by +inf there, get the top of the value band).
 	auto load_tile = [&](uint32_t t) -> uint32_t {
 		uint32_t trows = rows - t * SIMT_TILE_ROWS;
 		if (trows > SIMT_TILE_ROWS) trows = SIMT_TILE_ROWS;
-		if (tid == 0) {
-			const uint32_t bytes = trows * RS * (uint32_t)sizeof(float);
-			ptx::mbar_arrive_expect_tx(&bar, bytes);
-			ptx::bulk_g2s(tile, cprep + (size_t)t * SIMT_TILE_ROWS * RS, bytes, &bar);
-		}
-		ok = ptx::mbar_wait(&bar, phase) && ok;
-		phase ^= 1;
 		for (uint32_t r = tid; r < trows; r += SIMT_THREADS) {
-			const float c2 = tile[(size_t)r * RS];
-			tile[(size_t)r * RS] = c2 > 3.0e38f ? pad_value : c2 + kc.offset_c;
+			const float4* src = reinterpret_cast<const float4*>(cprep + ((size_t)t * SIMT_TILE_ROWS + r) * RS);
+			float* dst = tile + (r >> 1) * (2 * (D + 1)) + (r & 1u);
+			float v[RS];
+			#pragma unroll
+			for (int q = 0; q < RS / 4; ++q) {
+				const float4 w = src[q];
+				v[4 * q + 0] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
+			}
+			v[0] = v[0] > 3.0e38f ? pad_value : v[0] + kc.offset_c;
+			#pragma unroll
+			for (int j = 0; j <= D; ++j) dst[2 * j] = v[j];
 		}
 		__syncthreads();
 		return trows;
@@ -723,6 +719,11 @@ __global__ void __launch_bounds__(SIMT_THREADS) assign_simt_kernel(const float* 
 			#pragma unroll
 			for (int j = 0; j < D; ++j) x[p][j] = raw[p][j] - cen[j];
 		}
+		uint64_t xx[P][D];
+		#pragma unroll
+		for (int p = 0; p < P; ++p)
+			#pragma unroll
+			for (int j = 0; j < D; ++j) xx[p][j] = ptx::pack2(x[p][j], x[p][j]);
 		if (blk + gridDim.x < nblocks) load_points(blk + gridDim.x);
 
 		uint32_t best[P], second[P], bchunk[P];
@@ -739,21 +740,26 @@ __global__ void __launch_bounds__(SIMT_THREADS) assign_simt_kernel(const float* 
 			#pragma unroll 1
 			for (uint32_t ch = 0; ch < trows / 32; ++ch) {
 				uint32_t v[P][32];
-				const float4* rowp = reinterpret_cast<const float4*>(tile + (size_t)ch * 32 * RS);
+				const float4* rowp = reinterpret_cast<const float4*>(tile + (size_t)ch * 32 * (D + 1));
 				#pragma unroll
-				for (int m = 0; m < 32; ++m) {
-					float r[RS];
+				for (int m = 0; m < 32; m += 4) {
+					// four means = two interleaved pairs = D + 1 128-bit loads
+					float f[4 * (D + 1)];
 					#pragma unroll
-					for (int q = 0; q < RS / 4; ++q) {
-						const float4 w = rowp[m * (RS / 4) + q];
-						r[4 * q + 0] = w.x; r[4 * q + 1] = w.y; r[4 * q + 2] = w.z; r[4 * q + 3] = w.w;
+					for (int q = 0; q <= D; ++q) {
+						const float4 w = rowp[(m / 4) * (D + 1) + q];
+						f[4 * q + 0] = w.x; f[4 * q + 1] = w.y; f[4 * q + 2] = w.z; f[4 * q + 3] = w.w;
 					}
 					#pragma unroll
-					for (int p = 0; p < P; ++p) {
-						float val = r[0];
+					for (int h = 0; h < 2; ++h) {
+						const float* row = f + h * 2 * (D + 1);
 						#pragma unroll
-						for (int j = 0; j < D; ++j) val = fmaf(x[p][j], r[1 + j], val);
-						v[p][m] = __float_as_uint(val);
+						for (int p = 0; p < P; ++p) {
+							uint64_t val = ptx::pack2(row[0], row[1]);
+							#pragma unroll
+							for (int j = 0; j < D; ++j) val = ptx::fma2(xx[p][j], ptx::pack2(row[2 * j + 2], row[2 * j + 3]), val);
+							ptx::unpack2(val, v[p][m + 2 * h], v[p][m + 2 * h + 1]);
+						}
 					}
 				}
 				#pragma unroll
@@ -858,7 +864,6 @@ __global__ void __launch_bounds__(SIMT_THREADS) assign_simt_kernel(const float* 
 		}
 	}
 	flush_flag_buffer(flag_buf, flag_cnt, ctl, flag_list, n);
-	if (!ok && tid == 0) atomicOr(&ctl->status, (uint32_t)STATUS_WAIT_TIMEOUT);
 }
 
 bool assign_simt_supported(const Shape& s)
@@ -877,10 +882,9 @@ template<int D, int P>
 static cudaError_t launch_simt_d(const float* pts, const float* cprep, const float* center, uint32_t* asg, const Shape& s,
 	Control* ctl, int slot, uint32_t* flag_list, float margin_scale, int sm_count, cudaStream_t stream, const FusedAcc* fused)
 {
-	constexpr int RS = (D + 1 + 3) / 4 * 4;
 	const uint32_t rows = simt_rows(s.k);
 	const uint32_t trows = rows < (uint32_t)SIMT_TILE_ROWS ? rows : (uint32_t)SIMT_TILE_ROWS;
-	const size_t smem = (size_t)trows * RS * sizeof(float);
+	const size_t smem = (size_t)trows * (D + 1) * sizeof(float);
 	const uint64_t per_block = (uint64_t)SIMT_THREADS * P;
 	const uint64_t nblocks = (s.n + per_block - 1) / per_block;
 	// persistent grid: a whole number of resident blocks per SM
@@ -913,8 +917,8 @@ cudaError_t launch_assign_simt(const float* pts, const SimtMeans& sm, uint32_t* 
 	Control* ctl, int slot, uint32_t* flag_list, float margin_scale, int sm_count, cudaStream_t stream, const FusedAcc* fused)
 {
 	switch (s.dim) {
-	case 1: return launch_simt_d<1, 4>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 2: return launch_simt_d<2, 4>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 1: return launch_simt_d<1, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 2: return launch_simt_d<2, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
 	case 3: return launch_simt_d<3, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
 	case 4: return launch_simt_d<4, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
 	case 5: return launch_simt_d<5, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);

@@ -143,6 +143,26 @@ __device__ __forceinline__ void prefetch_tmap(const void* tmap)
 	asm volatile("prefetch.tensormap [%0];" :: "l"(tmap) : "memory");
 }
 
+// Two fp32 fused multiply-adds in one instruction; the operands are pairs in 64-bit registers.
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+	uint64_t d;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+	return d;
+}
+
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
+{
+	uint64_t d;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+	return d;
+}
+
+__device__ __forceinline__ void unpack2(uint64_t v, uint32_t& lo, uint32_t& hi)
+{
+	asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+}
+
 // ---- tcgen05 ----
 
 // Allocates `cols` TMEM columns (power of two, 32..512); the base address lands in *slot (shared).
