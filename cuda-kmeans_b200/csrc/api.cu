@@ -163,7 +163,8 @@ Workspace carve(char* base, uint64_t n, uint32_t k, uint32_t dim, bool with_tc_p
 		w.tp.a_hi = reinterpret_cast<float*>(take(aplane));
 		w.tp.a_lo = reinterpret_cast<float*>(take(aplane));
 		w.tp.xnorm = reinterpret_cast<float*>(take((size_t)w.tp.n_pad * sizeof(float)));
-		w.tp.partial = w.tp.d_pad > 32 ? reinterpret_cast<uint32_t*>(take((size_t)bkm::TC_JSPLIT * 3 * w.tp.n_pad * sizeof(uint32_t))) : nullptr;
+		w.tp.partial = w.tp.d_pad > 32 ? reinterpret_cast<uint32_t*>(take((size_t)bkm::TC_JSPLIT * 5 * w.tp.n_pad * sizeof(uint32_t))) : nullptr;
+		w.tp.pairs = w.tp.d_pad > 32 ? reinterpret_cast<uint32_t*>(take(2 * n * sizeof(uint32_t))) : nullptr;
 	}
 	w.bytes = off;
 	return w;
@@ -262,6 +263,8 @@ int enqueue_assign(int variant, const float* pts, const float* means, uint32_t* 
 	}
 	if (mid) CUDA_TRY(cudaEventRecord(mid, stream));
 	CUDA_TRY(bkm::launch_assign_exact(pts, means, asg, s, w.flag_list, &w.ctl->flag_count, sm_count, stream, fused, w.split_scratch));
+	if (variant == BKM_ASSIGN_TC && bkm::tc_plan_collects_pairs(plan))
+		CUDA_TRY(bkm::launch_assign_exact_pairs(pts, means, asg, s, w.tp.pairs, &w.ctl->pair_count, sm_count, stream));
 	return BKM_OK;
 }
 

@@ -335,6 +335,63 @@ __global__ void __launch_bounds__(LIST_THREADS, PB > LIST_PB ? 2 : 3) assign_exa
 	}
 }
 
+// Points with exactly two candidate means: a warp per point.  The lanes square the differences of 128
+// dimensions to both candidates (coalesced reads), lanes 0 and 1 add them up in dimension order, one
+// rounding per operation - two rows of means instead of all of them (a list of 4400 points of 512
+// dimensions against 4096 means took 1.5 ms in the list kernel above).
+template<bool SOA, bool SOAM>
+__global__ void __launch_bounds__(256) assign_exact_pairs_kernel(const float* __restrict__ pts, const float* __restrict__ means,
+	uint32_t* __restrict__ asg, uint64_t n, uint32_t k, uint32_t d, const uint32_t* __restrict__ pairs, const uint32_t* __restrict__ pair_count)
+{
+	__shared__ __align__(16) float squares[8][2][128];
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	uint64_t total = *pair_count;
+	if (total > n) total = n;
+	for (uint64_t w = (uint64_t)blockIdx.x * 8 + warp; w < total; w += (uint64_t)gridDim.x * 8) {
+		const uint64_t i = pairs[w];
+		const uint32_t c0 = asg[i], c1 = pairs[n + w];
+		const uint32_t lo = min(c0, c1), hi = max(c0, c1);
+		float sum = 0.0f;
+		for (uint32_t j0 = 0; j0 < d; j0 += 128) {
+			__syncwarp();
+			#pragma unroll
+			for (uint32_t r = 0; r < 4; ++r) {
+				const uint32_t j = j0 + r * 32 + lane;
+				if (j < d) {
+					const float x = pts[at<SOA>(i, j, n, d)];
+					const float d0 = __fsub_rn(x, means[at<SOAM>(lo, j, k, d)]), d1 = __fsub_rn(x, means[at<SOAM>(hi, j, k, d)]);
+					squares[warp][0][r * 32 + lane] = __fmul_rn(d0, d0);
+					squares[warp][1][r * 32 + lane] = __fmul_rn(d1, d1);
+				}
+			}
+			__syncwarp();
+			if (lane < 2) {
+				const uint32_t jn = d - j0 < 128 ? d - j0 : 128;
+				const float* sq = squares[warp][lane];
+				uint32_t j = 0;
+				for (; j + 4 <= jn; j += 4) {
+					const float4 v = *reinterpret_cast<const float4*>(sq + j);
+					sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
+				}
+				for (; j < jn; ++j) sum = __fadd_rn(sum, sq[j]);
+			}
+		}
+		const float dist = __fsqrt_rn(sum), other = __shfl_down_sync(0xffffffffu, dist, 1);
+		if (lane == 0) asg[i] = other < dist ? hi : lo;          // strictly smaller, the lower index first
+	}
+}
+
+cudaError_t launch_assign_exact_pairs(const float* pts, const float* means, uint32_t* asg, const Shape& s,
+	const uint32_t* pairs, const uint32_t* pair_count, int sm_count, cudaStream_t stream)
+{
+	const uint32_t grid = (uint32_t)sm_count * 8;
+	if (s.soa && s.soa_means) assign_exact_pairs_kernel<true, true><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, s.dim, pairs, pair_count);
+	else if (s.soa) assign_exact_pairs_kernel<true, false><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, s.dim, pairs, pair_count);
+	else if (s.soa_means) assign_exact_pairs_kernel<false, true><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, s.dim, pairs, pair_count);
+	else assign_exact_pairs_kernel<false, false><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, s.dim, pairs, pair_count);
+	return cudaGetLastError();
+}
+
 // The same arithmetic with all means in shared memory and the lanes of a warp shared out over points:
 // for mean sets of a few thousand floats and at most 16 dimensions, where a block per four points
 // spends its time in barriers and reductions.  A long list gives every point one thread and fills the

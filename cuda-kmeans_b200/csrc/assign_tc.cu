@@ -71,6 +71,7 @@ constexpr uint32_t SM_B_OFF = SM_A_OFF + TC_MA * A_TILE_BYTES;
 constexpr uint32_t SM_BAUG_OFF = SM_B_OFF + TC_NB * B_STAGE_BYTES; // |c|^2 K step per stage
 constexpr uint32_t SM_AAUG_OFF = SM_BAUG_OFF + TC_NB * AUG_BYTES;  // constant ones tile (128 rows)
 constexpr uint32_t SM_MERGE_OFF = SM_AAUG_OFF + TC_MTILE * 8 * 4;
+// (with THREE the same slots hold five words and extend over the flag buffers, which that form does not use)
 constexpr uint32_t MERGE_BYTES = 2 * 3 * TC_MA * TC_MTILE * 4;   // (best, second, chunk) of the upper column half, two slots
 constexpr uint32_t SM_FLAG_OFF = SM_MERGE_OFF + MERGE_BYTES;       // per epilogue warp: near-ties on their way to the list
 constexpr uint32_t SM_BAR_OFF = SM_FLAG_OFF + TC_EPI_WARPS * FLAG_BUFFER * 4;
@@ -341,39 +342,73 @@ struct TcBars {
 };
 static_assert(sizeof(TcBars) <= 256, "barrier block too large");
 static_assert(SM_ALLOC <= 227 * 1024, "shared memory budget exceeded");
+static_assert(2 * 5 * TC_MA * TC_MTILE * 4 <= SM_BAR_OFF - SM_MERGE_OFF, "merge slots of five words");
 static_assert(KL_AUG_OFF + 2 * AUG_BYTES <= SM_AAUG_OFF, "K-loop stages overlap the constant tile");
 
+template<bool THREE, bool MASKED>
+__device__ __forceinline__ void update_state(const uint32_t (&v)[32], uint32_t key_mult, uint32_t chunk_id, uint32_t nvalid, BestThree& st)
+{
+	if (THREE) chunk_update3<MASKED>(v, key_mult, chunk_id, nvalid, st);
+	else chunk_update<MASKED>(v, key_mult, chunk_id, nvalid, st.best, st.second, st.best_chunk);
+}
+
 // Combines the partial arg-min results of the CTAs that shared the mean tiles of a point block.
+// THREE: the partial results carry the third smallest key, and a near-tie between two means only goes
+// to the list of pairs.
+template<bool THREE>
 __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __restrict__ partial, uint64_t partial_stride, uint32_t parts,
 	const float* __restrict__ xnorm, uint32_t* __restrict__ asg, uint64_t n, uint32_t k, Control* __restrict__ ctl, int slot,
-	uint32_t* __restrict__ flag_list, float margin_coef, float sqrt_dim)
+	uint32_t* __restrict__ flag_list, float margin_coef, float sqrt_dim, uint32_t* __restrict__ pairs)
 {
+	constexpr uint32_t WORDS = THREE ? 5 : 3;
 	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
 	const KeyConsts kc = tc_key_consts(x2max, c2max);
 	const float ulp = kc.pow2 * 1.1920929e-07f;
 	const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim);
+	const uint32_t lane = threadIdx.x & 31u;
 	const uint64_t n32 = (n + 31) & ~(uint64_t)31;      // whole warps walk the loop together (the append is a warp operation)
 	for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n32; p += (uint64_t)gridDim.x * blockDim.x) {
-		bool flag = false;
+		bool flag = false, two = false;
+		uint32_t other = 0;
 		if (p < n) {
-			uint32_t best = 0xFFFFFFFFu, second = 0xFFFFFFFFu, bchunk = 0;
+			BestThree st;
 			for (uint32_t part = 0; part < parts; ++part) {
-				const uint32_t* src = partial + (size_t)part * 3 * partial_stride + p;
+				const uint32_t* src = partial + (size_t)part * WORDS * partial_stride + p;
 				const uint32_t ob = src[0], os = src[partial_stride], oc = src[2 * partial_stride];
-				second = umin3(second, os, max(best, ob));
-				bchunk = ob < best ? oc : bchunk;
-				best = min(best, ob);
+				if (THREE) st.merge(ob, os, src[3 * partial_stride], oc, src[4 * partial_stride]);
+				else st.merge(ob, os, 0xFFFFFFFFu, oc, 0u);
 			}
-			flag = finish_point(best, second, bchunk, kc.key_base, kc.key_mult, kc.key_magic, ulp, margin_coef * (xnorm[p] + c2max) + margin_floor, k, p, asg);
+			const float margin = margin_coef * (xnorm[p] + c2max) + margin_floor;
+			flag = finish_point(st.best, st.second, st.best_chunk, kc.key_base, kc.key_mult, kc.key_magic, ulp, margin, k, p, asg);
+			if (THREE && flag && st.second != 0xFFFFFFFFu) {
+				const uint32_t bm = div_key(st.best - kc.key_base, kc.key_magic);
+				const float gap3 = st.third == 0xFFFFFFFFu ? INFINITY : (float)(div_key(st.third - kc.key_base, kc.key_magic) - bm) * ulp;
+				other = key_column(st.second, st.second_chunk, kc.key_base, kc.key_mult, kc.key_magic);
+				two = margin < INFINITY && gap3 > margin && other < k;
+				flag = !two;
+			}
 		}
 		append_flagged(flag, (uint32_t)p, ctl, flag_list, n);
+		if (THREE) {
+			const uint32_t mask = __ballot_sync(0xffffffffu, two);
+			if (mask != 0) {
+				uint32_t base = 0;
+				if (lane == 0) base = atomicAdd(&ctl->pair_count, (uint32_t)__popc(mask));
+				base = __shfl_sync(0xffffffffu, base, 0) + (uint32_t)__popc(mask & ((1u << lane) - 1u));
+				if (two) {
+					if ((uint64_t)base < n) { pairs[base] = (uint32_t)p; pairs[n + base] = other; }
+					else atomicOr(&ctl->status, (uint32_t)STATUS_LIST_OVERFLOW);
+				}
+			}
+		}
 	}
 }
 
 // FULL: k is a whole number of mean tiles of 128 or 256 columns, so no accumulator column is padding
 // and every warp takes its columns in pairs of 32-column chunks: the epilogue runs without its masked
 // path and without the odd-chunk branches.
-template<bool FULL>
+// THREE (K loop with jsplit > 1): the partial results carry the three smallest keys.
+template<bool FULL, bool THREE>
 __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 	const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
 	const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
@@ -675,7 +710,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 		for (uint32_t blk = bid; blk < nblocks; blk += nbid, ++blk_count) {
 			const uint32_t tiles = min(TC_MA, n_tiles - blk * TC_MA);
 			if (i >= tiles) continue;              // odd tail: this accumulator is not used in the last block
-			uint32_t best = 0xFFFFFFFFu, second = 0xFFFFFFFFu, bchunk = 0;
+			BestThree st;
 			const uint64_t p = (uint64_t)(blk * TC_MA + i) * TC_MTILE + row;
 			float xn = 0.0f;                       // |x|^2 of this thread's point, needed at the end of the block
 			#pragma unroll 1
@@ -700,8 +735,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 						ptx::tmem_ld32(taddr, v0);
 						ptx::tmem_ld_wait();
 						if (two) ptx::tmem_ld32(taddr + 32, v1);
-						if (plain) chunk_update<false>(v0, key_mult, chunk0, 32, best, second, bchunk);
-						else if (left > 0) chunk_update<true>(v0, key_mult, chunk0, left, best, second, bchunk);
+						if (plain) update_state<THREE, false>(v0, key_mult, chunk0, 32, st);
+						else if (left > 0) update_state<THREE, true>(v0, key_mult, chunk0, left, st);
 						ptx::tmem_ld_wait();
 						if (c + 2 >= nchunks) {
 							// last load: the tensor cores may fill this accumulator again
@@ -713,9 +748,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 							if (j == j_end - 1 && half == 0 && p < n) xn = xnorm[p];
 						}
 						if (plain) {
-							if (two) chunk_update<false>(v1, key_mult, chunk0 + 1, 32, best, second, bchunk);
+							if (two) update_state<THREE, false>(v1, key_mult, chunk0 + 1, 32, st);
 						} else if (two && left > 32) {
-							chunk_update<true>(v1, key_mult, chunk0 + 1, left - 32, best, second, bchunk);
+							update_state<THREE, true>(v1, key_mult, chunk0 + 1, left - 32, st);
 						}
 					}
 				} else {
@@ -726,23 +761,25 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 			// The upper column half hands its state to the lower one through shared memory.  The slots
 			// alternate with the block count, so one barrier per block is enough: a slot is written
 			// again only after its reader has passed the barrier of the block in between.
-			uint32_t* mg = mg_state + ((blk_count & 1u) * TC_MA + i) * (3 * TC_MTILE);
+			constexpr uint32_t WORDS = THREE ? 5 : 3;
+			uint32_t* mg = mg_state + ((blk_count & 1u) * TC_MA + i) * (WORDS * TC_MTILE);
 			if (half == 1) {
-				mg[row] = best; mg[TC_MTILE + row] = second; mg[2 * TC_MTILE + row] = bchunk;
+				mg[row] = st.best; mg[TC_MTILE + row] = st.second; mg[2 * TC_MTILE + row] = st.best_chunk;
+				if (THREE) { mg[3 * TC_MTILE + row] = st.third; mg[4 * TC_MTILE + row] = st.second_chunk; }
 			}
 			asm volatile("bar.sync %0, 64;" :: "r"(bar_id) : "memory");
 			bool flag = false;
 			if (half == 0 && p < n && ok) {
 				const uint32_t ob = mg[row], os = mg[TC_MTILE + row], oc = mg[2 * TC_MTILE + row];
-				second = umin3(second, os, max(best, ob));
-				bchunk = ob < best ? oc : bchunk;
-				best = min(best, ob);
+				if (THREE) st.merge(ob, os, mg[3 * TC_MTILE + row], oc, mg[4 * TC_MTILE + row]);
+				else st.merge(ob, os, 0xFFFFFFFFu, oc, 0u);
 				if (partial != nullptr) {
 					// this CTA saw only its share of the mean tiles: the keys go out as they are
-					uint32_t* dst = partial + (size_t)jpart * 3 * partial_stride + p;
-					dst[0] = best; dst[partial_stride] = second; dst[2 * partial_stride] = bchunk;
+					uint32_t* dst = partial + (size_t)jpart * WORDS * partial_stride + p;
+					dst[0] = st.best; dst[partial_stride] = st.second; dst[2 * partial_stride] = st.best_chunk;
+					if (THREE) { dst[3 * partial_stride] = st.third; dst[4 * partial_stride] = st.second_chunk; }
 				} else {
-					flag = finish_point(best, second, bchunk, key_base, key_mult, key_magic, ulp, margin_coef * (xn + c2max) + margin_floor, k, p, asg);
+					flag = finish_point(st.best, st.second, st.best_chunk, key_base, key_mult, key_magic, ulp, margin_coef * (xn + c2max) + margin_floor, k, p, asg);
 				}
 			}
 			if (half == 0 && partial == nullptr) buffered_append(flag, (uint32_t)p, flag_buf, flag_cnt, ctl, flag_list, n);
@@ -854,8 +891,10 @@ TcPlan* tc_plan_create(const Shape& s, const TcPoints& tp, const TcMeans& tm, in
 		delete p;
 		return nullptr;
 	}
-	if (cudaFuncSetAttribute(assign_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess ||
-		cudaFuncSetAttribute(assign_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess) {
+	if (cudaFuncSetAttribute(assign_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess ||
+		cudaFuncSetAttribute(assign_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess ||
+		cudaFuncSetAttribute(assign_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess ||
+		cudaFuncSetAttribute(assign_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess) {
 		cudaGetLastError();
 		if (err) *err = e_attr;
 		delete p;
@@ -894,6 +933,11 @@ static uint32_t plan_jsplit(const TcPlan* p)
 	return (kloop && n_ctiles >= 2 * TC_JSPLIT && p->tp.partial != nullptr && p->sm_count >= (int)TC_JSPLIT) ? TC_JSPLIT : 1u;
 }
 
+// The three-key form costs the epilogue a third more minima; it pays where the multiplication is long
+// enough to make that small and the exact pass over all means long enough to matter (2^20 x 512 against
+// 4096: the pass 8.70 -> 9.06 ms, the re-check of 4400 points 1.49 -> 0.09 ms).
+bool tc_plan_collects_pairs(const TcPlan* p) { return plan_jsplit(p) > 1 && p->s.dim >= 256 && p->tp.pairs != nullptr; }
+
 void tc_plan_describe(const TcPlan* p, uint32_t out[4])
 {
 	out[1] = p->tm.k_pad / p->nt_cols;
@@ -931,14 +975,16 @@ cudaError_t launch_assign_tc(TcPlan* p, uint32_t* asg, Control* ctl, int slot, u
 			ranged ? (uint32_t)((std::min<uint64_t>(p_end, p->tp.n_pad) + 2 * TC_MTILE - 1) / (2 * TC_MTILE)) : 0u);
 	const uint32_t jsplit = plan_jsplit(p);
 	const uint32_t grid_j = jsplit * std::min<uint32_t>(nblocks, (uint32_t)p->sm_count / jsplit);
-	auto kern = (p->s.k == p->tm.k_pad && p->nt_cols % 128 == 0) ? assign_tc_kernel<true> : assign_tc_kernel<false>;
+	const bool full = p->s.k == p->tm.k_pad && p->nt_cols % 128 == 0, three = tc_plan_collects_pairs(p);
+	auto kern = three ? (full ? assign_tc_kernel<true, true> : assign_tc_kernel<false, true>) : (full ? assign_tc_kernel<true, false> : assign_tc_kernel<false, false>);
 	kern<<<jsplit > 1 ? grid_j : grid, TC_THREADS, SM_ALLOC, stream>>>(p->a_hi, p->a_lo, p->b_hi, p->b_lo,
 		p->tm.b_aug, p->tp.xnorm, asg, p->s.n, n_tiles, p->s.k, p->tm.k_pad, p->nt_cols, kw, kchunks, ksteps_last, idesc,
 		ctl, slot, flag_list, margin_coef, sqrt_dim, jsplit, jsplit > 1 ? p->tp.partial : nullptr, p->tp.n_pad);
 	if (jsplit > 1) {
 		const uint32_t mgrid = (uint32_t)std::min<uint64_t>((p->s.n + 255) / 256, (uint64_t)p->sm_count * 8);
-		merge_partials_kernel<<<mgrid, 256, 0, stream>>>(p->tp.partial, p->tp.n_pad, jsplit, p->tp.xnorm, asg, p->s.n, p->s.k, ctl, slot,
-			flag_list, margin_coef, sqrt_dim);
+		auto merge = three ? merge_partials_kernel<true> : merge_partials_kernel<false>;
+		merge<<<mgrid, 256, 0, stream>>>(p->tp.partial, p->tp.n_pad, jsplit, p->tp.xnorm, asg, p->s.n, p->s.k, ctl, slot,
+			flag_list, margin_coef, sqrt_dim, p->tp.pairs);
 	}
 	return cudaGetLastError();
 }

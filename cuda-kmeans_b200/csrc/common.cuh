@@ -26,6 +26,8 @@ struct Control {
 	                       // in units of the operand scale, see tc_scale, when the operands are the fp16 planes)
 	float xdev;            // largest |x_j - centre_j| over a sample of the points
 	uint32_t beyond;       // points that the fp16 planes cannot hold at the scale of that sample
+	uint32_t pair_count;   // number of points queued with exactly two candidate means
+	uint32_t pad[7];
 };
 
 // What a stateless workspace remembers about the point set its one-off operands (centre vector,

@@ -38,7 +38,8 @@ struct TcPoints {
 	float* xnorm;    // [n_pad] |x|^2 in units of the scale; +inf (and zero rows) for points the planes cannot hold
 	uint64_t n_pad;  // n rounded up to TC_MTILE
 	uint32_t d_pad;
-	uint32_t* partial; // K loop only (d_pad > 32): [TC_JSPLIT][3][n_pad] partial arg-min keys, else null
+	uint32_t* partial; // K loop only (d_pad > 32): [TC_JSPLIT][5][n_pad] partial arg-min keys, else null
+	uint32_t* pairs;   // K loop only: [2][n] points queued with two candidates, and the second candidate
 };
 constexpr uint32_t TC_JSPLIT = 2;   // CTAs that can share the mean tiles of one point block in the K loop
 
@@ -123,6 +124,10 @@ cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* 
 	const uint32_t* list, const uint32_t* list_count, int sm_count, cudaStream_t stream, const FusedAcc* fix = nullptr,
 	void* split_scratch = nullptr);
 
+// The same arithmetic for points that have two candidates only: asg[pairs[w]] and pairs[n + w].
+cudaError_t launch_assign_exact_pairs(const float* pts, const float* means, uint32_t* asg, const Shape& s,
+	const uint32_t* pairs, const uint32_t* pair_count, int sm_count, cudaStream_t stream);
+
 // Small-d fast pass (dim <= 8): approximate distances, near-ties appended to flag_list.
 bool assign_simt_supported(const Shape& s);
 // max |x - center|^2 over the points -> ctl->xmax2 (zero on entry); once per data set.
@@ -167,6 +172,10 @@ void tc_plan_describe(const TcPlan* plan, uint32_t out[4]);
 // the last point): only these points, so that the pass can follow a host upload chunk by chunk.
 cudaError_t launch_assign_tc(TcPlan* plan, uint32_t* asg, Control* ctl, int slot, uint32_t* flag_list,
 	float margin_scale, cudaStream_t stream, const FusedAcc* fused = nullptr, uint64_t p_begin = 0, uint64_t p_end = 0);
+
+// Whether the plan's kernels queue points that have exactly two candidate means (their number in
+// ctl->pair_count) in TcPoints::pairs, for launch_assign_exact_pairs.
+bool tc_plan_collects_pairs(const TcPlan* plan);
 
 // A wait that is made to run out (nothing ever arrives): sets STATUS_WAIT_TIMEOUT in `ctl` after `limit_ns`.
 cudaError_t launch_wait_timeout_selftest(Control* ctl, uint64_t limit_ns, cudaStream_t stream);

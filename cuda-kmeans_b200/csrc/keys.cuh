@@ -67,6 +67,57 @@ __device__ __forceinline__ void chunk_update(const uint32_t (&v)[32], uint32_t k
 }
 
 
+// The three smallest keys of a point so far, with the chunks (of 32 columns) of the first two.  A point
+// whose third smallest is far enough from the smallest has only two candidates for the exact re-check.
+struct BestThree {
+	uint32_t best = 0xFFFFFFFFu, second = 0xFFFFFFFFu, third = 0xFFFFFFFFu, best_chunk = 0, second_chunk = 0;
+
+	// Takes in another such triple, b <= s <= t.  Where keys of different chunks are equal, either may be
+	// called the second: the other is then the third and as close.
+	__device__ __forceinline__ void merge(uint32_t b, uint32_t s, uint32_t t, uint32_t b_chunk, uint32_t s_chunk)
+	{
+		const bool wins = b < best;
+		const uint32_t loser = max(best, b), loser_chunk = wins ? best_chunk : b_chunk;
+		const uint32_t middle = max(min(second, s), min(max(second, s), loser));      // second smallest of the three that are left
+		const uint32_t next = umin3(second, s, loser);
+		third = umin3(third, t, middle);
+		second_chunk = next == loser ? loser_chunk : (next == second ? second_chunk : s_chunk);
+		second = next;
+		best_chunk = wins ? b_chunk : best_chunk;
+		best = min(best, b);
+	}
+};
+
+// As chunk_update with the third smallest key as well: one more pass of add-and-minimum, in which the
+// two smallest wrap to the top (+28 instructions per chunk).
+template<bool MASKED>
+__device__ __forceinline__ void chunk_update3(const uint32_t (&v)[32], uint32_t key_mult, uint32_t chunk_id, uint32_t nvalid, BestThree& state)
+{
+	uint32_t p[32];
+	#pragma unroll
+	for (uint32_t t = 0; t < 32; ++t) p[t] = v[t] * key_mult + t;
+	if (MASKED && nvalid < 32) {
+		#pragma unroll
+		for (uint32_t t = 0; t < 32; ++t) p[t] = t < nvalid ? p[t] : 0xFFFFFFFFu;
+	}
+	auto min_above = [&p](uint32_t key) {          // the smallest key above `key`
+		const uint32_t shift = ~key;               // -(key + 1)
+		uint32_t r0 = p[0] + shift, r1 = p[1] + shift, r2 = p[2] + shift, r3 = p[3] + shift;
+		#pragma unroll
+		for (uint32_t t = 4; t < 32; t += 4) {
+			r0 = __viaddmin_u32(p[t], shift, r0);
+			r1 = __viaddmin_u32(p[t + 1], shift, r1);
+			r2 = __viaddmin_u32(p[t + 2], shift, r2);
+			r3 = __viaddmin_u32(p[t + 3], shift, r3);
+		}
+		return min(umin3(r0, r1, r2), r3) - shift;
+	};
+	const uint32_t b = min_of_32(p), s = min_above(b);
+	const uint32_t t = MASKED && s == 0xFFFFFFFFu ? 0xFFFFFFFFu : min_above(s);
+	state.merge(b, s, t, chunk_id, chunk_id);
+}
+
+
 // The constants that turn accumulator values into integer keys (see chunk_update).
 struct KeyConsts {
 	float pow2;          // P: every accumulator value lies in [P, 2P)
@@ -107,6 +158,13 @@ __device__ __forceinline__ uint32_t div_key(uint32_t x, uint32_t magic)
 {
 	const uint32_t t = __umulhi(magic, x);
 	return (t + ((x - t) >> 1)) >> 5;
+}
+
+// Index of the mean that a key stands for.
+__device__ __forceinline__ uint32_t key_column(uint32_t key, uint32_t chunk, uint32_t key_base, uint32_t key_mult, uint32_t key_magic)
+{
+	const uint32_t x = key - key_base;
+	return chunk * 32u + (x - div_key(x, key_magic) * key_mult);
 }
 
 // Appends the points whose `flag` is set to the near-tie list with ONE atomic per warp (a counter

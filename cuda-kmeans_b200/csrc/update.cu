@@ -121,8 +121,9 @@ __device__ __forceinline__ void finish_padding_row(const RowSinks& o, uint32_t c
 
 __device__ __forceinline__ void finish_control(Control* ctl, int slot)
 {
-	ctl->last_flag_count = ctl->flag_count;
+	ctl->last_flag_count = ctl->flag_count + ctl->pair_count;
 	ctl->flag_count = 0;
+	ctl->pair_count = 0;
 	ctl->cmax2[slot ^ 1] = 0.0f;
 }
 
@@ -470,7 +471,7 @@ __global__ void __launch_bounds__(256) stateless_begin_kernel(Control* ctl, Poin
 	const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
 	if (t == 0) {
 		// last_flag_count and what belongs to the points survive
-		ctl->status = 0; ctl->flag_count = 0; ctl->cmax2[0] = 0.0f; ctl->cmax2[1] = 0.0f;
+		ctl->status = 0; ctl->flag_count = 0; ctl->pair_count = 0; ctl->cmax2[0] = 0.0f; ctl->cmax2[1] = 0.0f;
 		if (key) { key->fp_new = 0; key->arrive = 0; }
 	}
 	#pragma unroll
