@@ -1291,7 +1291,8 @@ int bkm_assign_plan(bkm_handle_t h, uint32_t out[4])
 	else if (h->assign_variant == BKM_ASSIGN_SIMT) out[0] = BKM_PLAN_SIMT;
 	else {
 		if (!h->plan) return fail(BKM_ERR_STATE, "the tensor-core plan exists after initialize only");
-		bkm::tc_plan_describe(h->plan, out);
+		const bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(h->shape.k, h->shape.dim), h->ws.tm.center, h->d_points, h->shape.soa};
+		bkm::tc_plan_describe(h->plan, h->fuse_update && fuse_pays(h->assign_variant, h->update_variant, h->plan, fa, h->shape, h->fuse_update >= 2), out);
 	}
 	out[3] = h->last_fused ? 1u : 0u;
 	return BKM_OK;

@@ -915,13 +915,24 @@ TcPlan* tc_plan_create(const Shape& s, const TcPoints& tp, const TcMeans& tm, in
 void tc_plan_allow_pair(TcPlan* plan, bool allow) { if (plan) plan->pair_allowed = allow; }
 bool tc_plan_uses_pair(const TcPlan* plan) { return plan && plan->pair_ok && plan->pair_allowed; }
 
+// Where CTA pairs can run they serve what they are better at: the fused update sums, a range of the
+// points, and operand rows of 32 words (dim 33..64: 517 against 648 us for 2^21 points and 1024 means).
+// With 16-word rows the one-CTA kernel is the faster one (k = 512: 227 against 243 us, k = 1024: 427
+// against 440 us, 2^21 points of 32 dimensions).
+static bool launch_uses_pair(const TcPlan* p, bool fused, bool ranged) { return tc_plan_uses_pair(p) && (fused || ranged || p->tp.d_pad == TC_KCHUNK); }
+
 void tc_plan_destroy(TcPlan* plan) { delete plan; }
 
 // The pair kernel can accumulate the update sums when a point's row can go out as 128-bit vector
-// reductions: dim a multiple of 4 and 16-byte aligned accumulators.
+// reductions: dim a multiple of 4 and 16-byte aligned accumulators.  The reductions take as long however
+// few the means are, so with up to three mean tiles they pay for a launch less only (2^21 points of 32
+// dimensions: k = 512 404 us against 227 + 106 apart, k = 1024 509 us against 427 + 91).
+constexpr uint64_t PAIR_FUSE_SMALL_N = 1ull << 19;
+constexpr uint32_t PAIR_FUSE_LARGE_K = 3 * TC_NT_MAX;
+
 bool tc_plan_can_fuse(const TcPlan* p, const FusedAcc& f)
 {
-	return tc_plan_uses_pair(p) && assign_tc_pair_can_fuse(p->tm.k_pad, p->s.dim, p->tp.d_pad) && f.acc != nullptr && f.counts != nullptr && f.points != nullptr &&
+	return tc_plan_uses_pair(p) && (p->s.k > PAIR_FUSE_LARGE_K || p->s.n <= PAIR_FUSE_SMALL_N) && assign_tc_pair_can_fuse(p->tm.k_pad, p->s.dim, p->tp.d_pad) && f.acc != nullptr && f.counts != nullptr && f.points != nullptr &&
 		(reinterpret_cast<uintptr_t>(f.acc) & 15u) == 0 && (f.rep_stride * sizeof(float)) % 16 == 0;
 }
 
@@ -938,11 +949,11 @@ static uint32_t plan_jsplit(const TcPlan* p)
 // 4096: the pass 8.70 -> 9.06 ms, the re-check of 4400 points 1.49 -> 0.09 ms).
 bool tc_plan_collects_pairs(const TcPlan* p) { return plan_jsplit(p) > 1 && p->s.dim >= 256 && p->tp.pairs != nullptr; }
 
-void tc_plan_describe(const TcPlan* p, uint32_t out[4])
+void tc_plan_describe(const TcPlan* p, bool fused, uint32_t out[4])
 {
 	out[1] = p->tm.k_pad / p->nt_cols;
 	out[2] = 1;
-	if (tc_plan_uses_pair(p)) { out[0] = BKM_PLAN_TC_PAIR; return; }
+	if (launch_uses_pair(p, fused, false)) { out[0] = BKM_PLAN_TC_PAIR; return; }
 	out[0] = p->tp.d_pad > TC_KCHUNK ? BKM_PLAN_TC_KLOOP : BKM_PLAN_TC_RESIDENT;
 	out[2] = plan_jsplit(p);
 }
@@ -968,7 +979,7 @@ cudaError_t launch_assign_tc(TcPlan* p, uint32_t* asg, Control* ctl, int slot, u
 	const uint32_t kchunks = kloop ? p->tp.d_pad / kw : 1u;
 	const uint32_t ksteps_last = (p->s.dim - (kchunks - 1) * 2 * kw + 15) / 16;    // K steps (16 dimensions) of the last slice
 	const uint32_t idesc = p->idesc;
-	if (tc_plan_uses_pair(p))
+	if (launch_uses_pair(p, fused != nullptr, ranged))
 		return launch_assign_tc_pair(p->a_hi, p->a_lo, p->bh_hi, p->bh_lo, p->tm.b_aug, p->tp.xnorm, asg, p->s.n, n_tiles,
 			p->s.k, p->tm.k_pad, p->tp.d_pad, ksteps_last, p->max_pairs, ctl, slot, flag_list, margin_coef, sqrt_dim, stream, fused, p->s.dim,
 			ranged ? (uint32_t)(p_begin / (2 * TC_MTILE)) : 0u,

@@ -158,7 +158,7 @@ cudaError_t launch_compute_center(const float* pts, const Shape& s, float* cente
 struct TcPlan;
 TcPlan* tc_plan_create(const Shape& s, const TcPoints& tp, const TcMeans& tm, int device, const char** err);
 void tc_plan_destroy(TcPlan* plan);
-// The CTA-pair kernel (means resident in shared memory) is used where it applies unless disallowed.
+// The CTA-pair kernel (means resident in shared memory) is used where it applies and pays, unless disallowed.
 void tc_plan_allow_pair(TcPlan* plan, bool allow);
 bool tc_plan_uses_pair(const TcPlan* plan);
 // With `fused` set (allowed when tc_plan_can_fuse) the kernel also adds every point to the sum and
@@ -166,8 +166,9 @@ bool tc_plan_uses_pair(const TcPlan* plan);
 // exact re-check moves afterwards are corrected there.
 bool tc_plan_can_fuse(const TcPlan* plan, const FusedAcc& f);
 // out[0] = BKM_PLAN_* code of the kernel the plan launches, out[1] = mean tiles, out[2] = CTAs that
-// share one point block (1 = no split; > 1 implies the partial-result merge kernel).
-void tc_plan_describe(const TcPlan* plan, uint32_t out[4]);
+// share one point block (1 = no split; > 1 implies the partial-result merge kernel), for a launch with or
+// without the fused sums.
+void tc_plan_describe(const TcPlan* plan, bool fused, uint32_t out[4]);
 // `p_begin`, `p_end` (0, 0 = all; CTA-pair plans only; p_begin a multiple of 256, p_end too unless it is
 // the last point): only these points, so that the pass can follow a host upload chunk by chunk.
 cudaError_t launch_assign_tc(TcPlan* plan, uint32_t* asg, Control* ctl, int slot, uint32_t* flag_list,
