@@ -422,20 +422,20 @@ def roofline_of(ctx, job, phases, counters, plan, ms_step, tf32_peak):
                 traffic = C2_ASSIGN_TC_DRAM_BYTES_PER_POINT * job.count
             elif job.name == "c5" and plan["kernel"] == "tc_resident":
                 traffic = C5_ASSIGN_TC_DRAM_BYTES_PER_POINT * job.count
-            ksteps = (min(dim, 32) + 7) // 8 if dim <= 32 else None
-            issued = (3.0 * ksteps + 1.0) / ksteps if ksteps else 3.0 + 8.0 / dim
+            ksteps = (dim + 15) // 16               # K steps of 16 dimensions, each for three products, and one more step
+            issued = (3.0 * ksteps + 1.0) * 16.0 / dim
             roofline = {"bound": "tensor", "achieved": ach, "peak": tf32_peak, "unit": "TFLOP/s", "frac": ach / tf32_peak,
                         "peak_tf32_measured": tf32_peak,
-                        "frac_tensor_issued": issued * ach / tf32_peak,
+                        "frac_tensor_issued": issued * ach / peaks["bf16_tflops"],
                         "tensor_flops_per_algorithmic_flop": issued,
                         "frac_vs_half_bf16_burst": ach / (peaks["bf16_tflops"] * 0.5),
                         "traffic": traffic,
                         "traffic_unit": "bytes per launch (profiler DRAM read+write per point of a reduced-size capture x points of this launch)",
                         "kernel": "assignment (%s)" % plan["kernel"], "kernel_ms": assign_ms,
                         "peak_note": "peak = TF32 library GEMM (8192^3, best of 10) measured in this run; `frac` counts "
-                                     "algorithmic flops 2*N*k*d; the split-TF32 scheme issues `tensor_flops_per_algorithmic_flop` "
-                                     "tensor flops for each, `frac_tensor_issued` is that work against the same peak; half the %s "
-                                     "bf16 burst peak is %.1f TFLOP/s" % (peaks["source"], peaks["bf16_tflops"] * 0.5)}
+                                     "algorithmic flops 2*N*k*d; the fp16-pair scheme issues `tensor_flops_per_algorithmic_flop` "
+                                     "tensor flops at the 16-bit rate for each, `frac_tensor_issued` is that work against the %s "
+                                     "bf16 burst peak of %.1f TFLOP/s" % (peaks["source"], peaks["bf16_tflops"])}
         else:
             ach = bytes_iter / (assign_ms * 1e-3) / 1e9
             roofline = {"bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",

@@ -46,7 +46,7 @@ extern "C" {
 #define BKM_ASSIGN_AUTO 0   /* pick by shape */
 #define BKM_ASSIGN_EXACT 1  /* CUDA cores, reference arithmetic for every point (any shape) */
 #define BKM_ASSIGN_SIMT 2   /* CUDA cores, small-d fast path (dim <= 8), near-ties re-checked exactly */
-#define BKM_ASSIGN_TC 3     /* tcgen05 tensor cores, split-TF32 GEMM form, near-ties re-checked exactly */
+#define BKM_ASSIGN_TC 3     /* tcgen05 tensor cores, fp16-pair GEMM form, near-ties re-checked exactly */
 
 /* Update variants (the counterpart of choosing UPDATE_KERNEL). */
 #define BKM_UPDATE_AUTO 0
