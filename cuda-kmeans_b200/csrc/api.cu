@@ -257,11 +257,12 @@ int enqueue_assign(int variant, const float* pts, const float* means, uint32_t* 
 	if (fast_pass_done) {
 		// (the pass ran behind the upload of the points: only the near-ties are left)
 	} else if (variant == BKM_ASSIGN_SIMT) {
-		CUDA_TRY(bkm::launch_assign_simt(pts, w.sm, asg, s, w.ctl, slot, w.flag_list, margin_scale, sm_count, stream, fused));
+		CUDA_TRY(bkm::launch_assign_simt(pts, means, w.sm, asg, s, w.ctl, slot, w.flag_list, margin_scale, sm_count, stream, fused));
 	} else {
 		CUDA_TRY(bkm::launch_assign_tc(plan, asg, w.ctl, slot, w.flag_list, margin_scale, stream, fused));
 	}
 	if (mid) CUDA_TRY(cudaEventRecord(mid, stream));
+	if (variant == BKM_ASSIGN_SIMT && fused) return BKM_OK;       // (that form leaves no near-ties)
 	CUDA_TRY(bkm::launch_assign_exact(pts, means, asg, s, w.flag_list, &w.ctl->flag_count, sm_count, stream, fused, w.split_scratch));
 	if (variant == BKM_ASSIGN_TC && bkm::tc_plan_collects_pairs(plan))
 		CUDA_TRY(bkm::launch_assign_exact_pairs(pts, means, asg, s, w.tp.pairs, &w.ctl->pair_count, sm_count, stream));
@@ -1014,7 +1015,7 @@ static int enqueue_iteration(bkm_handle_t h, cudaEvent_t* ev)
 	bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(s.k, s.dim), h->ws.tm.center, h->d_points, s.soa};
 	const bool fused = h->fuse_update && fuse_pays(h->assign_variant, h->update_variant, h->plan, fa, s, h->fuse_update >= 2);
 	h->last_fused = fused;
-	h->launches_per_iter = (h->assign_variant == BKM_ASSIGN_EXACT ? 1u : 2u) + (fused ? 0u : 1u) + 1u;
+	h->launches_per_iter = (h->assign_variant == BKM_ASSIGN_EXACT || (h->assign_variant == BKM_ASSIGN_SIMT && fused) ? 1u : 2u) + (fused ? 0u : 1u) + 1u;
 	bool fast_pass_done = false;
 	if (h->first_pass_done) {
 		// usable if nothing has happened since bkm_initialize and the sums went where this iteration expects them

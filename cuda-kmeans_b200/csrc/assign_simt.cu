@@ -671,11 +671,38 @@ __device__ __forceinline__ void send_row(float* dst, const float (&sum)[D], floa
 	}
 }
 
+// One point's cluster by the reference's arithmetic, by a whole warp (lanes over the means; every lane
+// gets the result): what the exact kernels do for the queued points.
+template<int D, bool SOA>
+__device__ __forceinline__ uint32_t exact_cluster(const float* __restrict__ pts, uint64_t i, uint64_t n, const float* __restrict__ means, int soa_means, uint32_t k)
+{
+	float x[D];
+	#pragma unroll
+	for (int j = 0; j < D; ++j) x[j] = pts[at<SOA>(i, j, n, D)];
+	float best = INFINITY;
+	uint32_t bidx = 0xffffffffu;
+	for (uint32_t m = threadIdx.x & 31u; m < k; m += 32) {
+		float sum = 0.0f;
+		#pragma unroll
+		for (int j = 0; j < D; ++j) {
+			const float diff = __fsub_rn(x[j], means[at_rt(soa_means, m, j, k, D)]);
+			sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+		}
+		const float dist = __fsqrt_rn(sum);
+		if (dist < best || (dist == best && m < bidx)) { best = dist; bidx = m; }
+		// what is not a number never wins, but nothing replaces it as the first distance of the sequential scan
+		if (m == 0 && dist != dist) { best = 0.0f; bidx = 0; }
+	}
+	// distances are >= +0: their bit patterns order like the values
+	const uint32_t low = __reduce_min_sync(0xffffffffu, __float_as_uint(best));
+	return __reduce_min_sync(0xffffffffu, __float_as_uint(best) == low ? bidx : 0xffffffffu);
+}
+
 template<int D, bool SOA, int P, bool FUSE>
 __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const float* __restrict__ pts,
 	const float* __restrict__ cprep, const float* __restrict__ center, uint32_t* __restrict__ asg, uint64_t n, uint32_t rows,
 	Control* __restrict__ ctl, int slot, uint32_t* __restrict__ flag_list, float margin_ulps, int vec_ok,
-	uint32_t k, float* __restrict__ fuse_acc, uint32_t* __restrict__ fuse_counts)
+	uint32_t k, float* __restrict__ fuse_acc, uint32_t* __restrict__ fuse_counts, const float* __restrict__ means, int soa_means)
 {
 	constexpr int RS = (D + 1 + 3) / 4 * 4;      // floats of a prepared row in global memory
 	extern __shared__ __align__(128) float tile[];  // rows of two means interleaved: (D + 1) pairs
@@ -689,7 +716,7 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 		fuse_acc_rep += (blockIdx.x % acc_replicas(k, D)) * acc_replica_stride(k, D);
 		for (uint32_t c = threadIdx.x; c < SIMT_FUSE_MAX_K; c += SIMT_THREADS) s_cnt[c] = 0;
 	}
-	__shared__ uint32_t flag_bufs[SIMT_THREADS / 32][FLAG_BUFFER];     // per warp: near-ties on their way to the list
+	__shared__ uint32_t flag_bufs[SIMT_THREADS / 32][FUSE ? 1 : FLAG_BUFFER];     // per warp: near-ties on their way to the list
 	uint32_t* flag_buf = flag_bufs[threadIdx.x >> 5];
 	uint32_t flag_cnt = 0;
 
@@ -833,11 +860,24 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 				// key - key_base = M * mantissa + column
 				const uint32_t bm = div_key(best[p] - key_base, key_magic);
 				cl[p] = bchunk[p] * 32u + ((best[p] - key_base) - bm * key_mult);
-				asg[idx[p]] = cl[p];
+				if (!FUSE) asg[idx[p]] = cl[p];
 				const float gap = second[p] == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second[p] - key_base, key_magic) - bm);
 				flag = gap <= margin_ulps;
 			}
-			buffered_append(flag, (uint32_t)idx[p], flag_buf, flag_cnt, ctl, flag_list, n);
+			if (FUSE) {
+				// a near-tie is settled on the spot, before the point is added anywhere: no list, no
+				// launch for it, and nothing to move from one sum to another
+				uint32_t mask = __ballot_sync(0xffffffffu, flag);
+				flag_cnt += (uint32_t)__popc(mask);
+				for (; mask != 0; mask &= mask - 1) {
+					const int src = __ffs(mask) - 1;
+					const uint32_t c = exact_cluster<D, SOA>(pts, __shfl_sync(0xffffffffu, (unsigned long long)idx[p], src), n, means, soa_means, k);
+					if ((int)(tid & 31u) == src) cl[p] = c;
+				}
+				if (idx[p] < n) asg[idx[p]] = cl[p];
+			} else {
+				buffered_append(flag, (uint32_t)idx[p], flag_buf, flag_cnt, ctl, flag_list, n);
+			}
 		}
 
 		if (FUSE) {
@@ -920,7 +960,8 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 			if (v) atomicAdd(&cnt[c], v);
 		}
 	}
-	flush_flag_buffer(flag_buf, flag_cnt, ctl, flag_list, n);
+	if (!FUSE) flush_flag_buffer(flag_buf, flag_cnt, ctl, flag_list, n);
+	else if ((tid & 31u) == 0 && flag_cnt != 0) atomicAdd(&ctl->flag_count, flag_cnt);      // (for the report only)
 }
 
 bool assign_simt_supported(const Shape& s)
@@ -936,7 +977,7 @@ bool assign_simt_can_fuse(const Shape& s, const FusedAcc& f)
 }
 
 template<int D, int P>
-static cudaError_t launch_simt_d(const float* pts, const float* cprep, const float* center, uint32_t* asg, const Shape& s,
+static cudaError_t launch_simt_d(const float* pts, const float* means, const float* cprep, const float* center, uint32_t* asg, const Shape& s,
 	Control* ctl, int slot, uint32_t* flag_list, float margin_scale, int sm_count, cudaStream_t stream, const FusedAcc* fused)
 {
 	const uint32_t rows = simt_rows(s.k);
@@ -961,7 +1002,7 @@ static cudaError_t launch_simt_d(const float* pts, const float* cprep, const flo
 		uint32_t grid = (uint32_t)std::min<uint64_t>(nblocks, (uint64_t)sm_count * per_sm); \
 		if (grid < 1) grid = 1; \
 		kern<<<grid, SIMT_THREADS, smem, stream>>>(pts, cprep, center, asg, s.n, rows, ctl, slot, flag_list, margin_ulps, vec_ok, \
-			s.k, fused ? fused->acc : nullptr, fused ? fused->counts : nullptr); \
+			s.k, fused ? fused->acc : nullptr, fused ? fused->counts : nullptr, means, s.soa_means); \
 	} while (0)
 	if (fused && !assign_simt_can_fuse(s, *fused)) return cudaErrorInvalidValue;
 	if (fused) { if (s.soa) BKM_LAUNCH_SIMT(true, true); else BKM_LAUNCH_SIMT(false, true); }
@@ -970,18 +1011,18 @@ static cudaError_t launch_simt_d(const float* pts, const float* cprep, const flo
 	return cudaGetLastError();
 }
 
-cudaError_t launch_assign_simt(const float* pts, const SimtMeans& sm, uint32_t* asg, const Shape& s,
+cudaError_t launch_assign_simt(const float* pts, const float* means, const SimtMeans& sm, uint32_t* asg, const Shape& s,
 	Control* ctl, int slot, uint32_t* flag_list, float margin_scale, int sm_count, cudaStream_t stream, const FusedAcc* fused)
 {
 	switch (s.dim) {
-	case 1: return launch_simt_d<1, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 2: return launch_simt_d<2, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 3: return launch_simt_d<3, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 4: return launch_simt_d<4, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 5: return launch_simt_d<5, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 6: return launch_simt_d<6, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 7: return launch_simt_d<7, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 8: return launch_simt_d<8, 2>(pts, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 1: return launch_simt_d<1, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 2: return launch_simt_d<2, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 3: return launch_simt_d<3, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 4: return launch_simt_d<4, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 5: return launch_simt_d<5, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 6: return launch_simt_d<6, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 7: return launch_simt_d<7, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 8: return launch_simt_d<8, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
 	default: return cudaErrorInvalidValue;
 	}
 }
