@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __r
 	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
 	const KeyConsts kc = tc_key_consts(x2max, c2max);
 	const float ulp = kc.pow2 * 1.1920929e-07f;
-	const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim);
+	const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim, tc_scale(ctl->xdev));
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint64_t n32 = (n + 31) & ~(uint64_t)31;      // whole warps walk the loop together (the append is a warp operation)
 	for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n32; p += (uint64_t)gridDim.x * blockDim.x) {
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 		const uint32_t half = part & 1u;
 		const uint32_t row = q * 32 + lane;
 		const float ulp = pow2 * 1.1920929e-07f;   // spacing of the values inside [P, 2P)
-		const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim);
+		const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim, tc_scale(ctl->xdev));
 		const uint32_t chunks_total = nt_cols >> 5;                    // 1..8
 		const uint32_t per_half = (chunks_total + 1) / 2;              // 1..4
 		const uint32_t first_chunk = half * per_half;

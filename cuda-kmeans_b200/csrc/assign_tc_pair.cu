@@ -334,7 +334,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 		const uint32_t g = (warp - 2) >> 2;           // 0..3
 		const uint32_t row = q * 32 + lane;
 		const float ulp = kc.pow2 * 1.1920929e-07f;   // spacing of the values inside [P, 2P)
-		const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim);
+		const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim, tc_scale(ctl->xdev));
 		const uint32_t merger = 1u;                   // group 1, lower column half (fills per step are even in number)
 		const uint32_t acc_empty_base = ptx::map_to_cta(ptx::smem_u32(&bars->acc_empty[0]), 0);
 		uint32_t it = 0;
@@ -444,7 +444,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 					// (with means beyond the operands' range the keys mean nothing: any index, the exact kernel follows)
 					mine = min(bchunk * 32u + ((best - key_base) - bm * key_mult), k - 1);
 					// points that this pass cannot place are added by the exact kernel, which finds no previous cluster
-					if (fuse_acc != nullptr && !(fmaxf(xn, c2max) <= TC_NORM2_MAX && c2max == c2max)) mine = 0xFFFFFFFFu;
+					if (fuse_acc != nullptr && !(xn <= TC_NORM2_MAX && margin_floor < INFINITY)) mine = 0xFFFFFFFFu;
 					asg[p] = mine;
 					const float gap = second == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second - key_base, key_magic) - bm) * ulp;
 					const float margin = margin_coef * (xn + c2max) + margin_floor;

@@ -116,12 +116,19 @@ __device__ __forceinline__ KeyConsts tc_key_consts(float x2max, float c2max) { r
 
 // The part of the near-tie band that does not depend on the point: four value spacings, plus what the
 // absolute 2^-25 of small operand values can move a product sum by (2 * 2^-25 * sqrt(dim) * (|x| + |c|)
-// for each side).  Means beyond what the operands hold make it infinite: every point goes to the
-// exact kernel.  (A point beyond it has an infinite |x|^2, which does the same for that point.)
-__device__ __forceinline__ float tc_margin_floor(float ulp, float x2max, float c2max, float sqrt_dim)
+// for each side), plus what the reference's own squares lose where they are subnormal: half of 2^-149
+// for each dimension and distance, so dim * 2^-149 for a difference of two, twice that taken, in units of
+// `scale` squared (the values of this pass are scaled to the data, the reference's are not: where they
+// vanish its distances tie).
+// It is infinite - every point goes to the exact kernel - where the means lie beyond what the operands
+// hold, and where a squared distance of the reference, at most 2 * (|x|^2 + |c|^2) before the scaling, can
+// pass half the largest float: its distances are then infinite and tie.  (A point beyond the operands'
+// range has an infinite |x|^2, which does the same for that point.)
+__device__ __forceinline__ float tc_margin_floor(float ulp, float x2max, float c2max, float sqrt_dim, float scale)
 {
-	if (!(c2max <= TC_NORM2_MAX)) return INFINITY;
-	return 4.0f * ulp + 2.4e-7f * sqrt_dim * sqrtf(x2max + c2max);
+	const float s63 = scale * 9.223372e18f, s_74 = scale * 5.293956e-23f;            // scale * 2^63, scale * 2^-74
+	if (!(c2max <= TC_NORM2_MAX) || x2max + c2max >= s63 * s63) return INFINITY;
+	return 4.0f * ulp + 2.4e-7f * sqrt_dim * sqrtf(x2max + c2max) + (sqrt_dim * s_74) * (sqrt_dim * s_74);
 }
 
 // The three products of one operand-tile pair over KS steps of 16 dimensions: the small cross
