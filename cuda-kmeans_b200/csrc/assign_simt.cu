@@ -724,8 +724,13 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 	const uint32_t ntiles = (rows + SIMT_TILE_ROWS - 1) / SIMT_TILE_ROWS;
 	const uint64_t per_block = (uint64_t)SIMT_THREADS * P;
 	const uint64_t nblocks = (n + per_block - 1) / per_block;
-	const KeyConsts kc = make_key_consts(ctl->xmax2, ctl->cmax2[slot]);
+	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
+	const KeyConsts kc = make_key_consts(x2max, c2max);
 	const uint32_t key_mult = kc.key_mult, key_base = kc.key_base, key_magic = kc.key_magic;
+	// Up to 2^125 the binade of the values and the reference's squared distances (at most 2 * (|x|^2 + |c|^2))
+	// are inside the range of 32-bit floats; beyond, or with means that are not finite, the keys mean nothing
+	// and every point is settled by the exact arithmetic.
+	const float margin = x2max + c2max < 4.2535296e37f ? margin_ulps : INFINITY;
 	const float pad_value = kc.pow2 * (2.0f - 1.0f / 32.0f);     // padding rows: above every real value, inside [P, 2P)
 	float cen[D];
 	#pragma unroll
@@ -803,6 +808,14 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 			#pragma unroll
 			for (int j = 0; j < D; ++j) x[p][j] = raw[p][j] - cen[j];
 		}
+		uint32_t spoilt = 0;           // points that hold an infinity or what is not a number: their keys mean nothing either
+		#pragma unroll
+		for (int p = 0; p < P; ++p) {
+			float zero = 0.0f;
+			#pragma unroll
+			for (int j = 0; j < D; ++j) zero = fmaf(x[p][j], 0.0f, zero);
+			if (zero != 0.0f) spoilt |= 1u << p;
+		}
 		uint64_t xx[P][D];
 		#pragma unroll
 		for (int p = 0; p < P; ++p)
@@ -862,7 +875,8 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 				cl[p] = bchunk[p] * 32u + ((best[p] - key_base) - bm * key_mult);
 				if (!FUSE) asg[idx[p]] = cl[p];
 				const float gap = second[p] == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second[p] - key_base, key_magic) - bm);
-				flag = gap <= margin_ulps;
+				flag = !(gap > margin);
+				flag = flag || (spoilt >> p & 1u) != 0;
 			}
 			if (FUSE) {
 				// a near-tie is settled on the spot, before the point is added anywhere: no list, no

@@ -9,6 +9,7 @@ from helpers import DeviceArrays, rows_to_layout
 pytestmark = pytest.mark.gpu
 
 TC_SHAPES = [(1500, 40, 16), (1500, 40, 32), (900, 300, 32), (900, 300, 64), (700, 40, 97), (300, 300, 513), (300, 1100, 260)]
+SIMT_SHAPES = [(3001, 40, 1), (3000, 40, 3), (2000, 300, 8), (900, 1100, 4)]
 FACTORS = [1e-38, 1e-30, 1e-24, 1e-22, 1e-21, 1e-20, 1e-18, 1e17, 1e18, 1e19, 1e21, 1e30, 1e37]
 
 
@@ -106,3 +107,25 @@ def test_sums_of_the_cta_pair_pass_where_squares_leave_the_range(pkg, torch_cuda
     else:
         rows, means = _inputs(n, k, d, float(kind))
     _check_handle(pkg, oracle_mod, rows, means, layout, pkg.ASSIGN_TC, pkg.UPDATE_ROWS, "fused")
+
+
+@pytest.mark.parametrize("factor", FACTORS)
+@pytest.mark.parametrize("n,k,d", SIMT_SHAPES)
+def test_cuda_core_labels_where_squares_underflow_or_overflow(pkg, torch_cuda, oracle_mod, n, k, d, factor):
+    _check_assign(pkg, torch_cuda, oracle_mod, *_inputs(n, k, d, factor), pkg.ASSIGN_SIMT, ((0, 0), (1, 1)))
+
+
+@pytest.mark.parametrize("kind", ["p-nan", "p-+inf", "p--inf", "m-nan", "m-+inf", "m--inf"])
+@pytest.mark.parametrize("n,k,d", SIMT_SHAPES)
+def test_cuda_core_labels_of_values_that_are_not_finite(pkg, torch_cuda, oracle_mod, n, k, d, kind):
+    _check_assign(pkg, torch_cuda, oracle_mod, *_spoil(*_inputs(n, k, d, 1.0), kind), pkg.ASSIGN_SIMT, ((0, 0), (1, 1)))
+
+
+@pytest.mark.parametrize("kind", ["1e-30", "1e-22", "5e18", "1e19", "1e30", "p-nan", "p-+inf", "m-nan", "m--inf"])
+@pytest.mark.parametrize("n,k,d,layout", [(3001, 40, 1, 0), (3000, 60, 3, 1), (2000, 300, 8, 0)])
+def test_sums_of_the_cuda_core_pass_where_squares_leave_the_range(pkg, torch_cuda, oracle_mod, n, k, d, layout, kind):
+    if kind[0] in "pm":
+        rows, means = _spoil(*_inputs(n, k, d, 1.0), kind)
+    else:
+        rows, means = _inputs(n, k, d, float(kind))
+    _check_handle(pkg, oracle_mod, rows, means, layout, pkg.ASSIGN_SIMT, pkg.UPDATE_AUTO, "fused", (("fuse_update", 2),))
