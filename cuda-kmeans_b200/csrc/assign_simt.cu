@@ -49,14 +49,16 @@ __global__ void __launch_bounds__(256) assign_exact_kernel(const float* __restri
 				sum = __fadd_rn(sum, __fmul_rn(diff, diff));
 			}
 			float dist = __fsqrt_rn(sum);
-			if (dist < best || bidx == 0xffffffffu) { best = dist; bidx = m; }
+			if (dist < best || (dist == best && m < bidx)) { best = dist; bidx = m; }
+			// what is not a number never wins, but nothing replaces it as the first distance of the sequential scan
+			if (m == 0 && dist != dist) { best = 0.0f; bidx = 0; }
 		}
 		// lowest (distance, index) pair over the warp = what the sequential scan would keep
 		#pragma unroll
 		for (int off = 16; off > 0; off >>= 1) {
 			float ob = __shfl_xor_sync(0xffffffffu, best, off);
 			uint32_t oi = __shfl_xor_sync(0xffffffffu, bidx, off);
-			if (oi != 0xffffffffu && (bidx == 0xffffffffu || ob < best || (ob == best && oi < bidx))) { best = ob; bidx = oi; }
+			if (ob < best || (ob == best && oi < bidx)) { best = ob; bidx = oi; }
 		}
 		if (lane == 0) asg[i] = bidx;
 	}

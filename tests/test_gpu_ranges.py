@@ -129,3 +129,22 @@ def test_sums_of_the_cuda_core_pass_where_squares_leave_the_range(pkg, torch_cud
     else:
         rows, means = _inputs(n, k, d, float(kind))
     _check_handle(pkg, oracle_mod, rows, means, layout, pkg.ASSIGN_SIMT, pkg.UPDATE_AUTO, "fused", (("fuse_update", 2),))
+
+
+@pytest.mark.parametrize("kind", ["p-nan", "p-+inf", "m-nan", "m--inf", "1e-24", "1e19"])
+@pytest.mark.parametrize("n,k,d", [(301, 70, 3), (300, 70, 40), (201, 33, 513), (200, 1, 2)])
+def test_exact_variant_and_double_precision_outside_the_range(pkg, torch_cuda, oracle_mod, n, k, d, kind):
+    """A mean whose distance is not a number never wins, but must not hide the means behind it either."""
+    if kind[0] in "pm":
+        rows, means = _inputs(n, k, d, 1.0)
+        if k > 1:
+            rows, means = _spoil(rows, means, kind)
+    else:
+        rows, means = _inputs(n, k, d, float(kind))
+    _check_assign(pkg, torch_cuda, oracle_mod, rows, means, pkg.ASSIGN_EXACT)
+    if kind == "1e-24" or kind == "1e19":
+        rows, means = rows.astype(np.float64) * float(kind) ** 7.2, means.astype(np.float64) * float(kind) ** 7.2
+    for lay, laym in ((0, 0), (1, 1), (0, 1), (1, 0)):
+        data, m0 = (np.ascontiguousarray(a if lx == 0 else a.T, dtype=np.float64).reshape(-1) for a, lx in ((rows, lay), (means, laym)))
+        got = pkg.kmeans_host_f64(data, m0, n, k, d, 1, lay, laym)[1]
+        assert np.array_equal(got, oracle_mod.assign_f64(data, m0, n, k, d, lay, laym, threads=8)), (lay, laym)
