@@ -411,9 +411,14 @@ static bkm::TcPlan* cached_plan(const bkm::Shape& s, const Workspace& w, int dev
 	return plan;
 }
 
+static bkm::PointsKey* points_key(const Workspace& w)
+{
+	return reinterpret_cast<bkm::PointsKey*>(reinterpret_cast<char*>(w.ctl) + bkm::POINTS_KEY_OFFSET);
+}
+
 // One assignment pass on a caller's workspace.  The operands derived from the (immutable) points -
 // centre vector, largest norm, fp16 planes - stay in the workspace; a call that finds the same
-// point set there (address, shape and a fingerprint of a sample of the values) skips them.
+// point set there (address, shape, number of means and a fingerprint of a sample of the values) skips them.
 // Whether the fast assignment pass should accumulate the update sums itself.  On CTA pairs the
 // epilogue warps send the reductions, which pays where the update would otherwise be the row-wise
 // kernel (the sorted update of row-major points costs less than that).  In the CUDA-core pass every
@@ -440,7 +445,7 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 	if (fused_out) *fused_out = false;
 	bkm::TcPlan* plan = nullptr;
 	bool fused = false;
-	bkm::PointsKey* key = nullptr;
+	bkm::PointsKey* key = points_key(w);
 	if (v == BKM_ASSIGN_SIMT) {
 		fused = fa != nullptr && fuse_pays(v, variant_update, nullptr, *fa, s, true);     // the caller asked for the one-pass form
 	} else if (v == BKM_ASSIGN_TC) {
@@ -455,9 +460,8 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 	bkm::ClearRanges clear = {{w.split_scratch, w.acc, nullptr}, {bkm::list_split_scratch_bytes(), fa ? align256(w.acc_bytes) : 0, 0}};
 	if (v == BKM_ASSIGN_SIMT) { clear.base[2] = w.sm.rows; clear.bytes[2] = align256(w.cprep_bytes); }
 	if (v == BKM_ASSIGN_TC) { clear.base[2] = w.tm.b_hi; clear.bytes[2] = w.tm_bytes; }
-	if (v != BKM_ASSIGN_EXACT) key = reinterpret_cast<bkm::PointsKey*>(reinterpret_cast<char*>(w.ctl) + bkm::POINTS_KEY_OFFSET);
-	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, key, clear, sm_count, st));
-	if (key) {
+	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, key, s, clear, sm_count, st));
+	if (v != BKM_ASSIGN_EXACT) {
 		const uint32_t* skip = &key->valid;
 		CUDA_TRY(bkm::launch_points_fingerprint(points, s, v, key, w.ctl, sm_count, st));
 		CUDA_TRY(bkm::launch_compute_center(points, s, w.tm.center, w.ctl, st, skip));
@@ -481,7 +485,7 @@ static int stateless_update(const float* points, const uint32_t* assignment, flo
 	int rc = resolve_update(variant, s, device, &v);
 	if (rc) return rc;
 	// (an assignment in front of it has cleared the accumulators as well)
-	if (clear) CUDA_TRY(bkm::launch_stateless_begin(w.ctl, nullptr, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, sm_count, st));
+	if (clear) CUDA_TRY(bkm::launch_stateless_begin(w.ctl, points_key(w), s, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, sm_count, st));
 	bkm::launch_update(points, assignment, w.acc, w.counts, w.replicas, s, v, w.ctl, sm_count, st);
 	bkm::launch_finalize(w.acc, w.counts, w.replicas, means, sizes, s, nullptr, nullptr, w.ctl, 1, st);
 	CUDA_TRY(cudaGetLastError());
@@ -520,7 +524,7 @@ int bkm_bucket_sums_f32(const float* points, const uint32_t* indices, float* sum
 	int v = 0;
 	if ((rc = resolve_update(variant, s, device, &v))) return rc;
 	cudaStream_t st = static_cast<cudaStream_t>(stream);
-	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, nullptr, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, sm, st));
+	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, points_key(w), s, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, sm, st));
 	bkm::launch_update(points, indices, w.acc, w.counts, w.replicas, s, v, w.ctl, sm, st);
 	bkm::launch_finalize_sums(w.acc, w.counts, w.replicas, sums, s, w.ctl, st);
 	CUDA_TRY(cudaGetLastError());

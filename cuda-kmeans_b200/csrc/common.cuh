@@ -38,7 +38,8 @@ struct PointsKey {
 	unsigned long long fp_old;   // fingerprint the operands in the workspace belong to
 	unsigned long long ptr, n;
 	uint32_t dim, layout, variant, valid;
-	uint32_t arrive, pad;        // blocks of the fingerprint that are done
+	uint32_t arrive;             // blocks of the fingerprint that are done
+	uint32_t k;                  // the operands lie behind ranges whose sizes depend on it
 };
 constexpr size_t POINTS_KEY_OFFSET = 64;
 

@@ -85,10 +85,12 @@ cudaError_t launch_probe_atomics(float* result, uint64_t n, uint32_t k, uint32_t
 // ---- the beginning of a stateless call (update.cu) ----
 // Ranges of the workspace to clear (16-byte aligned, whole multiples of 16 bytes; 0 bytes = unused).
 struct ClearRanges { void* base[3]; size_t bytes[3]; };
-// Clears status, near-tie count, |c|^2 slots, the fingerprint of `key` (may be null) and the ranges.
-cudaError_t launch_stateless_begin(Control* ctl, PointsKey* key, const ClearRanges& ranges, int sm_count, cudaStream_t stream);
+// Clears status, near-tie count, |c|^2 slots, the fingerprint of `key` and the ranges.  A call that does not
+// look at the points (no fingerprint behind it) but lays the workspace out differently from the call that
+// `key` remembers writes over the operands derived then: it forgets them.
+cudaError_t launch_stateless_begin(Control* ctl, PointsKey* key, const Shape& s, const ClearRanges& ranges, int sm_count, cudaStream_t stream);
 // Fingerprints the points (every 16th 128-byte line and the last one; order-independent sum of mixed
-// (value, position) words), sets key->valid (same address, shape, variant and fingerprint as
+// (value, position) words), sets key->valid (same address, shape, number of means, variant and fingerprint as
 // remembered) and remembers the current call's; when the points are new it also clears what their
 // preprocessing refills in `ctl`.  Behind launch_stateless_begin with the same key.
 cudaError_t launch_points_fingerprint(const float* pts, const Shape& s, int variant, PointsKey* key, Control* ctl, int sm_count, cudaStream_t stream);

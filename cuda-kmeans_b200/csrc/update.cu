@@ -466,13 +466,14 @@ cudaError_t launch_probe_atomics(float* result, uint64_t n, uint32_t k, uint32_t
 // Clears what a stateless call needs cleared - status, near-tie count and |c|^2 slots, the fingerprint,
 // and up to three ranges of its scratch - in one launch (a call is bound by the number of its launches:
 // five memsets took a third of the 13 operations, 42 us together, of a small bkm_iterate_f32).
-__global__ void __launch_bounds__(256) stateless_begin_kernel(Control* ctl, PointsKey* key, ClearRanges ranges)
+__global__ void __launch_bounds__(256) stateless_begin_kernel(Control* ctl, PointsKey* key, unsigned long long n, uint32_t k, uint32_t dim, ClearRanges ranges)
 {
 	const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
 	if (t == 0) {
 		// last_flag_count and what belongs to the points survive
 		ctl->status = 0; ctl->flag_count = 0; ctl->pair_count = 0; ctl->cmax2[0] = 0.0f; ctl->cmax2[1] = 0.0f;
-		if (key) { key->fp_new = 0; key->arrive = 0; }
+		key->fp_new = 0; key->arrive = 0;
+		if (key->n != n || key->k != k || key->dim != dim) key->n = 0;      // (no call has 0 points)
 	}
 	#pragma unroll
 	for (uint32_t r = 0; r < 3; ++r) {
@@ -481,19 +482,19 @@ __global__ void __launch_bounds__(256) stateless_begin_kernel(Control* ctl, Poin
 	}
 }
 
-cudaError_t launch_stateless_begin(Control* ctl, PointsKey* key, const ClearRanges& ranges, int sm_count, cudaStream_t stream)
+cudaError_t launch_stateless_begin(Control* ctl, PointsKey* key, const Shape& s, const ClearRanges& ranges, int sm_count, cudaStream_t stream)
 {
 	uint64_t words = 0;
 	for (uint32_t r = 0; r < 3; ++r) words += ranges.bytes[r] / 16;
 	const uint32_t grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>((words + 511) / 512, 1), (uint64_t)sm_count * 4);
-	stateless_begin_kernel<<<grid, 256, 0, stream>>>(ctl, key, ranges);
+	stateless_begin_kernel<<<grid, 256, 0, stream>>>(ctl, key, s.n, s.k, s.dim, ranges);
 	return cudaGetLastError();
 }
 
 // Fingerprints the points (every 16th 128-byte line, and the last one); the block that finishes last
 // compares address, shape and fingerprint with what the workspace remembers.
 __global__ void __launch_bounds__(256) points_fingerprint_kernel(const uint32_t* __restrict__ bits, uint64_t words, PointsKey* __restrict__ key,
-	unsigned long long n, uint32_t dim, uint32_t layout, uint32_t variant, Control* __restrict__ ctl)
+	unsigned long long n, uint32_t k, uint32_t dim, uint32_t layout, uint32_t variant, Control* __restrict__ ctl)
 {
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint64_t lines = (words + 31) / 32;
@@ -517,10 +518,10 @@ __global__ void __launch_bounds__(256) points_fingerprint_kernel(const uint32_t*
 	if (threadIdx.x != 0 || atomicAdd(&key->arrive, 1u) != gridDim.x - 1) return;
 	__threadfence();
 	const unsigned long long fp = atomicAdd(&key->fp_new, 0ull), ptr = (unsigned long long)reinterpret_cast<uintptr_t>(bits);
-	const bool same = key->fp_old == fp && key->ptr == ptr && key->n == n && key->dim == dim && key->layout == layout && key->variant == variant;
+	const bool same = key->fp_old == fp && key->ptr == ptr && key->n == n && key->k == k && key->dim == dim && key->layout == layout && key->variant == variant;
 	key->valid = same ? 1u : 0u;
 	key->fp_old = fp;
-	key->ptr = ptr; key->n = n; key->dim = dim; key->layout = layout; key->variant = variant;
+	key->ptr = ptr; key->n = n; key->k = k; key->dim = dim; key->layout = layout; key->variant = variant;
 	if (!same) { ctl->xmax2 = 0.0f; ctl->xdev = 0.0f; ctl->beyond = 0u; }
 }
 
@@ -529,7 +530,7 @@ cudaError_t launch_points_fingerprint(const float* pts, const Shape& s, int vari
 	const uint64_t words = s.n * s.dim;
 	const uint64_t samples = ((words + 31) / 32 + 15) / 16 + 1;
 	const uint32_t grid = (uint32_t)std::min<uint64_t>((samples + 7) / 8, (uint64_t)sm_count * 8);
-	points_fingerprint_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(pts), words, key, s.n, s.dim, (uint32_t)s.soa,
+	points_fingerprint_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(pts), words, key, s.n, s.k, s.dim, (uint32_t)s.soa,
 		(uint32_t)variant, ctl);
 	return cudaGetLastError();
 }

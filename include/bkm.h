@@ -75,8 +75,9 @@ int bkm_device_count(void);
  * (headers/cuda.hpp:70-88).  bkm_assign_f32 and bkm_iterate_f32 therefore leave what they derive
  * from the points alone (a centre vector, the largest norm, fp16 operand planes) in the
  * workspace, and a later call on the same workspace skips that work when it finds the same
- * points: same address, shape and variant, and the same fingerprint of a sample of the values
- * (every 16th 128-byte line and the last).  New data at the same address is therefore noticed;
+ * points: same address, shape, number of means and variant, and the same fingerprint of a sample of
+ * the values (every 16th 128-byte line and the last).  New data at the same address is therefore noticed,
+ * and one workspace may serve calls of different n, k and dim (each change derives the operands again);
  * a caller that rewrites single coordinates in place, or scribbles over the workspace while
  * keeping its first 256 bytes, must clear those 256 bytes before the next call.
  * ------------------------------------------------------------------------------------------ */

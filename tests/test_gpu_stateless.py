@@ -75,3 +75,40 @@ def test_iterate_matches_oracle_iteration(pkg, torch_cuda, oracle_mod, n, k, d, 
         ok, err = means_close(got, want_means)
         assert ok, (it, err)
         cur = got.copy()
+
+
+@pytest.mark.parametrize("n,d,variant,small,large", [(5000, 24, 3, 40, 300), (3000, 70, 3, 40, 700), (9000, 4, 2, 20, 700)])
+@pytest.mark.parametrize("layout", [0, 1])
+def test_one_workspace_serves_calls_with_different_numbers_of_means(pkg, torch_cuda, oracle_mod, n, d, variant, small, large, layout):
+    """The operands kept in a workspace lie behind ranges whose sizes depend on k: the same points with another
+    k (a sweep over k on a workspace sized for the largest), and an update, a bucketing or an exact assignment
+    with another k in between, must have them derived again."""
+    torch = torch_cuda
+    rng = np.random.default_rng(n + d)
+    rows = rng.standard_normal((n, d)).astype(np.float32)
+    data = rows_to_layout(rows, layout)
+    dev = DeviceArrays(torch, pkg, data, rows_to_layout(rows[:large], layout), n, large, d)
+    means = {k: rows_to_layout(rng.standard_normal((k, d)).astype(np.float32), layout) for k in (small, large)}
+    want = {k: oracle_mod.assign(data, m, n, k, d, layout, layout, threads=8) for k, m in means.items()}
+
+    def assign(k, v=variant):
+        m = torch.from_numpy(means[k]).to("cuda:0")
+        pkg.assign(dev.points.data_ptr(), m.data_ptr(), dev.assignment.data_ptr(), n, k, d, layout, layout, dev.ws_ptr, dev.ws_bytes_avail, variant=v)
+        pkg.workspace_check(dev.ws_ptr)
+        got = dev.asg_host()
+        assert np.array_equal(got, want[k]), (k, v, int((got != want[k]).sum()))
+
+    for k in (large, small, large, large, small):
+        assign(k)
+    # the workspace now remembers the points for `small`
+    pkg.update(dev.points.data_ptr(), dev.assignment.data_ptr(), dev.means_out.data_ptr(), dev.sizes.data_ptr(), n, large, d, layout, layout,
+               dev.ws_ptr, dev.ws_bytes_avail)
+    assign(small)
+    pkg.bucket_sums(dev.points.data_ptr(), dev.assignment.data_ptr(), dev.means_out.data_ptr(), n, large, d, layout, dev.ws_ptr, dev.ws_bytes_avail)
+    assign(small)
+    assign(large, 1)
+    assign(small)
+    # fewer points: the same ranges mean something else again
+    pkg.update(dev.points.data_ptr(), dev.assignment.data_ptr(), dev.means_out.data_ptr(), dev.sizes.data_ptr(), n // 2, small, d, 0, layout,
+               dev.ws_ptr, dev.ws_bytes_avail)
+    assign(small)
