@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -383,16 +384,17 @@ static int stateless_common(uint64_t n, uint32_t k, uint32_t dim, int layout, in
 }
 
 // Tensor maps are a function of the workspace address and the shape, so the stateless calls keep
-// the few most recent plans instead of encoding six maps per call.
+// the few most recent plans instead of encoding six maps per call.  A plan is not changed once it is made, and
+// a call holds the one it uses: another thread may replace it in its slot meanwhile.
 struct PlanSlot {
 	void* ws = nullptr; uint64_t n = 0; uint32_t k = 0, dim = 0; int soa = 0, soa_means = 0, device = -1;
-	bkm::TcPlan* plan = nullptr; uint64_t stamp = 0;
+	std::shared_ptr<bkm::TcPlan> plan; uint64_t stamp = 0;
 };
 static std::mutex g_plan_mutex;
 static PlanSlot g_plan_slots[8];
 static uint64_t g_plan_clock = 0;
 
-static bkm::TcPlan* cached_plan(const bkm::Shape& s, const Workspace& w, int device, const char** err)
+static std::shared_ptr<bkm::TcPlan> cached_plan(const bkm::Shape& s, const Workspace& w, int device, const char** err)
 {
 	std::lock_guard<std::mutex> lock(g_plan_mutex);
 	PlanSlot* victim = &g_plan_slots[0];
@@ -403,9 +405,13 @@ static bkm::TcPlan* cached_plan(const bkm::Shape& s, const Workspace& w, int dev
 		}
 		if (p.stamp < victim->stamp) victim = &p;
 	}
-	bkm::TcPlan* plan = bkm::tc_plan_create(s, w.tp, w.tm, device, err);
+	std::shared_ptr<bkm::TcPlan> plan;
+	try {
+		plan.reset(bkm::tc_plan_create(s, w.tp, w.tm, device, err), bkm::tc_plan_destroy);
+	} catch (const std::bad_alloc&) {
+		if (err) *err = "out of host memory";
+	}
 	if (!plan) return nullptr;
-	if (victim->plan) bkm::tc_plan_destroy(victim->plan);
 	victim->ws = (void*)w.ctl; victim->n = s.n; victim->k = s.k; victim->dim = s.dim; victim->soa = s.soa; victim->soa_means = s.soa_means;
 	victim->device = device; victim->plan = plan; victim->stamp = ++g_plan_clock;
 	return plan;
@@ -443,7 +449,7 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 	int rc = resolve_assign(variant, s, &v);
 	if (rc) return rc;
 	if (fused_out) *fused_out = false;
-	bkm::TcPlan* plan = nullptr;
+	std::shared_ptr<bkm::TcPlan> plan;
 	bool fused = false;
 	bkm::PointsKey* key = points_key(w);
 	if (v == BKM_ASSIGN_SIMT) {
@@ -452,8 +458,7 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 		const char* err = nullptr;
 		plan = cached_plan(s, w, device, &err);
 		if (!plan) return fail(BKM_ERR_CUDA, "tensor-core plan: %s", err ? err : "unknown");
-		bkm::tc_plan_allow_pair(plan, true);
-		fused = fa != nullptr && fuse_pays(v, variant_update, plan, *fa, s);
+		fused = fa != nullptr && fuse_pays(v, variant_update, plan.get(), *fa, s);
 	}
 	// the re-check's scratch, the accumulators (also those of a separate update that follows) and the
 	// padding of the operands derived from the means (workspace ranges are multiples of 256 bytes)
@@ -475,7 +480,7 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 	}
 	CUDA_TRY(cudaGetLastError());
 	if (fused_out) *fused_out = fused;
-	return enqueue_assign(v, points, means, assignment, s, w, 0, plan, 1.0f, sm_count, st, nullptr, fused ? fa : nullptr);
+	return enqueue_assign(v, points, means, assignment, s, w, 0, plan.get(), 1.0f, sm_count, st, nullptr, fused ? fa : nullptr);
 }
 
 static int stateless_update(const float* points, const uint32_t* assignment, float* means, uint32_t* sizes,

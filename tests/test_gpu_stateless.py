@@ -112,3 +112,40 @@ def test_one_workspace_serves_calls_with_different_numbers_of_means(pkg, torch_c
     pkg.update(dev.points.data_ptr(), dev.assignment.data_ptr(), dev.means_out.data_ptr(), dev.sizes.data_ptr(), n // 2, small, d, 0, layout,
                dev.ws_ptr, dev.ws_bytes_avail)
     assign(small)
+
+
+def test_threads_that_replace_each_others_plans(pkg, torch_cuda, oracle_mod):
+    """The library keeps eight tensor-core plans; three threads with six shapes each keep replacing the others'
+    while their calls are being enqueued, each on a stream and workspaces of its own."""
+    import threading
+    torch = torch_cuda
+    n = 700
+
+    def job(t, errors):
+        try:
+            torch.cuda.set_device(0)
+            stream = torch.cuda.Stream()
+            rng = np.random.default_rng(t)
+            work = []
+            for k, d in ((20 + t, 16), (40 + t, 32), (300 + t, 32), (300 + t, 64), (40 + t, 90), (1030 + t, 260)):
+                data, means = (rng.standard_normal(m * d).astype(np.float32) for m in (n, k))
+                work.append((k, d, DeviceArrays(torch, pkg, data, means, n, k, d), oracle_mod.assign(data, means, n, k, d, 0, 0, threads=2)))
+            torch.cuda.synchronize()
+            for _ in range(20):
+                for k, d, dev, _want in work:
+                    pkg.assign(dev.points.data_ptr(), dev.means.data_ptr(), dev.assignment.data_ptr(), n, k, d, 0, 0, dev.ws_ptr, dev.ws_bytes_avail,
+                               variant=pkg.ASSIGN_TC, stream=stream.cuda_stream)
+            stream.synchronize()
+            for k, d, dev, want in work:
+                if not np.array_equal(dev.asg_host(), want):
+                    errors.append((t, k, d))
+        except Exception as e:  # noqa: BLE001 - reported by the main thread
+            errors.append((t, repr(e)))
+
+    errors = []
+    threads = [threading.Thread(target=job, args=(t, errors)) for t in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
