@@ -460,14 +460,26 @@ __device__ __forceinline__ void scan_means(const float* sm, const float (&x)[D],
 	}
 }
 
+// Lowest (distance, index) over the `lanes` lanes of a point, for the first of them, which has seen mean 0.
+__device__ __forceinline__ void lowest_of_lanes(float& best, uint32_t& bidx, uint32_t lanes)
+{
+	for (uint32_t off = lanes >> 1; off > 0; off >>= 1) {
+		const float ob = __shfl_down_sync(0xffffffffu, best, off, lanes);
+		const uint32_t oi = __shfl_down_sync(0xffffffffu, bidx, off, lanes);
+		if (oi != 0xffffffffu && (ob < best || (ob == best && oi < bidx))) { best = ob; bidx = oi; }
+	}
+}
+
+// Floats of a mean's row for scan_means, which reads it as vectors of 4, 2 or 1: an odd number of vectors, so
+// that lanes on neighbouring means meet different banks.
+__host__ __device__ constexpr uint32_t scan_row_floats(uint32_t dim) { return dim % 8 == 0 ? dim + 4 : dim; }
+
 template<int D, bool SOA, bool SOAM>
 __global__ void __launch_bounds__(256) assign_exact_list_small_kernel(const float* __restrict__ pts, const float* __restrict__ means,
 	uint32_t* __restrict__ asg, uint64_t n, uint32_t k, const uint32_t* __restrict__ list, const uint32_t* __restrict__ list_count,
 	float* __restrict__ fix_acc, uint32_t* __restrict__ fix_counts)
 {
-	// [mean][dimension], read as vectors of VW floats; a row is an odd number of them, so that lanes on
-	// neighbouring means meet different banks
-	constexpr uint32_t VW = D % 4 == 0 ? 4 : (D % 2 == 0 ? 2 : 1), RS = (D / VW) % 2 == 0 ? D + VW : D;
+	constexpr uint32_t RS = scan_row_floats(D);
 	__shared__ __align__(16) float sm[(LIST_SMALL_MAX_FLOATS / D + LIST_SMALL_SUMS - 1) * RS];
 	uint64_t total = *list_count;
 	if (total > n) total = n;
@@ -494,12 +506,7 @@ __global__ void __launch_bounds__(256) assign_exact_list_small_kernel(const floa
 		// (one lane per point: the stride is a constant and the four rows are one address away from each other)
 		if (lanes == 1) scan_means<D, RS>(sm, x, k, 0u, 1u, best, best_sum, bidx);
 		else scan_means<D, RS>(sm, x, k, sub, lanes, best, best_sum, bidx);
-		// lowest (distance, index) over the lanes of the point; lane 0 of them has seen mean 0
-		for (uint32_t off = lanes >> 1; off > 0; off >>= 1) {
-			const float ob = __shfl_down_sync(0xffffffffu, best, off, lanes);
-			const uint32_t oi = __shfl_down_sync(0xffffffffu, bidx, off, lanes);
-			if (oi != 0xffffffffu && (ob < best || (ob == best && oi < bidx))) { best = ob; bidx = oi; }
-		}
+		lowest_of_lanes(best, bidx, lanes);
 		if (sub != 0 || w >= total) continue;
 		if (fix_acc) {
 			// the fast pass has already added this point to the sum of the cluster it picked
@@ -638,6 +645,7 @@ cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* 
 // exact kernel; the final assignment is the reference's for every point.
 
 constexpr int SIMT_THREADS = 256;
+constexpr int SIMT_EVAL_POINTS = 2;  // points that a thread evaluates at a time
 constexpr int SIMT_TILE_ROWS = 1024; // means per shared-memory tile (a multiple of the 32-mean chunk)
 
 // Fused update sums (FUSE): every WARP sorts the 32 * P points it has just assigned by cluster, in
@@ -673,31 +681,32 @@ __device__ __forceinline__ void send_row(float* dst, const float (&sum)[D], floa
 	}
 }
 
-// One point's cluster by the reference's arithmetic, by a whole warp (lanes over the means; every lane
-// gets the result): what the exact kernels do for the queued points.
-template<int D, bool SOA>
-__device__ __forceinline__ uint32_t exact_cluster(const float* __restrict__ pts, uint64_t i, uint64_t n, const float* __restrict__ means, int soa_means, uint32_t k)
+// The near-ties of a warp, `count` (1 to 32 * P) point indices in `buf`, settled by the reference's arithmetic
+// against all means in shared memory (`rows`, see scan_means); every index is replaced by its cluster.  A few
+// points get many lanes each, so that the warp is soon done with them; many points get one or two lanes
+// each, which costs what the list kernel costs.  (A whole warp per point, one after another, over means in
+// global memory made the pass up to 4.2 times as long where many points are near-ties.)
+template<int D, bool SOA, uint32_t RS>
+__device__ __forceinline__ void settle(const float* __restrict__ pts, uint64_t n, const float* rows, uint32_t k, uint32_t* buf, uint32_t count)
 {
-	float x[D];
-	#pragma unroll
-	for (int j = 0; j < D; ++j) x[j] = pts[at<SOA>(i, j, n, D)];
-	float best = INFINITY;
-	uint32_t bidx = 0xffffffffu;
-	for (uint32_t m = threadIdx.x & 31u; m < k; m += 32) {
-		float sum = 0.0f;
+	const uint32_t lane = threadIdx.x & 31u;
+	uint32_t lanes = 1;
+	while (lanes < 32 && 2 * lanes * LIST_SMALL_SUMS <= k && 2 * lanes * count <= 64) lanes *= 2;
+	const uint32_t sub = lane & (lanes - 1u), per_round = 32 / lanes;
+	for (uint32_t e0 = 0; e0 < count; e0 += per_round) {
+		const uint32_t e = e0 + lane / lanes;
+		const uint64_t i = buf[e < count ? e : e0];
+		__syncwarp();                      // (entry e0 is read by the lanes without a point as well)
+		float x[D];
 		#pragma unroll
-		for (int j = 0; j < D; ++j) {
-			const float diff = __fsub_rn(x[j], means[at_rt(soa_means, m, j, k, D)]);
-			sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-		}
-		const float dist = __fsqrt_rn(sum);
-		if (dist < best || (dist == best && m < bidx)) { best = dist; bidx = m; }
-		// what is not a number never wins, but nothing replaces it as the first distance of the sequential scan
-		if (m == 0 && dist != dist) { best = 0.0f; bidx = 0; }
+		for (int j = 0; j < D; ++j) x[j] = pts[at<SOA>(i, j, n, D)];
+		float best = INFINITY, best_sum = INFINITY;
+		uint32_t bidx = 0xffffffffu;
+		if (lanes == 1) scan_means<D, RS>(rows, x, k, 0u, 1u, best, best_sum, bidx);
+		else scan_means<D, RS>(rows, x, k, sub, lanes, best, best_sum, bidx);
+		lowest_of_lanes(best, bidx, lanes);
+		if (sub == 0 && e < count) buf[e] = bidx;
 	}
-	// distances are >= +0: their bit patterns order like the values
-	const uint32_t low = __reduce_min_sync(0xffffffffu, __float_as_uint(best));
-	return __reduce_min_sync(0xffffffffu, __float_as_uint(best) == low ? bidx : 0xffffffffu);
 }
 
 template<int D, bool SOA, int P, bool FUSE>
@@ -706,6 +715,8 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 	Control* __restrict__ ctl, int slot, uint32_t* __restrict__ flag_list, float margin_ulps, int vec_ok,
 	uint32_t k, float* __restrict__ fuse_acc, uint32_t* __restrict__ fuse_counts, const float* __restrict__ means, int soa_means)
 {
+	constexpr int Q = SIMT_EVAL_POINTS;          // points evaluated at a time
+	static_assert(P % Q == 0 && (FUSE || P == Q), "points per thread");
 	constexpr int RS = (D + 1 + 3) / 4 * 4;      // floats of a prepared row in global memory
 	extern __shared__ __align__(128) float tile[];  // rows of two means interleaved: (D + 1) pairs
 	// fused update sums: see above
@@ -718,7 +729,7 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 		fuse_acc_rep += (blockIdx.x % acc_replicas(k, D)) * acc_replica_stride(k, D);
 		for (uint32_t c = threadIdx.x; c < SIMT_FUSE_MAX_K; c += SIMT_THREADS) s_cnt[c] = 0;
 	}
-	__shared__ uint32_t flag_bufs[SIMT_THREADS / 32][FUSE ? 1 : FLAG_BUFFER];     // per warp: near-ties on their way to the list
+	__shared__ uint32_t flag_bufs[SIMT_THREADS / 32][FUSE ? 32 * P : FLAG_BUFFER];  // per warp: near-ties to be settled, or on their way to the list
 	uint32_t* flag_buf = flag_bufs[threadIdx.x >> 5];
 	uint32_t flag_cnt = 0;
 
@@ -760,6 +771,16 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 		return trows;
 	};
 
+	// fused: the means as they are, for the near-ties, and the rows of infinities that scan_means wants behind them
+	constexpr uint32_t MS = scan_row_floats(D);
+	float* s_means = tile + rows * (D + 1);      // (a single tile, see assign_simt_can_fuse)
+	if (FUSE) {
+		for (uint32_t e = tid; e < k * D; e += SIMT_THREADS) {
+			const uint32_t m = e / D, j = e - m * D;
+			s_means[m * MS + j] = means[at_rt(soa_means, m, j, k, D)];
+		}
+		for (uint32_t e = tid; e < (LIST_SMALL_SUMS - 1) * MS; e += SIMT_THREADS) s_means[k * MS + e] = INFINITY;
+	}
 	uint32_t trows0 = 0;
 	if (ntiles == 1) trows0 = load_tile(0);
 
@@ -810,90 +831,110 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 			#pragma unroll
 			for (int j = 0; j < D; ++j) x[p][j] = raw[p][j] - cen[j];
 		}
-		uint32_t spoilt = 0;           // points that hold an infinity or what is not a number: their keys mean nothing either
+		uint32_t near = 0;             // bit p: point p is a near-tie
 		#pragma unroll
 		for (int p = 0; p < P; ++p) {
+			// an infinity or what is not a number in the point: its keys mean nothing
 			float zero = 0.0f;
 			#pragma unroll
 			for (int j = 0; j < D; ++j) zero = fmaf(x[p][j], 0.0f, zero);
-			if (zero != 0.0f) spoilt |= 1u << p;
+			if (zero != 0.0f) near |= 1u << p;
 		}
-		uint64_t xx[P][D];
-		#pragma unroll
-		for (int p = 0; p < P; ++p)
-			#pragma unroll
-			for (int j = 0; j < D; ++j) xx[p][j] = ptx::pack2(x[p][j], x[p][j]);
 		if (blk + gridDim.x < nblocks) load_points(blk + gridDim.x);
-
-		uint32_t best[P], second[P], bchunk[P];
-		#pragma unroll
-		for (int p = 0; p < P; ++p) { best[p] = 0xFFFFFFFFu; second[p] = 0xFFFFFFFFu; bchunk[p] = 0; }
-
-		for (uint32_t t = 0; t < ntiles; ++t) {
-			uint32_t trows = trows0;
-			if (ntiles > 1) {
-				__syncthreads();   // everyone is done reading the previous tile
-				trows = load_tile(t);
-			}
-			const uint32_t chunk_base = t * (SIMT_TILE_ROWS / 32);
-			#pragma unroll 1
-			for (uint32_t ch = 0; ch < trows / 32; ++ch) {
-				uint32_t v[P][32];
-				const float4* rowp = reinterpret_cast<const float4*>(tile + (size_t)ch * 32 * (D + 1));
-				#pragma unroll
-				for (int m = 0; m < 32; m += 4) {
-					// four means = two interleaved pairs = D + 1 128-bit loads
-					float f[4 * (D + 1)];
-					#pragma unroll
-					for (int q = 0; q <= D; ++q) {
-						const float4 w = rowp[(m / 4) * (D + 1) + q];
-						f[4 * q + 0] = w.x; f[4 * q + 1] = w.y; f[4 * q + 2] = w.z; f[4 * q + 3] = w.w;
-					}
-					#pragma unroll
-					for (int h = 0; h < 2; ++h) {
-						const float* row = f + h * 2 * (D + 1);
-						#pragma unroll
-						for (int p = 0; p < P; ++p) {
-							uint64_t val = ptx::pack2(row[0], row[1]);
-							#pragma unroll
-							for (int j = 0; j < D; ++j) val = ptx::fma2(xx[p][j], ptx::pack2(row[2 * j + 2], row[2 * j + 3]), val);
-							ptx::unpack2(val, v[p][m + 2 * h], v[p][m + 2 * h + 1]);
-						}
-					}
-				}
-				#pragma unroll
-				for (int p = 0; p < P; ++p) chunk_update<false>(v[p], key_mult, chunk_base + ch, 32, best[p], second[p], bchunk[p]);
-			}
-		}
 
 		uint32_t cl[P];
 		#pragma unroll
-		for (int p = 0; p < P; ++p) {
-			bool flag = false;
-			cl[p] = k;                     // rows behind the last point sort behind every cluster
-			if (idx[p] < n) {
-				// key - key_base = M * mantissa + column
-				const uint32_t bm = div_key(best[p] - key_base, key_magic);
-				cl[p] = bchunk[p] * 32u + ((best[p] - key_base) - bm * key_mult);
-				if (!FUSE) asg[idx[p]] = cl[p];
-				const float gap = second[p] == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second[p] - key_base, key_magic) - bm);
-				flag = !(gap > margin);
-				flag = flag || (spoilt >> p & 1u) != 0;
-			}
-			if (FUSE) {
-				// a near-tie is settled on the spot, before the point is added anywhere: no list, no
-				// launch for it, and nothing to move from one sum to another
-				uint32_t mask = __ballot_sync(0xffffffffu, flag);
-				flag_cnt += (uint32_t)__popc(mask);
-				for (; mask != 0; mask &= mask - 1) {
-					const int src = __ffs(mask) - 1;
-					const uint32_t c = exact_cluster<D, SOA>(pts, __shfl_sync(0xffffffffu, (unsigned long long)idx[p], src), n, means, soa_means, k);
-					if ((int)(tid & 31u) == src) cl[p] = c;
+		for (int g = 0; g < P; g += Q) {
+			uint64_t xx[Q][D];
+			#pragma unroll
+			for (int p = 0; p < Q; ++p)
+				#pragma unroll
+				for (int j = 0; j < D; ++j) xx[p][j] = ptx::pack2(x[g + p][j], x[g + p][j]);
+
+			uint32_t best[Q], second[Q], bchunk[Q];
+			#pragma unroll
+			for (int p = 0; p < Q; ++p) { best[p] = 0xFFFFFFFFu; second[p] = 0xFFFFFFFFu; bchunk[p] = 0; }
+
+			for (uint32_t t = 0; t < ntiles; ++t) {
+				uint32_t trows = trows0;
+				if (ntiles > 1) {
+					__syncthreads();   // everyone is done reading the previous tile
+					trows = load_tile(t);
 				}
-				if (idx[p] < n) asg[idx[p]] = cl[p];
-			} else {
-				buffered_append(flag, (uint32_t)idx[p], flag_buf, flag_cnt, ctl, flag_list, n);
+				const uint32_t chunk_base = t * (SIMT_TILE_ROWS / 32);
+				#pragma unroll 1
+				for (uint32_t ch = 0; ch < trows / 32; ++ch) {
+					uint32_t v[Q][32];
+					const float4* rowp = reinterpret_cast<const float4*>(tile + (size_t)ch * 32 * (D + 1));
+					#pragma unroll
+					for (int m = 0; m < 32; m += 4) {
+						// four means = two interleaved pairs = D + 1 128-bit loads
+						float f[4 * (D + 1)];
+						#pragma unroll
+						for (int q = 0; q <= D; ++q) {
+							const float4 w = rowp[(m / 4) * (D + 1) + q];
+							f[4 * q + 0] = w.x; f[4 * q + 1] = w.y; f[4 * q + 2] = w.z; f[4 * q + 3] = w.w;
+						}
+						#pragma unroll
+						for (int h = 0; h < 2; ++h) {
+							const float* row = f + h * 2 * (D + 1);
+							#pragma unroll
+							for (int p = 0; p < Q; ++p) {
+								uint64_t val = ptx::pack2(row[0], row[1]);
+								#pragma unroll
+								for (int j = 0; j < D; ++j) val = ptx::fma2(xx[p][j], ptx::pack2(row[2 * j + 2], row[2 * j + 3]), val);
+								ptx::unpack2(val, v[p][m + 2 * h], v[p][m + 2 * h + 1]);
+							}
+						}
+					}
+					#pragma unroll
+					for (int p = 0; p < Q; ++p) chunk_update<false>(v[p], key_mult, chunk_base + ch, 32, best[p], second[p], bchunk[p]);
+				}
 			}
+
+			#pragma unroll
+			for (int p = 0; p < Q; ++p) {
+				cl[g + p] = k;                 // rows behind the last point sort behind every cluster
+				bool flag = false;
+				if (idx[g + p] < n) {
+					// key - key_base = M * mantissa + column
+					const uint32_t bm = div_key(best[p] - key_base, key_magic);
+					cl[g + p] = bchunk[p] * 32u + ((best[p] - key_base) - bm * key_mult);
+					if (!FUSE) asg[idx[g + p]] = cl[g + p];
+					const float gap = second[p] == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second[p] - key_base, key_magic) - bm);
+					flag = !(gap > margin) || (near >> (g + p) & 1u) != 0;
+				}
+				if (FUSE) near = flag ? near | 1u << (g + p) : near & ~(1u << (g + p));
+				else buffered_append(flag, (uint32_t)idx[g + p], flag_buf, flag_cnt, ctl, flag_list, n);
+			}
+		}
+
+		if (FUSE) {
+			// near-ties are settled on the spot, before the points are added anywhere: no list, no launch
+			// for it, and nothing to move from one sum to another
+			const uint32_t before = (1u << (tid & 31u)) - 1u;
+			uint32_t count = 0;
+			#pragma unroll
+			for (int p = 0; p < P; ++p) {
+				const uint32_t mask = __ballot_sync(0xffffffffu, (near >> p & 1u) != 0);
+				if (near >> p & 1u) flag_buf[count + (uint32_t)__popc(mask & before)] = (uint32_t)idx[p];
+				count += (uint32_t)__popc(mask);
+			}
+			if (count != 0) {
+				__syncwarp();
+				settle<D, SOA, MS>(pts, n, s_means, k, flag_buf, count);
+				__syncwarp();
+				flag_cnt += count;
+				count = 0;
+				#pragma unroll
+				for (int p = 0; p < P; ++p) {
+					const uint32_t mask = __ballot_sync(0xffffffffu, (near >> p & 1u) != 0);
+					if (near >> p & 1u) cl[p] = flag_buf[count + (uint32_t)__popc(mask & before)];
+					count += (uint32_t)__popc(mask);
+				}
+			}
+			#pragma unroll
+			for (int p = 0; p < P; ++p) if (idx[p] < n) asg[idx[p]] = cl[p];
 		}
 
 		if (FUSE) {
@@ -992,14 +1033,16 @@ bool assign_simt_can_fuse(const Shape& s, const FusedAcc& f)
 		(reinterpret_cast<uintptr_t>(f.acc) & 15u) == 0 && (f.rep_stride * sizeof(float)) % 16 == 0;
 }
 
-template<int D, int P>
+template<int D>
 static cudaError_t launch_simt_d(const float* pts, const float* means, const float* cprep, const float* center, uint32_t* asg, const Shape& s,
 	Control* ctl, int slot, uint32_t* flag_list, float margin_scale, int sm_count, cudaStream_t stream, const FusedAcc* fused)
 {
+	constexpr int FUSE_P = 2;
+	const int points = fused ? FUSE_P : SIMT_EVAL_POINTS;
 	const uint32_t rows = simt_rows(s.k);
 	const uint32_t trows = rows < (uint32_t)SIMT_TILE_ROWS ? rows : (uint32_t)SIMT_TILE_ROWS;
-	const size_t smem = (size_t)trows * (D + 1) * sizeof(float);
-	const uint64_t per_block = (uint64_t)SIMT_THREADS * P;
+	const size_t smem = ((size_t)trows * (D + 1) + (fused ? (size_t)(s.k + LIST_SMALL_SUMS - 1) * scan_row_floats(D) : 0)) * sizeof(float);
+	const uint64_t per_block = (uint64_t)SIMT_THREADS * points;
 	const uint64_t nblocks = (s.n + per_block - 1) / per_block;
 	// persistent grid: a whole number of resident blocks per SM
 	int per_sm = 1;
@@ -1009,7 +1052,7 @@ static cudaError_t launch_simt_d(const float* pts, const float* means, const flo
 	const float margin_ulps = margin_scale * (float)(4 * D + 16);
 	const int vec_ok = ((reinterpret_cast<uintptr_t>(pts) & 15u) == 0) ? 1 : 0;
 #define BKM_LAUNCH_SIMT(SOA, FUSE) do { \
-		auto kern = assign_simt_kernel<D, SOA, P, FUSE>; \
+		auto kern = assign_simt_kernel<D, SOA, FUSE ? FUSE_P : SIMT_EVAL_POINTS, FUSE>; \
 		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
 		if (e != cudaSuccess) return e; \
 		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SIMT_THREADS, smem); \
@@ -1031,14 +1074,14 @@ cudaError_t launch_assign_simt(const float* pts, const float* means, const SimtM
 	Control* ctl, int slot, uint32_t* flag_list, float margin_scale, int sm_count, cudaStream_t stream, const FusedAcc* fused)
 {
 	switch (s.dim) {
-	case 1: return launch_simt_d<1, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 2: return launch_simt_d<2, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 3: return launch_simt_d<3, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 4: return launch_simt_d<4, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 5: return launch_simt_d<5, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 6: return launch_simt_d<6, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 7: return launch_simt_d<7, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
-	case 8: return launch_simt_d<8, 2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 1: return launch_simt_d<1>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 2: return launch_simt_d<2>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 3: return launch_simt_d<3>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 4: return launch_simt_d<4>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 5: return launch_simt_d<5>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 6: return launch_simt_d<6>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 7: return launch_simt_d<7>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
+	case 8: return launch_simt_d<8>(pts, means, sm.rows, sm.center, asg, s, ctl, slot, flag_list, margin_scale, sm_count, stream, fused);
 	default: return cudaErrorInvalidValue;
 	}
 }

@@ -76,3 +76,34 @@ def test_sorted_update_at_chunk_edges(pkg, torch_cuda, oracle_mod, chunk, extra)
     assert np.array_equal(dev.sizes.cpu().numpy().view(np.uint32), want_sizes)
     ok, err = means_close(dev.means_out.cpu().numpy(), want)
     assert ok, err
+
+
+@pytest.mark.parametrize("share", [0.02, 0.3, 1.0])
+@pytest.mark.parametrize("n", [1, 130, 1100, 9000])
+@pytest.mark.parametrize("k,d", [(1, 3), (2, 1), (7, 2), (9, 8), (64, 4), (600, 2), (1000, 8), (1024, 5)])
+def test_near_ties_settled_in_the_fused_pass(pkg, torch_cuda, oracle_mod, n, k, d, share):
+    """From one near-tie per warp to all of its points, each with as many lanes as that leaves: a share of the
+    points lies at means that exist twice (the lower index wins), the others far from them."""
+    rng = np.random.default_rng(n + 3 * k + d)
+    centres = rng.random((k, d), dtype=np.float32)
+    half = k // 2
+    centres[half:2 * half:2] = centres[:half:2]            # every second mean of the first half exists twice
+    twice, once = np.arange(0, max(half, 1), 2), np.arange(1 if half > 1 else 0, max(half, 1), 2 if half > 1 else 1)
+    pick = np.where(rng.random(n) < share, rng.choice(twice, n), rng.choice(once, n))
+    rows = (centres[pick] + np.float32(1e-3) * rng.standard_normal((n, d)).astype(np.float32)).astype(np.float32)
+    lay, laym = (n + k) % 2, d % 2
+    data, means = rows_to_layout(rows, lay), rows_to_layout(centres, laym)
+    km = pkg.KMeans(layout=lay, layout_means=laym, variant_assign=pkg.ASSIGN_SIMT)
+    km.initialize(d, k, n, 1, data, means)
+    km.set_option("fuse_update", 2)
+    km.run(1)
+    got, cur, sizes, info = km.getAssignment(), km.getMeans(), km.getSizes(), km.counters()
+    km.cleanup()
+    assert info["update_variant"] == "fused"
+    want = oracle_mod.assign(data, means, n, k, d, lay, laym, threads=8)
+    assert np.array_equal(got, want), int((got != want).sum())
+    assert info["rechecked"] >= (np.isin(pick, twice).sum() if half > 1 else 0)
+    want_means, want_sizes = oracle_mod.update(data, want, n, k, d, lay, laym)
+    assert np.array_equal(sizes, want_sizes)
+    ok, err = means_close(cur, want_means)
+    assert ok, err
