@@ -432,9 +432,18 @@ static bkm::PointsKey* points_key(const Workspace& w)
 static bool fuse_pays(int assign_variant, int update_variant, const bkm::TcPlan* plan, const bkm::FusedAcc& fa, const bkm::Shape& s, bool force = false)
 {
 	if (assign_variant == BKM_ASSIGN_SIMT) {
-		// measured: the warp-private sort adds 0.11 ms to a 0.32 ms pass over 2^24 two-dimensional points
-		// where the separate sorted update takes 0.10 ms, so it pays only where a launch less does
-		return bkm::assign_simt_can_fuse(s, fa) && (force || (double)s.n * s.k * s.dim <= 1.0e8);
+		// The fused form saves two launches (5 us per iteration of a graph) and pays for it in three ways.  Its
+		// warps settle their near-ties one warp at a time: with more means (64 for one or two dimensions, where
+		// near-ties are frequent, else 128) the list kernel is faster where they are many (20 011 clustered points,
+		// d = 2, k = 128 / 256: 34 / 48 against 30 / 34 us; d = 8: 36 / 44 against 35 / 39).  A row of sums
+		// goes out as one reduction for d = 1, 2 and 4, two for d = 8 and d or d / 2 of them otherwise, and with
+		// few clusters all rows meet (10 clusters: d = 4, 2^20 points 53 against 54; d = 8, 2^18 points 41 against
+		// 38; d = 3, 2^16 points 25 against 28 but 2^18 40 against 33; d = 5, 2^20 points 202 against 53).  Its
+		// sorting costs more than a separate pass over many points, unless few clusters make the sorted runs
+		// long (d = 2, 2^22 points, 10 / 32 / 128 clusters: 77 / 126 / 174 against 111 / 110 / 186).
+		const uint32_t log_n = s.dim <= 2 ? (s.k <= 16 ? 22 : 20) : (s.dim == 4 ? 20 : (s.dim == 8 ? 18 : 16));
+		const bool pays = s.k <= (s.dim <= 2 ? 64u : 128u) && s.n <= (1ull << log_n);
+		return bkm::assign_simt_can_fuse(s, fa) && (force || pays);
 	}
 	if (assign_variant != BKM_ASSIGN_TC) return false;
 	return update_variant == BKM_UPDATE_ROWS && bkm::tc_plan_can_fuse(plan, fa) && (size_t)s.dim * sizeof(float) * 4 <= 120 * 1024;
@@ -453,7 +462,7 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 	bool fused = false;
 	bkm::PointsKey* key = points_key(w);
 	if (v == BKM_ASSIGN_SIMT) {
-		fused = fa != nullptr && fuse_pays(v, variant_update, nullptr, *fa, s, true);     // the caller asked for the one-pass form
+		fused = fa != nullptr && fuse_pays(v, variant_update, nullptr, *fa, s);
 	} else if (v == BKM_ASSIGN_TC) {
 		const char* err = nullptr;
 		plan = cached_plan(s, w, device, &err);

@@ -151,7 +151,7 @@ def test_small_dim_fused_update_matches_separate_update(pkg, torch_cuda, oracle_
     for fuse in (1, 0):
         km = pkg.KMeans(layout=layout, variant_assign=pkg.ASSIGN_SIMT)
         km.initialize(d, k, n, 3, data, means)
-        km.set_option("fuse_update", 2 * fuse)     # 2 = wherever possible (the default takes it for launch-bound sizes only)
+        km.set_option("fuse_update", 2 * fuse)     # 2 = wherever possible (the default takes it where it pays)
         km.set_option("use_graph", 0)
         prev = np.asarray(means, dtype=np.float32).reshape(-1).copy()
         for it in range(3):

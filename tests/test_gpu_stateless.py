@@ -50,7 +50,9 @@ def test_repeated_calls_reuse_the_workspace_and_notice_new_points(pkg, torch_cud
     (7001, 512, 24, 1, 0, False),      # same, no assignment output, other means layout
     (9000, 300, 20, 0, 0, True),       # row-major points: two passes
     (30000, 64, 2, 0, 0, True),        # CUDA cores: single pass (every warp sorts its points by cluster)
-    (12345, 200, 7, 1, 0, False),      # same, dimension-major points, no assignment output
+    (12345, 100, 7, 1, 0, False),      # same, dimension-major points, no assignment output
+    (12345, 200, 7, 1, 0, False),      # more means: two passes
+    (70000, 10, 3, 0, 0, True),        # more points in few clusters: two passes
     (5000, 2000, 3, 0, 0, True),       # CUDA cores, more means than the single pass takes: two passes
 ])
 def test_iterate_matches_oracle_iteration(pkg, torch_cuda, oracle_mod, n, k, d, layout, layout_means, want_asg):
