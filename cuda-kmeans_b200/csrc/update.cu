@@ -761,8 +761,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) update_rows_kernel(const float* 
 // same and sending one row of reductions when it changes.  The number of reductions drops by
 // about the number of points per cluster and chunk (8 for 256 clusters), and the sums reach the
 // accumulators pre-added in a fixed small tree, which also keeps the rounding error down.
-// A walker has four rows in flight, so few blocks leave the kernel waiting for memory: the chunk is the
-// largest of 2048, 1024 and 512 points that still gives four blocks per SM (sorted_chunk).
+// A chunk has 2048, 1024 or 512 points (sorted_chunk).
 
 constexpr uint32_t SORT_THREADS = 256;
 constexpr uint32_t SORT_MAX_K = 1024;
@@ -770,9 +769,17 @@ constexpr uint32_t SORT_SCAN = (SORT_MAX_K + 1 + SORT_THREADS - 1) / SORT_THREAD
 
 bool update_sorted_supported(const Shape& s) { return s.k <= SORT_MAX_K; }
 
-static uint32_t sorted_chunk(uint64_t n, int sm_count)
+// A walker has four rows in flight, so few blocks leave the kernel waiting for memory, but smaller chunks send
+// more reductions, and with few clusters these wait for one another.  Rows of up to 8 floats are bound by the
+// latter (us for chunks of 512 / 1024 / 2048 points, mean over 2 to 1024 clusters; d = 1: 100 000 points 14.5 /
+// 14.8 / 15.0, 300 000 17.5 / 15.6 / 15.0; d = 4, 4 clusters, 1.2 million: 48 / 49 / 35): 2048 points as soon as
+// two thirds of the SMs or so get a block.  Longer rows wait for memory until there are two and a half blocks
+// per SM (d = 512: 300 000 points 141 / 157 / 240, 500 000 207 / 204 / 258, 800 000 304 / 341 / 307; d = 32: 150 000
+// 16.6 / 17.8 / 20.8, 600 000 25.2 / 21.8 / 22.9, 1.2 million 45.9 / 43.1 / 41.9).
+static uint32_t sorted_chunk(uint64_t n, uint32_t dim, int sm_count)
 {
-	const uint64_t blocks = (uint64_t)sm_count * 4;
+	if (dim <= 8) return n >= (uint64_t)sm_count * 1024 ? 2048u : 512u;
+	const uint64_t blocks = (uint64_t)sm_count * 5 / 2;
 	return n >= blocks * 2048 ? 2048u : (n >= blocks * 1024 ? 1024u : 512u);
 }
 
@@ -979,7 +986,7 @@ void launch_update(const float* pts, const uint32_t* asg, float* acc, uint32_t* 
 		const uint32_t per_point = s.dim / (uint32_t)vw;
 		uint32_t dg = vw == 1 ? 2 : 1;              // lanes per point: the power of two that covers a row, at most 32
 		while (dg < 32 && dg < per_point) dg <<= 1;
-		const uint32_t chunk = sorted_chunk(s.n, sm_count);
+		const uint32_t chunk = sorted_chunk(s.n, s.dim, sm_count);
 		const uint64_t chunks = (s.n + chunk - 1) / chunk;
 		const uint32_t grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(chunks, 1), (uint64_t)sm_count * 8);
 		const size_t rep_stride = acc_replica_stride(s.k, s.dim);

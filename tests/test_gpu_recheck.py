@@ -58,12 +58,13 @@ def test_near_ties_of_two_and_of_more_means_in_the_k_loop(pkg, torch_cuda, oracl
     assert np.array_equal(_assign(pkg, torch_cuda, data, means, n, k, d, lay, laym, pkg.ASSIGN_TC), want)
 
 
-@pytest.mark.parametrize("chunk", [512, 1024, 2048])
+@pytest.mark.parametrize("blocks_x2,chunk,d", [(2, 512, 2), (1, 2048, 2), (2, 2048, 2), (2, 512, 16), (5, 512, 16), (5, 1024, 16), (5, 2048, 16)])
 @pytest.mark.parametrize("extra", [-1, 0, 1])
-def test_sorted_update_at_chunk_edges(pkg, torch_cuda, oracle_mod, chunk, extra):
-    """Sizes around four blocks per SM, where the chunk of the sorted update changes."""
+def test_sorted_update_at_chunk_edges(pkg, torch_cuda, oracle_mod, blocks_x2, chunk, d, extra):
+    """Half a block of 2048 points per SM (up to 8 dimensions) and two and a half blocks per SM (longer rows), where
+    the chunk of the sorted update changes, and full last chunks of each size."""
     sms = torch_cuda.cuda.get_device_properties(0).multi_processor_count
-    n, k, d = 4 * sms * chunk + extra, 9, 2
+    n, k = sms * blocks_x2 // 2 * chunk + extra, 9
     rng = np.random.default_rng(chunk + extra)
     rows = rng.random((n, d), dtype=np.float32)
     asg = rng.integers(0, k, n).astype(np.uint32)
