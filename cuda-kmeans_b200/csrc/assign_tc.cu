@@ -916,23 +916,37 @@ void tc_plan_allow_pair(TcPlan* plan, bool allow) { if (plan) plan->pair_allowed
 bool tc_plan_uses_pair(const TcPlan* plan) { return plan && plan->pair_ok && plan->pair_allowed; }
 
 // Where CTA pairs can run they serve what they are better at: the fused update sums, a range of the
-// points, and operand rows of 32 words (dim 33..64: 517 against 648 us for 2^21 points and 1024 means).
-// With 16-word rows the one-CTA kernel is the faster one (k = 512: 227 against 243 us, k = 1024: 427
-// against 440 us, 2^21 points of 32 dimensions).
-static bool launch_uses_pair(const TcPlan* p, bool fused, bool ranged) { return tc_plan_uses_pair(p) && (fused || ranged || p->tp.d_pad == TC_KCHUNK); }
+// points, operand rows of 32 words (dim 33..64: 517 against 648 us for 2^21 points and 1024 means), and three
+// or four mean tiles that are not full, whose padding costs the one-CTA kernel column masks (iterations with
+// 2^21 points, pair / one CTA: k = 900 d = 24 556 / 571, k = 700 d = 32 464 / 469; k = 300, two tiles, 360 / 351).
+// With 16-word rows and full tiles the one-CTA kernel is the faster one (k = 512: 227 against 243 us, k = 1024:
+// 427 against 440 us, 2^21 points of 32 dimensions).
+static bool launch_uses_pair(const TcPlan* p, bool fused, bool ranged)
+{
+	return tc_plan_uses_pair(p) && (fused || ranged || p->tp.d_pad == TC_KCHUNK || (p->s.k > 2 * TC_NT_MAX && p->s.k < p->tm.k_pad));
+}
 
 void tc_plan_destroy(TcPlan* plan) { delete plan; }
 
 // The pair kernel can accumulate the update sums when a point's row can go out as 128-bit vector
 // reductions: dim a multiple of 4 and 16-byte aligned accumulators.  The reductions take as long however
-// few the means are, so with up to three mean tiles they pay for a launch less only (2^21 points of 32
-// dimensions: k = 512 404 us against 227 + 106 apart, k = 1024 509 us against 427 + 91).
-constexpr uint64_t PAIR_FUSE_SMALL_N = 1ull << 19;
-constexpr uint32_t PAIR_FUSE_LARGE_K = 3 * TC_NT_MAX;
+// few the means are, while the pass itself gets shorter with them, so up to three mean tiles the fused form pays
+// for the launches it saves only, and the sooner the shorter the rows.  Iterations in us, fused / one-CTA pass
+// and update apart: four tiles (k = 900) 2^21 points d = 20 537 / 565, d = 32 551 / 579, 2^17 points 81 / 87;
+// three tiles (k = 768) 2^21 points d = 24 447 / 443, d = 32 497 / 454, 2^17 points d = 32 77 / 79; two tiles (k = 512)
+// 2^17 / 2^18 / 2^19 / 2^21 points d = 20 66 / 71, 86 / 87, 128 / 127, 362 / 340, d = 24 68 / 71, 89 / 87, 136 / 127,
+// 390 / 344, d = 32 72 / 71, 97 / 87, 149 / 129, 442 / 351.  (After an upload in chunks the sums of the first
+// iteration are hidden behind it, which is why the bound for d = 20 serves for d = 24 as well.)
+static bool pair_fuse_pays(const Shape& s)
+{
+	if (s.k > 3 * TC_NT_MAX) return true;
+	if (s.k > 2 * TC_NT_MAX) return s.dim <= 28 || s.n <= 1u << 17;
+	return s.n <= (s.dim <= 24 ? 3u << 17 : 1u << 17);
+}
 
 bool tc_plan_can_fuse(const TcPlan* p, const FusedAcc& f)
 {
-	return tc_plan_uses_pair(p) && (p->s.k > PAIR_FUSE_LARGE_K || p->s.n <= PAIR_FUSE_SMALL_N) && assign_tc_pair_can_fuse(p->tm.k_pad, p->s.dim, p->tp.d_pad) && f.acc != nullptr && f.counts != nullptr && f.points != nullptr &&
+	return tc_plan_uses_pair(p) && pair_fuse_pays(p->s) && assign_tc_pair_can_fuse(p->tm.k_pad, p->s.dim, p->tp.d_pad) && f.acc != nullptr && f.counts != nullptr && f.points != nullptr &&
 		(reinterpret_cast<uintptr_t>(f.acc) & 15u) == 0 && (f.rep_stride * sizeof(float)) % 16 == 0;
 }
 

@@ -114,13 +114,21 @@ def test_variants_agree(pkg, torch_cuda, oracle_mod, workloads):
         assert ok, err
 
 
-@pytest.mark.parametrize("n,k,d,layout", [
-    (5000, 1024, 32, 1),      # four mean tiles, ragged last point tile, odd number of tiles
-    (4224, 300, 20, 0),       # k padded to 512: masked columns; dim padded to 32
-    (3000, 700, 12, 1),       # 16-float rows: one-CTA kernel either way
-    (130, 1000, 17, 0),       # fewer point tiles than SMs
+@pytest.mark.parametrize("n,k,d,layout,rows_update,pairs", [
+    (5000, 1024, 32, 1, True, True),     # with the fused sums: four full mean tiles, ragged last point tile, odd number of tiles
+    (4224, 300, 20, 0, True, True),      # k padded to 512: masked columns; dim padded to 32; row-major points
+    (4224, 300, 20, 0, False, False),    # two padded tiles and separate sums: one CTA either way
+    (3000, 700, 12, 1, True, False),     # 16-word rows with one K step per product: one-CTA kernel either way
+    (130, 1000, 17, 0, False, True),     # fewer point tiles than SMs
+    (130, 1000, 24, 0, True, True),      # fewer point tiles than SMs
+    (8000, 1024, 32, 0, False, False),   # full tiles and separate sums: one CTA either way
+    (4224, 700, 17, 0, False, True),     # three padded mean tiles, separate sums
+    (9000, 1000, 30, 1, True, True),     # four of them; a row of 30 floats does not go out as vectors
+    (4224, 300, 40, 0, False, True),     # 32-word rows
+    (777, 257, 33, 1, False, True),
+    (20000, 1024, 64, 1, False, True),
 ])
-def test_tc_pair_kernel_matches_single_cta_kernel(pkg, torch_cuda, oracle_mod, workloads, n, k, d, layout):
+def test_tc_pair_kernel_matches_single_cta_kernel(pkg, torch_cuda, oracle_mod, workloads, n, k, d, layout, rows_update, pairs):
     """The CTA-pair tensor-core kernel and the one-CTA kernel must both give the oracle's
     assignment (bit-exact) for the same means."""
     rows = workloads.generate_rows("mixture", n, d, 64, seed=11, sigma=0.05)
@@ -129,10 +137,11 @@ def test_tc_pair_kernel_matches_single_cta_kernel(pkg, torch_cuda, oracle_mod, w
     data, means = workloads.to_layout(rows, layout), workloads.to_layout(mrows, layout)
     want = oracle_mod.assign(data, means, n, k, d, layout, layout, threads=8)
     for pair in (0, 1):
-        km = pkg.KMeans(layout=layout, variant_assign=pkg.ASSIGN_TC)
+        km = pkg.KMeans(layout=layout, variant_assign=pkg.ASSIGN_TC, variant_update=pkg.UPDATE_ROWS if rows_update else pkg.UPDATE_SORTED)
         km.initialize(d, k, n, 1, data, means)
         km.set_option("tc_pair", pair)
         km.set_option("use_graph", 0)
+        assert km.assign_plan()["kernel"] == ("tc_pair" if pair and pairs else "tc_resident")
         km.run(1)
         got = km.getAssignment()
         km.cleanup()
@@ -168,15 +177,16 @@ def test_small_dim_fused_update_matches_separate_update(pkg, torch_cuda, oracle_
         km.cleanup()
 
 
-@pytest.mark.parametrize("n,k,d,layout", [(20000, 1024, 32, 1), (4224, 300, 20, 0), (777, 512, 24, 1)])
-def test_fused_update_matches_separate_update(pkg, torch_cuda, oracle_mod, workloads, n, k, d, layout):
+@pytest.mark.parametrize("n,k,d,layout,rows_update", [(20000, 1024, 32, 1, False), (4224, 300, 20, 0, False), (777, 512, 24, 1, False),
+                                                      (9001, 700, 28, 0, True), (4224, 300, 20, 0, True)])
+def test_fused_update_matches_separate_update(pkg, torch_cuda, oracle_mod, workloads, n, k, d, layout, rows_update):
     """The CTA-pair kernel can accumulate the update sums itself; means, sizes and assignment must
     agree with the run that uses the separate update pass, and with the oracle step by step."""
     rows = workloads.generate_rows("mixture", n, d, 64, seed=13, sigma=0.05)
     data, means = workloads.to_layout(rows, layout), workloads.to_layout(np.ascontiguousarray(rows[:k]), layout)
     outs = []
     for fuse in (1, 0):
-        km = pkg.KMeans(layout=layout, variant_assign=pkg.ASSIGN_TC)
+        km = pkg.KMeans(layout=layout, variant_assign=pkg.ASSIGN_TC, variant_update=pkg.UPDATE_ROWS if rows_update else pkg.UPDATE_AUTO)
         km.initialize(d, k, n, 3, data, means)
         km.set_option("fuse_update", fuse)
         km.set_option("use_graph", 0)
@@ -191,8 +201,8 @@ def test_fused_update_matches_separate_update(pkg, torch_cuda, oracle_mod, workl
             ok, err = means_close(cur, want)
             assert ok, (fuse, it, err)
             prev = cur
-        # fusion replaces the row-wise update only (dimension-major points)
-        assert (km.counters()["update_variant"] == "fused") == (fuse == 1 and layout == 1)
+        # fusion replaces the row-wise update only (the default of dimension-major points)
+        assert (km.counters()["update_variant"] == "fused") == (fuse == 1 and (layout == 1 or rows_update))
         outs.append(prev)
         km.cleanup()
 
