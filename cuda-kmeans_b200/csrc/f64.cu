@@ -51,59 +51,78 @@ __global__ void __launch_bounds__(256) assign_exact_f64_kernel(const double* __r
 	}
 }
 
-// Up to 32 dimensions: one THREAD per point, its coordinates in registers, the means in shared memory
-// (a tile of them at a time, every row read by the whole block at once), rows padded with zeros to DP
-// dimensions - a zero difference adds +0 and changes no bit.  The square root is taken only of sums
-// below the best sum: the correctly rounded root never decreases with its argument, so no other
-// candidate can be strictly smaller (equal roots of different sums keep the earlier mean, as the
-// reference's comparison does).  Bound by the fp64 pipe (three operations per coordinate); the form
-// with a warp per point that serves longer rows spends its time on loading the means again for every
-// point and on the reduction over the lanes.
+// Up to 32 dimensions: a THREAD per point, its coordinates in registers, the means in shared memory (a tile
+// of them at a time), rows padded with zeros to DP dimensions - a zero difference adds +0 and changes no
+// bit.  The square root is taken only of sums below the best sum: the correctly rounded root never decreases
+// with its argument, so no other candidate can be strictly smaller (equal roots of different sums keep the
+// earlier mean, as the reference's comparison does).  Bound by the fp64 pipe (three operations per
+// coordinate) where there are enough points.  Few points give too few threads, each in a chain of dependent
+// additions through all means: a point then gets 2 to 32 `lanes`, each of which walks every 2nd to 32nd mean
+// (see f64_lanes; iterations with 2000 points,
+// d = 2, k = 256: 48 us with one lane, 25 us now; 500 points, d = 32: 107 and 27 us).  The form with a warp per point that serves longer rows
+// spends its time on loading the means again for every point.
 constexpr uint32_t F64_TILE_DOUBLES = 4096;
 
 template<int DP, bool SOA>
 __global__ void __launch_bounds__(256) assign_f64_kernel(const double* __restrict__ pts, const double* __restrict__ means,
-	uint32_t* __restrict__ asg, uint64_t n, uint32_t k, uint32_t d, int soa_means)
+	uint32_t* __restrict__ asg, uint64_t n, uint32_t k, uint32_t d, int soa_means, uint32_t lanes)
 {
-	constexpr uint32_t TILE = F64_TILE_DOUBLES / DP;
+	// a row is an odd number of 16-byte vectors, so that lanes on neighbouring means meet different banks
+	constexpr uint32_t RS = (DP / 2) % 2 == 0 ? DP + 2 : DP, TILE = F64_TILE_DOUBLES / RS;
 	__shared__ __align__(16) double sm[F64_TILE_DOUBLES];
-	for (uint64_t i0 = (uint64_t)blockIdx.x * 256; i0 < n; i0 += (uint64_t)gridDim.x * 256) {
-		const uint64_t i = i0 + threadIdx.x;
+	const uint32_t sub = threadIdx.x & (lanes - 1u), per_block = 256 / lanes;
+	for (uint64_t i0 = (uint64_t)blockIdx.x * per_block; i0 < n; i0 += (uint64_t)gridDim.x * per_block) {
+		const uint64_t i = i0 + threadIdx.x / lanes;
 		double x[DP];
 		#pragma unroll
 		for (uint32_t j = 0; j < DP; ++j) x[j] = (i < n && j < d) ? pts[at<SOA>(i, j, n, d)] : 0.0;
-		double best = 0.0, best_sum = 0.0;
-		uint32_t bidx = 0;
+		double best = INFINITY, best_sum = INFINITY;
+		uint32_t bidx = 0xffffffffu;
 		for (uint32_t m0 = 0; m0 < k; m0 += TILE) {
 			const uint32_t rows = k - m0 < TILE ? k - m0 : TILE;
-			if (k > TILE || i0 == (uint64_t)blockIdx.x * 256) {          // a single tile stays
+			if (k > TILE || i0 == (uint64_t)blockIdx.x * per_block) {          // a single tile stays
 				__syncthreads();
 				for (uint32_t e = threadIdx.x; e < rows * DP; e += 256) {
 					const uint32_t m = e / DP, j = e % DP;
-					sm[e] = j < d ? means[at_rt(soa_means, m0 + m, j, k, d)] : 0.0;
+					sm[m * RS + j] = j < d ? means[at_rt(soa_means, m0 + m, j, k, d)] : 0.0;
 				}
 				__syncthreads();
 			}
-			for (uint32_t m = 0; m < rows; ++m) {
+			for (uint32_t m = sub; m < rows; m += lanes) {
 				double sum = 0.0;
 				#pragma unroll
 				for (uint32_t j = 0; j < DP; j += 2) {
-					const double2 c = *reinterpret_cast<const double2*>(&sm[m * DP + j]);
+					const double2 c = *reinterpret_cast<const double2*>(&sm[m * RS + j]);
 					const double d0 = __dsub_rn(x[j], c.x), d1 = __dsub_rn(x[j + 1], c.y);
 					sum = __dadd_rn(sum, __dmul_rn(d0, d0));
 					sum = __dadd_rn(sum, __dmul_rn(d1, d1));
 				}
-				if (m0 + m == 0) {
+				if (m0 + m == 0) {                      // taken whatever its distance, as in the sequential scan
 					best_sum = sum;
 					best = __dsqrt_rn(sum);
+					bidx = 0;
 				} else if (sum < best_sum) {
 					const double dist = __dsqrt_rn(sum);
 					if (dist < best) { best = dist; best_sum = sum; bidx = m0 + m; }
 				}
 			}
 		}
-		if (i < n) asg[i] = bidx;
+		// lowest (distance, index) over the lanes of the point, for the first of them, which has seen mean 0
+		for (uint32_t off = lanes >> 1; off > 0; off >>= 1) {
+			const double ob = __shfl_down_sync(0xffffffffu, best, off, lanes);
+			const uint32_t oi = __shfl_down_sync(0xffffffffu, bidx, off, lanes);
+			if (oi != 0xffffffffu && (ob < best || (ob == best && oi < bidx))) { best = ob; bidx = oi; }
+		}
+		if (sub == 0 && i < n) asg[i] = bidx;
 	}
+}
+
+// Lanes per point: as many as fill the machine with 1024 threads per SM, and at least two means for each.
+static uint32_t f64_lanes(uint64_t n, uint32_t k, int sms)
+{
+	uint32_t lanes = 1;
+	while (lanes < 32 && 4 * lanes <= k && n * lanes * 2 <= (uint64_t)sms * 1024) lanes *= 2;
+	return lanes;
 }
 
 // sums[c][:] += x_i, sizes[c] += 1 (row-major sums, zero on entry); one thread per coordinate.  The
@@ -189,15 +208,16 @@ extern "C" int bkm_kmeans_host_f64(const double* host_points, double* means, uin
 		F64_TRY(cudaMemsetAsync(d_sums, 0, off_asg - off_sums));
 		const size_t smem = (size_t)8 * dim * sizeof(double);
 		const uint32_t grid_a = (uint32_t)std::min<uint64_t>((n + 7) / 8, (uint64_t)sms * 16);
-		const uint32_t grid_t = (uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 16);
+		const uint32_t lanes = bkm::f64_lanes(n, k, sms);
+		const uint32_t grid_t = (uint32_t)std::min<uint64_t>((n * lanes + 255) / 256, (uint64_t)sms * 16);
 		const uint32_t grid_u = (uint32_t)std::min<uint64_t>((nd + 255) / 256, (uint64_t)sms * 16);
 		const uint32_t grid_d = (uint32_t)std::min<uint64_t>(((uint64_t)k + 7) / 8, (uint64_t)sms * 8);
 		int cur = 0;
 		for (uint32_t it = 0; it < iters; ++it) {
 			const int next = cur ^ 1;
 #define F64_ASSIGN(DP) do { \
-				if (soa) bkm::assign_f64_kernel<DP, true><<<grid_t, 256>>>(d_pts, d_means[cur], d_asg, n, k, dim, soam); \
-				else bkm::assign_f64_kernel<DP, false><<<grid_t, 256>>>(d_pts, d_means[cur], d_asg, n, k, dim, soam); \
+				if (soa) bkm::assign_f64_kernel<DP, true><<<grid_t, 256>>>(d_pts, d_means[cur], d_asg, n, k, dim, soam, lanes); \
+				else bkm::assign_f64_kernel<DP, false><<<grid_t, 256>>>(d_pts, d_means[cur], d_asg, n, k, dim, soam, lanes); \
 			} while (0)
 #define F64_ASSIGN_LONG(SOA, SOAM) do { \
 				auto ka = bkm::assign_exact_f64_kernel<SOA, SOAM>; \
