@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) assign_exact_f64_kernel(const double* __r
 // coordinate) where there are enough points.  Few points give too few threads, each in a chain of dependent
 // additions through all means: a point then gets 2 to 32 `lanes`, each of which walks every 2nd to 32nd mean
 // (see f64_lanes; iterations with 2000 points,
-// d = 2, k = 256: 48 us with one lane, 25 us now; 500 points, d = 32: 107 and 27 us).  The form with a warp per point that serves longer rows
+// d = 2, k = 256: 48 us with one lane, 14 us now; 500 points, d = 32: 107 and 25 us).  The form with a warp per point that serves longer rows
 // spends its time on loading the means again for every point.
 constexpr uint32_t F64_TILE_DOUBLES = 4096;
 
@@ -159,12 +159,15 @@ __global__ void __launch_bounds__(256) divide_f64_kernel(double* __restrict__ su
 		count = __reduce_add_sync(0xffffffffu, count);
 		if (lane < replicas) sizes[(size_t)lane * k + c] = 0u;
 		for (uint32_t j = lane; j < d; j += 32) {
-			double sum = 0.0;
-			#pragma unroll 4
-			for (uint32_t r = 0; r < replicas; ++r) {
-				double* src = sums + ((size_t)r * k + c) * d + j;
-				sum += *src;
-				*src = 0.0;
+			// all copies on their way together, cleared only after that (one after another: 14 us for 256 x 2)
+			double part[F64_REPLICAS], sum = 0.0;
+			double* src = sums + (size_t)c * d + j;
+			#pragma unroll
+			for (uint32_t r = 0; r < F64_REPLICAS; ++r) part[r] = r < replicas ? src[(size_t)r * k * d] : 0.0;
+			#pragma unroll
+			for (uint32_t r = 0; r < F64_REPLICAS; ++r) {
+				sum += part[r];
+				if (r < replicas) src[(size_t)r * k * d] = 0.0;
 			}
 			means[at_rt(soa_means, c, j, k, d)] = count ? __ddiv_rn(sum, (double)count) : 0.0;
 		}
