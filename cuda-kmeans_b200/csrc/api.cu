@@ -151,7 +151,6 @@ Workspace carve(char* base, uint64_t n, uint32_t k, uint32_t dim, bool with_tc_p
 	w.tm_bytes = 2 * align256(plane);
 	w.tm.b_hi = reinterpret_cast<float*>(take(plane));
 	w.tm.b_lo = reinterpret_cast<float*>(take(plane));
-	w.tm.cnorm = reinterpret_cast<float*>(take((size_t)w.tm.k_pad * sizeof(float)));
 	w.tm.b_aug = reinterpret_cast<float*>(take((size_t)w.tm.k_pad * 8 * sizeof(float)));
 	w.tm.center = reinterpret_cast<float*>(take((size_t)dim * sizeof(float)));
 	w.sm.center = w.tm.center;
@@ -164,8 +163,9 @@ Workspace carve(char* base, uint64_t n, uint32_t k, uint32_t dim, bool with_tc_p
 		w.tp.a_hi = reinterpret_cast<float*>(take(aplane));
 		w.tp.a_lo = reinterpret_cast<float*>(take(aplane));
 		w.tp.xnorm = reinterpret_cast<float*>(take((size_t)w.tp.n_pad * sizeof(float)));
-		w.tp.partial = w.tp.d_pad > 32 ? reinterpret_cast<uint32_t*>(take((size_t)bkm::TC_JSPLIT * 5 * w.tp.n_pad * sizeof(uint32_t))) : nullptr;
-		w.tp.pairs = w.tp.d_pad > 32 ? reinterpret_cast<uint32_t*>(take(2 * n * sizeof(uint32_t))) : nullptr;
+		const uint32_t words = bkm::tc_partial_words(k, dim);
+		if (words) w.tp.partial = reinterpret_cast<uint32_t*>(take((size_t)bkm::TC_JSPLIT * words * w.tp.n_pad * sizeof(uint32_t)));
+		if (words == 5) w.tp.pairs = reinterpret_cast<uint32_t*>(take(2 * n * sizeof(uint32_t)));
 	}
 	w.bytes = off;
 	return w;
@@ -571,7 +571,7 @@ int bkm_iterate_f32(const float* points, const float* means_in, float* means_out
 	// otherwise be the row-wise kernel) the points are read once.
 	int vu = 0;
 	if ((rc = resolve_update(variant_update, s, device, &vu))) return rc;
-	bkm::FusedAcc fa{w.acc, w.counts, w.replicas, bkm::acc_replica_stride(k, dim), w.tm.center, points, s.soa};
+	bkm::FusedAcc fa{w.acc, w.counts, w.replicas, bkm::acc_replica_stride(k, dim), points, s.soa};
 	bool fused = false;
 	rc = stateless_assign(points, means_in, asg, s, w, variant_assign, device, sm, st, &fa, vu, &fused);
 	if (rc) return rc;
@@ -898,7 +898,7 @@ static int upload_and_split(bkm_handle_t h, const float* host_points)
 	for (cudaEvent_t& e : h->copy_ev)
 		if (!e) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
 	const uint64_t chunk = bkm::round_up64((s.n + bkm_handle_s::UPLOAD_CHUNKS - 1) / bkm_handle_s::UPLOAD_CHUNKS, 4096);
-	bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(s.k, s.dim), h->ws.tm.center, h->d_points, s.soa};
+	bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(s.k, s.dim), h->d_points, s.soa};
 	bool fused = false, early_pass = false;
 	// the copies must not overtake the clearing of the workspace and of what the previous use left in the planes' consumers
 	CUDA_TRY(cudaEventRecord(h->copy_ev[0], h->stream));
@@ -1030,7 +1030,7 @@ static int enqueue_iteration(bkm_handle_t h, cudaEvent_t* ev)
 	if (ev) CUDA_TRY(cudaEventRecord(ev[0], st));
 	// The CTA-pair tensor-core pass and the CUDA-core pass can add every point to its cluster's sum on
 	// the way (the accumulators are zero between iterations: the finalize pass clears what it has read).
-	bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(s.k, s.dim), h->ws.tm.center, h->d_points, s.soa};
+	bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(s.k, s.dim), h->d_points, s.soa};
 	const bool fused = h->fuse_update && fuse_pays(h->assign_variant, h->update_variant, h->plan, fa, s, h->fuse_update >= 2);
 	h->last_fused = fused;
 	h->launches_per_iter = (h->assign_variant == BKM_ASSIGN_EXACT || (h->assign_variant == BKM_ASSIGN_SIMT && fused) ? 1u : 2u) + (fused ? 0u : 1u) + 1u;
@@ -1310,7 +1310,7 @@ int bkm_assign_plan(bkm_handle_t h, uint32_t out[4])
 	else if (h->assign_variant == BKM_ASSIGN_SIMT) out[0] = BKM_PLAN_SIMT;
 	else {
 		if (!h->plan) return fail(BKM_ERR_STATE, "the tensor-core plan exists after initialize only");
-		const bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(h->shape.k, h->shape.dim), h->ws.tm.center, h->d_points, h->shape.soa};
+		const bkm::FusedAcc fa{h->ws.acc, h->ws.counts, h->ws.replicas, bkm::acc_replica_stride(h->shape.k, h->shape.dim), h->d_points, h->shape.soa};
 		bkm::tc_plan_describe(h->plan, h->fuse_update && fuse_pays(h->assign_variant, h->update_variant, h->plan, fa, h->shape, h->fuse_update >= 2), out);
 	}
 	out[3] = h->last_fused ? 1u : 0u;

@@ -476,8 +476,7 @@ __host__ __device__ constexpr uint32_t scan_row_floats(uint32_t dim) { return di
 
 template<int D, bool SOA, bool SOAM>
 __global__ void __launch_bounds__(256) assign_exact_list_small_kernel(const float* __restrict__ pts, const float* __restrict__ means,
-	uint32_t* __restrict__ asg, uint64_t n, uint32_t k, const uint32_t* __restrict__ list, const uint32_t* __restrict__ list_count,
-	float* __restrict__ fix_acc, uint32_t* __restrict__ fix_counts)
+	uint32_t* __restrict__ asg, uint64_t n, uint32_t k, const uint32_t* __restrict__ list, const uint32_t* __restrict__ list_count)
 {
 	constexpr uint32_t RS = scan_row_floats(D);
 	__shared__ __align__(16) float sm[(LIST_SMALL_MAX_FLOATS / D + LIST_SMALL_SUMS - 1) * RS];
@@ -512,36 +511,21 @@ __global__ void __launch_bounds__(256) assign_exact_list_small_kernel(const floa
 		else scan_means<D, RS>(sm, x, k, sub, lanes, best, best_sum, bidx);
 		lowest_of_lanes(best, bidx, lanes);
 		if (sub != 0 || w >= total) continue;
-		if (fix_acc) {
-			// the fast pass has already added this point to the sum of the cluster it picked
-			const uint32_t from = asg[i];
-			if (from != bidx) {
-				#pragma unroll
-				for (int j = 0; j < D; ++j) {
-					if (from < k) atomicAdd(&fix_acc[(size_t)from * D + j], -x[j]);
-					atomicAdd(&fix_acc[(size_t)bidx * D + j], x[j]);
-				}
-				if (from < k) atomicSub(&fix_counts[from], 1u);
-				atomicAdd(&fix_counts[bidx], 1u);
-			}
-		}
 		asg[i] = bidx;
 	}
 }
 
 template<int D>
 static cudaError_t launch_list_small(const float* pts, const float* means, uint32_t* asg, const Shape& s,
-	const uint32_t* list, const uint32_t* list_count, int sm_count, cudaStream_t stream, const FusedAcc* fix)
+	const uint32_t* list, const uint32_t* list_count, int sm_count, cudaStream_t stream)
 {
 	// a thread's point is a dependent gather behind its list entry: many threads in flight hide that,
 	// so a long list gets one or two points per thread rather than a loop
 	const uint32_t grid = (uint32_t)sm_count * 16;
-	float* fa = fix ? fix->acc : nullptr;
-	uint32_t* fc = fix ? fix->counts : nullptr;
-	if (s.soa && s.soa_means) assign_exact_list_small_kernel<D, true, true><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, list, list_count, fa, fc);
-	else if (s.soa) assign_exact_list_small_kernel<D, true, false><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, list, list_count, fa, fc);
-	else if (s.soa_means) assign_exact_list_small_kernel<D, false, true><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, list, list_count, fa, fc);
-	else assign_exact_list_small_kernel<D, false, false><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, list, list_count, fa, fc);
+	if (s.soa && s.soa_means) assign_exact_list_small_kernel<D, true, true><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, list, list_count);
+	else if (s.soa) assign_exact_list_small_kernel<D, true, false><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, list, list_count);
+	else if (s.soa_means) assign_exact_list_small_kernel<D, false, true><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, list, list_count);
+	else assign_exact_list_small_kernel<D, false, false><<<grid, 256, 0, stream>>>(pts, means, asg, s.n, s.k, list, list_count);
 	return cudaGetLastError();
 }
 
@@ -556,24 +540,25 @@ cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* 
 	unsigned long long* split_keys = reinterpret_cast<unsigned long long*>(split_scratch);
 	uint32_t* split_arrive = split_scratch ? reinterpret_cast<uint32_t*>(split_keys + (size_t)LIST_SPLIT_MAX_BLOCKS * LIST_PB_WIDE) : nullptr;
 	if (fix != nullptr && (list == nullptr || (size_t)s.dim * sizeof(float) * LIST_PB > 120 * 1024)) return cudaErrorInvalidValue;
-	if (list != nullptr && s.dim <= LIST_SMALL_MAX_DIM && (uint64_t)s.k * s.dim <= LIST_SMALL_MAX_FLOATS) {
+	// (the passes that leave sums to be corrected, `fix`, serve longer rows or settle their near-ties themselves)
+	if (list != nullptr && fix == nullptr && s.dim <= LIST_SMALL_MAX_DIM && (uint64_t)s.k * s.dim <= LIST_SMALL_MAX_FLOATS) {
 		switch (s.dim) {
-		case 1: return launch_list_small<1>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 2: return launch_list_small<2>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 3: return launch_list_small<3>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 4: return launch_list_small<4>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 5: return launch_list_small<5>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 6: return launch_list_small<6>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 7: return launch_list_small<7>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 8: return launch_list_small<8>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 9: return launch_list_small<9>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 10: return launch_list_small<10>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 11: return launch_list_small<11>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 12: return launch_list_small<12>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 13: return launch_list_small<13>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 14: return launch_list_small<14>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		case 15: return launch_list_small<15>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
-		default: return launch_list_small<16>(pts, means, asg, s, list, list_count, sm_count, stream, fix);
+		case 1: return launch_list_small<1>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 2: return launch_list_small<2>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 3: return launch_list_small<3>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 4: return launch_list_small<4>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 5: return launch_list_small<5>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 6: return launch_list_small<6>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 7: return launch_list_small<7>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 8: return launch_list_small<8>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 9: return launch_list_small<9>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 10: return launch_list_small<10>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 11: return launch_list_small<11>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 12: return launch_list_small<12>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 13: return launch_list_small<13>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 14: return launch_list_small<14>(pts, means, asg, s, list, list_count, sm_count, stream);
+		case 15: return launch_list_small<15>(pts, means, asg, s, list, list_count, sm_count, stream);
+		default: return launch_list_small<16>(pts, means, asg, s, list, list_count, sm_count, stream);
 		}
 	}
 	if (list != nullptr && (size_t)s.dim * sizeof(float) * LIST_PB <= 120 * 1024) {

@@ -81,6 +81,15 @@ constexpr uint32_t SM_ALLOC = SM_TOTAL + 1024;                   // slack for 10
 uint32_t tc_nt_cols(uint32_t k) { return k >= TC_NT_MAX ? TC_NT_MAX : round_up(k, 32); }
 uint32_t tc_kpad(uint32_t k) { return round_up(k, tc_nt_cols(k)); }
 
+// The three-key form costs the epilogue a third more minima; it pays where the multiplication is long
+// enough to make that small and the exact pass over all means long enough to matter (2^20 x 512 against
+// 4096: the pass 8.70 -> 9.06 ms, the re-check of 4400 points 1.49 -> 0.09 ms).
+uint32_t tc_partial_words(uint32_t k, uint32_t dim)
+{
+	if (tc_dpad(dim) <= TC_KCHUNK || tc_kpad(k) / tc_nt_cols(k) < 2 * TC_JSPLIT) return 0;
+	return dim >= 256 ? 5 : 3;
+}
+
 bool assign_tc_supported(const Shape& s)
 {
 	return s.dim <= 4096 && tc_kpad(s.k) <= TC_MAX_KPAD && s.n < (1ull << 32) - 1024;
@@ -601,12 +610,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 							}
 							ptx::tc_fence_after();
 							const uint32_t base = ptx::smem_u32(smem + s * KL_STAGE_BYTES);
-							const uint64_t b_hi = make_desc_kw(base + KL_B_OFF, KL_KW), b_lo = make_desc_kw(base + KL_B_OFF + KL_B_PLANE, KL_KW);
+							const uint64_t b_hi = make_desc_sw64(base + KL_B_OFF), b_lo = make_desc_sw64(base + KL_B_OFF + KL_B_PLANE);
 							const uint32_t steps = last ? ksteps : 2u;
 							if (ptx::elect_one()) {
 								for (uint32_t i = 0; i < tiles; ++i) {
 									const uint32_t d_tmem = tmem_base + i * TC_NT_MAX;
-									const uint64_t a_hi = make_desc_kw(base + i * KL_A1_OFF, KL_KW), a_lo = make_desc_kw(base + i * KL_A1_OFF + KL_A_PLANE, KL_KW);
+									const uint64_t a_hi = make_desc_sw64(base + i * KL_A1_OFF), a_lo = make_desc_sw64(base + i * KL_A1_OFF + KL_A_PLANE);
 									#pragma unroll
 									for (uint32_t ks = 0; ks < 2; ++ks)
 										if (ks < steps) ptx::mma_f16(d_tmem, a_lo + 2 * ks, b_hi + 2 * ks, idesc, (kc | ks) > 0);
@@ -953,15 +962,10 @@ bool tc_plan_can_fuse(const TcPlan* p, const FusedAcc& f)
 // K loop with several mean tiles: pairs of neighbouring CTAs share a point block (see the kernel)
 static uint32_t plan_jsplit(const TcPlan* p)
 {
-	const bool kloop = p->tp.d_pad > TC_KCHUNK;
-	const uint32_t n_ctiles = p->tm.k_pad / p->nt_cols;
-	return (kloop && n_ctiles >= 2 * TC_JSPLIT && p->tp.partial != nullptr && p->sm_count >= (int)TC_JSPLIT) ? TC_JSPLIT : 1u;
+	return p->tp.partial != nullptr && p->sm_count >= (int)TC_JSPLIT ? TC_JSPLIT : 1u;
 }
 
-// The three-key form costs the epilogue a third more minima; it pays where the multiplication is long
-// enough to make that small and the exact pass over all means long enough to matter (2^20 x 512 against
-// 4096: the pass 8.70 -> 9.06 ms, the re-check of 4400 points 1.49 -> 0.09 ms).
-bool tc_plan_collects_pairs(const TcPlan* p) { return plan_jsplit(p) > 1 && p->s.dim >= 256 && p->tp.pairs != nullptr; }
+bool tc_plan_collects_pairs(const TcPlan* p) { return plan_jsplit(p) > 1 && p->tp.pairs != nullptr; }
 
 void tc_plan_describe(const TcPlan* p, bool fused, uint32_t out[4])
 {

@@ -17,7 +17,6 @@ struct Shape {
 struct TcMeans {
 	float* b_hi;     // [k_pad][d_pad words] fp16 high part of -2*mean (centred, scaled by tc_scale), K-major
 	float* b_lo;     // [k_pad][d_pad words] fp16 low part
-	float* cnorm;    // [k_pad] |mean|^2 in units of the scale, +inf for padding rows
 	float* b_aug;    // [k_pad x 8 words] one K step of |mean|^2 (aug_offset layout, see tc_aug_row); padding rows: 0
 	float* center;   // [dim] vector subtracted from points and means alike before the split (distances do
 	                 // not change; the norms, and with them the cancellation of the GEMM form, shrink)
@@ -38,8 +37,8 @@ struct TcPoints {
 	float* xnorm;    // [n_pad] |x|^2 in units of the scale; +inf (and zero rows) for points the planes cannot hold
 	uint64_t n_pad;  // n rounded up to TC_MTILE
 	uint32_t d_pad;
-	uint32_t* partial; // K loop only (d_pad > 32): [TC_JSPLIT][5][n_pad] partial arg-min keys, else null
-	uint32_t* pairs;   // K loop only: [2][n] points queued with two candidates, and the second candidate
+	uint32_t* partial; // [TC_JSPLIT][tc_partial_words][n_pad] partial arg-min keys, or null
+	uint32_t* pairs;   // with five words only: [2][n] points queued with two candidates, and the second candidate
 };
 constexpr uint32_t TC_JSPLIT = 2;   // CTAs that can share the mean tiles of one point block in the K loop
 
@@ -115,7 +114,6 @@ struct FusedAcc {
 	uint32_t* counts;
 	uint32_t replicas;
 	size_t rep_stride;
-	const float* center;  // the vector the split operands were centred by
 	const float* points;  // the points themselves (in the layout `soa`): what the tensor-core pass adds up
 	int soa;
 };
@@ -147,6 +145,9 @@ cudaError_t launch_assign_simt(const float* pts, const float* means, const SimtM
 // ---- assignment on tensor cores (assign_tc.cu) ----
 bool assign_tc_supported(const Shape& s);
 uint32_t tc_kpad(uint32_t k);
+// Words that each of the CTAs that share a point block leaves per point: 0 = they do not share (short rows or few
+// mean tiles), 3 = (best, second, chunk), 5 = the third smallest key too, for lists of points with two candidates.
+uint32_t tc_partial_words(uint32_t k, uint32_t dim);
 // One-off split of the points into fp16 hi/lo K-major planes + |x|^2 (after launch_compute_center).
 // `p_begin`, `p_end` (multiples of 32; 0, 0 = all): only these rows of the planes, so that a host upload
 // can be split chunk by chunk while the next chunk is on its way.

@@ -324,18 +324,7 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols)
 // One MMA over both CTAs of the pair (M = 256: 128 accumulator rows in each CTA's tensor memory;
 // each CTA's shared memory holds its 128 rows of A and its half of the N rows of B at the
 // descriptor's address).  Issued by one thread of the pair's first CTA.
-__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
-{
-	asm volatile(
-		"{\n"
-		".reg .pred p;\n"
-		"setp.ne.b32 p, %4, 0;\n"
-		"tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-		"}\n"
-		:: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// The same with the two 64-bit shared-memory descriptors given as 32-bit halves.  Within one
+// The two 64-bit shared-memory descriptors are given as 32-bit halves: within one
 // operand tile only the low half (the address field) changes from instruction to instruction and
 // the high half is a constant of the layout, which leaves the issuing thread one 32-bit add per
 // operand and MMA instead of 64-bit descriptor arithmetic.  ACC = accumulate onto the destination.

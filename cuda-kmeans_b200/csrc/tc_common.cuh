@@ -66,18 +66,10 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
 	return false;
 }
 
-// K-major operand, 128-byte swizzle: rows of 128 B, 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr)
+// K-major operand, 64-byte swizzle: rows of 64 B, 8-row groups 512 B apart.
+__device__ __forceinline__ uint64_t make_desc_sw64(uint32_t smem_addr)
 {
-	return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-
-// Same for rows of `kw` words: kw = 32 as above, kw = 16 -> 64-byte swizzle, rows of 64 B,
-// 8-row groups 512 B apart.
-__device__ __forceinline__ uint64_t make_desc_kw(uint32_t smem_addr, uint32_t kw)
-{
-	return kw == 32 ? make_desc(smem_addr)
-		: ((uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61));
+	return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
 }
 
 // K-major operand without swizzle, one K step (16 fp16 = two 16-byte chunks) wide: 8x16-byte core
@@ -87,7 +79,7 @@ __device__ __forceinline__ uint64_t make_desc_aug(uint32_t smem_addr)
 	return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (8ull << 16) | (16ull << 32) | (1ull << 46);
 }
 
-// The two 32-bit halves of those descriptors: the low half holds the address field (>> 4) and the
+// The two 32-bit halves of such descriptors: the low half holds the address field (>> 4) and the
 // leading byte offset, the high half is a constant of the layout.
 constexpr uint32_t DESC_HI_SW128 = 64u | (1u << 14) | (2u << 29);     // 128-byte swizzle, 8-row groups 1024 B apart
 constexpr uint32_t DESC_HI_AUG = 16u | (1u << 14);                    // no swizzle, row groups 256 B apart

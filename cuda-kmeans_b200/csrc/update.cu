@@ -58,7 +58,7 @@ struct RowSinks {
 	float* means_out; uint32_t* sizes_out;
 	uint32_t k, d; int soa_means;
 	float* cprep; uint32_t rs, srows;
-	__half* b_hi; __half* b_lo; float* cnorm; float* b_aug; const float* center; uint32_t k_pad, d_pad;   // d_pad in words
+	__half* b_hi; __half* b_lo; float* b_aug; const float* center; uint32_t k_pad, d_pad;   // d_pad in words
 	Control* ctl; int slot;
 	int divide;            // 0: the rows are written as sums (bucketing), 1: as means
 };
@@ -98,7 +98,6 @@ __device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32
 	__syncwarp();
 	if (lane == 0) {
 		if (o.cprep) o.cprep[(size_t)c * o.rs] = s2;
-		if (o.cnorm) o.cnorm[c] = s2;
 		if (o.b_aug) {
 			*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 0)) = tc_aug_row(s2);
 			*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 1)) = make_uint4(0u, 0u, 0u, 0u);
@@ -112,7 +111,6 @@ __device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32
 __device__ __forceinline__ void finish_padding_row(const RowSinks& o, uint32_t c)
 {
 	if (o.cprep && c < o.srows) o.cprep[(size_t)c * o.rs] = INFINITY;
-	if (o.cnorm && c < o.k_pad) o.cnorm[c] = INFINITY;
 	if (o.b_aug && c < o.k_pad) {
 		*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 0)) = tc_aug_row(0.0f);
 		*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 1)) = make_uint4(0u, 0u, 0u, 0u);
@@ -131,7 +129,7 @@ __device__ __forceinline__ uint32_t rows_to_finish(const RowSinks& o)
 {
 	uint32_t rows_total = o.k;
 	if (o.cprep && o.srows > rows_total) rows_total = o.srows;
-	if (o.cnorm && o.k_pad > rows_total) rows_total = o.k_pad;
+	if (o.b_aug && o.k_pad > rows_total) rows_total = o.k_pad;
 	return rows_total;
 }
 
@@ -340,7 +338,7 @@ static RowSinks make_sinks(float* means_out, uint32_t* sizes_out, const Shape& s
 	o.k = s.k; o.d = s.dim; o.soa_means = s.soa_means;
 	o.cprep = sm ? sm->rows : nullptr; o.rs = simt_row_stride(s.dim); o.srows = simt_rows(s.k);
 	o.b_hi = tc ? reinterpret_cast<__half*>(tc->b_hi) : nullptr; o.b_lo = tc ? reinterpret_cast<__half*>(tc->b_lo) : nullptr;
-	o.cnorm = tc ? tc->cnorm : nullptr; o.b_aug = tc ? tc->b_aug : nullptr;
+	o.b_aug = tc ? tc->b_aug : nullptr;
 	o.center = tc ? tc->center : (sm ? sm->center : nullptr);
 	o.k_pad = tc ? tc->k_pad : 0; o.d_pad = tc ? tc->d_pad : 0;
 	o.ctl = ctl; o.slot = slot;
