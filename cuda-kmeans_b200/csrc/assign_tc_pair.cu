@@ -202,7 +202,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 		// so that the arg-min needs no column masks.
 		uint4* dst = reinterpret_cast<uint4*>(smem + baug_off);
 		const uint32_t per_tile = P2_AUG_HALF_BYTES / 16;
-		const uint4 pad_row = tc_aug_row(kc.pow2 - x2max - kc.pow2 * (1.0f / 16.0f));
+		const uint4 pad_row = tc_aug_row(kc.pow2 - fmaxf(x2max, 1.0f) - kc.pow2 * (1.0f / 16.0f));     // (the offset takes the norm as at least 1, too)
 		for (uint32_t e = threadIdx.x; e < n_ctiles * per_tile; e += TC_THREADS) {
 			const uint32_t j = e / per_tile, r = e - j * per_tile;
 			// 16-byte chunk r of a tile half: row (r / 16) * 8 + r % 8, K positions 8 * ((r / 8) % 2) ..
