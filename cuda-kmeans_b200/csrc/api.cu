@@ -474,7 +474,7 @@ static int stateless_assign(const float* points, const float* means, uint32_t* a
 	bkm::ClearRanges clear = {{w.split_scratch, w.acc, nullptr}, {bkm::list_split_scratch_bytes(), fa ? align256(w.acc_bytes) : 0, 0}};
 	if (v == BKM_ASSIGN_SIMT) { clear.base[2] = w.sm.rows; clear.bytes[2] = align256(w.cprep_bytes); }
 	if (v == BKM_ASSIGN_TC) { clear.base[2] = w.tm.b_hi; clear.bytes[2] = w.tm_bytes; }
-	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, key, s, clear, sm_count, st));
+	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, key, s, clear, v != BKM_ASSIGN_EXACT, sm_count, st));
 	if (v != BKM_ASSIGN_EXACT) {
 		const uint32_t* skip = &key->valid;
 		CUDA_TRY(bkm::launch_points_fingerprint(points, s, v, key, w.ctl, sm_count, st));
@@ -499,7 +499,7 @@ static int stateless_update(const float* points, const uint32_t* assignment, flo
 	int rc = resolve_update(variant, s, device, &v);
 	if (rc) return rc;
 	// (an assignment in front of it has cleared the accumulators as well)
-	if (clear) CUDA_TRY(bkm::launch_stateless_begin(w.ctl, points_key(w), s, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, sm_count, st));
+	if (clear) CUDA_TRY(bkm::launch_stateless_begin(w.ctl, points_key(w), s, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, false, sm_count, st));
 	bkm::launch_update(points, assignment, w.acc, w.counts, w.replicas, s, v, w.ctl, sm_count, st);
 	bkm::launch_finalize(w.acc, w.counts, w.replicas, means, sizes, s, nullptr, nullptr, w.ctl, 1, st);
 	CUDA_TRY(cudaGetLastError());
@@ -538,7 +538,7 @@ int bkm_bucket_sums_f32(const float* points, const uint32_t* indices, float* sum
 	int v = 0;
 	if ((rc = resolve_update(variant, s, device, &v))) return rc;
 	cudaStream_t st = static_cast<cudaStream_t>(stream);
-	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, points_key(w), s, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, sm, st));
+	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, points_key(w), s, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, false, sm, st));
 	bkm::launch_update(points, indices, w.acc, w.counts, w.replicas, s, v, w.ctl, sm, st);
 	bkm::launch_finalize_sums(w.acc, w.counts, w.replicas, sums, s, w.ctl, st);
 	CUDA_TRY(cudaGetLastError());

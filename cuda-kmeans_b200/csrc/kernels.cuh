@@ -85,9 +85,10 @@ cudaError_t launch_probe_atomics(float* result, uint64_t n, uint32_t k, uint32_t
 // Ranges of the workspace to clear (16-byte aligned, whole multiples of 16 bytes; 0 bytes = unused).
 struct ClearRanges { void* base[3]; size_t bytes[3]; };
 // Clears status, near-tie count, |c|^2 slots, the fingerprint of `key` and the ranges.  A call that does not
-// look at the points (no fingerprint behind it) but lays the workspace out differently from the call that
-// `key` remembers writes over the operands derived then: it forgets them.
-cudaError_t launch_stateless_begin(Control* ctl, PointsKey* key, const Shape& s, const ClearRanges& ranges, int sm_count, cudaStream_t stream);
+// look at the points (no fingerprint behind it: `fingerprint_follows` = false) but lays the workspace out
+// differently from the call that `key` remembers writes over the operands derived then: it forgets them.
+cudaError_t launch_stateless_begin(Control* ctl, PointsKey* key, const Shape& s, const ClearRanges& ranges, bool fingerprint_follows,
+	int sm_count, cudaStream_t stream);
 // Fingerprints the points (every 16th 128-byte line and the last one; order-independent sum of mixed
 // (value, position) words), sets key->valid (same address, shape, number of means, variant and fingerprint as
 // remembered) and remembers the current call's; when the points are new it also clears what their

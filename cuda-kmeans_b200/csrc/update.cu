@@ -464,15 +464,17 @@ cudaError_t launch_probe_atomics(float* result, uint64_t n, uint32_t k, uint32_t
 // Clears what a stateless call needs cleared - status, near-tie count and |c|^2 slots, the fingerprint,
 // and up to three ranges of its scratch - in one launch (a call is bound by the number of its launches:
 // five memsets took a third of the 13 operations, 42 us together, of a small bkm_iterate_f32).
-__global__ void __launch_bounds__(256) stateless_begin_kernel(Control* ctl, PointsKey* key, unsigned long long n, uint32_t k, uint32_t dim, ClearRanges ranges)
+__global__ void __launch_bounds__(256) stateless_begin_kernel(Control* ctl, PointsKey* key, unsigned long long n, uint32_t k, uint32_t dim, ClearRanges ranges, int check)
 {
 	const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
 	if (t == 0) {
 		// last_flag_count and what belongs to the points survive
 		ctl->status = 0; ctl->flag_count = 0; ctl->pair_count = 0; ctl->cmax2[0] = 0.0f; ctl->cmax2[1] = 0.0f;
 		key->fp_new = 0; key->arrive = 0;
-		if (key->n != n || key->k != k || key->dim != dim) key->n = 0;      // (no call has 0 points)
 	}
+	// (by another warp: the round trip of the loads is not waited for behind the stores, and where the fingerprint
+	// compares anyway it is saved, 1 us per call)
+	if (check && t == 32 && (key->n != n || key->k != k || key->dim != dim)) key->n = 0;      // (no call has 0 points)
 	#pragma unroll
 	for (uint32_t r = 0; r < 3; ++r) {
 		uint4* dst = static_cast<uint4*>(ranges.base[r]);
@@ -480,12 +482,12 @@ __global__ void __launch_bounds__(256) stateless_begin_kernel(Control* ctl, Poin
 	}
 }
 
-cudaError_t launch_stateless_begin(Control* ctl, PointsKey* key, const Shape& s, const ClearRanges& ranges, int sm_count, cudaStream_t stream)
+cudaError_t launch_stateless_begin(Control* ctl, PointsKey* key, const Shape& s, const ClearRanges& ranges, bool fingerprint_follows, int sm_count, cudaStream_t stream)
 {
 	uint64_t words = 0;
 	for (uint32_t r = 0; r < 3; ++r) words += ranges.bytes[r] / 16;
 	const uint32_t grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>((words + 511) / 512, 1), (uint64_t)sm_count * 4);
-	stateless_begin_kernel<<<grid, 256, 0, stream>>>(ctl, key, s.n, s.k, s.dim, ranges);
+	stateless_begin_kernel<<<grid, 256, 0, stream>>>(ctl, key, s.n, s.k, s.dim, ranges, fingerprint_follows ? 0 : 1);
 	return cudaGetLastError();
 }
 
