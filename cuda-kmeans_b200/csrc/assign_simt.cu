@@ -740,38 +740,38 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 
 	// Brings tile t of the prepared means into shared memory, interleaved by pairs, and adds the offset
 	// constant to its |c|^2 column (padding rows, marked by +inf there, get the top of the value band).
+	// Fused (a single tile, see assign_simt_can_fuse): beside it the means as they are, for the near-ties, and the
+	// rows of infinities that scan_means wants behind them.
+	constexpr uint32_t MS = scan_row_floats(D);
+	float* s_means = tile + rows * (D + 1);
 	auto load_tile = [&](uint32_t t) -> uint32_t {
 		uint32_t trows = rows - t * SIMT_TILE_ROWS;
 		if (trows > SIMT_TILE_ROWS) trows = SIMT_TILE_ROWS;
 		for (uint32_t r = tid; r < trows; r += SIMT_THREADS) {
 			const float4* src = reinterpret_cast<const float4*>(cprep + ((size_t)t * SIMT_TILE_ROWS + r) * RS);
 			float* dst = tile + (r >> 1) * (2 * (D + 1)) + (r & 1u);
-			float v[RS];
+			float v[RS], mean[FUSE ? D : 1];
 			#pragma unroll
 			for (int q = 0; q < RS / 4; ++q) {
 				const float4 w = src[q];
 				v[4 * q + 0] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
 			}
+			if (FUSE) {
+				#pragma unroll
+				for (int j = 0; j < D; ++j) if (r < k) mean[j] = means[at_rt(soa_means, r, j, k, D)];
+			}
 			v[0] = v[0] > 3.0e38f ? pad_value : v[0] + kc.offset_c;
 			#pragma unroll
 			for (int j = 0; j <= D; ++j) dst[2 * j] = v[j];
+			if (FUSE && r < k) {
+				#pragma unroll
+				for (int j = 0; j < D; ++j) s_means[r * MS + j] = mean[j];
+			}
 		}
+		if (FUSE) for (uint32_t e = tid; e < (LIST_SMALL_SUMS - 1) * MS; e += SIMT_THREADS) s_means[k * MS + e] = INFINITY;
 		__syncthreads();
 		return trows;
 	};
-
-	// fused: the means as they are, for the near-ties, and the rows of infinities that scan_means wants behind them
-	constexpr uint32_t MS = scan_row_floats(D);
-	float* s_means = tile + rows * (D + 1);      // (a single tile, see assign_simt_can_fuse)
-	if (FUSE) {
-		for (uint32_t e = tid; e < k * D; e += SIMT_THREADS) {
-			const uint32_t m = e / D, j = e - m * D;
-			s_means[m * MS + j] = means[at_rt(soa_means, m, j, k, D)];
-		}
-		for (uint32_t e = tid; e < (LIST_SMALL_SUMS - 1) * MS; e += SIMT_THREADS) s_means[k * MS + e] = INFINITY;
-	}
-	uint32_t trows0 = 0;
-	if (ntiles == 1) trows0 = load_tile(0);
 
 	// The points of a block of work, as they lie in memory (slots behind the last point read as the
 	// centre).  The next block's points are fetched while the current block is being evaluated.
@@ -808,7 +808,9 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 			}
 		}
 	};
-	if (blockIdx.x < nblocks) load_points(blockIdx.x);
+	if (blockIdx.x < nblocks) load_points(blockIdx.x);     // (on their way while the means are brought in)
+	uint32_t trows0 = 0;
+	if (ntiles == 1) trows0 = load_tile(0);
 
 	for (uint64_t blk = blockIdx.x; blk < nblocks; blk += gridDim.x) {
 		float x[P][D];
@@ -1028,9 +1030,11 @@ static cudaError_t launch_simt_d(const float* pts, const float* means, const flo
 {
 	// The fused sums are sent per warp and run of sorted points, and with few clusters all of them meet on a few
 	// rows: where the coordinates fit, a warp sorts 128 points instead of 64 (2^21 points in 5 clusters, per
-	// iteration: 81 -> 55 us for d = 1, 80 -> 50 us for d = 2).
-	constexpr int FUSE_P = D <= 2 ? 4 : 2;
-	const int points = fused ? FUSE_P : SIMT_EVAL_POINTS;
+	// iteration: 81 -> 55 us for d = 1, 80 -> 50 us for d = 2), unless that leaves SMs without a block (20 000
+	// points, d = 2: 18 instead of 16 us).
+	constexpr int MANY_P = D <= 2 ? 4 : 2;
+	const bool many = MANY_P != SIMT_EVAL_POINTS && s.n >= (uint64_t)sm_count * SIMT_THREADS * MANY_P;
+	const int points = fused && many ? MANY_P : SIMT_EVAL_POINTS;
 	const uint32_t rows = simt_rows(s.k);
 	const uint32_t trows = rows < (uint32_t)SIMT_TILE_ROWS ? rows : (uint32_t)SIMT_TILE_ROWS;
 	const size_t smem = ((size_t)trows * (D + 1) + (fused ? (size_t)(s.k + LIST_SMALL_SUMS - 1) * scan_row_floats(D) : 0)) * sizeof(float);
@@ -1044,7 +1048,7 @@ static cudaError_t launch_simt_d(const float* pts, const float* means, const flo
 	const float margin_ulps = margin_scale * (float)(4 * D + 16);
 	const int vec_ok = ((reinterpret_cast<uintptr_t>(pts) & 15u) == 0) ? 1 : 0;
 #define BKM_LAUNCH_SIMT(SOA, FUSE) do { \
-		auto kern = assign_simt_kernel<D, SOA, FUSE ? FUSE_P : SIMT_EVAL_POINTS, FUSE>; \
+		auto kern = FUSE && many ? assign_simt_kernel<D, SOA, FUSE ? MANY_P : SIMT_EVAL_POINTS, FUSE> : assign_simt_kernel<D, SOA, SIMT_EVAL_POINTS, FUSE>; \
 		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
 		if (e != cudaSuccess) return e; \
 		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SIMT_THREADS, smem); \
