@@ -425,6 +425,27 @@ static bkm::PointsKey* points_key(const Workspace& w)
 // One assignment pass on a caller's workspace.  The operands derived from the (immutable) points -
 // centre vector, largest norm, fp16 planes - stay in the workspace; a call that finds the same
 // point set there (address, shape, number of means and a fingerprint of a sample of the values) skips them.
+// Whether the CUDA-core pass should.  The fused form saves two launches (5 us per iteration of a graph, 8 us
+// per stateless call) and pays for it in three ways; microseconds per stateless call, fused / apart.
+//  - Its warps settle their own near-ties, the list kernel shares them out over the machine: with many means the
+//    fused form wins where near-ties are few and loses where they are many (20 011 points, d = 3, k = 400:
+//    uniform 46 / 52, clustered 64 / 54, means that exist twice 83 / 60), with one dimension, where they are
+//    frequent, from 100 means on (43 / 43, 46 / 43, 46 / 45).
+//  - A row of sums goes out as one reduction for d = 1, 2 and 4, two for d = 8 and d or d / 2 of them otherwise,
+//    and with few clusters all rows meet (10 clusters, 2^18 points: d = 3 55 / 50, d = 5 82 / 58, d = 8 56 / 53;
+//    d = 4 2^20 points 76 / 74; 64 clusters, 2^18 points: d = 5 57 / 60, 2^19 points d = 8 67 / 73).
+//  - Its sorting costs more than a separate pass over many points, unless few clusters make the sorted runs long
+//    (iterations with 2^22 points, d = 2, 10 / 32 clusters: 77 / 111, 126 / 110).
+static bool simt_fuse_pays(const bkm::Shape& s)
+{
+	const uint32_t d = s.dim, k = s.k;
+	if (d == 1) return k <= 64 && s.n <= (k <= 16 ? 1u << 22 : 1u << 20);
+	if (s.n <= 1u << 16) return k <= (d == 2 ? 256u : 512u);
+	if (k > (s.n <= 1u << 18 ? 256u : (d == 2 ? 64u : 128u))) return false;
+	if (d == 2 || d == 4) return s.n <= (d == 2 && k <= 16 ? 1u << 22 : 1u << 20);
+	return s.n <= (d == 8 ? (k < 64 ? 1u << 17 : 1u << 19) : (k < 64 ? 1u << 16 : 1u << 18));
+}
+
 // Whether the fast assignment pass should accumulate the update sums itself.  On CTA pairs the
 // epilogue warps send the reductions, which pays where the update would otherwise be the row-wise
 // kernel (the sorted update of row-major points costs less than that).  In the CUDA-core pass every
@@ -432,18 +453,7 @@ static bkm::PointsKey* points_key(const Workspace& w)
 static bool fuse_pays(int assign_variant, int update_variant, const bkm::TcPlan* plan, const bkm::FusedAcc& fa, const bkm::Shape& s, bool force = false)
 {
 	if (assign_variant == BKM_ASSIGN_SIMT) {
-		// The fused form saves two launches (5 us per iteration of a graph) and pays for it in three ways.  Its
-		// warps settle their near-ties one warp at a time: with more means (64 for one or two dimensions, where
-		// near-ties are frequent, else 128) the list kernel is faster where they are many (20 011 clustered points,
-		// d = 2, k = 128 / 256: 34 / 48 against 30 / 34 us; d = 8: 36 / 44 against 35 / 39).  A row of sums
-		// goes out as one reduction for d = 1, 2 and 4, two for d = 8 and d or d / 2 of them otherwise, and with
-		// few clusters all rows meet (10 clusters: d = 4, 2^20 points 53 against 54; d = 8, 2^18 points 41 against
-		// 38; d = 3, 2^16 points 25 against 28 but 2^18 40 against 33; d = 5, 2^20 points 202 against 53).  Its
-		// sorting costs more than a separate pass over many points, unless few clusters make the sorted runs
-		// long (d = 2, 2^22 points, 10 / 32 / 128 clusters: 77 / 126 / 174 against 111 / 110 / 186).
-		const uint32_t log_n = s.dim <= 2 ? (s.k <= 16 ? 22 : 20) : (s.dim == 4 ? 20 : (s.dim == 8 ? 18 : 16));
-		const bool pays = s.k <= (s.dim <= 2 ? 64u : 128u) && s.n <= (1ull << log_n);
-		return bkm::assign_simt_can_fuse(s, fa) && (force || pays);
+		return bkm::assign_simt_can_fuse(s, fa) && (force || simt_fuse_pays(s));
 	}
 	if (assign_variant != BKM_ASSIGN_TC) return false;
 	return update_variant == BKM_UPDATE_ROWS && bkm::tc_plan_can_fuse(plan, fa) && (size_t)s.dim * sizeof(float) * 4 <= 120 * 1024;

@@ -51,7 +51,9 @@ def test_repeated_calls_reuse_the_workspace_and_notice_new_points(pkg, torch_cud
     (9000, 300, 20, 0, 0, True),       # row-major points: two passes
     (30000, 64, 2, 0, 0, True),        # CUDA cores: single pass (every warp sorts its points by cluster)
     (12345, 100, 7, 1, 0, False),      # same, dimension-major points, no assignment output
-    (12345, 200, 7, 1, 0, False),      # more means: two passes
+    (12345, 300, 2, 1, 0, False),      # more means: two passes
+    (12345, 512, 7, 0, 1, True),       # longer rows, as many as the single pass takes by itself
+    (65537, 257, 4, 0, 0, True),       # one more point and mean than that: two passes
     (70000, 10, 3, 0, 0, True),        # more points in few clusters: two passes
     (5000, 2000, 3, 0, 0, True),       # CUDA cores, more means than the single pass takes: two passes
 ])
