@@ -41,13 +41,13 @@ if ROOT not in sys.path:
 
 V100_PUBLISHED_GEVALS = 84.4  # reference's best variant, N=2M d=32 k=1024, V100 (results/README.md:20)
 # DRAM bytes (read + write, from one profiler capture) that one assignment launch on workload c2
-# moves per point: the capture ran on 2^19 points (138.81 MB read + 6.79 MB written); the traffic is
-# the point operands, read once, so it grows in proportion to the points.
-C2_ASSIGN_TC_DRAM_BYTES_PER_POINT = (138.81e6 + 6.79e6) / (1 << 19)
-# the same for the one-CTA tensor-core kernel on c5's shape (2^24-point capture: 2.215 GB read, 67.8 MB written)
+# moves per point: the capture ran on 2^19 points (138.74 MB read + 3.68 MB written, fp16 operands and raw
+# rows); the traffic is the points, read once, so it grows in proportion to them.
+C2_ASSIGN_TC_DRAM_BYTES_PER_POINT = (138.74e6 + 3.68e6) / (1 << 19)
+# the same for the one-CTA tensor-core kernel on c5's shape (2^22-point capture: 554 MB read, 17.5 MB written)
 # and for the CUDA-core kernel on c3's shape (2^22-point capture: 33.6 MB read; the 16.8 MB of assignments
 # stayed in L2 at that size and are counted as written)
-C5_ASSIGN_TC_DRAM_BYTES_PER_POINT = (2.215e9 + 67.8e6) / (1 << 24)
+C5_ASSIGN_TC_DRAM_BYTES_PER_POINT = (554.0e6 + 17.5e6) / (1 << 22)
 C3_ASSIGN_SIMT_DRAM_BYTES_PER_POINT = (33.6e6 + 16.8e6) / (1 << 22)
 PARITY_SAMPLE = 4096
 PHASE_STEPS = 8     # instrumented iterations behind the timed ones, for `phases_ms`
