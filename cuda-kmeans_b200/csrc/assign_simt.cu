@@ -625,10 +625,10 @@ cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* 
 // point's coordinate in both halves): the pass is bound by instruction issue, and this halves the D
 // instructions per mean and point.  The constant C (from the
 // largest |x|^2 and |c|^2, see make_key_consts) puts all values into one binade, where their bit
-// patterns order like the values.  The 32 values of a chunk become integer keys (bits * M + column)
-// and are reduced to the smallest and second smallest with plain integer minima (chunk_update):
-// about 1.75 integer instructions per point and mean where a (best, second, index) tournament on
-// floats takes five, and D instead of 2D arithmetic instructions.  The form cancels where the
+// patterns order like the values.  The values go into minima over two partitions of the means (RowMin):
+// about one integer instruction per point and mean where keys with a pass each for the smallest and the
+// second smallest took 1.75 and a multiply-add (2^24 points of two dimensions against 64 means: 0.278 ->
+// 0.261 ms), and D instead of 2D arithmetic instructions.  The form cancels where the
 // difference form does not, so a point whose best and second-best keys are closer than the
 // rounding band of the pass (and of the reference's own sum and square root) is queued for the
 // exact kernel; the final assignment is the reference's for every point.
@@ -842,9 +842,9 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 				#pragma unroll
 				for (int j = 0; j < D; ++j) xx[p][j] = ptx::pack2(x[g + p][j], x[g + p][j]);
 
-			uint32_t best[Q], second[Q], bchunk[Q];
+			RowMin row[Q];
 			#pragma unroll
-			for (int p = 0; p < Q; ++p) { best[p] = 0xFFFFFFFFu; second[p] = 0xFFFFFFFFu; bchunk[p] = 0; }
+			for (int p = 0; p < Q; ++p) row[p].reset();
 
 			for (uint32_t t = 0; t < ntiles; ++t) {
 				uint32_t trows = trows0;
@@ -855,44 +855,61 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 				const uint32_t chunk_base = t * (SIMT_TILE_ROWS / 32);
 				#pragma unroll 1
 				for (uint32_t ch = 0; ch < trows / 32; ++ch) {
-					uint32_t v[Q][32];
+					// Columns m .. m + 3 and m + 16 .. m + 19 together: they meet in the same position minima.
 					const float4* rowp = reinterpret_cast<const float4*>(tile + (size_t)ch * 32 * (D + 1));
+					uint32_t group[Q][2];
 					#pragma unroll
-					for (int m = 0; m < 32; m += 4) {
-						// four means = two interleaved pairs = D + 1 128-bit loads
-						float f[4 * (D + 1)];
+					for (int p = 0; p < Q; ++p) group[p][0] = group[p][1] = 0xFFFFFFFFu;
+					#pragma unroll
+					for (int m = 0; m < 16; m += 4) {
+						uint32_t v[Q][2][4];
 						#pragma unroll
-						for (int q = 0; q <= D; ++q) {
-							const float4 w = rowp[(m / 4) * (D + 1) + q];
-							f[4 * q + 0] = w.x; f[4 * q + 1] = w.y; f[4 * q + 2] = w.z; f[4 * q + 3] = w.w;
+						for (int half = 0; half < 2; ++half) {
+							// four means = two interleaved pairs = D + 1 128-bit loads
+							float f[4 * (D + 1)];
+							#pragma unroll
+							for (int q = 0; q <= D; ++q) {
+								const float4 w = rowp[(m / 4 + half * 4) * (D + 1) + q];
+								f[4 * q + 0] = w.x; f[4 * q + 1] = w.y; f[4 * q + 2] = w.z; f[4 * q + 3] = w.w;
+							}
+							#pragma unroll
+							for (int h = 0; h < 2; ++h) {
+								const float* mean2 = f + h * 2 * (D + 1);
+								#pragma unroll
+								for (int p = 0; p < Q; ++p) {
+									uint64_t val = ptx::pack2(mean2[0], mean2[1]);
+									#pragma unroll
+									for (int j = 0; j < D; ++j) val = ptx::fma2(xx[p][j], ptx::pack2(mean2[2 * j + 2], mean2[2 * j + 3]), val);
+									ptx::unpack2(val, v[p][half][2 * h], v[p][half][2 * h + 1]);
+								}
+							}
 						}
 						#pragma unroll
-						for (int h = 0; h < 2; ++h) {
-							const float* row = f + h * 2 * (D + 1);
+						for (int p = 0; p < Q; ++p) {
 							#pragma unroll
-							for (int p = 0; p < Q; ++p) {
-								uint64_t val = ptx::pack2(row[0], row[1]);
-								#pragma unroll
-								for (int j = 0; j < D; ++j) val = ptx::fma2(xx[p][j], ptx::pack2(row[2 * j + 2], row[2 * j + 3]), val);
-								ptx::unpack2(val, v[p][m + 2 * h], v[p][m + 2 * h + 1]);
-							}
+							for (int u = 0; u < 4; ++u) row[p].position[m + u] = umin3(row[p].position[m + u], v[p][0][u], v[p][1][u]);
+							#pragma unroll
+							for (int half = 0; half < 2; ++half)
+								group[p][half] = umin3(umin3(group[p][half], v[p][half][0], v[p][half][1]), v[p][half][2], v[p][half][3]);
 						}
 					}
 					#pragma unroll
-					for (int p = 0; p < Q; ++p) chunk_update<false>(v[p], key_mult, chunk_base + ch, 32, best[p], second[p], bchunk[p]);
+					for (int p = 0; p < Q; ++p) row[p].take_groups(group[p][0], group[p][1], key_mult, chunk_base + ch);
 				}
 			}
 
 			#pragma unroll
 			for (int p = 0; p < Q; ++p) {
+				uint32_t best, second, bchunk;
+				row[p].finish(key_base, key_mult, key_magic, best, second, bchunk);
 				cl[g + p] = k;                 // rows behind the last point sort behind every cluster
 				bool flag = false;
 				if (idx[g + p] < n) {
 					// key - key_base = M * mantissa + column
-					const uint32_t bm = div_key(best[p] - key_base, key_magic);
-					cl[g + p] = bchunk[p] * 32u + ((best[p] - key_base) - bm * key_mult);
+					const uint32_t bm = div_key(best - key_base, key_magic);
+					cl[g + p] = bchunk * 32u + ((best - key_base) - bm * key_mult);
 					if (!FUSE) asg[idx[g + p]] = cl[g + p];
-					const float gap = second[p] == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second[p] - key_base, key_magic) - bm);
+					const float gap = second == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second - key_base, key_magic) - bm);
 					flag = !(gap > margin) || (near >> (g + p) & 1u) != 0;
 				}
 				if (FUSE) near = flag ? near | 1u << (g + p) : near & ~(1u << (g + p));

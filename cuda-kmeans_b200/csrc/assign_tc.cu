@@ -27,9 +27,9 @@
 //   warps 2..17 : epilogue.  Eight warps per accumulator (TMEM lane quarter x column half), so
 //                 that one accumulator is reduced while the other is being multiplied.  A warp
 //                 reads its columns with tcgen05.ld two 32-column chunks at a time, hands the
-//                 accumulator back after its last load, and reduces each chunk to (best, second)
-//                 on integer keys; (best, second, chunk of best) per point stay in registers
-//                 across all mean tiles and are merged through shared memory at the end.
+//                 accumulator back after its last load, and reduces each chunk with integer minima
+//                 (RowMin); what it keeps per point stays in registers across all mean tiles and
+//                 is merged through shared memory at the end.
 // Mean sets of 2..4 tiles of 256 with 17 <= dim <= 64 run on CTA pairs instead, with all means
 // resident in shared memory (assign_tc_pair.cu).
 // All mbarrier waits are bounded; a wait that runs out sets STATUS_WAIT_TIMEOUT and lets every
@@ -354,12 +354,27 @@ static_assert(SM_ALLOC <= 227 * 1024, "shared memory budget exceeded");
 static_assert(2 * 5 * TC_MA * TC_MTILE * 4 <= SM_BAR_OFF - SM_MERGE_OFF, "merge slots of five words");
 static_assert(KL_AUG_OFF + 2 * AUG_BYTES <= SM_AAUG_OFF, "K-loop stages overlap the constant tile");
 
-template<bool THREE, bool MASKED>
-__device__ __forceinline__ void update_state(const uint32_t (&v)[32], uint32_t key_mult, uint32_t chunk_id, uint32_t nvalid, BestThree& st)
+// Columns at or behind `nvalid` of a chunk are padding: their keys lie above every key of a value, whatever the column.
+__device__ __forceinline__ void mask_columns(uint32_t (&v)[32], uint32_t nvalid)
 {
-	if (THREE) chunk_update3<MASKED>(v, key_mult, chunk_id, nvalid, st);
-	else chunk_update<MASKED>(v, key_mult, chunk_id, nvalid, st.best, st.second, st.best_chunk);
+	#pragma unroll
+	for (uint32_t t = 0; t < 32; ++t) v[t] = t < nvalid ? v[t] : 0xFFFFFFFFu;
 }
+
+// What an epilogue warp keeps of a point's row: the two smallest values, or (THREE) the three smallest.
+template<bool THREE> struct RowState;
+template<> struct RowState<false> {
+	RowMin row;
+	__device__ __forceinline__ void reset() { row.reset(); }
+	__device__ __forceinline__ void take_chunk(const uint32_t (&v)[32], uint32_t key_mult, uint32_t chunk_id) { row.take_chunk(v, key_mult, chunk_id); }
+	__device__ __forceinline__ void finish(uint32_t key_base, uint32_t key_mult, uint32_t key_magic, BestThree& st) const { row.finish(key_base, key_mult, key_magic, st.best, st.second, st.best_chunk); }
+};
+template<> struct RowState<true> {
+	BestThree three;
+	__device__ __forceinline__ void reset() { three = BestThree(); }
+	__device__ __forceinline__ void take_chunk(const uint32_t (&v)[32], uint32_t key_mult, uint32_t chunk_id) { chunk_update3(v, key_mult, chunk_id, three); }
+	__device__ __forceinline__ void finish(uint32_t, uint32_t, uint32_t, BestThree& st) const { st = three; }
+};
 
 // Combines the partial arg-min results of the CTAs that shared the mean tiles of a point block.
 // THREE: the partial results carry the third smallest key, and a near-tie between two means only goes
@@ -719,7 +734,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 		for (uint32_t blk = bid; blk < nblocks; blk += nbid, ++blk_count) {
 			const uint32_t tiles = min(TC_MA, n_tiles - blk * TC_MA);
 			if (i >= tiles) continue;              // odd tail: this accumulator is not used in the last block
-			BestThree st;
+			RowState<THREE> rows;
+			rows.reset();
 			const uint64_t p = (uint64_t)(blk * TC_MA + i) * TC_MTILE + row;
 			float xn = 0.0f;                       // |x|^2 of this thread's point, needed at the end of the block
 			#pragma unroll 1
@@ -739,13 +755,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 						const uint32_t col0 = chunk0 * 32u;
 						// columns at or behind k are padding
 						const uint32_t left = FULL ? 64u : (k > col0 ? k - col0 : 0u);
-						const bool plain = FULL || left >= 64 || (!two && left >= 32);
 						// the second chunk travels from tensor memory while the first is reduced
 						ptx::tmem_ld32(taddr, v0);
 						ptx::tmem_ld_wait();
 						if (two) ptx::tmem_ld32(taddr + 32, v1);
-						if (plain) update_state<THREE, false>(v0, key_mult, chunk0, 32, st);
-						else if (left > 0) update_state<THREE, true>(v0, key_mult, chunk0, left, st);
+						if (!FULL && left < 32) mask_columns(v0, left);
+						rows.take_chunk(v0, key_mult, chunk0);
 						ptx::tmem_ld_wait();
 						if (c + 2 >= nchunks) {
 							// last load: the tensor cores may fill this accumulator again
@@ -756,10 +771,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 							// the chunks just loaded covers the latency
 							if (j == j_end - 1 && half == 0 && p < n) xn = xnorm[p];
 						}
-						if (plain) {
-							if (two) update_state<THREE, false>(v1, key_mult, chunk0 + 1, 32, st);
-						} else if (two && left > 32) {
-							update_state<THREE, true>(v1, key_mult, chunk0 + 1, left - 32, st);
+						if (two) {
+							if (!FULL && left < 64) mask_columns(v1, left > 32 ? left - 32 : 0u);
+							rows.take_chunk(v1, key_mult, chunk0 + 1);
 						}
 					}
 				} else {
@@ -770,6 +784,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 			// The upper column half hands its state to the lower one through shared memory.  The slots
 			// alternate with the block count, so one barrier per block is enough: a slot is written
 			// again only after its reader has passed the barrier of the block in between.
+			BestThree st;
+			rows.finish(key_base, key_mult, key_magic, st);
 			constexpr uint32_t WORDS = THREE ? 5 : 3;
 			uint32_t* mg = mg_state + ((blk_count & 1u) * TC_MA + i) * (WORDS * TC_MTILE);
 			if (half == 1) {

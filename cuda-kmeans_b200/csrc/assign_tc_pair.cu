@@ -375,7 +375,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 			pending = false;
 		};
 		for (uint32_t step = step_begin + pair; step < steps_total; step += n_pairs, ++it) {
-			uint32_t best = 0xFFFFFFFFu, second = 0xFFFFFFFFu, bchunk = 0;
+			RowMin rows;
+			rows.reset();
 			const uint64_t p = (uint64_t)(2 * step + rank) * TC_MTILE + row;
 			float xn = 0.0f;
 			if (g == merger && p < n) xn = xnorm[p];      // needed at the end of the step only: fetch early
@@ -401,12 +402,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 					ptx::tmem_ld32(taddr, v0);
 					ptx::tmem_ld_wait();
 					ptx::tmem_ld32(taddr + 32, v1);
-					chunk_update<false>(v0, key_mult, chunk0, 32, best, second, bchunk);
+					rows.take_chunk(v0, key_mult, chunk0);
 					ptx::tmem_ld_wait();
 					ptx::tc_fence_before();
 					__syncwarp();
 					if (lane == 0) ptx::mbar_arrive_cluster(acc_release);
-					chunk_update<false>(v1, key_mult, chunk0 + 1, 32, best, second, bchunk);
+					rows.take_chunk(v1, key_mult, chunk0 + 1);
 				} else {
 					__syncwarp();
 					if (lane == 0) ptx::mbar_arrive_cluster(acc_release);
@@ -420,6 +421,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 			// step ahead of another: every accumulator fill needs all warps of both groups to have
 			// released the fill four before it.  The merging warp belongs to the group that serves the
 			// last fill of a step (it is the last to finish anyway) and has the second fill of the next.
+			uint32_t best, second, bchunk;
+			rows.finish(key_base, key_mult, key_magic, best, second, bchunk);
 			uint32_t* mg = mg_state + (it & 1u) * (3 * 3 * TC_MTILE);
 			const uint32_t merge_bar = 1u + (it & 1u) * 4u + q;
 			uint32_t mine = 0xFFFFFFFFu;                  // cluster of this thread's point (merging warp)

@@ -13,7 +13,7 @@ namespace bkm {
 
 __device__ __forceinline__ uint32_t umin3(uint32_t a, uint32_t b, uint32_t c) { return __vimin3_u32(a, b, c); }
 
-// One 32-column chunk of an accumulator row.  The kernel adds a constant to every value so that
+// Keys of accumulator values.  The kernel adds a constant to every value so that
 // all of them are positive floats with the SAME exponent; their bit patterns then order like the
 // values, the upper exponent bits carry no information, and bits * M + column (M odd, > column:
 // one integer multiply-add, off the min/max pipe) is a key that keeps the full 23-bit mantissa
@@ -33,39 +33,61 @@ __device__ __forceinline__ uint32_t min_of_32(const uint32_t (&p)[32])
 	return min(umin3(c[0], c[1], c[2]), c[3]);
 }
 
-template<bool MASKED>
-__device__ __forceinline__ void chunk_update(const uint32_t (&v)[32], uint32_t key_mult, uint32_t chunk_id, uint32_t nvalid,
-	uint32_t& best, uint32_t& second, uint32_t& best_chunk)
+// Smallest of 16 values (8 instructions).
+__device__ __forceinline__ uint32_t min_of_16(const uint32_t* p)
 {
-	uint32_t p[32];
-	#pragma unroll
-	for (uint32_t t = 0; t < 32; ++t) p[t] = v[t] * key_mult + t;
-	if (MASKED && nvalid < 32) {
-		#pragma unroll
-		for (uint32_t t = 0; t < 32; ++t) p[t] = t < nvalid ? p[t] : 0xFFFFFFFFu;
-	}
-	// Two passes of plain minima instead of a (best, second) tournament.  The keys are distinct
-	// (they carry the column), so key - (smallest + 1) wraps to the top of the unsigned range for
-	// the smallest key only, and the minimum of these differences belongs to the second smallest.
-	// The second pass is 32 fused add-and-minimum instructions in four independent chains;
-	// 16 + 32 + 8 integer instructions per chunk where a tournament takes 77 + 5.
-	const uint32_t b = min_of_32(p);
-	const uint32_t nb1 = ~b;                       // -(b + 1)
-	// (the chains start from their first keys: an add each instead of a constant and an add-and-minimum)
-	uint32_t r0 = p[0] + nb1, r1 = p[1] + nb1, r2 = p[2] + nb1, r3 = p[3] + nb1;
-	#pragma unroll
-	for (uint32_t t = 4; t < 32; t += 4) {
-		r0 = __viaddmin_u32(p[t], nb1, r0);
-		r1 = __viaddmin_u32(p[t + 1], nb1, r1);
-		r2 = __viaddmin_u32(p[t + 2], nb1, r2);
-		r3 = __viaddmin_u32(p[t + 3], nb1, r3);
-	}
-	const uint32_t s2 = min(umin3(r0, r1, r2), r3) - nb1;      // + (b + 1); a lone valid key gives 0xFFFFFFFF again
-	second = umin3(second, max(best, b), s2);
-	best_chunk = b < best ? chunk_id : best_chunk;
-	best = min(best, b);
+	const uint32_t a0 = umin3(p[0], p[1], p[2]), a1 = umin3(p[3], p[4], p[5]), a2 = umin3(p[6], p[7], p[8]);
+	const uint32_t a3 = umin3(p[9], p[10], p[11]), a4 = umin3(p[12], p[13], p[14]);
+	return min(umin3(a0, a1, a2), umin3(a3, a4, p[15]));
 }
 
+// The two smallest values of a point's row, and the column of the smallest, from minima alone.  The
+// columns are partitioned twice: by their position (column mod 16) and into groups of 16 neighbours.  Two
+// columns of one position lie in different groups, so the second smallest value of the row is the
+// second smallest of the 16 position minima or the second smallest of the group minima, whichever is
+// less; the smallest one has its position from the one partition and its group from the other.  A value thus
+// takes part in two three-input minima (which each take in two values) and needs no key of its own: 32 of them
+// for a chunk of 32 columns and nine instructions to rank its two groups, where 32 keys with a pass for
+// the smallest and one for the second took 88 (and no final ranking of positions, about 60 per row and warp).  The
+// epilogues are bound by the ALU pipe (two clocks per instruction): 2^26 x 16 against 256 means 3.35 -> 2.82 ms,
+// 2^21 x 32 against 1024 with update sums 0.510 -> 0.419 ms.  Equal values give a difference of zero, a near-tie.
+// Positions and groups become keys of the usual form (bits * M + column) only for ranking.
+struct RowMin {
+	uint32_t position[16];
+	uint32_t best, second;      // the two smallest group minima so far, as keys bits * M + group within the chunk
+	uint32_t chunk;             // chunk (of 32 columns) of the first
+
+	__device__ __forceinline__ void reset()
+	{
+		#pragma unroll
+		for (int t = 0; t < 16; ++t) position[t] = 0xFFFFFFFFu;
+		best = second = 0xFFFFFFFFu;
+		chunk = 0;
+	}
+
+	// Ranks the minima of the two groups of a chunk.
+	__device__ __forceinline__ void take_groups(uint32_t g0, uint32_t g1, uint32_t key_mult, uint32_t chunk_id)
+	{
+		const uint32_t k0 = g0 * key_mult, k1 = g1 * key_mult + 1u;
+		const uint32_t lo = min(k0, k1), hi = max(k0, k1);
+		second = umin3(second, hi, max(best, lo));
+		chunk = lo < best ? chunk_id : chunk;
+		best = min(best, lo);
+	}
+
+	// One chunk of 32 columns.
+	__device__ __forceinline__ void take_chunk(const uint32_t (&v)[32], uint32_t key_mult, uint32_t chunk_id)
+	{
+		#pragma unroll
+		for (int t = 0; t < 16; ++t) position[t] = umin3(position[t], v[t], v[t + 16]);
+		take_groups(min_of_16(v), min_of_16(v + 16), key_mult, chunk_id);
+	}
+
+	// (best, second, chunk of best) with keys bits * M + column within the chunk.  What stands for "nothing" -
+	// padding, or no second column at all - lies above every key of a value.  Values outside the binade (means
+	// beyond what the pass can hold) give meaningless, but harmless keys.
+	__device__ __forceinline__ void finish(uint32_t key_base, uint32_t key_mult, uint32_t key_magic, uint32_t& best_out, uint32_t& second_out, uint32_t& chunk_out) const;
+};
 
 // The three smallest keys of a point so far, with the chunks (of 32 columns) of the first two.  A point
 // whose third smallest is far enough from the smallest has only two candidates for the exact re-check.
@@ -88,18 +110,15 @@ struct BestThree {
 	}
 };
 
-// As chunk_update with the third smallest key as well: one more pass of add-and-minimum, in which the
-// two smallest wrap to the top (+28 instructions per chunk).
-template<bool MASKED>
-__device__ __forceinline__ void chunk_update3(const uint32_t (&v)[32], uint32_t key_mult, uint32_t chunk_id, uint32_t nvalid, BestThree& state)
+// Takes a chunk of 32 columns into the three smallest keys.  Plain minima instead of a tournament: the keys are
+// distinct (they carry the column), so key - (smallest + 1) wraps to the top of the unsigned range for the
+// smallest key only, and the minimum of these differences - 28 fused add-and-minimum instructions in four
+// independent chains - belongs to the second smallest; once more from there for the third.
+__device__ __forceinline__ void chunk_update3(const uint32_t (&v)[32], uint32_t key_mult, uint32_t chunk_id, BestThree& state)
 {
 	uint32_t p[32];
 	#pragma unroll
 	for (uint32_t t = 0; t < 32; ++t) p[t] = v[t] * key_mult + t;
-	if (MASKED && nvalid < 32) {
-		#pragma unroll
-		for (uint32_t t = 0; t < 32; ++t) p[t] = t < nvalid ? p[t] : 0xFFFFFFFFu;
-	}
 	auto min_above = [&p](uint32_t key) {          // the smallest key above `key`
 		const uint32_t shift = ~key;               // -(key + 1)
 		uint32_t r0 = p[0] + shift, r1 = p[1] + shift, r2 = p[2] + shift, r3 = p[3] + shift;
@@ -113,12 +132,11 @@ __device__ __forceinline__ void chunk_update3(const uint32_t (&v)[32], uint32_t 
 		return min(umin3(r0, r1, r2), r3) - shift;
 	};
 	const uint32_t b = min_of_32(p), s = min_above(b);
-	const uint32_t t = MASKED && s == 0xFFFFFFFFu ? 0xFFFFFFFFu : min_above(s);
-	state.merge(b, s, t, chunk_id, chunk_id);
+	state.merge(b, s, min_above(s), chunk_id, chunk_id);
 }
 
 
-// The constants that turn accumulator values into integer keys (see chunk_update).
+// The constants that turn accumulator values into integer keys.
 struct KeyConsts {
 	float pow2;          // P: every accumulator value lies in [P, 2P)
 	float offset_c;      // constant added to every |c|^2 - 2 x.c by the extra K step
@@ -165,6 +183,30 @@ __device__ __forceinline__ uint32_t key_column(uint32_t key, uint32_t chunk, uin
 {
 	const uint32_t x = key - key_base;
 	return chunk * 32u + (x - div_key(x, key_magic) * key_mult);
+}
+
+__device__ __forceinline__ void RowMin::finish(uint32_t key_base, uint32_t key_mult, uint32_t key_magic, uint32_t& best_out, uint32_t& second_out, uint32_t& chunk_out) const
+{
+	uint32_t p[16];
+	#pragma unroll
+	for (uint32_t t = 0; t < 16; ++t) p[t] = position[t] * key_mult + t;
+	const uint32_t b = min_of_16(p);
+	// The keys are distinct (they carry the position), so key - (smallest + 1) wraps to the top of the unsigned
+	// range for the smallest only, and the minimum of these differences belongs to the second smallest.
+	const uint32_t shift = ~b;
+	uint32_t r0 = p[0] + shift, r1 = p[1] + shift, r2 = p[2] + shift, r3 = p[3] + shift;
+	#pragma unroll
+	for (uint32_t t = 4; t < 16; t += 4) {
+		r0 = __viaddmin_u32(p[t], shift, r0);
+		r1 = __viaddmin_u32(p[t + 1], shift, r1);
+		r2 = __viaddmin_u32(p[t + 2], shift, r2);
+		r3 = __viaddmin_u32(p[t + 3], shift, r3);
+	}
+	second_out = min(min(umin3(r0, r1, r2), r3) - shift, second);
+	// both smallest keys have the same value part: what is left of the group's key is its number
+	const uint32_t value = div_key(b - key_base, key_magic) * key_mult + key_base;
+	best_out = b + ((best - value) & 1u) * 16u;
+	chunk_out = chunk;
 }
 
 // Appends the points whose `flag` is set to the near-tie list with ONE atomic per warp (a counter
