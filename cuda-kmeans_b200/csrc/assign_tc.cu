@@ -354,13 +354,6 @@ static_assert(SM_ALLOC <= 227 * 1024, "shared memory budget exceeded");
 static_assert(2 * 5 * TC_MA * TC_MTILE * 4 <= SM_BAR_OFF - SM_MERGE_OFF, "merge slots of five words");
 static_assert(KL_AUG_OFF + 2 * AUG_BYTES <= SM_AAUG_OFF, "K-loop stages overlap the constant tile");
 
-// Columns at or behind `nvalid` of a chunk are padding: their keys lie above every key of a value, whatever the column.
-__device__ __forceinline__ void mask_columns(uint32_t (&v)[32], uint32_t nvalid)
-{
-	#pragma unroll
-	for (uint32_t t = 0; t < 32; ++t) v[t] = t < nvalid ? v[t] : 0xFFFFFFFFu;
-}
-
 // What an epilogue warp keeps of a point's row: the two smallest values, or (THREE) the three smallest.
 template<bool THREE> struct RowState;
 template<> struct RowState<false> {
@@ -428,11 +421,10 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __r
 	}
 }
 
-// FULL: k is a whole number of mean tiles of 128 or 256 columns, so no accumulator column is padding
-// and every warp takes its columns in pairs of 32-column chunks: the epilogue runs without its masked
-// path and without the odd-chunk branches.
+// EVEN: mean tiles of 128 or 256 columns, so every warp takes its columns in pairs of 32-column chunks and the
+// epilogue runs without the odd-chunk branches.
 // THREE (K loop with jsplit > 1): the partial results carry the three smallest keys.
-template<bool FULL, bool THREE>
+template<bool EVEN, bool THREE>
 __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 	const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
 	const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
@@ -497,7 +489,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 	const KeyConsts kc = tc_key_consts(x2max, c2max);
 	const float pow2 = kc.pow2;
 	const uint32_t key_mult = kc.key_mult, key_base = kc.key_base, key_magic = kc.key_magic;
-	fill_a_aug(smem + SM_AAUG_OFF, kc.offset_c, threadIdx.x, TC_THREADS);
+	fill_a_aug(smem + SM_AAUG_OFF, kc, x2max, threadIdx.x, TC_THREADS);
 	ptx::fence_proxy_async();
 	ptx::tc_fence_before();
 	__syncthreads();
@@ -750,16 +742,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 						const uint32_t colbase = (first_chunk + c) * 32u;
 						const uint32_t taddr = tmem_base + ((q * 32u) << 16) + i * TC_NT_MAX + colbase;
 						const uint32_t chunk0 = (j * nt_cols + colbase) >> 5;
-						const bool two = FULL ? true : c + 1 < nchunks;
+						const bool two = EVEN ? true : c + 1 < nchunks;
 						uint32_t v0[32], v1[32];
-						const uint32_t col0 = chunk0 * 32u;
-						// columns at or behind k are padding
-						const uint32_t left = FULL ? 64u : (k > col0 ? k - col0 : 0u);
 						// the second chunk travels from tensor memory while the first is reduced
 						ptx::tmem_ld32(taddr, v0);
 						ptx::tmem_ld_wait();
-						if (two) ptx::tmem_ld32(taddr + 32, v1);
-						if (!FULL && left < 32) mask_columns(v0, left);
+						ptx::tmem_ld32(taddr + 32, v1);            // (a chunk that is not there lies inside the accumulator's columns, and is not used)
 						rows.take_chunk(v0, key_mult, chunk0);
 						ptx::tmem_ld_wait();
 						if (c + 2 >= nchunks) {
@@ -771,10 +759,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 							// the chunks just loaded covers the latency
 							if (j == j_end - 1 && half == 0 && p < n) xn = xnorm[p];
 						}
-						if (two) {
-							if (!FULL && left < 64) mask_columns(v1, left > 32 ? left - 32 : 0u);
-							rows.take_chunk(v1, key_mult, chunk0 + 1);
-						}
+						if (two) rows.take_chunk(v1, key_mult, chunk0 + 1);
 					}
 				} else {
 					__syncwarp();
@@ -942,7 +927,7 @@ bool tc_plan_uses_pair(const TcPlan* plan) { return plan && plan->pair_ok && pla
 
 // Where CTA pairs can run they serve what they are better at: the fused update sums, a range of the
 // points, operand rows of 32 words (dim 33..64: 517 against 648 us for 2^21 points and 1024 means), and three
-// or four mean tiles that are not full, whose padding costs the one-CTA kernel column masks (iterations with
+// or four mean tiles that are not full (iterations with
 // 2^21 points, pair / one CTA: k = 900 d = 24 556 / 571, k = 700 d = 32 464 / 469; k = 300, two tiles, 360 / 351).
 // With 16-word rows and full tiles the one-CTA kernel is the faster one (k = 512: 227 against 243 us, k = 1024:
 // 427 against 440 us, 2^21 points of 32 dimensions).
@@ -1020,8 +1005,8 @@ cudaError_t launch_assign_tc(TcPlan* p, uint32_t* asg, Control* ctl, int slot, u
 			ranged ? (uint32_t)((std::min<uint64_t>(p_end, p->tp.n_pad) + 2 * TC_MTILE - 1) / (2 * TC_MTILE)) : 0u);
 	const uint32_t jsplit = plan_jsplit(p);
 	const uint32_t grid_j = jsplit * std::min<uint32_t>(nblocks, (uint32_t)p->sm_count / jsplit);
-	const bool full = p->s.k == p->tm.k_pad && p->nt_cols % 128 == 0, three = tc_plan_collects_pairs(p);
-	auto kern = three ? (full ? assign_tc_kernel<true, true> : assign_tc_kernel<false, true>) : (full ? assign_tc_kernel<true, false> : assign_tc_kernel<false, false>);
+	const bool even = p->nt_cols % 128 == 0, three = tc_plan_collects_pairs(p);
+	auto kern = three ? (even ? assign_tc_kernel<true, true> : assign_tc_kernel<false, true>) : (even ? assign_tc_kernel<true, false> : assign_tc_kernel<false, false>);
 	kern<<<jsplit > 1 ? grid_j : grid, TC_THREADS, SM_ALLOC, stream>>>(p->a_hi, p->a_lo, p->b_hi, p->b_lo,
 		p->tm.b_aug, p->tp.xnorm, asg, p->s.n, n_tiles, p->s.k, p->tm.k_pad, p->nt_cols, kw, kchunks, ksteps_last, idesc,
 		ctl, slot, flag_list, margin_coef, sqrt_dim, jsplit, jsplit > 1 ? p->tp.partial : nullptr, p->tp.n_pad);

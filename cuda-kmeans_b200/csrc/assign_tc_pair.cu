@@ -194,22 +194,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
 	const KeyConsts kc = tc_key_consts(x2max, c2max);
 	const uint32_t key_mult = kc.key_mult, key_base = kc.key_base, key_magic = kc.key_magic;
-	fill_a_aug(smem + P2_AAUG_OFF, kc.offset_c, threadIdx.x, TC_THREADS);
+	fill_a_aug(smem + P2_AAUG_OFF, kc, x2max, threadIdx.x, TC_THREADS);
 	{
 		// This CTA's half of every tile's |c|^2 K step: 128 rows = 4 KiB, contiguous in global memory.
-		// Rows behind the last mean are padding (their operand rows are zero); they get the |c|^2 that
-		// puts their value at 2P - P/32, above every real value (at most 1.83 P) and inside [P, 2P),
-		// so that the arg-min needs no column masks.
 		uint4* dst = reinterpret_cast<uint4*>(smem + baug_off);
 		const uint32_t per_tile = P2_AUG_HALF_BYTES / 16;
-		const uint4 pad_row = tc_aug_row(kc.pow2 - fmaxf(x2max, 1.0f) - kc.pow2 * (1.0f / 16.0f));     // (the offset takes the norm as at least 1, too)
 		for (uint32_t e = threadIdx.x; e < n_ctiles * per_tile; e += TC_THREADS) {
 			const uint32_t j = e / per_tile, r = e - j * per_tile;
-			// 16-byte chunk r of a tile half: row (r / 16) * 8 + r % 8, K positions 8 * ((r / 8) % 2) ..
-			const uint32_t mean = j * TC_NT_MAX + rank * P2_HALF + (r >> 4) * 8 + (r & 7u);
-			uint4 v = reinterpret_cast<const uint4*>(b_aug + ((size_t)j * TC_NT_MAX + rank * P2_HALF) * 8)[r];
-			if (mean >= k && ((r >> 3) & 1u) == 0) v = pad_row;
-			dst[e] = v;
+			dst[e] = reinterpret_cast<const uint4*>(b_aug + ((size_t)j * TC_NT_MAX + rank * P2_HALF) * 8)[r];
 		}
 	}
 	ptx::fence_proxy_async();

@@ -17,7 +17,7 @@ struct Shape {
 struct TcMeans {
 	float* b_hi;     // [k_pad][d_pad words] fp16 high part of -2*mean (centred, scaled by tc_scale), K-major
 	float* b_lo;     // [k_pad][d_pad words] fp16 low part
-	float* b_aug;    // [k_pad x 8 words] one K step of |mean|^2 (aug_offset layout, see tc_aug_row); padding rows: 0
+	float* b_aug;    // [k_pad x 8 words] one K step of |mean|^2 (aug_offset layout, see tc_aug_row and tc_aug_padding_row)
 	float* center;   // [dim] vector subtracted from points and means alike before the split (distances do
 	                 // not change; the norms, and with them the cancellation of the GEMM form, shrink)
 	uint32_t k_pad;  // k rounded up to the centroid tile

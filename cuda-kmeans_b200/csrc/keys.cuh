@@ -17,8 +17,7 @@ __device__ __forceinline__ uint32_t umin3(uint32_t a, uint32_t b, uint32_t c) { 
 // all of them are positive floats with the SAME exponent; their bit patterns then order like the
 // values, the upper exponent bits carry no information, and bits * M + column (M odd, > column:
 // one integer multiply-add, off the min/max pipe) is a key that keeps the full 23-bit mantissa
-// and carries the column position.  The keys are reduced to the two smallest and merged into the running
-// (best, second, chunk of best).  `nvalid` < 32 masks the padding columns behind the last mean.
+// and carries the column position.
 // Smallest of 32 keys with three-input minima (16 instructions).
 __device__ __forceinline__ uint32_t min_of_32(const uint32_t (&p)[32])
 {

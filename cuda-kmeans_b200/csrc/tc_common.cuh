@@ -87,13 +87,16 @@ constexpr uint32_t DESC_HI_SW64 = 32u | (1u << 14) | (4u << 29);      // 64-byte
 __device__ __forceinline__ uint32_t desc_lo_sw128(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3FFFu) | (1u << 16); }
 __device__ __forceinline__ uint32_t desc_lo_aug(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3FFFu) | (8u << 16); }
 
-// The constant A operand of the extra K step (128 rows, no-swizzle layout): see tc_aug_row.
-__device__ __forceinline__ void fill_a_aug(uint8_t* a_aug, float offset_c, uint32_t tid, uint32_t nthreads)
+// The constant A operand of the extra K step (128 rows, no-swizzle layout): see tc_aug_row.  Padding columns get the value
+// 2P - P/32 (and the rounding of two fp16 values), above every real value (at most 1.83 P) and inside [P, 2P), so
+// that the arg-min needs no column masks.
+__device__ __forceinline__ void fill_a_aug(uint8_t* a_aug, const KeyConsts& kc, float x2max, uint32_t tid, uint32_t nthreads)
 {
+	const float offset_c = kc.offset_c, padding = kc.pow2 - fmaxf(x2max, 1.0f) - kc.pow2 * (1.0f / 16.0f);     // (the offset takes the norm as at least 1, too)
 	const __half a0 = __float2half_rn(TC_AUG_A0), a1 = __float2half_rn(TC_AUG_A1), a2 = __float2half_rn(TC_AUG_A2);
-	const __half a3 = __float2half_rn(offset_c * (1.0f / TC_AUG_B3));
+	const __half a3 = __float2half_rn(offset_c * (1.0f / TC_AUG_B3)), a4 = __float2half_rn(padding * (1.0f / TC_AUG_B3));
 	const uint4 row = make_uint4((uint32_t)__half_as_ushort(a0) | ((uint32_t)__half_as_ushort(a1) << 16),
-		(uint32_t)__half_as_ushort(a2) | ((uint32_t)__half_as_ushort(a3) << 16), 0u, 0u);
+		(uint32_t)__half_as_ushort(a2) | ((uint32_t)__half_as_ushort(a3) << 16), (uint32_t)__half_as_ushort(a4), 0u);
 	uint32_t* words = reinterpret_cast<uint32_t*>(a_aug);
 	for (uint32_t r = tid; r < TC_MTILE; r += nthreads) {
 		*reinterpret_cast<uint4*>(words + aug_offset(r, 0)) = row;

@@ -30,7 +30,8 @@ __device__ __forceinline__ void tc_split2(float x0, float x1, uint32_t& hi, uint
 
 // The extra K step.  Columns 0..2 carry v = |c|^2 (at most TC_NORM2_MAX): fp16 values on the mean's
 // side against 2^15, 2^4 and 2^-7 on the points' side, exact to 33 bits; column 3 carries the offset
-// constant of the keys as an fp16 value on the points' side against 2^15 on the mean's side.
+// constant of the keys as an fp16 value on the points' side against 2^15 on the mean's side.  Column 4 is for the padding
+// rows behind the last mean: 2^15 there and 0 for the means, against what puts their value above that of every mean.
 constexpr float TC_AUG_A0 = 32768.0f, TC_AUG_A1 = 16.0f, TC_AUG_A2 = 0.0078125f, TC_AUG_B3 = 32768.0f;
 
 __device__ __forceinline__ uint4 tc_aug_row(float v)
@@ -43,6 +44,12 @@ __device__ __forceinline__ uint4 tc_aug_row(float v)
 	const __half b2 = __float2half_rn(r2 * (1.0f / TC_AUG_A2));
 	return make_uint4((uint32_t)__half_as_ushort(b0) | ((uint32_t)__half_as_ushort(b1) << 16),
 		(uint32_t)__half_as_ushort(b2) | ((uint32_t)__half_as_ushort(__float2half_rn(TC_AUG_B3)) << 16), 0u, 0u);
+}
+
+__device__ __forceinline__ uint4 tc_aug_padding_row()
+{
+	const uint32_t b = (uint32_t)__half_as_ushort(__float2half_rn(TC_AUG_B3));
+	return make_uint4(0u, b << 16, b, 0u);
 }
 
 } // namespace bkm

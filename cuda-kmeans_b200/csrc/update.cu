@@ -112,7 +112,7 @@ __device__ __forceinline__ void finish_padding_row(const RowSinks& o, uint32_t c
 {
 	if (o.cprep && c < o.srows) o.cprep[(size_t)c * o.rs] = INFINITY;
 	if (o.b_aug && c < o.k_pad) {
-		*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 0)) = tc_aug_row(0.0f);
+		*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 0)) = tc_aug_padding_row();
 		*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 1)) = make_uint4(0u, 0u, 0u, 0u);
 	}
 }
