@@ -1,6 +1,6 @@
 // Assignment on CUDA cores.
 //
-//  * assign_exact_kernel: one warp per point, lanes over the means, the reference's arithmetic
+//  * assign_exact_kernel: tiles of points and means, the reference's arithmetic
 //    (sequential subtract / multiply / add without fusing, square root, strictly-smaller
 //    comparison in ascending index order).  Used for every point by the EXACT variant and
 //    for the queued near-ties of the fast passes.  Replaces baseAssignmentKernel
@@ -21,313 +21,248 @@ namespace bkm {
 // ------------------------------------------------------------------------------------------
 // exact kernel
 // ------------------------------------------------------------------------------------------
+//
+// The reference's arithmetic for a list of queued points, or for all points (list == null): subtract,
+// multiply, add in dimension order with one rounding each, square root, strictly smaller in ascending
+// index order.  A block takes 64 points and 128 means at a time, a thread four points and eight means of them; the
+// operands lie dimension-major in shared memory, and additions work on two neighbouring means at a time
+// (add.rn.f32x2: each half is rounded like the scalar operation), so a dimension costs a thread 64 arithmetic
+// instructions and four 128-bit loads.  Lists too short to fill the machine in that way go through tiles of 32
+// means, as many blocks to a group of points as there are.  The kernel before (one mean and 4 or 16 points per
+// thread, scalar) spent more instructions on loads and barriers than on arithmetic: list of 58 800 points of 50
+// dimensions against 1000 means 818 us, now 427 (its 9.0e9 dimension pairs are 176 us of issue slots at 68
+// instructions for 32); 51 900 of 200 against 300 1261 -> 553 us; 22 900 of 32 against 512 106 -> 70 us; 44
+// points of 512 against 4096 46 -> 43 us.
+constexpr int EX_THREADS = 256;
+constexpr uint32_t EX_POINTS = 64, EX_DIMS = 32;                       // of a block: points, dimensions per slab
+constexpr uint32_t EX_PSTRIDE = 2 * EX_POINTS + 8;                     // floats per dimension: every coordinate twice (the two halves of an operand)
+constexpr uint32_t EX_MSTRIDE = 128 + 4;                               // floats per dimension: up to 128 negated means
+constexpr uint32_t EX_RESIDENT_DIMS = 2 * EX_DIMS;                     // up to here a block's points stay in shared memory for all means
+constexpr uint32_t EX_MAX_BLOCKS = 512;                                // for lists whose groups of points are shared between blocks
 
-template<bool SOA, bool SOAM>
-__global__ void __launch_bounds__(256) assign_exact_kernel(const float* __restrict__ pts,
-	const float* __restrict__ means, uint32_t* __restrict__ asg, uint64_t n, uint32_t k, uint32_t d,
-	const uint32_t* __restrict__ list, const uint32_t* __restrict__ list_count)
+// The nearest of the mean tiles [t_begin, t_end), PAIRS * 32 means each, for the block's 64 points: the thread's
+// four points (4 ty ..) against its means of every tile, as (distance, index) of the nearest it has seen.
+// Strides of both arrays put the 8 dimensions x 4 items that a warp stores at a time (row-major sources: 32-byte pieces of
+// four rows) into different banks.
+template<bool SOA, bool SOAM, bool RESIDENT, int PAIRS>
+__device__ __forceinline__ void exact_scan(const float* __restrict__ pts, const float* __restrict__ means, uint64_t n, uint32_t k, uint32_t d,
+	const uint32_t* s_index, float* s_points, float* s_means, uint32_t t_begin, uint32_t t_end, unsigned long long (&key)[4])
 {
-	extern __shared__ float sx[];
-	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-	float* x = sx + (size_t)warp * d;
-	uint64_t total = n;
-	if (list != nullptr) {
-		uint64_t c = *list_count;
-		total = c < n ? c : n;
-	}
-	for (uint64_t w = (uint64_t)blockIdx.x * wpb + warp; w < total; w += (uint64_t)gridDim.x * wpb) {
-		const uint64_t i = list ? (uint64_t)list[w] : w;
-		__syncwarp();
-		for (uint32_t j = lane; j < d; j += 32) x[j] = pts[at<SOA>(i, j, n, d)];
-		__syncwarp();
-		float best = INFINITY;
-		uint32_t bidx = 0xffffffffu;
-		for (uint32_t m = lane; m < k; m += 32) {
-			float sum = 0.0f;
-			for (uint32_t j = 0; j < d; ++j) {
-				float diff = __fsub_rn(x[j], means[at<SOAM>(m, j, k, d)]);
-				sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-			}
-			float dist = __fsqrt_rn(sum);
-			if (dist < best || (dist == best && m < bidx)) { best = dist; bidx = m; }
-			// what is not a number never wins, but nothing replaces it as the first distance of the sequential scan
-			if (m == 0 && dist != dist) { best = 0.0f; bidx = 0; }
-		}
-		// lowest (distance, index) pair over the warp = what the sequential scan would keep
+	static_assert(PAIRS == 1 || PAIRS == 4, "pairs of means per thread");
+	constexpr uint32_t TILE = PAIRS * 32;               // means of a tile
+	constexpr uint32_t LOADS = TILE * EX_DIMS / EX_THREADS;
+	const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, tx = tid & 15u, ty = tid >> 4;
+	const uint32_t slabs = (d + EX_DIMS - 1) / EX_DIMS;
+
+	// slab of the points / of a mean tile -> registers; registers -> shared memory
+	auto fetch_points = [&](uint32_t j0, float (&r)[8]) {
 		#pragma unroll
-		for (int off = 16; off > 0; off >>= 1) {
-			float ob = __shfl_xor_sync(0xffffffffu, best, off);
-			uint32_t oi = __shfl_xor_sync(0xffffffffu, bidx, off);
-			if (ob < best || (ob == best && oi < bidx)) { best = ob; bidx = oi; }
-		}
-		if (lane == 0) asg[i] = bidx;
-	}
-}
-
-
-// Four consecutive dimensions of one mean against the LIST_PB staged points: each point's four
-// coordinates come with one 128-bit shared load (the same address for the whole warp), and the
-// squares are added in dimension order, one rounding per operation, as in the scalar loop.
-template<int PB>
-__device__ __forceinline__ void add_four_dims(float (&sum)[PB], const float* sx, uint32_t dpad, uint32_t j,
-	float c0, float c1, float c2, float c3)
-{
-	#pragma unroll
-	for (int p = 0; p < PB; ++p) {
-		const float4 x = *reinterpret_cast<const float4*>(sx + p * dpad + j);
-		const float d0 = __fsub_rn(x.x, c0), d1 = __fsub_rn(x.y, c1), d2 = __fsub_rn(x.z, c2), d3 = __fsub_rn(x.w, c3);
-		sum[p] = __fadd_rn(sum[p], __fmul_rn(d0, d0));
-		sum[p] = __fadd_rn(sum[p], __fmul_rn(d1, d1));
-		sum[p] = __fadd_rn(sum[p], __fmul_rn(d2, d2));
-		sum[p] = __fadd_rn(sum[p], __fmul_rn(d3, d3));
-	}
-}
-
-// The same arithmetic for a list of queued points: one block per PB points, one mean per
-// thread at a time, so that a short list still fills the machine and every mean that is
-// fetched serves PB points (4, or 16 for long rows and many means, where the re-reads of the means
-// for every group of points are what the kernel spends its time on).  Each distance is still summed in dimension order by a single
-// thread.  AoS means are staged through a shared tile (32 dimensions of 256 means at a time,
-// loaded along the dimensions) so that the global loads stay coalesced; SoA means are read
-// directly (consecutive threads = consecutive means).
-constexpr int LIST_THREADS = 256;
-constexpr int LIST_PB = 4;          // points per block (the default)
-constexpr int LIST_PB_WIDE = 16;    // ... when every fetched mean should serve more points (long rows, many means)
-constexpr uint32_t LIST_SPLIT_MAX_BLOCKS = 2048;   // grid size up to which a short list is shared between blocks
-
-template<bool SOA, bool SOAM, int PB>
-__global__ void __launch_bounds__(LIST_THREADS, PB > LIST_PB ? 2 : 3) assign_exact_list_kernel(const float* __restrict__ pts,
-	const float* __restrict__ means, uint32_t* __restrict__ asg, uint64_t n, uint32_t k, uint32_t d,
-	const uint32_t* __restrict__ list, const uint32_t* __restrict__ list_count,
-	float* __restrict__ fix_acc, uint32_t* __restrict__ fix_counts, uint32_t resident_ok,
-	unsigned long long* __restrict__ split_keys, uint32_t* __restrict__ split_arrive)
-{
-	extern __shared__ __align__(16) float sx[];         // PB points (dpad floats each), then the means tile
-	__shared__ uint32_t smoved[PB][2];             // (old, new) cluster of a point that changed, else old == new
-	__shared__ uint32_t s_last;                         // this block is the last of its group's blocks to finish
-	const uint32_t dpad = (d + 3) & ~3u;
-	float (*tile)[33] = reinterpret_cast<float (*)[33]>(sx + (size_t)PB * dpad);
-	__shared__ float sbest[PB][LIST_THREADS / 32];
-	__shared__ uint32_t sidx[PB][LIST_THREADS / 32];
-	const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-	uint64_t total = *list_count;
-	if (total > n) total = n;
-	// A long list and few means: every block copies all means to shared memory once (rows of an
-	// odd number of floats, one mean per thread -> conflict-free) instead of fetching them again
-	// for every group of points.
-	const uint32_t ds = d | 1u;
-	float* mres = sx + (size_t)PB * dpad;
-	const bool resident = resident_ok != 0 && total >= (uint64_t)gridDim.x * PB * 4;
-	if (resident) {
-		for (uint32_t e = tid; e < k * d; e += LIST_THREADS) {
-			// e walks the means array in memory order (coalesced)
-			const uint32_t m = SOAM ? e % k : e / d, j = SOAM ? e / k : e % d;
-			mres[m * ds + j] = means[e];
-		}
-	}
-	// Staging of a group's points: two dependent global reads (the list entry, then the coordinate)
-	// for each of the PB * d floats, all of them in flight together.  With few dimensions
-	// (at most two floats per thread) a thread fetches the NEXT group's floats into registers
-	// while the block works on the current group, which takes both reads off the block's
-	// critical path.  Unused slots of the last group repeat its first point.
-	const uint32_t pe = PB * d;
-	const bool prefetch = pe <= 2 * LIST_THREADS;
-	uint32_t pf_p[2], pf_j[2];
-	float pf[2] = {0.0f, 0.0f};
-	#pragma unroll
-	for (uint32_t r = 0; r < 2; ++r) {
-		const uint32_t e = tid + r * LIST_THREADS;
-		pf_p[r] = e / d;
-		pf_j[r] = e - pf_p[r] * d;
-	}
-	auto fetch = [&](uint64_t g0) {
-		#pragma unroll
-		for (uint32_t r = 0; r < 2; ++r) {
-			if (tid + r * LIST_THREADS < pe) {
-				const uint64_t idx = g0 + pf_p[r] < total ? g0 + pf_p[r] : g0;
-				pf[r] = pts[at<SOA>((uint64_t)list[idx], pf_j[r], n, d)];
-			}
+		for (uint32_t e = 0; e < 8; ++e) {
+			const uint32_t j = j0 + (SOA ? e * 4 + (tid >> 6) : (e & 3u) * 8 + (lane >> 2));
+			const uint32_t p = SOA ? tid & 63u : (e >> 2) * 32 + warp * 4 + (lane & 3u);
+			r[e] = j < d ? pts[at<SOA>((uint64_t)s_index[p], j, n, d)] : 0.0f;
 		}
 	};
-	// A short list (fewer groups than blocks) would leave most of the machine idle while a few
-	// blocks walk all k means one after another.  The blocks then share the groups: `splits`
-	// blocks take one group, each a contiguous range of the means, and combine their results in
-	// global memory (see below); every block has at most one piece of work.
-	const uint64_t groups = (total + PB - 1) / PB;
-	const uint32_t mchunks = (k + LIST_THREADS - 1) / LIST_THREADS;
-	uint32_t splits = 1;
-	if (split_keys != nullptr && groups > 0 && groups < gridDim.x && gridDim.x <= LIST_SPLIT_MAX_BLOCKS && mchunks > 1) {
-		splits = gridDim.x / (uint32_t)groups;
-		if (splits > mchunks) splits = mchunks;
+	auto store_points = [&](float* dst, const float (&r)[8]) {
+		#pragma unroll
+		for (uint32_t e = 0; e < 8; ++e) {
+			const uint32_t j = SOA ? e * 4 + (tid >> 6) : (e & 3u) * 8 + (lane >> 2);
+			const uint32_t p = SOA ? tid & 63u : (e >> 2) * 32 + warp * 4 + (lane & 3u);
+			*reinterpret_cast<float2*>(dst + j * EX_PSTRIDE + 2 * p) = make_float2(r[e], r[e]);
+		}
+	};
+	auto fetch_means = [&](uint32_t m0, uint32_t j0, float (&r)[LOADS]) {
+		#pragma unroll
+		for (uint32_t e = 0; e < LOADS; ++e) {
+			const uint32_t j = j0 + (SOAM ? (e * EX_THREADS + tid) / TILE : (e & 3u) * 8 + (lane >> 2));
+			const uint32_t m = m0 + (SOAM ? tid % TILE : (e >> 2) * 32 + warp * 4 + (lane & 3u));
+			// (a distance to what lies behind the last mean is infinite, or not a number: it never wins)
+			r[e] = m < k ? (j < d ? -means[at<SOAM>(m, j, k, d)] : 0.0f) : -INFINITY;
+		}
+	};
+	auto store_means = [&](float* dst, const float (&r)[LOADS]) {
+		#pragma unroll
+		for (uint32_t e = 0; e < LOADS; ++e) {
+			const uint32_t j = SOAM ? (e * EX_THREADS + tid) / TILE : (e & 3u) * 8 + (lane >> 2);
+			const uint32_t m = SOAM ? tid % TILE : (e >> 2) * 32 + warp * 4 + (lane & 3u);
+			dst[j * EX_MSTRIDE + m] = r[e];
+		}
+	};
+
+	float rp[8], rm[LOADS];
+	fetch_means(t_begin * TILE, 0, rm);
+	if (RESIDENT) {
+		for (uint32_t sl = 0; sl < slabs; ++sl) {
+			fetch_points(sl * EX_DIMS, rp);
+			store_points(s_points + sl * EX_DIMS * EX_PSTRIDE, rp);
+		}
+	} else {
+		fetch_points(0, rp);
 	}
-	const uint32_t split_group = blockIdx.x / splits, split_part = blockIdx.x - split_group * splits;
-	const uint32_t m_begin = splits > 1 ? (split_part * mchunks / splits) * LIST_THREADS : 0u;
-	const uint32_t m_end = splits > 1 ? min(k, ((split_part + 1) * mchunks / splits) * LIST_THREADS) : k;
-	const uint32_t n_chunks = (m_end - m_begin + LIST_THREADS - 1) / LIST_THREADS;
-	const uint32_t chunk_rot = (splits > 1 ? split_group : blockIdx.x) % n_chunks;
-	const uint64_t stride = (uint64_t)gridDim.x * PB;        // with splits > 1 one step leaves the list
-	const uint64_t w_first = (uint64_t)(splits > 1 ? split_group : blockIdx.x) * PB;
-	if (prefetch && w_first < total) fetch(w_first);
-	for (uint64_t w0 = w_first; w0 < total; w0 += stride) {
-		const uint32_t np = total - w0 < PB ? (uint32_t)(total - w0) : PB;
-		__syncthreads();
-		if (prefetch) {
-			#pragma unroll
-			for (uint32_t r = 0; r < 2; ++r)
-				if (tid + r * LIST_THREADS < pe) sx[pf_p[r] * dpad + pf_j[r]] = pf[r];
-		} else {
-			for (uint32_t e = tid; e < pe; e += LIST_THREADS) {
-				const uint32_t p = e / d, j = e - p * d;
-				const uint64_t idx = w0 + p < total ? w0 + p : w0;
-				sx[p * dpad + j] = pts[at<SOA>((uint64_t)list[idx], j, n, d)];
-			}
-		}
-		__syncthreads();
-		if (prefetch && w0 + stride < total) fetch(w0 + stride);
-		float best[PB];
-		uint32_t bidx[PB];
+
+	float best[4], best_sum[4];
+	uint32_t bidx[4];
+	#pragma unroll
+	for (int p = 0; p < 4; ++p) { best[p] = best_sum[p] = INFINITY; bidx[p] = 0xffffffffu; }
+	uint32_t buf = 0;
+	for (uint32_t t = t_begin; t < t_end; ++t) {
+		uint64_t sum[4][PAIRS];                         // means 4 tx + 0..3 and 64 + 4 tx + 0..3, or 2 tx + 0..1
 		#pragma unroll
-		for (int p = 0; p < PB; ++p) { best[p] = INFINITY; bidx[p] = 0xffffffffu; }
-		// The blocks walk their chunks of 256 means starting at different chunks, so that blocks
-		// working at the same time do not all ask the L2 for the same rows at once.
-		for (uint32_t c = 0; c < n_chunks; ++c) {
-			const uint32_t m0 = m_begin + (c + chunk_rot < n_chunks ? c + chunk_rot : c + chunk_rot - n_chunks) * LIST_THREADS;
-			const uint32_t m = m0 + tid;
-			float sum[PB];
+		for (int p = 0; p < 4; ++p)
 			#pragma unroll
-			for (int p = 0; p < PB; ++p) sum[p] = 0.0f;
-			if (resident) {
-				if (m < k) {
-					const float* cm = mres + m * ds;
-					uint32_t j = 0;
-					for (; j + 4 <= d; j += 4) add_four_dims<PB>(sum, sx, dpad, j, cm[j], cm[j + 1], cm[j + 2], cm[j + 3]);
-					for (; j < d; ++j) {
-						const float c = cm[j];
-						#pragma unroll
-						for (int p = 0; p < PB; ++p) {
-							const float diff = __fsub_rn(sx[p * dpad + j], c);
-							sum[p] = __fadd_rn(sum[p], __fmul_rn(diff, diff));
-						}
-					}
-				}
-			} else if (SOAM) {
-				if (m < k) {
-					const float* cm = means + m;
-					uint32_t j = 0;
-					for (; j + 4 <= d; j += 4)
-						add_four_dims<PB>(sum, sx, dpad, j, cm[(size_t)j * k], cm[(size_t)(j + 1) * k], cm[(size_t)(j + 2) * k], cm[(size_t)(j + 3) * k]);
-					for (; j < d; ++j) {
-						const float c = cm[(size_t)j * k];
-						#pragma unroll
-						for (int p = 0; p < PB; ++p) {
-							const float diff = __fsub_rn(sx[p * dpad + j], c);
-							sum[p] = __fadd_rn(sum[p], __fmul_rn(diff, diff));
-						}
-					}
-				}
-			} else {
-				// 32 dimensions of the chunk's 256 means at a time go through the shared tile (read along
-				// the rows, used along the means).  The next slab's row segments are fetched into registers
-				// while the current slab is evaluated, so their latency does not sit between two barriers.
-				float seg[32];
-				auto fetch_slab = [&](uint32_t j0) {
-					#pragma unroll
-					for (uint32_t r = 0; r < 32; ++r) {
-						const uint32_t row = warp * 32 + r;
-						seg[r] = (m0 + row < k && j0 + lane < d) ? means[(size_t)(m0 + row) * d + j0 + lane] : 0.0f;
-					}
-				};
-				fetch_slab(0);
-				for (uint32_t j0 = 0; j0 < d; j0 += 32) {
-					__syncthreads();                    // the previous slab has been read by everyone
-					#pragma unroll
-					for (uint32_t r = 0; r < 32; ++r) tile[warp * 32 + r][lane] = seg[r];
-					__syncthreads();
-					if (j0 + 32 < d) fetch_slab(j0 + 32);
-					const uint32_t jn = d - j0 < 32 ? d - j0 : 32;
-					uint32_t jj = 0;
-					for (; jj + 4 <= jn; jj += 4)
-						add_four_dims<PB>(sum, sx, dpad, j0 + jj, tile[tid][jj], tile[tid][jj + 1], tile[tid][jj + 2], tile[tid][jj + 3]);
-					for (; jj < jn; ++jj) {
-						const float c = tile[tid][jj];
-						#pragma unroll
-						for (int p = 0; p < PB; ++p) {
-							const float diff = __fsub_rn(sx[p * dpad + j0 + jj], c);
-							sum[p] = __fadd_rn(sum[p], __fmul_rn(diff, diff));
-						}
-					}
-				}
+			for (int q = 0; q < PAIRS; ++q) sum[p][q] = 0;
+		for (uint32_t sl = 0; sl < slabs; ++sl) {
+			float* mslab = s_means + buf * EX_DIMS * EX_MSTRIDE;
+			float* pslab = s_points + (RESIDENT ? sl : buf) * EX_DIMS * EX_PSTRIDE;
+			store_means(mslab, rm);
+			if (!RESIDENT) store_points(pslab, rp);
+			// (one barrier per slab: the slab before the previous one has been read by all when this one is written)
+			__syncthreads();
+			const bool same = sl + 1 < slabs;
+			if (same || t + 1 < t_end) {
+				fetch_means((same ? t : t + 1) * TILE, same ? (sl + 1) * EX_DIMS : 0u, rm);
+				if (!RESIDENT) fetch_points(same ? (sl + 1) * EX_DIMS : 0u, rp);
 			}
-			if (m < k) {
+			const uint32_t jn = min(EX_DIMS, d - sl * EX_DIMS);
+			const float* mrow = mslab + (PAIRS == 4 ? 4 : 2) * tx;
+			const float* prow = pslab + 8 * ty;
+			#pragma unroll 4
+			for (uint32_t j = 0; j < jn; ++j) {
+				uint64_t mm[PAIRS];
+				if (PAIRS == 4) {
+					const ulonglong2 m0 = *reinterpret_cast<const ulonglong2*>(mrow + j * EX_MSTRIDE);
+					const ulonglong2 m1 = *reinterpret_cast<const ulonglong2*>(mrow + j * EX_MSTRIDE + 64);
+					mm[0] = m0.x; mm[PAIRS / 4] = m0.y; mm[PAIRS / 2] = m1.x; mm[PAIRS - 1] = m1.y;
+				} else {
+					mm[0] = *reinterpret_cast<const unsigned long long*>(mrow + j * EX_MSTRIDE);
+				}
+				const ulonglong2 p0 = *reinterpret_cast<const ulonglong2*>(prow + j * EX_PSTRIDE);
+				const ulonglong2 p1 = *reinterpret_cast<const ulonglong2*>(prow + j * EX_PSTRIDE + 4);
+				const uint64_t pp[4] = {p0.x, p0.y, p1.x, p1.y};
 				#pragma unroll
-				for (int p = 0; p < PB; ++p) {
-					const float dist = __fsqrt_rn(sum[p]);
-					// (the chunks come in rotated order: the lower index wins a tie explicitly)
-					if (dist < best[p] || (dist == best[p] && m < bidx[p])) { best[p] = dist; bidx[p] = m; }
-					// what is not a number never wins, but nothing replaces it as the first distance of the sequential scan
-					if (m == 0 && dist != dist) { best[p] = 0.0f; bidx[p] = 0; }
+				for (int p = 0; p < 4; ++p)
+					#pragma unroll
+					for (int q = 0; q < PAIRS; ++q) sum[p][q] = ptx::add2(sum[p][q], ptx::square2(ptx::add2(pp[p], mm[q])));
+			}
+			buf ^= 1u;
+		}
+		// The reference compares square roots.  The correctly rounded square root never decreases with its
+		// argument, so only a sum below the best sum can give a smaller root (equal roots of different sums keep
+		// the earlier mean, as the reference's strict comparison does).
+		const uint32_t m_first = t * TILE + (PAIRS == 4 ? 4 : 2) * tx;
+		#pragma unroll
+		for (int p = 0; p < 4; ++p) {
+			float v[2 * PAIRS];
+			#pragma unroll
+			for (int q = 0; q < PAIRS; ++q) {
+				uint32_t lo, hi;
+				ptx::unpack2(sum[p][q], lo, hi);
+				v[2 * q] = __uint_as_float(lo);
+				v[2 * q + 1] = __uint_as_float(hi);
+			}
+			if (m_first == 0 && !(v[0] < INFINITY)) {
+				// the first mean is taken whatever its distance; nothing replaces what is not a number
+				bidx[p] = 0;
+				if (v[0] != v[0]) best[p] = best_sum[p] = 0.0f;
+			}
+			#pragma unroll
+			for (int q = 0; q < 2 * PAIRS; ++q) {
+				if (v[q] < best_sum[p]) {
+					const float dist = __fsqrt_rn(v[q]);
+					if (dist < best[p]) { best[p] = dist; best_sum[p] = v[q]; bidx[p] = m_first + (q < 4 ? q : 60 + q); }
 				}
 			}
 		}
-		#pragma unroll
-		for (int p = 0; p < PB; ++p) {
-			// Distances are >= +0, so their bit patterns order like the values: the warp's smallest
-			// distance, then the lowest index among the means that have it (a thread without a mean
-			// holds infinity and the index 0xffffffff).
-			const uint32_t bits = __float_as_uint(best[p]);
-			const uint32_t mn = __reduce_min_sync(0xffffffffu, bits);
-			const uint32_t mi = __reduce_min_sync(0xffffffffu, bits == mn ? bidx[p] : 0xffffffffu);
-			if (lane == 0) { sbest[p][warp] = __uint_as_float(mn); sidx[p][warp] = mi; }
+	}
+	// distances are >= +0, so their bit patterns order like the values
+	#pragma unroll
+	for (int p = 0; p < 4; ++p) key[p] = ((unsigned long long)__float_as_uint(best[p]) << 32) | bidx[p];
+}
+
+template<bool SOA, bool SOAM, bool RESIDENT>
+__global__ void __launch_bounds__(EX_THREADS, 2) assign_exact_kernel(const float* __restrict__ pts,
+	const float* __restrict__ means, uint32_t* __restrict__ asg, uint64_t n, uint32_t k, uint32_t d,
+	const uint32_t* __restrict__ list, const uint32_t* __restrict__ list_count,
+	float* __restrict__ fix_acc, uint32_t* __restrict__ fix_counts,
+	unsigned long long* __restrict__ split_keys, uint32_t* __restrict__ split_arrive)
+{
+	extern __shared__ __align__(16) float sx[];         // points: all dimensions, or two slabs of them; then two slabs of means
+	__shared__ uint32_t s_index[EX_POINTS];
+	__shared__ uint32_t s_moved[EX_POINTS][2];          // (old, new) cluster of a point that changed, else old == new
+	__shared__ uint32_t s_last;                         // this block is the last of its group's blocks to finish
+	const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
+	uint64_t total = n;
+	if (list != nullptr) {
+		const uint64_t c = *list_count;
+		total = c < n ? c : n;
+	}
+	float* s_means = sx + (RESIDENT ? (d + EX_DIMS - 1) / EX_DIMS : 2u) * EX_DIMS * EX_PSTRIDE;
+	const uint64_t groups = (total + EX_POINTS - 1) / EX_POINTS;
+	// Few points would leave most of the machine idle while a few blocks walk all means.  The blocks then share
+	// the groups: `splits` blocks take one group, each a contiguous range of the means in narrow tiles, and
+	// combine their results in global memory; every block has at most one piece of work.
+	uint32_t splits = 1, mtiles = (k + 127) / 128;
+	const bool narrow = split_keys != nullptr && gridDim.x <= EX_MAX_BLOCKS && groups * mtiles < gridDim.x;
+	if (narrow) mtiles = (k + 31) / 32;
+	if (split_keys != nullptr && gridDim.x <= EX_MAX_BLOCKS && groups > 0 && groups < gridDim.x) splits = min(gridDim.x / (uint32_t)groups, mtiles);
+	const uint32_t part = blockIdx.x % splits;
+	const uint32_t t_begin = part * mtiles / splits, t_end = (part + 1) * mtiles / splits;
+	const uint64_t stride = splits > 1 ? groups : gridDim.x;   // (shared groups: one piece of work per block)
+
+	for (uint64_t grp = blockIdx.x / splits; grp < groups; grp += stride) {
+		const uint64_t w0 = grp * EX_POINTS;
+		const uint32_t np = total - w0 < EX_POINTS ? (uint32_t)(total - w0) : EX_POINTS;
+		__syncthreads();                                // the previous group is done with the shared arrays
+		if (tid < EX_POINTS) {
+			const uint64_t e = tid < np ? w0 + tid : w0;  // unused slots repeat the first point
+			s_index[tid] = list ? list[e] : (uint32_t)e;
 		}
 		__syncthreads();
-		if (tid < np) {
-			float b = sbest[tid][0];
-			uint32_t bi = sidx[tid][0];
-			for (uint32_t v = 1; v < LIST_THREADS / 32; ++v) {
-				const float ob = sbest[tid][v];
-				const uint32_t oi = sidx[tid][v];
-				if (oi != 0xffffffffu && (bi == 0xffffffffu || ob < b || (ob == b && oi < bi))) { b = ob; bi = oi; }
+		unsigned long long key[4], mine = 0;
+		if (narrow) exact_scan<SOA, SOAM, RESIDENT, 1>(pts, means, n, k, d, s_index, sx, s_means, t_begin, t_end, key);
+		else exact_scan<SOA, SOAM, RESIDENT, 4>(pts, means, n, k, d, s_index, sx, s_means, t_begin, t_end, key);
+
+		// lowest (distance, index) over the sixteen threads of a point
+		#pragma unroll
+		for (int p = 0; p < 4; ++p) {
+			#pragma unroll
+			for (int off = 8; off > 0; off >>= 1) {
+				const unsigned long long o = __shfl_xor_sync(0xffffffffu, key[p], off);
+				key[p] = o < key[p] ? o : key[p];
 			}
-			if (splits > 1) {
-				// (distance, index) as one 64-bit key whose minimum is the smallest distance and, among
-				// equal distances, the lowest index; stored inverted so that zero means "nothing yet"
-				const unsigned long long key = ((unsigned long long)__float_as_uint(b) << 32) | bi;
-				atomicMax(&split_keys[w0 + tid], ~key);
-			} else {
-				const uint32_t i = list[w0 + tid];
-				smoved[tid][0] = fix_acc ? asg[i] : bi;
-				smoved[tid][1] = bi;
-				asg[i] = bi;
-			}
+			if ((uint32_t)p == tx) mine = key[p];
 		}
+		const uint32_t q = ty * 4 + tx;                 // the point that this thread (tx < 4) reports
+		const bool reports = tx < 4 && q < np;
 		if (splits > 1) {
+			// stored inverted, so that zero means "nothing yet"
+			if (reports) atomicMax(&split_keys[w0 + q], ~mine);
 			// The block that arrives last for its group finds all partial results in place; it
 			// writes the assignment and leaves keys and counter zeroed for the next launch.
 			__threadfence();
 			__syncthreads();
-			if (tid == 0) s_last = atomicAdd(&split_arrive[split_group], 1u) == splits - 1 ? 1u : 0u;
+			if (tid == 0) s_last = atomicAdd(&split_arrive[grp], 1u) == splits - 1 ? 1u : 0u;
 			__syncthreads();
 			if (s_last == 0) break;
 			__threadfence();
-			if (tid < np) {
-				const unsigned long long key = ~atomicExch(&split_keys[w0 + tid], 0ull);
-				const uint32_t bi = (uint32_t)key;
-				const uint32_t i = list[w0 + tid];
-				smoved[tid][0] = fix_acc ? asg[i] : bi;
-				smoved[tid][1] = bi;
-				asg[i] = bi;
-			}
-			if (tid == 0) split_arrive[split_group] = 0;
+			if (reports) mine = ~atomicExch(&split_keys[w0 + q], 0ull);
+			if (tid == 0) split_arrive[grp] = 0;
+		}
+		if (reports) {
+			const uint32_t to = (uint32_t)mine, i = s_index[q];
+			s_moved[q][0] = fix_acc ? asg[i] : to;
+			s_moved[q][1] = to;
+			asg[i] = to;
 		}
 		if (fix_acc) {
 			// the fast pass has already added these points to the sums of the clusters it picked
 			__syncthreads();
 			for (uint32_t p = 0; p < np; ++p) {
-				const uint32_t from = smoved[p][0], to = smoved[p][1];
+				const uint32_t from = s_moved[p][0], to = s_moved[p][1];
 				if (from == to) continue;
 				// (no previous cluster: the fast pass could not hold the point and has not added it)
-				for (uint32_t j = tid; j < d; j += LIST_THREADS) {
-					const float x = sx[p * dpad + j];
+				for (uint32_t j = tid; j < d; j += EX_THREADS) {
+					const float x = pts[at<SOA>((uint64_t)s_index[p], j, n, d)];
 					if (from < k) atomicAdd(&fix_acc[(size_t)from * d + j], -x);
 					atomicAdd(&fix_acc[(size_t)to * d + j], x);
 				}
@@ -531,15 +466,15 @@ static cudaError_t launch_list_small(const float* pts, const float* means, uint3
 
 size_t list_split_scratch_bytes()
 {
-	return (size_t)LIST_SPLIT_MAX_BLOCKS * LIST_PB_WIDE * sizeof(unsigned long long) + (size_t)LIST_SPLIT_MAX_BLOCKS * sizeof(uint32_t);
+	return (size_t)EX_MAX_BLOCKS * EX_POINTS * sizeof(unsigned long long) + (size_t)EX_MAX_BLOCKS * sizeof(uint32_t);
 }
 
 cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* asg, const Shape& s,
 	const uint32_t* list, const uint32_t* list_count, int sm_count, cudaStream_t stream, const FusedAcc* fix, void* split_scratch)
 {
 	unsigned long long* split_keys = reinterpret_cast<unsigned long long*>(split_scratch);
-	uint32_t* split_arrive = split_scratch ? reinterpret_cast<uint32_t*>(split_keys + (size_t)LIST_SPLIT_MAX_BLOCKS * LIST_PB_WIDE) : nullptr;
-	if (fix != nullptr && (list == nullptr || (size_t)s.dim * sizeof(float) * LIST_PB > 120 * 1024)) return cudaErrorInvalidValue;
+	uint32_t* split_arrive = split_scratch ? reinterpret_cast<uint32_t*>(split_keys + (size_t)EX_MAX_BLOCKS * EX_POINTS) : nullptr;
+	if (fix != nullptr && list == nullptr) return cudaErrorInvalidValue;
 	// (the passes that leave sums to be corrected, `fix`, serve longer rows or settle their near-ties themselves)
 	if (list != nullptr && fix == nullptr && s.dim <= LIST_SMALL_MAX_DIM && (uint64_t)s.k * s.dim <= LIST_SMALL_MAX_FLOATS) {
 		switch (s.dim) {
@@ -561,54 +496,23 @@ cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* 
 		default: return launch_list_small<16>(pts, means, asg, s, list, list_count, sm_count, stream);
 		}
 	}
-	if (list != nullptr && (size_t)s.dim * sizeof(float) * LIST_PB <= 120 * 1024) {
-		// Every group of points walks all means: with long rows and many means (megabytes of them) the
-		// re-reads through L2 dominate, and sixteen points per group cut them fourfold (from 64 KiB of
-		// means on: 51 instead of 49 us for 1000 x 50, 19 instead of 11.5 us for 1024 x 128).
-		const bool wide = fix == nullptr && (size_t)s.k * s.dim * sizeof(float) >= (1u << 20) &&
-			(size_t)LIST_PB_WIDE * ((s.dim + 3) & ~3u) * sizeof(float) <= 64 * 1024;
-		const int pb = wide ? LIST_PB_WIDE : LIST_PB;
-		const size_t points_bytes = (size_t)pb * ((s.dim + 3) & ~3u) * sizeof(float);
-		size_t lsmem = points_bytes + (s.soa_means ? 0 : (size_t)LIST_THREADS * 33 * sizeof(float));
-		// room for all means (the kernel uses it when the list is long): at most 64 KiB, so that
-		// several blocks still share an SM
-		const size_t resident_bytes = points_bytes + (size_t)s.k * (s.dim | 1u) * sizeof(float);
-		const uint32_t resident_ok = resident_bytes <= 64 * 1024 ? 1u : 0u;
-		if (resident_ok && resident_bytes > lsmem) lsmem = resident_bytes;
-		const uint32_t lgrid = (uint32_t)sm_count * 8;
-		// (the 48 KiB that need no permission include the kernel's static arrays, less than 4 KiB)
-#define BKM_LAUNCH_LIST_PB(SOA, SOAM, PBV) do { \
-		auto kern = assign_exact_list_kernel<SOA, SOAM, PBV>; \
-		if (lsmem > 44 * 1024) { cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem); if (e != cudaSuccess) return e; } \
-		kern<<<lgrid, LIST_THREADS, lsmem, stream>>>(pts, means, asg, s.n, s.k, s.dim, list, list_count, \
-			fix ? fix->acc : nullptr, fix ? fix->counts : nullptr, resident_ok, split_keys, split_arrive); \
-	} while (0)
-#define BKM_LAUNCH_LIST(SOA, SOAM) do { if (wide) BKM_LAUNCH_LIST_PB(SOA, SOAM, LIST_PB_WIDE); else BKM_LAUNCH_LIST_PB(SOA, SOAM, LIST_PB); } while (0)
-		if (s.soa && s.soa_means) BKM_LAUNCH_LIST(true, true);
-		else if (s.soa && !s.soa_means) BKM_LAUNCH_LIST(true, false);
-		else if (!s.soa && s.soa_means) BKM_LAUNCH_LIST(false, true);
-		else BKM_LAUNCH_LIST(false, false);
-#undef BKM_LAUNCH_LIST_PB
-#undef BKM_LAUNCH_LIST
-		return cudaGetLastError();
-	}
-
-	// shared memory: one copy of the point per warp
-	uint32_t warps = 8;
-	while (warps > 1 && (size_t)warps * s.dim * sizeof(float) > 96 * 1024) warps >>= 1;
-	size_t smem = (size_t)warps * s.dim * sizeof(float);
-	if (smem > 200 * 1024) return cudaErrorInvalidValue;
-	uint64_t want = list ? (uint64_t)sm_count * 8 : (s.n + warps - 1) / warps;
-	uint32_t grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(want, 1), (uint64_t)sm_count * 16);
-	dim3 block(warps * 32);
+	if ((size_t)s.dim * sizeof(float) > 200 * 1024) return cudaErrorInvalidValue;
+	// Two blocks per SM are resident; a list's length is known on the device only.
+	const uint64_t groups = (s.n + EX_POINTS - 1) / EX_POINTS;
+	const uint32_t grid = (uint32_t)std::min<uint64_t>(list ? (uint64_t)sm_count * 2 : groups, (uint64_t)sm_count * 2);
+	const uint32_t slabs = (s.dim + EX_DIMS - 1) / EX_DIMS;
+	const bool resident = s.dim <= EX_RESIDENT_DIMS;
+	const size_t smem = (size_t)((resident ? slabs : 2u) * EX_PSTRIDE + 2 * EX_MSTRIDE) * EX_DIMS * sizeof(float);
 #define BKM_LAUNCH_EXACT(SOA, SOAM) do { \
-		auto kern = assign_exact_kernel<SOA, SOAM>; \
-		if (smem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) return e; } \
-		kern<<<grid, block, smem, stream>>>(pts, means, asg, s.n, s.k, s.dim, list, list_count); \
+		auto kern = resident ? assign_exact_kernel<SOA, SOAM, true> : assign_exact_kernel<SOA, SOAM, false>; \
+		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+		if (e != cudaSuccess) return e; \
+		kern<<<grid, EX_THREADS, smem, stream>>>(pts, means, asg, s.n, s.k, s.dim, list, list_count, \
+			fix ? fix->acc : nullptr, fix ? fix->counts : nullptr, list ? split_keys : nullptr, split_arrive); \
 	} while (0)
 	if (s.soa && s.soa_means) BKM_LAUNCH_EXACT(true, true);
-	else if (s.soa && !s.soa_means) BKM_LAUNCH_EXACT(true, false);
-	else if (!s.soa && s.soa_means) BKM_LAUNCH_EXACT(false, true);
+	else if (s.soa) BKM_LAUNCH_EXACT(true, false);
+	else if (s.soa_means) BKM_LAUNCH_EXACT(false, true);
 	else BKM_LAUNCH_EXACT(false, false);
 #undef BKM_LAUNCH_EXACT
 	return cudaGetLastError();

@@ -151,6 +151,14 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
 	return d;
 }
 
+// Two fp32 additions in one instruction, each rounded as by itself.
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+	uint64_t d;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+	return d;
+}
+
 __device__ __forceinline__ uint64_t pack2(float lo, float hi)
 {
 	uint64_t d;
@@ -161,6 +169,16 @@ __device__ __forceinline__ uint64_t pack2(float lo, float hi)
 __device__ __forceinline__ void unpack2(uint64_t v, uint32_t& lo, uint32_t& hi)
 {
 	asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+}
+
+// The squares of both halves.  Scalar multiplications: a packed one was contracted with the addition behind it
+// (mul.rn.f32x2 and add.rn.f32x2 gave the result of a fused multiply-add).
+__device__ __forceinline__ uint64_t square2(uint64_t v)
+{
+	uint32_t lo, hi;
+	unpack2(v, lo, hi);
+	const float a = __uint_as_float(lo), b = __uint_as_float(hi);
+	return pack2(__fmul_rn(a, a), __fmul_rn(b, b));
 }
 
 // ---- tcgen05 ----
