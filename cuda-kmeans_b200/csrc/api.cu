@@ -163,6 +163,10 @@ Workspace carve(char* base, uint64_t n, uint32_t k, uint32_t dim, bool with_tc_p
 		w.tp.a_hi = reinterpret_cast<float*>(take(aplane));
 		w.tp.a_lo = reinterpret_cast<float*>(take(aplane));
 		w.tp.xnorm = reinterpret_cast<float*>(take((size_t)w.tp.n_pad * sizeof(float)));
+		if (bkm::tc_screen_fits(k, dim)) {
+			w.tp.xlow = reinterpret_cast<float*>(take((size_t)w.tp.n_pad * sizeof(float)));
+			w.tp.screen_list = reinterpret_cast<uint32_t*>(take(n * sizeof(uint32_t)));
+		}
 		const uint32_t words = bkm::tc_partial_words(k, dim);
 		if (words) w.tp.partial = reinterpret_cast<uint32_t*>(take((size_t)bkm::TC_JSPLIT * words * w.tp.n_pad * sizeof(uint32_t)));
 		if (words == 5) w.tp.pairs = reinterpret_cast<uint32_t*>(take(2 * n * sizeof(uint32_t)));
@@ -322,6 +326,7 @@ struct bkm_handle_s {
 	// CUDA graph of two iterations (launch-bound problem sizes)
 	int use_graph = 2;                 // 0 = never, 1 = always (single GPU), 2 = by problem size
 	bool tc_pair = true;               // let the tensor-core assignment use its CTA-pair kernel where it applies
+	int tc_screen = 1;                 // screening pass in front of the K loop: 0 never, 1 where it pays, 2 wherever it can
 	int fuse_update = 1;               // fast pass accumulates the update sums: 0 never, 1 where it pays, 2 wherever it can
 	bool last_fused = false;
 	cudaGraphExec_t graph_exec = nullptr;
@@ -803,6 +808,13 @@ int bkm_set_option(bkm_handle_t h, const char* name, double value)
 		drop_graph(h);
 		return BKM_OK;
 	}
+	if (!strcmp(name, "tc_screen")) {
+		if (value != 0.0 && value != 1.0 && value != 2.0) return fail(BKM_ERR_INVALID, "tc_screen is 0 (never), 1 (where it pays) or 2 (wherever it can)");
+		h->tc_screen = (int)value;
+		bkm::tc_plan_screen(h->plan, h->tc_screen);
+		drop_graph(h);
+		return BKM_OK;
+	}
 	if (!strcmp(name, "exchange_wait_ms")) {
 		if (!(value >= 1.0 && value <= 600000.0)) return fail(BKM_ERR_INVALID, "exchange_wait_ms must be 1..600000");
 		h->exchange_wait_ns = (uint64_t)(value * 1.0e6);
@@ -845,6 +857,7 @@ static int prepare_plan_and_means(bkm_handle_t h)
 		h->plan = bkm::tc_plan_create(s, h->ws.tp, h->ws.tm, h->cfg.device, &err);
 		if (!h->plan) return fail(BKM_ERR_CUDA, "tensor-core plan: %s", err ? err : "unknown");
 		bkm::tc_plan_allow_pair(h->plan, h->tc_pair);
+		bkm::tc_plan_screen(h->plan, h->tc_screen);
 	}
 	bkm::launch_prepare_means(h->d_means[0], s,
 		h->assign_variant == BKM_ASSIGN_SIMT ? &h->ws.sm : nullptr,
@@ -1020,8 +1033,8 @@ int bkm_set_means(bkm_handle_t h, const float* host_means)
 	cudaStream_t st = h->stream;
 	{ const int rc = drop_first_pass(h); if (rc) return rc; }
 	CUDA_TRY(cudaMemcpyAsync(h->d_means[h->cur], host_means, (size_t)s.k * s.dim * sizeof(float), cudaMemcpyHostToDevice, st));
-	// the preparation fills cmax2[slot] with atomicMax, so the slot starts from zero
-	CUDA_TRY(cudaMemsetAsync(&h->ws.ctl->cmax2[h->slot], 0, sizeof(float), st));
+	// the preparation fills the slot with atomicMax, so it starts from zero
+	CUDA_TRY(cudaMemsetAsync(&h->ws.ctl->mean_max[h->slot], 0, sizeof(bkm::MeanMax), st));
 	bkm::launch_prepare_means(h->d_means[h->cur], s,
 		h->assign_variant == BKM_ASSIGN_SIMT ? &h->ws.sm : nullptr,
 		h->assign_variant == BKM_ASSIGN_TC ? &h->ws.tm : nullptr, h->ws.ctl, h->slot, st);

@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 	const uint32_t ntiles = (rows + SIMT_TILE_ROWS - 1) / SIMT_TILE_ROWS;
 	const uint64_t per_block = (uint64_t)SIMT_THREADS * P;
 	const uint64_t nblocks = (n + per_block - 1) / per_block;
-	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
+	const float x2max = ctl->xmax2, c2max = ctl->mean_max[slot].c2;
 	const KeyConsts kc = make_key_consts(x2max, c2max);
 	const uint32_t key_mult = kc.key_mult, key_base = kc.key_base, key_magic = kc.key_magic;
 	// Up to 2^125 the binade of the values and the reference's squared distances (at most 2 * (|x|^2 + |c|^2))

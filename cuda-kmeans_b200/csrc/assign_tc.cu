@@ -121,7 +121,7 @@ __device__ __forceinline__ void block_norm_max(float local_max, Control* __restr
 constexpr uint32_t SPLIT_ROWS = 4;
 
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ pts, uint32_t* __restrict__ a_hi,
-	uint32_t* __restrict__ a_lo, float* __restrict__ xnorm, uint64_t n, uint64_t p_begin, uint64_t p_end, uint32_t d, uint32_t d_pad, int vec,
+	uint32_t* __restrict__ a_lo, float* __restrict__ xnorm, float* __restrict__ xlow, uint64_t n, uint64_t p_begin, uint64_t p_end, uint32_t d, uint32_t d_pad, int vec,
 	const float* __restrict__ center, Control* __restrict__ ctl, const uint32_t* __restrict__ skip_if)
 {
 	if (skip_if && *skip_if) return;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
 	float local_max = 0.0f;
 	for (uint64_t r0 = p_begin + ((uint64_t)blockIdx.x * 8 + warp) * per_warp; r0 < p_end; r0 += (uint64_t)gridDim.x * 8 * per_warp) {
 		const uint64_t first = r0 + (lane >= lanes ? SPLIT_ROWS : 0u);
-		float norm[SPLIT_ROWS] = {};
+		float norm[SPLIT_ROWS] = {}, rest[SPLIT_ROWS] = {};
 		for (uint32_t w = word; w < d_pad; w += lanes) {
 			const uint32_t j = 2 * w;
 			const float c0 = j < d ? center[j] : 0.0f, c1 = j + 1 < d ? center[j + 1] : 0.0f;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
 			for (uint32_t u = 0; u < SPLIT_ROWS; ++u) {
 				const float y0 = (x0[u] - c0) * scale, y1 = (x1[u] - c1) * scale;
 				uint32_t hi, lo;
-				tc_split2(y0, y1, hi, lo);
+				tc_split2(y0, y1, hi, lo, rest[u]);
 				const size_t o = (size_t)(first + u) * d_pad + w;
 				a_hi[o] = hi;
 				a_lo[o] = lo;
@@ -168,6 +168,12 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
 			for (uint32_t off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
 			const float other = __shfl_xor_sync(0xffffffffu, s, 16);
 			if (lanes == 32) s += other;
+			if (xlow) {                                  // (rows of 32 lanes, see tc_screen_fits)
+				float r = rest[u];
+				#pragma unroll
+				for (uint32_t off = 16; off > 0; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
+				if (lane == 0) xlow[first + u] = sqrtf(r);
+			}
 			if (!(s <= TC_NORM2_MAX)) {
 				// beyond what the planes hold, or not a number: a zero row whose |x|^2 sends the point to the exact kernel
 				s = INFINITY;
@@ -187,7 +193,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
 // neither side meets a bank twice) and leave as whole rows: written straight from the lanes, 16 bytes
 // every 64, the stores cost 1.3 ms for 2^21 points of 32 dimensions.
 __global__ void __launch_bounds__(256) split_columns_kernel(const float* __restrict__ pts, uint32_t* __restrict__ a_hi,
-	uint32_t* __restrict__ a_lo, float* __restrict__ xnorm, uint64_t n, uint64_t p_begin, uint64_t p_end, uint32_t d, uint32_t d_pad,
+	uint32_t* __restrict__ a_lo, float* __restrict__ xnorm, float* __restrict__ xlow, uint64_t n, uint64_t p_begin, uint64_t p_end, uint32_t d, uint32_t d_pad,
 	const float* __restrict__ center, Control* __restrict__ ctl, const uint32_t* __restrict__ skip_if)
 {
 	if (skip_if && *skip_if) return;
@@ -200,7 +206,7 @@ __global__ void __launch_bounds__(256) split_columns_kernel(const float* __restr
 		uint4* out_hi = reinterpret_cast<uint4*>(a_hi + (size_t)p0 * d_pad);
 		uint4* out_lo = reinterpret_cast<uint4*>(a_lo + (size_t)p0 * d_pad);
 		const uint32_t pitch = d_pad / 4;           // 16-byte pieces of a row
-		float s = 0.0f;
+		float s = 0.0f, rest = 0.0f;
 		for (uint32_t w0 = 0; w0 < d_pad; w0 += 16) {
 			float x[32];
 			#pragma unroll
@@ -218,10 +224,10 @@ __global__ void __launch_bounds__(256) split_columns_kernel(const float* __restr
 			#pragma unroll
 			for (uint32_t q = 0; q < 4; ++q) {
 				uint4 hi, lo;
-				tc_split2(x[8 * q + 0], x[8 * q + 1], hi.x, lo.x);
-				tc_split2(x[8 * q + 2], x[8 * q + 3], hi.y, lo.y);
-				tc_split2(x[8 * q + 4], x[8 * q + 5], hi.z, lo.z);
-				tc_split2(x[8 * q + 6], x[8 * q + 7], hi.w, lo.w);
+				tc_split2(x[8 * q + 0], x[8 * q + 1], hi.x, lo.x, rest);
+				tc_split2(x[8 * q + 2], x[8 * q + 3], hi.y, lo.y, rest);
+				tc_split2(x[8 * q + 4], x[8 * q + 5], hi.z, lo.z, rest);
+				tc_split2(x[8 * q + 6], x[8 * q + 7], hi.w, lo.w, rest);
 				const uint32_t e = lane * 4 + (q ^ ((lane >> 1) & 3u));
 				s_hi[warp][e] = hi;
 				s_lo[warp][e] = lo;
@@ -242,6 +248,7 @@ __global__ void __launch_bounds__(256) split_columns_kernel(const float* __restr
 			atomicAdd(&ctl->beyond, 1u);
 		}
 		xnorm[p] = s;
+		if (xlow) xlow[p] = sqrtf(rest);
 	}
 	block_norm_max(local_max, ctl);
 }
@@ -326,8 +333,8 @@ cudaError_t launch_split_points(const float* pts, const Shape& s, const TcPoints
 	const uint64_t rows_pb = s.soa ? 256 : 8 * SPLIT_ROWS * (tp.d_pad == 16 ? 2 : 1);
 	const uint32_t grid = (uint32_t)std::min<uint64_t>((p_end - p_begin + rows_pb - 1) / rows_pb, (uint64_t)current_sm_count() * 8);
 	const int vec = s.dim % 2 == 0 && (reinterpret_cast<uintptr_t>(pts) & 7u) == 0 ? 1 : 0;
-	if (s.soa) split_columns_kernel<<<grid, 256, 0, stream>>>(pts, a_hi, a_lo, tp.xnorm, s.n, p_begin, p_end, s.dim, tp.d_pad, center, ctl, skip_if);
-	else split_rows_kernel<<<grid, 256, 0, stream>>>(pts, a_hi, a_lo, tp.xnorm, s.n, p_begin, p_end, s.dim, tp.d_pad, vec, center, ctl, skip_if);
+	if (s.soa) split_columns_kernel<<<grid, 256, 0, stream>>>(pts, a_hi, a_lo, tp.xnorm, tp.xlow, s.n, p_begin, p_end, s.dim, tp.d_pad, center, ctl, skip_if);
+	else split_rows_kernel<<<grid, 256, 0, stream>>>(pts, a_hi, a_lo, tp.xnorm, tp.xlow, s.n, p_begin, p_end, s.dim, tp.d_pad, vec, center, ctl, skip_if);
 	return cudaGetLastError();
 }
 
@@ -372,22 +379,25 @@ template<> struct RowState<true> {
 // Combines the partial arg-min results of the CTAs that shared the mean tiles of a point block.
 // THREE: the partial results carry the third smallest key, and a near-tie between two means only goes
 // to the list of pairs.
-template<bool THREE>
+// LIST: the points are list[0 .. *list_count) (the partial results lie in the order of the list).
+template<bool THREE, bool LIST>
 __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __restrict__ partial, uint64_t partial_stride, uint32_t parts,
 	const float* __restrict__ xnorm, uint32_t* __restrict__ asg, uint64_t n, uint32_t k, Control* __restrict__ ctl, int slot,
-	uint32_t* __restrict__ flag_list, float margin_coef, float sqrt_dim, uint32_t* __restrict__ pairs)
+	uint32_t* __restrict__ flag_list, float margin_coef, float sqrt_dim, uint32_t* __restrict__ pairs, const uint32_t* __restrict__ list)
 {
 	constexpr uint32_t WORDS = THREE ? 5 : 3;
-	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
+	const uint64_t total = LIST ? min((uint64_t)ctl->screen_count, n) : n;
+	const float x2max = ctl->xmax2, c2max = ctl->mean_max[slot].c2;
 	const KeyConsts kc = tc_key_consts(x2max, c2max);
 	const float ulp = kc.pow2 * 1.1920929e-07f;
 	const float margin_floor = tc_margin_floor(ulp, x2max, c2max, sqrt_dim, tc_scale(ctl->xdev));
 	const uint32_t lane = threadIdx.x & 31u;
-	const uint64_t n32 = (n + 31) & ~(uint64_t)31;      // whole warps walk the loop together (the append is a warp operation)
+	const uint64_t n32 = (total + 31) & ~(uint64_t)31;  // whole warps walk the loop together (the append is a warp operation)
 	for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n32; p += (uint64_t)gridDim.x * blockDim.x) {
 		bool flag = false, two = false;
-		uint32_t other = 0;
-		if (p < n) {
+		uint32_t other = 0, i = 0;
+		if (p < total) {
+			i = LIST ? list[p] : (uint32_t)p;
 			BestThree st;
 			for (uint32_t part = 0; part < parts; ++part) {
 				const uint32_t* src = partial + (size_t)part * WORDS * partial_stride + p;
@@ -395,8 +405,8 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __r
 				if (THREE) st.merge(ob, os, src[3 * partial_stride], oc, src[4 * partial_stride]);
 				else st.merge(ob, os, 0xFFFFFFFFu, oc, 0u);
 			}
-			const float margin = margin_coef * (xnorm[p] + c2max) + margin_floor;
-			flag = finish_point(st.best, st.second, st.best_chunk, kc.key_base, kc.key_mult, kc.key_magic, ulp, margin, k, p, asg);
+			const float margin = margin_coef * (xnorm[i] + c2max) + margin_floor;
+			flag = finish_point(st.best, st.second, st.best_chunk, kc.key_base, kc.key_mult, kc.key_magic, ulp, margin, k, i, asg);
 			if (THREE && flag && st.second != 0xFFFFFFFFu) {
 				const uint32_t bm = div_key(st.best - kc.key_base, kc.key_magic);
 				const float gap3 = st.third == 0xFFFFFFFFu ? INFINITY : (float)(div_key(st.third - kc.key_base, kc.key_magic) - bm) * ulp;
@@ -405,7 +415,7 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __r
 				flag = !two;
 			}
 		}
-		append_flagged(flag, (uint32_t)p, ctl, flag_list, n);
+		append_flagged(flag, i, ctl, flag_list, n);
 		if (THREE) {
 			const uint32_t mask = __ballot_sync(0xffffffffu, two);
 			if (mask != 0) {
@@ -413,7 +423,7 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __r
 				if (lane == 0) base = atomicAdd(&ctl->pair_count, (uint32_t)__popc(mask));
 				base = __shfl_sync(0xffffffffu, base, 0) + (uint32_t)__popc(mask & ((1u << lane) - 1u));
 				if (two) {
-					if ((uint64_t)base < n) { pairs[base] = (uint32_t)p; pairs[n + base] = other; }
+					if ((uint64_t)base < n) { pairs[base] = i; pairs[n + base] = other; }
 					else atomicOr(&ctl->status, (uint32_t)STATUS_LIST_OVERFLOW);
 				}
 			}
@@ -424,15 +434,22 @@ __global__ void __launch_bounds__(256) merge_partials_kernel(const uint32_t* __r
 // EVEN: mean tiles of 128 or 256 columns, so every warp takes its columns in pairs of 32-column chunks and the
 // epilogue runs without the odd-chunk branches.
 // THREE (K loop with jsplit > 1): the partial results carry the three smallest keys.
-template<bool EVEN, bool THREE>
+// LIST (K loop): the points are list[0 .. ctl->screen_count), and their rows (of row_words words) are gathered from the planes.
+template<bool EVEN, bool THREE, bool LIST>
 __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 	const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
 	const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
 	const float* __restrict__ b_aug, const float* __restrict__ xnorm, uint32_t* __restrict__ asg,
-	uint64_t n, uint32_t n_tiles, uint32_t k, uint32_t k_pad, uint32_t nt_cols, uint32_t kw, uint32_t kchunks, uint32_t ksteps, uint32_t idesc,
+	uint64_t n_all, uint32_t n_tiles, uint32_t k, uint32_t k_pad, uint32_t nt_cols, uint32_t kw, uint32_t kchunks, uint32_t ksteps, uint32_t idesc,
 	Control* __restrict__ ctl, int slot, uint32_t* __restrict__ flag_list, float margin_coef, float sqrt_dim,
-	uint32_t jsplit, uint32_t* __restrict__ partial, uint64_t partial_stride)
+	uint32_t jsplit, uint32_t* __restrict__ partial, uint64_t partial_stride, const uint32_t* __restrict__ list,
+	const float* __restrict__ a_hi, const float* __restrict__ a_lo, uint32_t row_words)
 {
+	const uint64_t n = LIST ? min((uint64_t)ctl->screen_count, n_all) : n_all;
+	if (LIST) {
+		n_tiles = (uint32_t)((n + TC_MTILE - 1) / TC_MTILE);
+		if ((blockIdx.x / jsplit) * TC_MA >= n_tiles) return;     // nothing to do for this block (most of them, with a short list)
+	}
 	extern __shared__ uint8_t smem_raw[];
 	uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 	TcBars* bars = reinterpret_cast<TcBars*>(smem + SM_BAR_OFF);
@@ -471,7 +488,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 			ptx::mbar_init(&bars->acc_empty[i], TC_EPI_WARPS / TC_MA);
 		}
 		for (uint32_t i = 0; i < KL_STAGES; ++i) {
-			ptx::mbar_init(&bars->b_full[i], 1);
+			ptx::mbar_init(&bars->b_full[i], LIST ? 33 : 1);     // (and the lanes that gather)
 			ptx::mbar_init(&bars->b_empty[i], 1);
 		}
 		for (uint32_t i = 0; i < 2; ++i) {
@@ -485,7 +502,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 		ptx::tmem_alloc(&bars->tmem_slot, TC_TMEM_COLS);
 		ptx::tmem_relinquish();
 	}
-	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
+	const float x2max = ctl->xmax2, c2max = ctl->mean_max[slot].c2;
 	const KeyConsts kc = tc_key_consts(x2max, c2max);
 	const float pow2 = kc.pow2;
 	const uint32_t key_mult = kc.key_mult, key_base = kc.key_base, key_magic = kc.key_magic;
@@ -498,7 +515,81 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 
 	if (warp == 0) {
 		// ---------------- TMA producer ----------------
-		if (lane == 0) {
+		if (LIST) {
+			// The whole warp gathers the rows of the listed points with asynchronous 16-byte copies, in the swizzle
+			// that the tensor maps give the other operands; the first lane loads the means.  Row piece lane % 4 of the
+			// rows lane / 4, + 8, + 16 ..  (Gathering by TMA, four rows of 64 bytes an instruction, took 68
+			// clocks each: 18 900 points of 512 dimensions against 4096 means 600 us, a quarter of that now.)
+			uint32_t b_count = 0, aug_count = 0;
+			bool ok = true;
+			const uint32_t sub = lane >> 2, piece = lane & 3u;
+			const uint32_t swizzled = sub * (KL_KW * 4) + ((piece ^ ((sub >> 1) & 3u)) * 16);
+			auto landed = [&](uint32_t count) {
+				// this lane's copies of stage `count` are complete: visible to the tensor cores, then announced
+				ptx::fence_proxy_async();
+				ptx::mbar_arrive(&bars->b_full[count % KL_STAGES]);
+			};
+			for (uint32_t blk = bid; blk < nblocks && ok; blk += nbid) {
+				const uint32_t tiles = min(TC_MA, n_tiles - blk * TC_MA);
+				uint32_t row[TC_MA][TC_MTILE / 8];
+				#pragma unroll
+				for (uint32_t t = 0; t < TC_MA; ++t)
+					#pragma unroll
+					for (uint32_t r = 0; r < TC_MTILE / 8; ++r) {
+						const uint64_t e = (uint64_t)(blk * TC_MA + t) * TC_MTILE + r * 8 + sub;
+						row[t][r] = list[e < n ? e : n - 1];       // (rows behind the last point repeat it)
+					}
+				for (uint32_t j = j_begin; j < j_end && ok; ++j) {
+					const uint32_t as = aug_count & 1u;
+					ok = __all_sync(0xffffffffu, wait_or_abort<100>(&bars->aug_empty[as], ((aug_count >> 1) & 1u) ^ 1u, abort_flag)) != 0;
+					if (!ok) break;
+					if (lane == 0) {
+						ptx::mbar_arrive_expect_tx(&bars->aug_full[as], nt_cols * 8 * 4);
+						ptx::bulk_g2s(smem + KL_AUG_OFF + as * AUG_BYTES, b_aug + (size_t)j * nt_cols * 8, nt_cols * 8 * 4, &bars->aug_full[as]);
+					}
+					++aug_count;
+					for (uint32_t kc = 0; kc < kchunks; ++kc) {
+						const uint32_t s = b_count % KL_STAGES, u = b_count / KL_STAGES;
+						ok = __all_sync(0xffffffffu, wait_or_abort<100>(&bars->b_empty[s], (u & 1u) ^ 1u, abort_flag)) != 0;
+						if (!ok) break;
+						uint8_t* dst = smem + s * KL_STAGE_BYTES;
+						if (lane == 0) {
+							const int32_t x = (int32_t)(kc * KL_KW);
+							ptx::mbar_arrive_expect_tx(&bars->b_full[s], 2 * nt_cols * KL_KW * 4);
+							ptx::tma_load_2d(dst + KL_B_OFF, &tm_b_hi, x, (int32_t)(j * nt_cols), &bars->b_full[s]);
+							ptx::tma_load_2d(dst + KL_B_OFF + KL_B_PLANE, &tm_b_lo, x, (int32_t)(j * nt_cols), &bars->b_full[s]);
+						}
+						const uint32_t at = ptx::smem_u32(dst) + swizzled;
+						const size_t column = (size_t)kc * KL_KW + piece * 4;
+						#pragma unroll
+						for (uint32_t t = 0; t < TC_MA; ++t) {
+							if (t >= tiles) break;
+							#pragma unroll
+							for (uint32_t r = 0; r < TC_MTILE / 8; ++r) {
+								const size_t o = (size_t)row[t][r] * row_words + column;
+								ptx::cp_async16(at + t * KL_A1_OFF + r * (8 * KL_KW * 4), a_hi + o);
+								ptx::cp_async16(at + t * KL_A1_OFF + KL_A_PLANE + r * (8 * KL_KW * 4), a_lo + o);
+							}
+						}
+						ptx::cp_async_commit();
+						if (b_count != 0) { ptx::cp_async_wait_all_but_one(); landed(b_count - 1); }
+						++b_count;
+					}
+				}
+			}
+			ptx::cp_async_wait_all();
+			if (b_count != 0) landed(b_count - 1);
+			// (do not leave while an own copy may still be in flight)
+			__syncwarp();
+			for (uint32_t back = 0; back < KL_STAGES && back < b_count; ++back) {
+				const uint32_t c = b_count - 1 - back;
+				ptx::mbar_wait(&bars->b_full[c % KL_STAGES], (c / KL_STAGES) & 1u);
+			}
+			for (uint32_t back = 0; back < 2 && back < aug_count; ++back) {
+				const uint32_t c = aug_count - 1 - back;
+				ptx::mbar_wait(&bars->aug_full[c & 1u], (c >> 1) & 1u);
+			}
+		} else if (lane == 0) {
 			ptx::prefetch_tmap(&tm_a_hi); ptx::prefetch_tmap(&tm_a_lo);
 			ptx::prefetch_tmap(&tm_b_hi); ptx::prefetch_tmap(&tm_b_lo);
 			uint32_t a_use[TC_NA_MAX] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -730,6 +821,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 			rows.reset();
 			const uint64_t p = (uint64_t)(blk * TC_MA + i) * TC_MTILE + row;
 			float xn = 0.0f;                       // |x|^2 of this thread's point, needed at the end of the block
+			uint32_t point = (uint32_t)p;
 			#pragma unroll 1
 			for (uint32_t j = j_begin; j < j_end; ++j) {
 				// the whole warp polls (one warp instruction either way, and no divergent region around it)
@@ -757,7 +849,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 							if (lane == 0) ptx::mbar_arrive(&bars->acc_empty[i]);
 							// fetched behind the hand-back of the block's last accumulator: the arithmetic on
 							// the chunks just loaded covers the latency
-							if (j == j_end - 1 && half == 0 && p < n) xn = xnorm[p];
+							if (j == j_end - 1 && half == 0 && p < n) {
+								if (LIST) point = list[p];
+								xn = xnorm[LIST ? point : p];
+							}
 						}
 						if (two) rows.take_chunk(v1, key_mult, chunk0 + 1);
 					}
@@ -789,12 +884,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 					dst[0] = st.best; dst[partial_stride] = st.second; dst[2 * partial_stride] = st.best_chunk;
 					if (THREE) { dst[3 * partial_stride] = st.third; dst[4 * partial_stride] = st.second_chunk; }
 				} else {
-					flag = finish_point(st.best, st.second, st.best_chunk, key_base, key_mult, key_magic, ulp, margin_coef * (xn + c2max) + margin_floor, k, p, asg);
+					flag = finish_point(st.best, st.second, st.best_chunk, key_base, key_mult, key_magic, ulp, margin_coef * (xn + c2max) + margin_floor, k, LIST ? point : p, asg);
 				}
 			}
-			if (half == 0 && partial == nullptr) buffered_append(flag, (uint32_t)p, flag_buf, flag_cnt, ctl, flag_list, n);
+			if (half == 0 && partial == nullptr) buffered_append(flag, point, flag_buf, flag_cnt, ctl, flag_list, n_all);
 		}
-		flush_flag_buffer(flag_buf, flag_cnt, ctl, flag_list, n);
+		flush_flag_buffer(flag_buf, flag_cnt, ctl, flag_list, n_all);
 	}
 
 	ptx::tc_fence_before();
@@ -839,6 +934,10 @@ struct TcPlan {
 	bool pair_ok;                   // the CTA-pair kernel covers this shape
 	bool pair_allowed;
 	int max_pairs;                  // CTA pairs the device holds at once
+	CUtensorMap as_hi, bs_hi, bs_aug;   // screening pass: planes of high parts in slices of 32 words, |c|^2 steps of 128 means
+	bool screen_ok;                 // ... can run
+	int screen_mode;                // see tc_plan_screen
+	int screen_pairs;               // CTA pairs of the screening pass the device holds at once
 	Shape s;
 	TcPoints tp;
 	TcMeans tm;
@@ -865,9 +964,9 @@ static PFN_cuTensorMapEncodeTiled_v12000 get_encode()
 // [rows][cols] 32-bit words (two fp16 each) row-major, box = box_rows x 32 columns with 128-byte
 // swizzle, or, when the rows are only 16 words long or the K loop runs (rows longer than 32 words,
 // 16-word slices), box_rows x 16 columns with 64-byte swizzle.
-static bool encode_plane(CUtensorMap* out, const float* base, uint64_t rows, uint32_t cols, uint32_t box_rows)
+static bool encode_plane(CUtensorMap* out, const float* base, uint64_t rows, uint32_t cols, uint32_t box_rows, uint32_t kw = 0, bool swizzle = true)
 {
-	const uint32_t kw = (cols == 16 || cols > TC_KCHUNK) ? 16u : TC_KCHUNK;
+	if (kw == 0) kw = (cols == 16 || cols > TC_KCHUNK) ? 16u : TC_KCHUNK;
 	auto enc = get_encode();
 	if (!enc) return false;
 	cuuint64_t dims[2] = {cols, rows};
@@ -875,7 +974,7 @@ static bool encode_plane(CUtensorMap* out, const float* base, uint64_t rows, uin
 	cuuint32_t box[2] = {kw, box_rows};
 	cuuint32_t estr[2] = {1, 1};
 	CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr,
-		CU_TENSOR_MAP_INTERLEAVE_NONE, kw == 16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+		CU_TENSOR_MAP_INTERLEAVE_NONE, !swizzle ? CU_TENSOR_MAP_SWIZZLE_NONE : (kw == 16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
 		CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 	return r == CUDA_SUCCESS;
 }
@@ -901,10 +1000,9 @@ TcPlan* tc_plan_create(const Shape& s, const TcPoints& tp, const TcMeans& tm, in
 		delete p;
 		return nullptr;
 	}
-	if (cudaFuncSetAttribute(assign_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess ||
-		cudaFuncSetAttribute(assign_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess ||
-		cudaFuncSetAttribute(assign_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess ||
-		cudaFuncSetAttribute(assign_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) != cudaSuccess) {
+	auto allow = [](auto kern) { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_ALLOC) == cudaSuccess; };
+	if (!allow(assign_tc_kernel<true, false, false>) || !allow(assign_tc_kernel<false, false, false>) || !allow(assign_tc_kernel<true, true, false>) ||
+		!allow(assign_tc_kernel<false, true, false>) || !allow(assign_tc_kernel<true, false, true>) || !allow(assign_tc_kernel<true, true, true>)) {
 		cudaGetLastError();
 		if (err) *err = e_attr;
 		delete p;
@@ -919,10 +1017,22 @@ TcPlan* tc_plan_create(const Shape& s, const TcPoints& tp, const TcMeans& tm, in
 		cudaGetLastError();
 		p->pair_ok = false;
 	}
+	// (a screening pass that cannot be set up is left out: the pass with all three products serves every shape)
+	p->screen_mode = 1;
+	p->screen_ok = tp.xlow != nullptr && tp.screen_list != nullptr &&
+		encode_plane(&p->as_hi, tp.a_hi, tp.n_pad, tp.d_pad, TC_MTILE, TC_KCHUNK) &&
+		encode_plane(&p->bs_hi, tm.b_hi, tm.k_pad, tm.d_pad, TC_NT_MAX / 2, TC_KCHUNK) &&
+		encode_plane(&p->bs_aug, tm.b_aug, tm.k_pad / 4, 32, TC_NT_MAX / 8, 32, false);
+	p->screen_pairs = 0;
+	if (p->screen_ok && (assign_tc_screen_prepare(p->sm_count, &p->screen_pairs) != cudaSuccess || p->screen_pairs < 1)) {
+		cudaGetLastError();
+		p->screen_ok = false;
+	}
 	return p;
 }
 
 void tc_plan_allow_pair(TcPlan* plan, bool allow) { if (plan) plan->pair_allowed = allow; }
+void tc_plan_screen(TcPlan* plan, int mode) { if (plan) plan->screen_mode = mode; }
 bool tc_plan_uses_pair(const TcPlan* plan) { return plan && plan->pair_ok && plan->pair_allowed; }
 
 // Where CTA pairs can run they serve what they are better at: the fused update sums, a range of the
@@ -1006,16 +1116,30 @@ cudaError_t launch_assign_tc(TcPlan* p, uint32_t* asg, Control* ctl, int slot, u
 	const uint32_t jsplit = plan_jsplit(p);
 	const uint32_t grid_j = jsplit * std::min<uint32_t>(nblocks, (uint32_t)p->sm_count / jsplit);
 	const bool even = p->nt_cols % 128 == 0, three = tc_plan_collects_pairs(p);
-	auto kern = three ? (even ? assign_tc_kernel<true, true> : assign_tc_kernel<false, true>) : (even ? assign_tc_kernel<true, false> : assign_tc_kernel<false, false>);
-	kern<<<jsplit > 1 ? grid_j : grid, TC_THREADS, SM_ALLOC, stream>>>(p->a_hi, p->a_lo, p->b_hi, p->b_lo,
-		p->tm.b_aug, p->tp.xnorm, asg, p->s.n, n_tiles, p->s.k, p->tm.k_pad, p->nt_cols, kw, kchunks, ksteps_last, idesc,
-		ctl, slot, flag_list, margin_coef, sqrt_dim, jsplit, jsplit > 1 ? p->tp.partial : nullptr, p->tp.n_pad);
-	if (jsplit > 1) {
-		const uint32_t mgrid = (uint32_t)std::min<uint64_t>((p->s.n + 255) / 256, (uint64_t)p->sm_count * 8);
-		auto merge = three ? merge_partials_kernel<true> : merge_partials_kernel<false>;
-		merge<<<mgrid, 256, 0, stream>>>(p->tp.partial, p->tp.n_pad, jsplit, p->tp.xnorm, asg, p->s.n, p->s.k, ctl, slot,
-			flag_list, margin_coef, sqrt_dim, p->tp.pairs);
+	const bool screens = p->screen_ok && (p->screen_mode == 2 || (p->screen_mode == 1 && tc_screen_pays(p->s)));
+	const uint32_t* list = screens ? p->tp.screen_list : nullptr;
+	if (screens) {
+		// the high parts alone first; what they leave open goes through the pass with all three products
+		const cudaError_t e = launch_assign_tc_screen(p->as_hi, p->bs_hi, p->bs_aug, p->tp, asg, p->s.n, p->s.k, p->tm.k_pad, p->s.dim, p->screen_pairs,
+			ctl, slot, margin_coef, margin_scale, sqrt_dim, stream);
+		if (e != cudaSuccess) return e;
 	}
+#define BKM_LAUNCH_TC(LIST) do { \
+		/* (a list has mean tiles of 256) */ \
+		auto kern = three ? (even || LIST ? assign_tc_kernel<true, true, LIST> : assign_tc_kernel<LIST, true, LIST>) : (even || LIST ? assign_tc_kernel<true, false, LIST> : assign_tc_kernel<LIST, false, LIST>); \
+		kern<<<jsplit > 1 ? grid_j : grid, TC_THREADS, SM_ALLOC, stream>>>(p->a_hi, p->a_lo, p->b_hi, p->b_lo, \
+			p->tm.b_aug, p->tp.xnorm, asg, p->s.n, n_tiles, p->s.k, p->tm.k_pad, p->nt_cols, kw, kchunks, ksteps_last, idesc, \
+			ctl, slot, flag_list, margin_coef, sqrt_dim, jsplit, jsplit > 1 ? p->tp.partial : nullptr, p->tp.n_pad, list, p->tp.a_hi, p->tp.a_lo, p->tp.d_pad); \
+		if (jsplit > 1) { \
+			const uint32_t mgrid = (uint32_t)std::min<uint64_t>((p->s.n + 255) / 256, (uint64_t)p->sm_count * 8); \
+			auto merge = three ? merge_partials_kernel<true, LIST> : merge_partials_kernel<false, LIST>; \
+			merge<<<mgrid, 256, 0, stream>>>(p->tp.partial, p->tp.n_pad, jsplit, p->tp.xnorm, asg, p->s.n, p->s.k, ctl, slot, \
+				flag_list, margin_coef, sqrt_dim, p->tp.pairs, list); \
+		} \
+	} while (0)
+	if (screens) BKM_LAUNCH_TC(true);
+	else BKM_LAUNCH_TC(false);
+#undef BKM_LAUNCH_TC
 	return cudaGetLastError();
 }
 

@@ -118,15 +118,6 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
 	asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" :: "l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// Like wait_or_abort, and a wait that runs out also raises the flag of the other CTA.
-template<uint32_t SLEEP_NS = 100>
-__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t peer_abort_addr)
-{
-	if (wait_or_abort<SLEEP_NS, true>(bar, parity, abort_flag)) return true;
-	ptx::st_cluster_u32(peer_abort_addr, 1u);
-	return false;
-}
-
 // KSTEPS = K steps of 16 dimensions per product (2 for dim 17..32, 3 and 4 up to 48 and 64): a template
 // parameter so that the MMA-issuing warp runs a straight line of instructions.
 template<uint32_t KSTEPS>
@@ -191,7 +182,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 		fuse_acc += rep * rep_stride;
 		fuse_counts += rep * rep_stride;
 	}
-	const float x2max = ctl->xmax2, c2max = ctl->cmax2[slot];
+	const float x2max = ctl->xmax2, c2max = ctl->mean_max[slot].c2;
 	const KeyConsts kc = tc_key_consts(x2max, c2max);
 	const uint32_t key_mult = kc.key_mult, key_base = kc.key_base, key_magic = kc.key_magic;
 	fill_a_aug(smem + P2_AAUG_OFF, kc, x2max, threadIdx.x, TC_THREADS);

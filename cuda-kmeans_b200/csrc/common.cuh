@@ -15,19 +15,26 @@ enum : uint32_t {
 	STATUS_LIST_OVERFLOW = 4u,  // the near-tie list was too short (cannot happen when sized n)
 };
 
+// Largest values over the means.
+struct MeanMax {
+	float c2;              // |mean|^2 (centred, in units of the operand scale where there is one)
+	float bl2;             // squared length of what the fp16 high parts of -2 mean leave over
+};
+
 // Device-resident control block shared by the kernels of one handle / one stateless call.
 struct Control {
 	uint32_t status;       // STATUS_* bits
 	uint32_t flag_count;   // number of points queued for the exact re-check
-	float cmax2[2];        // max over clusters of |mean|^2; the preparation of iteration t
-	                       // writes slot (t+1)&1 with atomicMax and clears slot t&1
+	MeanMax mean_max[2];   // the preparation of iteration t writes slot (t+1)&1 with atomicMax and clears slot t&1
 	uint32_t last_flag_count; // flag_count of the last finished iteration (for reporting)
 	float xmax2;           // max over the points of |x|^2 (written by the one-off preprocessing of the points;
 	                       // in units of the operand scale, see tc_scale, when the operands are the fp16 planes)
 	float xdev;            // largest |x_j - centre_j| over a sample of the points
 	uint32_t beyond;       // points that the fp16 planes cannot hold at the scale of that sample
 	uint32_t pair_count;   // number of points queued with exactly two candidate means
-	uint32_t pad[7];
+	uint32_t screen_count; // number of points that the screening pass left open
+	uint32_t probe_count;  // ... that its first launch left open
+	uint32_t pad[3];
 };
 
 // What a stateless workspace remembers about the point set its one-off operands (centre vector,
@@ -42,6 +49,7 @@ struct PointsKey {
 	uint32_t k;                  // the operands lie behind ranges whose sizes depend on it
 };
 constexpr size_t POINTS_KEY_OFFSET = 64;
+static_assert(sizeof(Control) <= POINTS_KEY_OFFSET, "the control block ends where the key begins");
 
 // Element offset of (item, dim) in a buffer of `items` vectors of `dims` floats.
 // AoS: item*dims + dim, SoA: dim*items + item (the reference's layout policies, ALIGN = 1).

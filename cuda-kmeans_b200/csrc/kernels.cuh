@@ -37,6 +37,8 @@ struct TcPoints {
 	float* xnorm;    // [n_pad] |x|^2 in units of the scale; +inf (and zero rows) for points the planes cannot hold
 	uint64_t n_pad;  // n rounded up to TC_MTILE
 	uint32_t d_pad;
+	float* xlow;       // [n_pad] length of what the high parts leave over, or null (no screening pass)
+	uint32_t* screen_list; // [n] points that the screening pass leaves open, or null
 	uint32_t* partial; // [TC_JSPLIT][tc_partial_words][n_pad] partial arg-min keys, or null
 	uint32_t* pairs;   // with five words only: [2][n] points queued with two candidates, and the second candidate
 };
@@ -149,6 +151,9 @@ uint32_t tc_kpad(uint32_t k);
 // Words that each of the CTAs that share a point block leaves per point: 0 = they do not share (short rows or few
 // mean tiles), 3 = (best, second, chunk), 5 = the third smallest key too, for lists of points with two candidates.
 uint32_t tc_partial_words(uint32_t k, uint32_t dim);
+// Whether a pass with the fp16 high parts alone can go first (assign_tc_screen.cu), and whether it pays.
+bool tc_screen_fits(uint32_t k, uint32_t dim);
+bool tc_screen_pays(const Shape& s);
 // One-off split of the points into fp16 hi/lo K-major planes + |x|^2 (after launch_compute_center).
 // `p_begin`, `p_end` (multiples of 32; 0, 0 = all): only these rows of the planes, so that a host upload
 // can be split chunk by chunk while the next chunk is on its way.
@@ -167,6 +172,8 @@ void tc_plan_destroy(TcPlan* plan);
 // The CTA-pair kernel (means resident in shared memory) is used where it applies and pays, unless disallowed.
 void tc_plan_allow_pair(TcPlan* plan, bool allow);
 bool tc_plan_uses_pair(const TcPlan* plan);
+// 0: no screening pass, 1: where it pays (the default), 2: wherever it can.
+void tc_plan_screen(TcPlan* plan, int mode);
 // With `fused` set (allowed when tc_plan_can_fuse) the kernel also adds every point to the sum and
 // the size of the cluster it picked, so that no separate update pass is needed; points that the
 // exact re-check moves afterwards are corrected there.

@@ -126,6 +126,17 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar)
 	asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
 
+__device__ __forceinline__ void cp_async_commit()
+{
+	asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// All groups of copies but the latest are complete.
+__device__ __forceinline__ void cp_async_wait_all_but_one()
+{
+	asm volatile("cp.async.wait_group 1;" ::: "memory");
+}
+
 __device__ __forceinline__ void cp_async_wait_all()
 {
 	asm volatile("cp.async.wait_all;" ::: "memory");

@@ -66,6 +66,15 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
 	return false;
 }
 
+// Like wait_or_abort, and a wait that runs out also raises the flag of the other CTA.
+template<uint32_t SLEEP_NS = 100>
+__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t peer_abort_addr)
+{
+	if (wait_or_abort<SLEEP_NS, true>(bar, parity, abort_flag)) return true;
+	ptx::st_cluster_u32(peer_abort_addr, 1u);
+	return false;
+}
+
 // K-major operand, 64-byte swizzle: rows of 64 B, 8-row groups 512 B apart.
 __device__ __forceinline__ uint64_t make_desc_sw64(uint32_t smem_addr)
 {
@@ -168,5 +177,11 @@ cudaError_t launch_assign_tc_pair(const CUtensorMap& a_hi, const CUtensorMap& a_
 	const float* b_aug, const float* xnorm, uint32_t* asg, uint64_t n, uint32_t n_tiles, uint32_t k, uint32_t k_pad, uint32_t d_pad,
 	uint32_t ksteps, int max_pairs, Control* ctl, int slot, uint32_t* flag_list, float margin_coef, float sqrt_dim, cudaStream_t stream,
 	const FusedAcc* fused, uint32_t dim, uint32_t step_begin = 0, uint32_t step_end = 0);
+
+// ---- the screening pass (assign_tc_screen.cu), likewise ----
+cudaError_t assign_tc_screen_prepare(int sm_count, int* max_pairs);
+cudaError_t launch_assign_tc_screen(const CUtensorMap& a_hi, const CUtensorMap& b_hi, const CUtensorMap& b_aug, const TcPoints& tp, uint32_t* asg,
+	uint64_t n, uint32_t k, uint32_t k_pad, uint32_t dim, int max_pairs, Control* ctl, int slot, float margin_coef, float margin_scale, float sqrt_dim,
+	cudaStream_t stream);
 
 } // namespace bkm

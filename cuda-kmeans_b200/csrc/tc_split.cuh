@@ -18,12 +18,14 @@ __device__ __forceinline__ void tc_split(float x, __half& hi, __half& lo)
 	lo = __float2half_rn(c - __half2float(hi));
 }
 
-// Two neighbouring dimensions as the words of the two planes.
-__device__ __forceinline__ void tc_split2(float x0, float x1, uint32_t& hi, uint32_t& lo)
+// Two neighbouring dimensions as the words of the two planes; what the high parts leave over is added to `rest2`, squared.
+__device__ __forceinline__ void tc_split2(float x0, float x1, uint32_t& hi, uint32_t& lo, float& rest2)
 {
 	__half h0, l0, h1, l1;
 	tc_split(x0, h0, l0);
 	tc_split(x1, h1, l1);
+	const float r0 = x0 - __half2float(h0), r1 = x1 - __half2float(h1);
+	rest2 = fmaf(r0, r0, fmaf(r1, r1, rest2));
 	hi = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
 	lo = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
 }

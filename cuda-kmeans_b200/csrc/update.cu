@@ -69,7 +69,7 @@ struct RowSinks {
 template<class MEANS>
 __device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32_t lane, bool write_means, uint32_t cnt, MEANS means_of)
 {
-	float s2 = 0.0f;
+	float s2 = 0.0f, rest2 = 0.0f;
 	const float scale = o.b_hi ? tc_scale(o.ctl->xdev) : 1.0f;
 	for (uint32_t j0 = lane; j0 < o.d; j0 += 128) {
 		float m[4];
@@ -88,6 +88,8 @@ __device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32
 			if (o.b_hi) {
 				__half hi, lo;
 				tc_split(b, hi, lo);
+				const float rest = b - __half2float(hi);
+				rest2 = fmaf(rest, rest, rest2);
 				o.b_hi[(size_t)c * o.d_pad * 2 + j] = hi;
 				o.b_lo[(size_t)c * o.d_pad * 2 + j] = lo;
 			}
@@ -95,6 +97,10 @@ __device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32
 	}
 	#pragma unroll
 	for (int off = 16; off > 0; off >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, off);
+	if (o.b_hi) {
+		#pragma unroll
+		for (int off = 16; off > 0; off >>= 1) rest2 += __shfl_xor_sync(0xffffffffu, rest2, off);
+	}
 	__syncwarp();
 	if (lane == 0) {
 		if (o.cprep) o.cprep[(size_t)c * o.rs] = s2;
@@ -102,7 +108,8 @@ __device__ __forceinline__ void finish_row(const RowSinks& o, uint32_t c, uint32
 			*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 0)) = tc_aug_row(s2);
 			*reinterpret_cast<uint4*>(o.b_aug + aug_offset(c, 1)) = make_uint4(0u, 0u, 0u, 0u);
 		}
-		atomicMax(reinterpret_cast<int*>(&o.ctl->cmax2[o.slot]), __float_as_int(s2));
+		atomicMax(reinterpret_cast<int*>(&o.ctl->mean_max[o.slot].c2), __float_as_int(s2));
+		if (o.b_hi) atomicMax(reinterpret_cast<int*>(&o.ctl->mean_max[o.slot].bl2), __float_as_int(rest2));
 		if (write_means && o.sizes_out) o.sizes_out[c] = cnt;
 	}
 }
@@ -122,7 +129,9 @@ __device__ __forceinline__ void finish_control(Control* ctl, int slot)
 	ctl->last_flag_count = ctl->flag_count + ctl->pair_count;
 	ctl->flag_count = 0;
 	ctl->pair_count = 0;
-	ctl->cmax2[slot ^ 1] = 0.0f;
+	ctl->screen_count = 0;
+	ctl->probe_count = 0;
+	ctl->mean_max[slot ^ 1] = MeanMax{0.0f, 0.0f};
 }
 
 __device__ __forceinline__ uint32_t rows_to_finish(const RowSinks& o)
@@ -469,7 +478,8 @@ __global__ void __launch_bounds__(256) stateless_begin_kernel(Control* ctl, Poin
 	const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
 	if (t == 0) {
 		// last_flag_count and what belongs to the points survive
-		ctl->status = 0; ctl->flag_count = 0; ctl->pair_count = 0; ctl->cmax2[0] = 0.0f; ctl->cmax2[1] = 0.0f;
+		ctl->status = 0; ctl->flag_count = 0; ctl->pair_count = 0; ctl->screen_count = 0; ctl->probe_count = 0;
+		ctl->mean_max[0] = ctl->mean_max[1] = MeanMax{0.0f, 0.0f};
 		key->fp_new = 0; key->arrive = 0;
 	}
 	// (by another warp: the round trip of the loads is not waited for behind the stores, and where the fingerprint
