@@ -451,7 +451,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 		if ((blockIdx.x / jsplit) * TC_MA >= n_tiles) return;     // nothing to do for this block (most of them, with a short list)
 	}
 	extern __shared__ uint8_t smem_raw[];
-	uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+	// (an offset from the array, so that the compiler still knows it for shared memory: 32-bit addresses in the epilogue)
+	uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
 	TcBars* bars = reinterpret_cast<TcBars*>(smem + SM_BAR_OFF);
 	uint32_t* mg_state = reinterpret_cast<uint32_t*>(smem + SM_MERGE_OFF);
 	volatile uint32_t* abort_flag = &bars->abort_flag;

@@ -133,7 +133,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 	constexpr uint32_t kw = KSTEPS <= 2 ? 16u : TC_KCHUNK;         // words per operand row: 64-byte or 128-byte swizzle
 	constexpr uint32_t DESC_HI_ROWS = KSTEPS <= 2 ? DESC_HI_SW64 : DESC_HI_SW128;
 	extern __shared__ uint8_t smem_raw[];
-	uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+	// (an offset from the array, so that the compiler still knows it for shared memory: 32-bit addresses in the epilogue)
+	uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
 	PairBars* bars = reinterpret_cast<PairBars*>(smem + P2_BAR_OFF);
 	uint32_t* mg_state = reinterpret_cast<uint32_t*>(smem + P2_MERGE_OFF);
 	volatile uint32_t* abort_flag = &bars->abort_flag;

@@ -91,7 +91,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 	Control* __restrict__ ctl, int slot, float margin_coef, float margin_scale, float sqrt_dim, uint32_t step_begin, uint32_t step_end, uint32_t probe_points)
 {
 	extern __shared__ uint8_t smem_raw[];
-	uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+	// (an offset from the array, so that the compiler still knows it for shared memory: 32-bit addresses in the epilogue)
+	uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
 	ScreenBars* bars = reinterpret_cast<ScreenBars*>(smem + SC_BAR_OFF);
 	uint32_t* mg_state = reinterpret_cast<uint32_t*>(smem + SC_MERGE_OFF);
 	volatile uint32_t* abort_flag = &bars->abort_flag;
