@@ -118,6 +118,7 @@ struct Workspace {
 	bkm::TcMeans tm{};
 	size_t tm_bytes = 0;           // b_hi + b_lo
 	uint32_t* flag_list = nullptr; // n entries
+	uint32_t* group_cursor = nullptr; // k + 1 entries, or null (see update_grouped_supported; the near-tie list holds the order)
 	uint32_t* asg_scratch = nullptr; // n entries (iterate without an assignment output)
 	bkm::TcPoints tp{};
 	size_t bytes = 0;
@@ -156,6 +157,7 @@ Workspace carve(char* base, uint64_t n, uint32_t k, uint32_t dim, bool with_tc_p
 	w.sm.center = w.tm.center;
 	w.flag_list = reinterpret_cast<uint32_t*>(take(n * sizeof(uint32_t)));
 	w.asg_scratch = reinterpret_cast<uint32_t*>(take(n * sizeof(uint32_t)));
+	if (bkm::update_grouped_supported(n, k, dim)) w.group_cursor = reinterpret_cast<uint32_t*>(take(((size_t)k + 1) * sizeof(uint32_t)));
 	if (with_tc_points) {
 		w.tp.n_pad = bkm::round_up64(n, bkm::TC_MTILE);
 		w.tp.d_pad = w.tm.d_pad;
@@ -515,7 +517,7 @@ static int stateless_update(const float* points, const uint32_t* assignment, flo
 	if (rc) return rc;
 	// (an assignment in front of it has cleared the accumulators as well)
 	if (clear) CUDA_TRY(bkm::launch_stateless_begin(w.ctl, points_key(w), s, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, false, sm_count, st));
-	bkm::launch_update(points, assignment, w.acc, w.counts, w.replicas, s, v, w.ctl, sm_count, st);
+	bkm::launch_update(points, assignment, w.acc, w.counts, w.replicas, s, v, w.ctl, sm_count, st, w.flag_list, w.group_cursor);
 	bkm::launch_finalize(w.acc, w.counts, w.replicas, means, sizes, s, nullptr, nullptr, w.ctl, 1, st);
 	CUDA_TRY(cudaGetLastError());
 	return BKM_OK;
@@ -554,7 +556,7 @@ int bkm_bucket_sums_f32(const float* points, const uint32_t* indices, float* sum
 	if ((rc = resolve_update(variant, s, device, &v))) return rc;
 	cudaStream_t st = static_cast<cudaStream_t>(stream);
 	CUDA_TRY(bkm::launch_stateless_begin(w.ctl, points_key(w), s, {{w.acc, nullptr, nullptr}, {align256(w.acc_bytes), 0, 0}}, false, sm, st));
-	bkm::launch_update(points, indices, w.acc, w.counts, w.replicas, s, v, w.ctl, sm, st);
+	bkm::launch_update(points, indices, w.acc, w.counts, w.replicas, s, v, w.ctl, sm, st, w.flag_list, w.group_cursor);
 	bkm::launch_finalize_sums(w.acc, w.counts, w.replicas, sums, s, w.ctl, st);
 	CUDA_TRY(cudaGetLastError());
 	return BKM_OK;
@@ -1073,7 +1075,7 @@ static int enqueue_iteration(bkm_handle_t h, cudaEvent_t* ev)
 	if (rc) return rc;
 	if (ev) CUDA_TRY(cudaEventRecord(ev[2], st));
 	if (!fused)
-		bkm::launch_update(h->d_points, h->d_asg, h->ws.acc, h->ws.counts, h->ws.replicas, s, h->update_variant, h->ws.ctl, h->sm_count, st);
+		bkm::launch_update(h->d_points, h->d_asg, h->ws.acc, h->ws.counts, h->ws.replicas, s, h->update_variant, h->ws.ctl, h->sm_count, st, h->ws.flag_list, h->ws.group_cursor);
 	if (ev) CUDA_TRY(cudaEventRecord(ev[3], st));
 	if (h->peer_on) {
 		// one kernel: publish this rank's sums, read the peers', add in rank order, divide, next operands

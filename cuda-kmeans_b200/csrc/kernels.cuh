@@ -102,8 +102,11 @@ cudaError_t launch_points_fingerprint(const float* pts, const Shape& s, int vari
 // Returns false when the shared variant cannot hold k*dim in shared memory.
 bool update_shared_fits(const Shape& s, int device);
 bool update_sorted_supported(const Shape& s);
+// `order` (n words) and `cursor` (k + 1 words), optional: scratch of the row-wise variant for long rows and many clusters
+// (update_grouped_supported).
+bool update_grouped_supported(uint64_t n, uint32_t k, uint32_t dim);
 void launch_update(const float* pts, const uint32_t* asg, float* acc, uint32_t* counts, uint32_t replicas, const Shape& s,
-	int variant, Control* ctl, int sm_count, cudaStream_t stream);
+	int variant, Control* ctl, int sm_count, cudaStream_t stream, uint32_t* order = nullptr, uint32_t* cursor = nullptr);
 // Folds accumulator replicas 1.. into replica 0 (before an all-reduce of replica 0).
 void launch_merge_replicas(float* acc, uint32_t* counts, uint32_t replicas, const Shape& s, cudaStream_t stream);
 
