@@ -537,6 +537,19 @@ cudaError_t launch_assign_exact(const float* pts, const float* means, uint32_t* 
 // rounding band of the pass (and of the reference's own sum and square root) is queued for the
 // exact kernel; the final assignment is the reference's for every point.
 
+//
+// The band, in spacings of the values (ulp = P * 2^-23 in the binade [P, 2P), P at least 2.5 times the largest |x|^2 plus the
+// largest |c|^2; u = 2^-24), for the difference of two values:
+//   D + 1     roundings of the D multiply-adds and of |c|^2 + C, half an ulp each, for two values;
+//   1.6       |c|^2 itself: four roundings of at most 0.4 P, for two values;
+//   and, with r the distance to the mean in question, relative to what is small for a point near its mean:
+//   the centring of both operands, 2 r u (|x| + |c|) for each, |c| <= |x| + r, and the reference's own sum (D + 2) u r^2
+//   for each and the collapse of its square root, 4 u r^2: together (2 D + 12) u r^2 + 8 u |x| r.
+// A flat band of 4 D + 16 spacings, which covers all of that at any distance, queued 6.3 % of 2^24 points in tight two-dimensional
+// clusters, and the list took 60 us; 1.5 % and 24 us now.  The flat band stays where near-ties are few, with more
+// dimensions (batches of 250 000 x 8 against 256: 298.8 us with it, 310.3 with the other, whose sums of squares cost registers), and
+// in the fused form, which settles its near-ties on the spot (66.3 / 66.8 us per iteration).
+
 constexpr int SIMT_THREADS = 256;
 constexpr int SIMT_EVAL_POINTS = 2;  // points that a thread evaluates at a time
 constexpr int SIMT_TILE_ROWS = 1024; // means per shared-memory tile (a multiple of the 32-mean chunk)
@@ -605,10 +618,11 @@ __device__ __forceinline__ void settle(const float* __restrict__ pts, uint64_t n
 template<int D, bool SOA, int P, bool FUSE>
 __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const float* __restrict__ pts,
 	const float* __restrict__ cprep, const float* __restrict__ center, uint32_t* __restrict__ asg, uint64_t n, uint32_t rows,
-	Control* __restrict__ ctl, int slot, uint32_t* __restrict__ flag_list, float margin_ulps, int vec_ok,
+	Control* __restrict__ ctl, int slot, uint32_t* __restrict__ flag_list, float margin_scale, int vec_ok,
 	uint32_t k, float* __restrict__ fuse_acc, uint32_t* __restrict__ fuse_counts, const float* __restrict__ means, int soa_means)
 {
 	constexpr int Q = SIMT_EVAL_POINTS;          // points evaluated at a time
+	constexpr bool TIGHT = !FUSE && D <= 4;      // the band follows a point's distance to its mean (see above)
 	static_assert(P % Q == 0 && (FUSE || P == Q), "points per thread");
 	constexpr int RS = (D + 1 + 3) / 4 * 4;      // floats of a prepared row in global memory
 	extern __shared__ __align__(128) float tile[];  // rows of two means interleaved: (D + 1) pairs
@@ -636,7 +650,8 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 	// Up to 2^125 the binade of the values and the reference's squared distances (at most 2 * (|x|^2 + |c|^2))
 	// are inside the range of 32-bit floats; beyond, or with means that are not finite, the keys mean nothing
 	// and every point is settled by the exact arithmetic.
-	const float margin = x2max + c2max < 4.2535296e37f ? margin_ulps : INFINITY;
+	const float margin_floor = x2max + c2max < 4.2535296e37f ? margin_scale * (float)(TIGHT ? D + 3 : 4 * D + 16) : INFINITY;
+	const float value_ulp = kc.pow2 * 1.1920929e-07f, per_value = margin_scale * 0.5f / kc.pow2;
 	const float pad_value = kc.pow2 * (2.0f - 1.0f / 32.0f);     // padding rows: above every real value, inside [P, 2P)
 	float cen[D];
 	#pragma unroll
@@ -814,6 +829,15 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 					cl[g + p] = bchunk * 32u + ((best - key_base) - bm * key_mult);
 					if (!FUSE) asg[idx[g + p]] = cl[g + p];
 					const float gap = second == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second - key_base, key_magic) - bm);
+					float margin = margin_floor;
+					if (TIGHT) {
+						float x2 = 0.0f;
+						#pragma unroll
+						for (int j = 0; j < D; ++j) x2 = fmaf(x[g + p][j], x[g + p][j], x2);
+						// the squared distance to the winner, a little more than that
+						const float dist2 = fmaxf(__uint_as_float(__float_as_uint(kc.pow2) + bm) - kc.offset_c + x2, 0.0f) + 32.0f * value_ulp;
+						margin += per_value * ((float)(2 * D + 12) * dist2 + 8.0f * sqrtf(x2 * dist2));
+					}
 					flag = !(gap > margin) || (near >> (g + p) & 1u) != 0;
 				}
 				if (FUSE) near = flag ? near | 1u << (g + p) : near & ~(1u << (g + p));
@@ -963,10 +987,6 @@ static cudaError_t launch_simt_d(const float* pts, const float* means, const flo
 	const uint64_t nblocks = (s.n + per_block - 1) / per_block;
 	// persistent grid: a whole number of resident blocks per SM
 	int per_sm = 1;
-	// Near-tie band in value spacings (ulps of the common binade): roundings of this pass (|c|^2,
-	// the offset, D fused steps, the centring of both operands), doubled for a difference of two
-	// values, plus the reference's own sum and the collapse of its square root.
-	const float margin_ulps = margin_scale * (float)(4 * D + 16);
 	const int vec_ok = ((reinterpret_cast<uintptr_t>(pts) & 15u) == 0) ? 1 : 0;
 #define BKM_LAUNCH_SIMT(SOA, FUSE) do { \
 		auto kern = FUSE && many ? assign_simt_kernel<D, SOA, FUSE ? MANY_P : SIMT_EVAL_POINTS, FUSE> : assign_simt_kernel<D, SOA, SIMT_EVAL_POINTS, FUSE>; \
@@ -977,7 +997,7 @@ static cudaError_t launch_simt_d(const float* pts, const float* means, const flo
 		if (per_sm < 1) per_sm = 1; \
 		uint32_t grid = (uint32_t)std::min<uint64_t>(nblocks, (uint64_t)sm_count * per_sm); \
 		if (grid < 1) grid = 1; \
-		kern<<<grid, SIMT_THREADS, smem, stream>>>(pts, cprep, center, asg, s.n, rows, ctl, slot, flag_list, margin_ulps, vec_ok, \
+		kern<<<grid, SIMT_THREADS, smem, stream>>>(pts, cprep, center, asg, s.n, rows, ctl, slot, flag_list, margin_scale, vec_ok, \
 			s.k, fused ? fused->acc : nullptr, fused ? fused->counts : nullptr, means, s.soa_means); \
 	} while (0)
 	if (fused && !assign_simt_can_fuse(s, *fused)) return cudaErrorInvalidValue;
