@@ -65,6 +65,23 @@ bool tc_screen_fits(uint32_t k, uint32_t dim) { return tc_dpad(dim) > TC_KCHUNK 
 // 30 000 points x 1024 x 128 83 / 77.  Where the first wave leaves most points open: 3141 / 3056 (99.5 % of 10^6 x 1000 x 100).
 bool tc_screen_pays(const Shape& s) { return s.n >= 1u << 15 && (double)s.n * s.k * s.dim >= 1.2e10; }
 
+// Place in a ring of buffers.  (Counted up with a wrap: remainder and quotient by a ring size that is known at run time cost the
+// loading lane 800 clocks per slice, beside four busy warps, where a slice's multiplication takes 512.)
+struct RingPos {
+	uint32_t slot = 0, phase = 0;
+	__device__ __forceinline__ void next(uint32_t slots) { if (++slot == slots) { slot = 0; phase ^= 1u; } }
+};
+
+// Waits for the last fill of every buffer that has been filled (a lap at most); `pos` is the next one to be filled.
+__device__ __forceinline__ void drain_ring(uint64_t* full, RingPos pos, uint32_t slots, uint32_t fills)
+{
+	for (uint32_t back = 0; back < slots && back < fills; ++back) {
+		if (pos.slot == 0) { pos.slot = slots; pos.phase ^= 1u; }
+		--pos.slot;
+		ptx::mbar_wait(&full[pos.slot], pos.phase);
+	}
+}
+
 // Appends the points whose `flag` is set to the list of open points, one atomic per warp.
 __device__ __forceinline__ uint32_t append_open(bool flag, uint32_t point, Control* __restrict__ ctl, uint32_t* __restrict__ list, uint64_t n)
 {
@@ -150,41 +167,45 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 		// ---------------- TMA producer (both CTAs) ----------------
 		if (lane == 0) {
 			ptx::prefetch_tmap(&tm_a); ptx::prefetch_tmap(&tm_b); ptx::prefetch_tmap(&tm_aug);
-			uint32_t a_count = 0, b_count = 0, c = 0;
+			RingPos a_pos, b_pos, aug_pos;
+			uint32_t a_fills = 0, b_fills = 0, aug_fills = 0;
+			const uint32_t a_full0 = ptx::leader_cta_addr(ptx::smem_u32(bars->a_full)), b_full0 = ptx::leader_cta_addr(ptx::smem_u32(bars->b_full));
+			const uint32_t aug_full0 = ptx::leader_cta_addr(ptx::smem_u32(bars->aug_full));
 			bool ok = true;
-			auto load = [&](uint64_t* full, uint64_t* empty, uint32_t count, uint32_t slots, uint8_t* ring, const CUtensorMap* map, uint32_t x, uint32_t row) {
-				const uint32_t s = count % slots, u = count / slots;
-				ok = pair_wait<20>(&empty[s], (u & 1u) ^ 1u, abort_flag, peer_abort_addr);
-				if (!ok) return;
-				if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], 2 * SC_PLANE_BYTES);
-				ptx::tma_load_2d_pair(ring + s * SC_PLANE_BYTES, map, (int32_t)x, (int32_t)row, ptx::leader_cta_addr(ptx::smem_u32(&full[s])));
-			};
 			for (uint32_t step = step_begin + pair; step < step_end && ok; step += n_pairs) {
-				for (uint32_t j = 0; j < n_ctiles && ok; ++j, ++c) {
-					const uint32_t as = c % SC_AUG_SLOTS, mean = j * TC_NT_MAX + rank * (TC_NT_MAX / 2);
-					ok = pair_wait<20>(&bars->aug_empty[as], ((c / SC_AUG_SLOTS) & 1u) ^ 1u, abort_flag, peer_abort_addr);
+				for (uint32_t j = 0; j < n_ctiles && ok; ++j) {
+					const uint32_t mean = j * TC_NT_MAX + rank * (TC_NT_MAX / 2);
+					ok = pair_wait<20>(&bars->aug_empty[aug_pos.slot], aug_pos.phase ^ 1u, abort_flag, peer_abort_addr);
 					if (!ok) break;
-					if (rank == 0) ptx::mbar_arrive_expect_tx(&bars->aug_full[as], 2 * SC_AUG_BYTES);
-					ptx::tma_load_2d_pair(smem + SC_AUG_OFF + as * SC_AUG_BYTES, &tm_aug, 0, (int32_t)(mean / 4), ptx::leader_cta_addr(ptx::smem_u32(&bars->aug_full[as])));
-					for (uint32_t sl = 0; sl < slices && ok; ++sl) {
+					if (rank == 0) ptx::mbar_arrive_expect_tx(&bars->aug_full[aug_pos.slot], 2 * SC_AUG_BYTES);
+					ptx::tma_load_2d_pair(smem + SC_AUG_OFF + aug_pos.slot * SC_AUG_BYTES, &tm_aug, 0, (int32_t)(mean / 4), aug_full0 + aug_pos.slot * 8u);
+					aug_pos.next(SC_AUG_SLOTS);
+					++aug_fills;
+					for (uint32_t sl = 0; sl < slices; ++sl) {
 						if (!resident || j == 0) {
-							// (rows behind the last tile read as zeros)
-							load(bars->a_full, bars->a_empty, a_count, a_slots, smem, &tm_a, sl * TC_KCHUNK, (2 * step + rank) * TC_MTILE);
+							ok = pair_wait<20>(&bars->a_empty[a_pos.slot], a_pos.phase ^ 1u, abort_flag, peer_abort_addr);
 							if (!ok) break;
-							++a_count;
+							if (rank == 0) ptx::mbar_arrive_expect_tx(&bars->a_full[a_pos.slot], 2 * SC_PLANE_BYTES);
+							// (rows behind the last tile read as zeros)
+							ptx::tma_load_2d_pair(smem + a_pos.slot * SC_PLANE_BYTES, &tm_a, (int32_t)(sl * TC_KCHUNK), (int32_t)((2 * step + rank) * TC_MTILE), a_full0 + a_pos.slot * 8u);
+							a_pos.next(a_slots);
+							++a_fills;
 						}
-						load(bars->b_full, bars->b_empty, b_count, b_slots, b_ring, &tm_b, sl * TC_KCHUNK, mean);
+						ok = pair_wait<20>(&bars->b_empty[b_pos.slot], b_pos.phase ^ 1u, abort_flag, peer_abort_addr);
 						if (!ok) break;
-						++b_count;
+						if (rank == 0) ptx::mbar_arrive_expect_tx(&bars->b_full[b_pos.slot], 2 * SC_PLANE_BYTES);
+						ptx::tma_load_2d_pair(b_ring + b_pos.slot * SC_PLANE_BYTES, &tm_b, (int32_t)(sl * TC_KCHUNK), (int32_t)mean, b_full0 + b_pos.slot * 8u);
+						b_pos.next(b_slots);
+						++b_fills;
 					}
 				}
 			}
 			if (rank == 0) {
 				// Nobody leaves while a copy may still be in flight: the first CTA's barriers count
 				// the bytes of both CTAs, and the second CTA stays until the final cluster barrier.
-				for (uint32_t back = 0; back < a_slots && back < a_count; ++back) { const uint32_t t = a_count - 1 - back; ptx::mbar_wait(&bars->a_full[t % a_slots], (t / a_slots) & 1u); }
-				for (uint32_t back = 0; back < b_slots && back < b_count; ++back) { const uint32_t t = b_count - 1 - back; ptx::mbar_wait(&bars->b_full[t % b_slots], (t / b_slots) & 1u); }
-				for (uint32_t back = 0; back < SC_AUG_SLOTS && back < c; ++back) { const uint32_t t = c - 1 - back; ptx::mbar_wait(&bars->aug_full[t % SC_AUG_SLOTS], (t / SC_AUG_SLOTS) & 1u); }
+				drain_ring(bars->a_full, a_pos, a_slots, a_fills);
+				drain_ring(bars->b_full, b_pos, b_slots, b_fills);
+				drain_ring(bars->aug_full, aug_pos, SC_AUG_SLOTS, aug_fills);
 			}
 		}
 	} else if (warp == 1) {
@@ -196,20 +217,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 				ptx::mma_commit_pair(own);
 				ptx::mma_commit_pair(ptx::map_to_cta(own, 1u));
 			};
-			uint32_t a_count = 0, b_count = 0, c = 0;    // a_count: resident, first slice of the step's points
+			RingPos a_pos, b_pos, aug_pos, acc_pos;      // a_pos: resident, the first slice of the step's points
 			bool ok = true;
 			for (uint32_t step = step_begin + pair; step < step_end && ok; step += n_pairs) {
-				for (uint32_t j = 0; j < n_ctiles && ok; ++j, ++c) {
-					const uint32_t acc = c & 1u, d_tmem = tmem_base + acc * TC_NT_MAX;
-					ok = pair_wait<20>(&bars->acc_empty[acc], ((c >> 1) & 1u) ^ 1u, abort_flag, peer_abort_addr);
+				RingPos next_points = a_pos;
+				for (uint32_t j = 0; j < n_ctiles && ok; ++j) {
+					const uint32_t d_tmem = tmem_base + acc_pos.slot * TC_NT_MAX;
+					ok = pair_wait<20>(&bars->acc_empty[acc_pos.slot], acc_pos.phase ^ 1u, abort_flag, peer_abort_addr);
 					if (!ok) break;
+					RingPos points = a_pos;
 					for (uint32_t sl = 0; sl < slices; ++sl) {
-						const uint32_t ac = a_count + (resident ? sl : 0u), as = ac % a_slots, bs = b_count % b_slots;
-						if (!resident || j == 0) ok = pair_wait<20>(&bars->a_full[as], (ac / a_slots) & 1u, abort_flag, peer_abort_addr);
-						if (ok) ok = pair_wait<20>(&bars->b_full[bs], (b_count / b_slots) & 1u, abort_flag, peer_abort_addr);
+						if (!resident || j == 0) ok = pair_wait<20>(&bars->a_full[points.slot], points.phase, abort_flag, peer_abort_addr);
+						if (ok) ok = pair_wait<20>(&bars->b_full[b_pos.slot], b_pos.phase, abort_flag, peer_abort_addr);
 						if (!ok) break;
 						ptx::tc_fence_after();
-						const uint32_t a_lo = desc_lo_sw128(ptx::smem_u32(smem + as * SC_PLANE_BYTES)), b_lo = desc_lo_sw128(ptx::smem_u32(b_ring + bs * SC_PLANE_BYTES));
+						const uint32_t a_lo = desc_lo_sw128(ptx::smem_u32(smem + points.slot * SC_PLANE_BYTES)), b_lo = desc_lo_sw128(ptx::smem_u32(b_ring + b_pos.slot * SC_PLANE_BYTES));
 						const uint32_t steps = sl + 1 == slices ? ksteps_last : 4u;
 						if (ptx::elect_one()) {
 							if (sl == 0) ptx::mma_f16_pair_halves<false>(d_tmem, a_lo, DESC_HI_SW128, b_lo, DESC_HI_SW128, idesc);
@@ -217,26 +239,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 							#pragma unroll
 							for (uint32_t ks = 1; ks < 4; ++ks)
 								if (ks < steps) ptx::mma_f16_pair_halves<true>(d_tmem, a_lo + 2 * ks, DESC_HI_SW128, b_lo + 2 * ks, DESC_HI_SW128, idesc);
-							commit_both(&bars->b_empty[bs]);
-							if (!resident || j + 1 == n_ctiles) commit_both(&bars->a_empty[as]);
+							commit_both(&bars->b_empty[b_pos.slot]);
+							if (!resident || j + 1 == n_ctiles) commit_both(&bars->a_empty[points.slot]);
 						}
 						__syncwarp();
-						++b_count;
-						if (!resident) ++a_count;
+						b_pos.next(b_slots);
+						points.next(a_slots);
 					}
 					if (!ok) break;
-					const uint32_t gs = c % SC_AUG_SLOTS;
-					ok = pair_wait<20>(&bars->aug_full[gs], (c / SC_AUG_SLOTS) & 1u, abort_flag, peer_abort_addr);
+					if (!resident) a_pos = points;
+					next_points = points;
+					ok = pair_wait<20>(&bars->aug_full[aug_pos.slot], aug_pos.phase, abort_flag, peer_abort_addr);
 					if (!ok) break;
 					ptx::tc_fence_after();
 					if (ptx::elect_one()) {
-						ptx::mma_f16_pair_halves<true>(d_tmem, a_aug_lo, DESC_HI_AUG, desc_lo_aug(ptx::smem_u32(smem + SC_AUG_OFF + gs * SC_AUG_BYTES)), DESC_HI_AUG, idesc);
-						commit_both(&bars->acc_full[acc]);
-						commit_both(&bars->aug_empty[gs]);
+						ptx::mma_f16_pair_halves<true>(d_tmem, a_aug_lo, DESC_HI_AUG, desc_lo_aug(ptx::smem_u32(smem + SC_AUG_OFF + aug_pos.slot * SC_AUG_BYTES)), DESC_HI_AUG, idesc);
+						commit_both(&bars->acc_full[acc_pos.slot]);
+						commit_both(&bars->aug_empty[aug_pos.slot]);
 					}
 					__syncwarp();
+					aug_pos.next(SC_AUG_SLOTS);
+					acc_pos.next(2);
 				}
-				if (resident) a_count += slices;
+				a_pos = next_points;
 			}
 		}
 	} else {
