@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 					}
 				}
 			} else {
-				uint32_t g = 0;                       // position of the block's first tile in the A ring
+				RingPos ring;                         // of point tiles: the block's first
 				bool b_ready = false;
 				for (uint32_t blk = bid; blk < nblocks && ok; blk += nbid) {
 					const uint32_t tiles = min(TC_MA, n_tiles - blk * TC_MA);
@@ -753,8 +753,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 						const uint32_t b_addr = ptx::smem_u32(smem + sm_b_off + s * b_stage);
 						const uint32_t b_hi = desc_lo_sw128(b_addr), b_lo = desc_lo_sw128(b_addr + b_plane);
 						const uint32_t b_aug_lo = desc_lo_aug(ptx::smem_u32(smem + sm_baug_off + s * AUG_BYTES));
-						for (uint32_t i = 0; i < tiles; ++i) {
-							const uint32_t buf = (g + i) % n_abuf, ua = (g + i) / n_abuf;
+						RingPos tile = ring;
+						for (uint32_t i = 0; i < tiles; ++i, tile.next(n_abuf)) {
+							const uint32_t buf = tile.slot, ua = tile.phase;
 							if (j == j_begin) {
 								ok = wait_or_abort<100>(&bars->a_full[buf], ua & 1u, abort_flag);
 								if (!ok) break;
@@ -786,7 +787,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(
 							++b_count;
 						}
 					}
-					g += tiles;
+					for (uint32_t i = 0; i < tiles; ++i) ring.next(n_abuf);
 				}
 			}
 		}

@@ -218,9 +218,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 		}
 		__syncwarp();
 		uint32_t it = 0;
+		RingPos ring;
 		bool ok = true;
-		for (uint32_t step = step_begin + pair; step < steps_total; step += n_pairs, ++it) {
-			const uint32_t buf = it % n_abuf, u = it / n_abuf;
+		for (uint32_t step = step_begin + pair; step < steps_total; step += n_pairs, ++it, ring.next(n_abuf)) {
+			const uint32_t buf = ring.slot, u = ring.phase;
 			// the raw rows need the whole warp; otherwise the other lanes have nothing to wait for
 			if (fuse_acc != nullptr) ok = __all_sync(0xffffffffu, pair_wait<400>(&bars->a_empty[buf], (u & 1u) ^ 1u, abort_flag, peer_abort_addr)) != 0;
 			else if (lane == 0) ok = pair_wait<400>(&bars->a_empty[buf], (u & 1u) ^ 1u, abort_flag, peer_abort_addr);
@@ -264,9 +265,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 			const uint32_t acc_full_own = ptx::smem_u32(&bars->acc_full[0]);
 			const uint32_t acc_full_peer = ptx::map_to_cta(acc_full_own, peer);
 			bool ok = pair_wait(&bars->b_full, 0, abort_flag, peer_abort_addr);
-			uint32_t it = 0, c = 0;                 // c counts units: accumulator c % 4, use c / 4
-			for (uint32_t step = step_begin + pair; step < steps_total && ok; step += n_pairs, ++it) {
-				const uint32_t buf = it % n_abuf, ua = it / n_abuf;
+			uint32_t c = 0;                         // counts units: accumulator c % 4, use c / 4
+			RingPos ring;
+			for (uint32_t step = step_begin + pair; step < steps_total && ok; step += n_pairs, ring.next(n_abuf)) {
+				const uint32_t buf = ring.slot, ua = ring.phase;
 				ok = pair_wait(&bars->a_full[buf], ua & 1u, abort_flag, peer_abort_addr);
 				if (!ok) break;
 				// descriptor halves (see desc_lo_sw128): +2 in the address field = 32 bytes = one K step
@@ -332,13 +334,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 		// last of them has read it.
 		bool pending = false;
 		uint32_t pend_it = 0;
+		RingPos pend_ring;                            // buffer of the step whose sums are pending
 		auto flush_sums = [&]() {
 			if (g != merger) asm volatile("bar.sync %0, 128;" :: "r"(9u + q) : "memory");   // the final clusters are written
 			const uint32_t* s_mine = mg_state + 2 * 3 * 3 * TC_MTILE + (pend_it & 1u) * TC_MTILE;
-			const uint32_t buf = pend_it % n_abuf;
+			const uint32_t buf = pend_ring.slot;
 			const float* raw = reinterpret_cast<const float*>(smem + raw_off + buf * P2_RAW_BYTES);
 			const uint32_t sub = lane >> 3, c4 = lane & 7u;
-			if (ok) ok = __all_sync(0xffffffffu, pair_wait(&bars->raw_full[buf], (pend_it / n_abuf) & 1u, abort_flag, peer_abort_addr)) != 0;
+			if (ok) ok = __all_sync(0xffffffffu, pair_wait(&bars->raw_full[buf], pend_ring.phase, abort_flag, peer_abort_addr)) != 0;
 			#pragma unroll
 			for (uint32_t r4 = 0; r4 < 2; ++r4) {
 				const uint32_t trow = q * 32 + g * 8 + r4 * 4 + sub;
@@ -357,6 +360,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) assig
 			__syncwarp();
 			if (lane == 0) ptx::mbar_arrive(&bars->a_empty[buf]);
 			pending = false;
+			pend_ring.next(n_abuf);
 		};
 		for (uint32_t step = step_begin + pair; step < steps_total; step += n_pairs, ++it) {
 			RowMin rows;

@@ -65,13 +65,6 @@ bool tc_screen_fits(uint32_t k, uint32_t dim) { return tc_dpad(dim) > TC_KCHUNK 
 // 30 000 points x 1024 x 128 83 / 77.  Where the first wave leaves most points open: 3141 / 3056 (99.5 % of 10^6 x 1000 x 100).
 bool tc_screen_pays(const Shape& s) { return s.n >= 1u << 15 && (double)s.n * s.k * s.dim >= 1.2e10; }
 
-// Place in a ring of buffers.  (Counted up with a wrap: remainder and quotient by a ring size that is known at run time cost the
-// loading lane 800 clocks per slice, beside four busy warps, where a slice's multiplication takes 512.)
-struct RingPos {
-	uint32_t slot = 0, phase = 0;
-	__device__ __forceinline__ void next(uint32_t slots) { if (++slot == slots) { slot = 0; phase ^= 1u; } }
-};
-
 // Waits for the last fill of every buffer that has been filled (a lap at most); `pos` is the next one to be filled.
 __device__ __forceinline__ void drain_ring(uint64_t* full, RingPos pos, uint32_t slots, uint32_t fills)
 {

@@ -75,6 +75,13 @@ __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, volati
 	return false;
 }
 
+// Place in a ring of buffers.  (Counted up with a wrap: remainder and quotient by a ring size that is known at run time cost the
+// loading lane of the screening pass 800 clocks per slice, beside four busy warps, where a slice's multiplication takes 512.)
+struct RingPos {
+	uint32_t slot = 0, phase = 0;
+	__device__ __forceinline__ void next(uint32_t slots) { if (++slot == slots) { slot = 0; phase ^= 1u; } }
+};
+
 // K-major operand, 64-byte swizzle: rows of 64 B, 8-row groups 512 B apart.
 __device__ __forceinline__ uint64_t make_desc_sw64(uint32_t smem_addr)
 {
