@@ -226,7 +226,8 @@ int bkm_set_stream(bkm_handle_t h, void* stream);
  * latency; single GPU only), "tc_pair" (0/1, default 1: let the tensor-core assignment run on CTA
  * pairs with all means resident in shared memory where the shape allows, i.e. 257..1024 means
  * of 17..32 dimensions), "tc_screen" (0 never, 1 = default: where it pays, 2
- * wherever possible: rows longer than 64 dimensions are screened with the fp16 high parts first), "fuse_update" (0 never, 1 = default: where it pays, 2 wherever possible:
+ * wherever possible: rows longer than 64 dimensions are screened with the fp16 high parts first),
+ * "fuse_update" (0 never, 1 = default: where it pays, 2 wherever possible:
  * let the fast assignment pass add every point to the sum of the cluster it picks, which replaces
  * the update pass of bkm_run; possible on CTA pairs with dim % 4 == 0 and in the CUDA-core pass
  * for dim <= 8 and at most 1024 means; by default the latter only for launch-bound sizes),
