@@ -15,6 +15,7 @@
 #include "keys.cuh"
 
 #include <cmath>
+#include <type_traits>
 
 namespace bkm {
 
@@ -692,6 +693,31 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 		return trows;
 	};
 
+	// Values of the means m .. m + 3 of a chunk (two interleaved pairs, D + 1 128-bit loads) for Q points.
+	auto four_means = [&](const float* chunk, int m, const uint64_t (&xx)[Q][D], auto&& put) {
+		const float4* rowp = reinterpret_cast<const float4*>(chunk) + (m / 4) * (D + 1);
+		float f[4 * (D + 1)];
+		#pragma unroll
+		for (int q = 0; q <= D; ++q) {
+			const float4 w = rowp[q];
+			f[4 * q + 0] = w.x; f[4 * q + 1] = w.y; f[4 * q + 2] = w.z; f[4 * q + 3] = w.w;
+		}
+		#pragma unroll
+		for (int h = 0; h < 2; ++h) {
+			const float* mean2 = f + h * 2 * (D + 1);
+			#pragma unroll
+			for (int p = 0; p < Q; ++p) {
+				uint64_t val = ptx::pack2(mean2[0], mean2[1]);
+				#pragma unroll
+				for (int j = 0; j < D; ++j) val = ptx::fma2(xx[p][j], ptx::pack2(mean2[2 * j + 2], mean2[2 * j + 3]), val);
+				uint32_t lo, hi;
+				ptx::unpack2(val, lo, hi);
+				put(p, 2 * h, lo);
+				put(p, 2 * h + 1, hi);
+			}
+		}
+	};
+
 	// The points of a block of work, as they lie in memory (slots behind the last point read as the
 	// centre).  The next block's points are fetched while the current block is being evaluated.
 	float raw[P][D];
@@ -761,6 +787,26 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 				#pragma unroll
 				for (int j = 0; j < D; ++j) xx[p][j] = ptx::pack2(x[g + p][j], x[g + p][j]);
 
+			uint32_t best[Q], second[Q], bchunk[Q];
+			// Means 0 .. N - 1 at once, straight to keys: for up to 16 or 32 means that is shorter than minima over two partitions
+			// and their ranking (ten iterations of 65 536 x 4 against 16 means, 2 % less).
+			auto few_means = [&](auto count) {
+				constexpr int N = decltype(count)::value;
+				uint32_t v[Q][N];
+				#pragma unroll
+				for (int m = 0; m < N; m += 4) four_means(tile, m, xx, [&](int p, int u, uint32_t bits) { v[p][m + u] = bits; });
+				#pragma unroll
+				for (int p = 0; p < Q; ++p) {
+					#pragma unroll
+					for (int t = 0; t < N; ++t) v[p][t] = v[p][t] * key_mult + (uint32_t)t;
+					two_smallest(v[p], best[p], second[p]);
+					bchunk[p] = 0;
+				}
+			};
+			if (rows == 32) {
+				if (k <= 16) few_means(std::integral_constant<int, 16>());
+				else few_means(std::integral_constant<int, 32>());
+			} else {
 			RowMin row[Q];
 			#pragma unroll
 			for (int p = 0; p < Q; ++p) row[p].reset();
@@ -775,7 +821,6 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 				#pragma unroll 1
 				for (uint32_t ch = 0; ch < trows / 32; ++ch) {
 					// Columns m .. m + 3 and m + 16 .. m + 19 together: they meet in the same position minima.
-					const float4* rowp = reinterpret_cast<const float4*>(tile + (size_t)ch * 32 * (D + 1));
 					uint32_t group[Q][2];
 					#pragma unroll
 					for (int p = 0; p < Q; ++p) group[p][0] = group[p][1] = 0xFFFFFFFFu;
@@ -783,26 +828,8 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 					for (int m = 0; m < 16; m += 4) {
 						uint32_t v[Q][2][4];
 						#pragma unroll
-						for (int half = 0; half < 2; ++half) {
-							// four means = two interleaved pairs = D + 1 128-bit loads
-							float f[4 * (D + 1)];
-							#pragma unroll
-							for (int q = 0; q <= D; ++q) {
-								const float4 w = rowp[(m / 4 + half * 4) * (D + 1) + q];
-								f[4 * q + 0] = w.x; f[4 * q + 1] = w.y; f[4 * q + 2] = w.z; f[4 * q + 3] = w.w;
-							}
-							#pragma unroll
-							for (int h = 0; h < 2; ++h) {
-								const float* mean2 = f + h * 2 * (D + 1);
-								#pragma unroll
-								for (int p = 0; p < Q; ++p) {
-									uint64_t val = ptx::pack2(mean2[0], mean2[1]);
-									#pragma unroll
-									for (int j = 0; j < D; ++j) val = ptx::fma2(xx[p][j], ptx::pack2(mean2[2 * j + 2], mean2[2 * j + 3]), val);
-									ptx::unpack2(val, v[p][half][2 * h], v[p][half][2 * h + 1]);
-								}
-							}
-						}
+						for (int half = 0; half < 2; ++half)
+							four_means(tile + (size_t)ch * 32 * (D + 1), m + half * 16, xx, [&](int p, int u, uint32_t bits) { v[p][half][u] = bits; });
 						#pragma unroll
 						for (int p = 0; p < Q; ++p) {
 							#pragma unroll
@@ -818,17 +845,19 @@ __global__ void __launch_bounds__(SIMT_THREADS, 2) assign_simt_kernel(const floa
 			}
 
 			#pragma unroll
+			for (int p = 0; p < Q; ++p) row[p].finish(key_base, key_mult, key_magic, best[p], second[p], bchunk[p]);
+			}
+
+			#pragma unroll
 			for (int p = 0; p < Q; ++p) {
-				uint32_t best, second, bchunk;
-				row[p].finish(key_base, key_mult, key_magic, best, second, bchunk);
 				cl[g + p] = k;                 // rows behind the last point sort behind every cluster
 				bool flag = false;
 				if (idx[g + p] < n) {
 					// key - key_base = M * mantissa + column
-					const uint32_t bm = div_key(best - key_base, key_magic);
-					cl[g + p] = bchunk * 32u + ((best - key_base) - bm * key_mult);
+					const uint32_t bm = div_key(best[p] - key_base, key_magic);
+					cl[g + p] = bchunk[p] * 32u + ((best[p] - key_base) - bm * key_mult);
 					if (!FUSE) asg[idx[g + p]] = cl[g + p];
-					const float gap = second == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second - key_base, key_magic) - bm);
+					const float gap = second[p] == 0xFFFFFFFFu ? INFINITY : (float)(div_key(second[p] - key_base, key_magic) - bm);
 					float margin = margin_floor;
 					if (TIGHT) {
 						float x2 = 0.0f;

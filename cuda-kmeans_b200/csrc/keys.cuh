@@ -40,6 +40,27 @@ __device__ __forceinline__ uint32_t min_of_16(const uint32_t* p)
 	return min(umin3(a0, a1, a2), umin3(a3, a4, p[15]));
 }
 
+__device__ __forceinline__ uint32_t min_of(const uint32_t (&p)[16]) { return min_of_16(p); }
+__device__ __forceinline__ uint32_t min_of(const uint32_t (&p)[32]) { return min_of_32(p); }
+
+// The two smallest of N distinct keys: key - (smallest + 1) wraps to the top of the unsigned range for the smallest only, and the
+// minimum of these differences belongs to the second smallest.
+template<int N>
+__device__ __forceinline__ void two_smallest(const uint32_t (&p)[N], uint32_t& best, uint32_t& second)
+{
+	best = min_of(p);
+	const uint32_t shift = ~best;                  // -(smallest + 1)
+	uint32_t r0 = p[0] + shift, r1 = p[1] + shift, r2 = p[2] + shift, r3 = p[3] + shift;
+	#pragma unroll
+	for (uint32_t t = 4; t < N; t += 4) {
+		r0 = __viaddmin_u32(p[t], shift, r0);
+		r1 = __viaddmin_u32(p[t + 1], shift, r1);
+		r2 = __viaddmin_u32(p[t + 2], shift, r2);
+		r3 = __viaddmin_u32(p[t + 3], shift, r3);
+	}
+	second = min(umin3(r0, r1, r2), r3) - shift;
+}
+
 // The two smallest values of a point's row, and the column of the smallest, from minima alone.  The
 // columns are partitioned twice: by their position (column mod 16) and into groups of 16 neighbours.  Two
 // columns of one position lie in different groups, so the second smallest value of the row is the
@@ -189,19 +210,9 @@ __device__ __forceinline__ void RowMin::finish(uint32_t key_base, uint32_t key_m
 	uint32_t p[16];
 	#pragma unroll
 	for (uint32_t t = 0; t < 16; ++t) p[t] = position[t] * key_mult + t;
-	const uint32_t b = min_of_16(p);
-	// The keys are distinct (they carry the position), so key - (smallest + 1) wraps to the top of the unsigned
-	// range for the smallest only, and the minimum of these differences belongs to the second smallest.
-	const uint32_t shift = ~b;
-	uint32_t r0 = p[0] + shift, r1 = p[1] + shift, r2 = p[2] + shift, r3 = p[3] + shift;
-	#pragma unroll
-	for (uint32_t t = 4; t < 16; t += 4) {
-		r0 = __viaddmin_u32(p[t], shift, r0);
-		r1 = __viaddmin_u32(p[t + 1], shift, r1);
-		r2 = __viaddmin_u32(p[t + 2], shift, r2);
-		r3 = __viaddmin_u32(p[t + 3], shift, r3);
-	}
-	second_out = min(min(umin3(r0, r1, r2), r3) - shift, second);
+	uint32_t b, next;
+	two_smallest(p, b, next);
+	second_out = min(next, second);
 	// both smallest keys have the same value part: what is left of the group's key is its number
 	const uint32_t value = div_key(b - key_base, key_magic) * key_mult + key_base;
 	best_out = b + ((best - value) & 1u) * 16u;
