@@ -10,7 +10,7 @@
 // together against their distance from the centre of all points) go to a list and through the pass with all
 // three products, K loop of assign_tc.cu, and from there to the exact kernel as ever: the labels are the same.
 // Long rows are bound by the tensor pipe, and at three products by the power limit as well: 2^20 x 512
-// against 4096 means 9.06 ms per iteration in one pass, SCREEN_B with the list.
+// against 4096 means 9.06 ms per iteration in one pass, 3.10 with screening and list.
 //
 // One CTA pair (cta_group::2) multiplies 256 points by 256 means at a time: each CTA holds its 128 points and half of
 // the means, and gets the 128 x 256 block of its points in tensor memory, twice over, so that one block
